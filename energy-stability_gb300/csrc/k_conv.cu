@@ -34,7 +34,7 @@
 #include "sclet_internal.cuh"
 #include "sclet_tc.cuh"
 #include "sclet_tc_ptx.cuh"
-#include "sclet_conv.cuh"
+#include "sclet_conv_tc.cuh"
 
 namespace sclet {
 namespace conv {
@@ -51,13 +51,10 @@ using tc::smem_desc;
 using tc::smem_u32;
 using tc::tmem_ld32;
 
-constexpr int ROWS = 128;                  // cells per tile (MMA M)
-constexpr int MAX_STAGES = 3;              // tiles of input runs in flight
 constexpr int WTILE = CH * CH * 2;         // 2 KB: one tap's 32 x 32 weights
 constexpr int NACC = 4;                    // TMEM accumulators of 32 columns
 constexpr int TMEM_COLS = NACC * CH;       // 128
 constexpr int THREADS = 192;
-constexpr int SMEM_LIMIT = 226 * 1024;  // dynamic shared memory: 227 KB per CTA less the static part
 
 // Per-launch geometry.  ny = 1: per stencil plane and channel chunk one run
 // of 128 + 2 Np + 2 slots serves all nine in-plane taps (twelve runs a tile);
@@ -86,39 +83,6 @@ static Geom geom_of(int N) {
   if (forced == 1 && a.stages >= 1) return a;
   if (forced == 3) return b;
   return a.stages >= 1 && a.stage_bytes <= b.stage_bytes ? a : b;
-}
-
-// Shared-memory matrix descriptor, K-major without swizzle: 8-row core
-// matrices 128 bytes apart (rows 16 bytes apart), K chunks lbo bytes apart.
-__device__ __forceinline__ uint64_t smem_desc_plain(uint32_t addr, uint32_t lbo) {
-  uint64_t d = 0;
-  d |= (uint64_t)((addr & 0x3FFFFu) >> 4);
-  d |= (uint64_t)((lbo >> 4) & 0x3FFFu) << 16;  // leading byte offset: next K chunk
-  d |= (uint64_t)(128 >> 4) << 32;              // stride byte offset: next 8 rows
-  d |= (uint64_t)1 << 46;                       // descriptor version
-  return d;                                     // layout type 0: no swizzle
-}
-
-__device__ __forceinline__ void tma_load_2d(void *dst, const CUtensorMap *map, int x, int y, uint64_t *bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
-          smem_u32(dst)),
-      "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(smem_u32(bar))
-      : "memory");
-}
-
-// tile -> (sample b, plane zh in 1..N, first slot s0 of the plane)
-struct Tile {
-  int b, zh, s0;
-};
-__device__ __forceinline__ Tile tile_of(int t, int N, int Np, int per_plane) {
-  Tile x;
-  const int j = t % per_plane;
-  const int bz = t / per_plane;
-  x.zh = 1 + bz % N;
-  x.b = bz / N;
-  x.s0 = Np + j * ROWS;
-  return x;
 }
 
 __device__ __forceinline__ float bf(uint32_t w, int hi) {
@@ -239,7 +203,7 @@ __global__ void __launch_bounds__(THREADS, 1)
         // descriptors of the stage's first run and of the first weight tile;
         // a tap adds its run and row offsets (16-byte units) to the address
         // field, which stays below 2^14 inside the shared memory
-        const uint64_t dab = smem_desc_plain(a0 + (uint32_t)(s * stage_bytes), box_bytes);
+        const uint64_t dab = smem_desc_lin(a0 + (uint32_t)(s * stage_bytes), box_bytes, 128);
         const uint64_t dwb = smem_desc(w0);
         const uint32_t run16 = (uint32_t)box_bytes >> 4;
 #pragma unroll
@@ -353,22 +317,6 @@ static cudaError_t make_map_rows(CUtensorMap *map, const void *ptr, long long ro
   return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
 }
 
-// 2-D BF16 tensor map over an activation buffer as lines of 128 bytes (8 slots
-// of 16 bytes), no swizzle, boxes of box_rows lines; lines outside the buffer
-// read as zeros.
-static cudaError_t make_map_lines(CUtensorMap *map, const void *ptr, long long lines, int box_rows) {
-  auto fn = encode_fn();
-  if (!fn) return cudaErrorNotSupported;
-  cuuint64_t dims[2] = {64, (cuuint64_t)lines};
-  cuuint64_t strides[1] = {128};
-  cuuint32_t box[2] = {64, (cuuint32_t)box_rows};
-  cuuint32_t estr[2] = {1, 1};
-  CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void *>(ptr), dims, strides, box, estr,
-                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
-}
-
 // per device: the shared-memory attribute and the resident CTA count
 static cudaError_t conv_setup(int *ctas) {
   constexpr int MAXDEV = 64;
@@ -400,6 +348,8 @@ int conv_set_runs(int runs_per_plane) {
   if (runs_per_plane != 0 && runs_per_plane != 1 && runs_per_plane != 3) return -1;
   return conv::g_runs_per_plane.exchange(runs_per_plane);
 }
+
+int conv_runs() { return conv::g_runs_per_plane.load(); }
 
 cudaError_t launch_conv(const __nv_bfloat16 *in, const __nv_bfloat16 *w, const ConvArgs &args, cudaStream_t s) {
   int ctas = 0;

@@ -1,7 +1,6 @@
 // Element-wise and reduction kernels of the corrector network: periodic halo,
-// packing FP32 fields into haloed BF16 activations, the weight gradient of a
-// 3x3x3 convolution (FP32 accumulation), the BF16 weight copies, Adam and the
-// training residual.  Activations in the chunk-planar layout of
+// packing FP32 fields into haloed BF16 activations, the BF16 weight copies,
+// Adam and the training residual.  Activations in the chunk-planar layout of
 // sclet_conv.cuh (conv_at).
 #include <cuda_bf16.h>
 #include <stdint.h>
@@ -79,80 +78,6 @@ __global__ void pack_kernel(const float *__restrict__ in, int cin, float scale, 
     const long long c0 = conv_at(N, b, z, 0, (long long)y * Np + x), cs = conv_chunk_slots(N);
 #pragma unroll
     for (int k = 0; k < 4; k++) dst[c0 + k * cs] = make_uint4(w[4 * k], w[4 * k + 1], w[4 * k + 2], w[4 * k + 3]);
-  }
-}
-
-// Weight gradient: one tap per blockIdx.y; a CTA of 64 threads walks its
-// share of the owned cells 64 at a time, the gradient and the shifted input
-// of those cells in shared memory as FP32; thread (co4, ci4) accumulates a
-// 4 x 4 block of dW over them, then adds it to the FP32 accumulator.
-constexpr int WG_CELLS = 64;
-__global__ void __launch_bounds__(64) wgrad_kernel(const __nv_bfloat16 *__restrict__ in,
-                                                   const __nv_bfloat16 *__restrict__ g, int N, int batch,
-                                                   float *__restrict__ dw, float *__restrict__ db) {
-  __shared__ __align__(16) float gs[WG_CELLS][CH];
-  __shared__ __align__(16) float xs[WG_CELLS][CH];
-  const int tap = blockIdx.y;
-  const int dz = tap / 9 - 1, dy = (tap / 3) % 3 - 1, dx = tap % 3 - 1;
-  const int Np = N + 2;
-  const long long n3 = (long long)N * N * N;
-  const long long total = n3 * batch;
-  const int tid = threadIdx.x;
-  const int co0 = (tid >> 3) * 4, ci0 = (tid & 7) * 4;
-  float acc[4][4] = {};
-  float bacc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-  const long long nblk = (total + WG_CELLS - 1) / WG_CELLS;
-  for (long long blk = blockIdx.x; blk < nblk; blk += gridDim.x) {
-    // 64 cells x 4 chunks of 8 channels per array: 4 chunk loads per thread each
-#pragma unroll
-    for (int r = 0; r < 4; r++) {
-      const int idx = tid + 64 * r;  // 0..255
-      const int c = idx >> 2, k = idx & 3;
-      const long long i = blk * WG_CELLS + c;
-      uint4 gv = make_uint4(0, 0, 0, 0), xv = make_uint4(0, 0, 0, 0);
-      if (i < total) {
-        const int b = (int)(i / n3);
-        long long rr = i - (long long)b * n3;
-        const int z = (int)(rr / ((long long)N * N));
-        rr -= (long long)z * N * N;
-        const int y = (int)(rr / N), x = (int)(rr - (long long)y * N);
-        gv = reinterpret_cast<const uint4 *>(g)[conv_at(N, b, z + 1, k, (long long)(y + 1) * Np + x + 1)];
-        xv = reinterpret_cast<const uint4 *>(in)[conv_at(N, b, z + 1 + dz, k, (long long)(y + 1 + dy) * Np + x + 1 + dx)];
-      }
-      const uint32_t gw[4] = {gv.x, gv.y, gv.z, gv.w}, xw[4] = {xv.x, xv.y, xv.z, xv.w};
-#pragma unroll
-      for (int h = 0; h < 4; h++) {
-        gs[c][k * 8 + 2 * h] = __uint_as_float(gw[h] << 16);
-        gs[c][k * 8 + 2 * h + 1] = __uint_as_float(gw[h] & 0xffff0000u);
-        xs[c][k * 8 + 2 * h] = __uint_as_float(xw[h] << 16);
-        xs[c][k * 8 + 2 * h + 1] = __uint_as_float(xw[h] & 0xffff0000u);
-      }
-    }
-    __syncthreads();
-#pragma unroll 8
-    for (int c = 0; c < WG_CELLS; c++) {
-      const float4 gv = *reinterpret_cast<const float4 *>(&gs[c][co0]);
-      const float4 xv = *reinterpret_cast<const float4 *>(&xs[c][ci0]);
-      const float gg[4] = {gv.x, gv.y, gv.z, gv.w}, xx[4] = {xv.x, xv.y, xv.z, xv.w};
-#pragma unroll
-      for (int a = 0; a < 4; a++)
-#pragma unroll
-        for (int b = 0; b < 4; b++) acc[a][b] = fmaf(gg[a], xx[b], acc[a][b]);
-      if (tap == 13 && ci0 == 0) {
-#pragma unroll
-        for (int a = 0; a < 4; a++) bacc[a] += gg[a];
-      }
-    }
-    __syncthreads();
-  }
-  float *d = dw + (long long)tap * CH * CH;
-#pragma unroll
-  for (int a = 0; a < 4; a++)
-#pragma unroll
-    for (int b = 0; b < 4; b++) atomicAdd(&d[(co0 + a) * CH + ci0 + b], acc[a][b]);
-  if (tap == 13 && ci0 == 0 && db) {
-#pragma unroll
-    for (int a = 0; a < 4; a++) atomicAdd(&db[co0 + a], bacc[a]);
   }
 }
 
@@ -252,15 +177,6 @@ cudaError_t launch_conv_relu_mask(__nv_bfloat16 *g, const __nv_bfloat16 *act, in
   const long long chunks = conv_units(N, batch);
   relu_mask_kernel<<<grid_for(chunks, 256), 256, 0, s>>>(reinterpret_cast<uint4 *>(g),
                                                           reinterpret_cast<const uint4 *>(act), chunks);
-  launch_counter()++;
-  return cudaGetLastError();
-}
-
-cudaError_t launch_conv_wgrad(const __nv_bfloat16 *in, const __nv_bfloat16 *g, int N, int batch, float *dw, float *db,
-                              cudaStream_t s) {
-  const long long blocks = ((long long)N * N * N * batch + WG_CELLS - 1) / WG_CELLS;
-  const int gx = (int)(blocks < 256 ? blocks : 256);
-  wgrad_kernel<<<dim3(gx, TAPS), 64, 0, s>>>(in, g, N, batch, dw, db);
   launch_counter()++;
   return cudaGetLastError();
 }

@@ -1,0 +1,307 @@
+// Weight gradient of the corrector's 3x3x3 convolutions on the 5th-generation
+// tensor cores:
+//   dW[tap][co][ci] += sum over owned cells of g[cell][co] x[cell + off(tap)][ci]
+//   db[co]          += sum over owned cells of g[cell][co]
+// A GEMM whose contraction runs over the cells.  A tile is 128 consecutive
+// slots of one haloed plane (as in k_conv.cu).  The activation layout
+// (chunk-planar, 8 channels of a cell in 16 bytes, consecutive cells 16 bytes
+// apart) is the MN-major operand layout as it lies in memory, so both
+// operands go from TMA to the MMA without a transpose, and a tap is an offset
+// of the operand's start address.
+//   M = 128: the three stencil planes dz x 32 input channels (twelve runs, a
+//       run apart), then one run of ones, whose row sums g: the bias gradient
+//   N = 32 output channels, K = the tile's 128 cells in steps of 16
+// The nine in-plane taps (dy, dx) have one 32-column accumulator each in
+// tensor memory, kept across tiles, and are drained into FP32 registers every
+// DRAIN tiles with round-to-nearest adds (the accumulator's own rounding then
+// acts on at most 8 DRAIN sums); each CTA adds its sums to the gradient once,
+// at the end.  Warp 0 issues TMA, warp 1 the 72 MMAs of a tile, warp 2 clears
+// the gradient's slots outside the owned cells (the halo holds periodic
+// images, which the data gradient needs), warps 3-14 drain.
+//
+// Bound by the L2 -> shared-memory ingest of the three planes (61 KB a tile
+// at 64^3): 0.14 ms a layer on 4 x 64^3, where the FP32-issue kernel it
+// replaces took 2.22 ms.
+#include <mutex>
+
+#include "sclet_conv_tc.cuh"
+#include "sclet_internal.cuh"
+
+namespace sclet {
+namespace conv {
+namespace wg {
+
+using namespace tc;
+
+constexpr int TAPS2 = 9;                    // in-plane taps, one accumulator each
+constexpr int G_ROWS = (ROWS + 7 + 7) / 8;  // 128-byte lines of one gradient run
+constexpr int G_BYTES = G_ROWS * 128;
+constexpr int EPI = 12;                     // draining warps, three per TMEM lane quadrant
+constexpr int TAPS_PER_WARP = TAPS2 / 3;
+constexpr int WG_THREADS = 32 * (3 + EPI);
+constexpr int WG_TMEM = 512;                // 288 columns used; allocations are powers of two
+constexpr int DRAIN = 8;                    // tiles per drain
+
+// Runs of the input per stage as in k_conv.cu's ny: 1 one run of 128 + 2 Np + 2
+// slots per plane and chunk, 3 one run of 130 slots per stencil row.  A stage:
+// for each of ny rows the twelve runs (dz, chunk), the ones run, three run
+// lengths that rows 104..127 of M read and drop (they overlay what follows),
+// and the four gradient runs at the end.
+struct Geom {
+  int ny, box_rows, box_bytes, row_bytes, stage_bytes, stages, smem;
+};
+static Geom geom_for(int N, int ny) {
+  Geom g;
+  g.ny = ny;
+  const int R = ny == 1 ? ROWS + 2 * (N + 2) + 2 : ROWS + 2;
+  g.box_rows = (R + 7 + 7) / 8;
+  g.box_bytes = g.box_rows * 128;
+  g.row_bytes = 13 * g.box_bytes;
+  g.stage_bytes = ny * g.row_bytes + 4 * G_BYTES;
+  const int tail = 3 * g.box_bytes + 128;  // the dropped rows' reads past the last stage
+  g.stages = (SMEM_LIMIT - 1024 - tail) / g.stage_bytes;
+  if (g.stages > MAX_STAGES) g.stages = MAX_STAGES;
+  g.smem = (g.stages > 0 ? g.stages : 1) * g.stage_bytes + tail + 1024;
+  return g;
+}
+
+__global__ void __launch_bounds__(WG_THREADS, 1)
+    wgrad_tc_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmG, int N, int batch,
+                    float *__restrict__ dw, float *__restrict__ db, int *err, Geom gm) {
+  extern __shared__ uint8_t smem_raw[];
+  __shared__ __align__(8) uint64_t full_bar[MAX_STAGES];
+  __shared__ __align__(8) uint64_t ready_bar[MAX_STAGES];  // gradient slots outside the owned cells cleared
+  __shared__ __align__(8) uint64_t empty_bar[MAX_STAGES];
+  __shared__ __align__(8) uint64_t acc_full, acc_empty, done_bar;
+  __shared__ uint32_t tmem_slot;
+  __shared__ int failed;
+
+  uint8_t *base = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int Np = N + 2, ny = gm.ny, stages = gm.stages;
+  const int per_plane = (N * Np + ROWS - 1) / ROWS;
+  const int total = batch * N * per_plane;
+  const int mine = (int)blockIdx.x < total ? (total - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
+  const int g_off = ny * gm.row_bytes;  // gradient runs within a stage
+
+  // shared memory starts as zeros, the ones runs as ones: what the dropped
+  // rows read is initialised too
+  {
+    const int n16 = (stages * gm.stage_bytes + 3 * gm.box_bytes + 128) / 16;
+    const uint4 z = make_uint4(0, 0, 0, 0);
+    for (int i = threadIdx.x; i < n16; i += WG_THREADS) reinterpret_cast<uint4 *>(base)[i] = z;
+    __syncthreads();
+    const uint32_t one2 = 0x3f803f80u;  // two BF16 ones
+    const int per = gm.box_bytes / 16;
+    for (int i = threadIdx.x; i < stages * ny * per; i += WG_THREADS) {
+      const int r = i / per, q = i - r * per, s = r / ny, y = r - s * ny;
+      reinterpret_cast<uint4 *>(base + s * gm.stage_bytes + y * gm.row_bytes + 12 * gm.box_bytes)[q] =
+          make_uint4(one2, one2, one2, one2);
+    }
+  }
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < MAX_STAGES; s++) {
+      mbar_init(&full_bar[s], 1);
+      mbar_init(&ready_bar[s], 1);
+      mbar_init(&empty_bar[s], 1);
+    }
+    mbar_init(&acc_full, 1);
+    mbar_init(&acc_empty, EPI);
+    mbar_init(&done_bar, 1);
+    failed = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)),
+                 "r"(WG_TMEM)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  fence_before();
+  __syncthreads();
+  fence_after();
+  const uint32_t tmem = tmem_slot;
+
+  if (warp == 0) {
+    if (lane == 0) {
+      int it = 0;
+      for (; it < mine && !*(volatile int *)&failed; it++) {
+        const Tile ti = tile_of(blockIdx.x + it * gridDim.x, N, Np, per_plane);
+        const int s = it % stages;
+        if (it >= stages && !mbar_wait(&empty_bar[s], ((it / stages) & 1) ^ 1)) {
+          failed = 1;
+          break;
+        }
+        uint8_t *st = base + s * gm.stage_bytes;
+        mbar_expect_tx(&full_bar[s], 12 * ny * gm.box_bytes + 4 * G_BYTES);
+        for (int r = 0; r < ny; r++)
+          for (int dz = 0; dz < 3; dz++)
+            for (int k = 0; k < 4; k++) {
+              const long long first = (long long)ti.s0 + (ny == 1 ? -Np : (r - 1) * Np) - 1;
+              const long long flat = conv_at(N, ti.b, ti.zh + dz - 1, k, first);
+              tma_load_2d(st + r * gm.row_bytes + (dz * 4 + k) * gm.box_bytes, &tmX, 0, (int)(flat >> 3), &full_bar[s]);
+            }
+        for (int k = 0; k < 4; k++)
+          tma_load_2d(st + g_off + k * G_BYTES, &tmG, 0, (int)(conv_at(N, ti.b, ti.zh, k, ti.s0) >> 3), &full_bar[s]);
+      }
+      if (*(volatile int *)&failed)  // drain (bounded) the copies still in flight
+        for (int i = it - stages < 0 ? 0 : it - stages; i < it; i++) mbar_wait(&full_bar[i % stages], (i / stages) & 1);
+    }
+  } else if (warp == 1) {
+    if (lane == 0) {
+      const uint32_t idesc = idesc_bf16(ROWS, CH) | (1u << 15) | (1u << 16);  // both operands MN-major
+      const uint32_t a0 = smem_u32(base);
+      for (int it = 0; it < mine && !*(volatile int *)&failed; it++) {
+        const int grp = it / DRAIN;
+        if (it % DRAIN == 0 && grp > 0 && !mbar_wait(&acc_empty, (grp - 1) & 1)) {
+          failed = 1;
+          break;
+        }
+        const int s = it % stages;
+        if (!mbar_wait(&ready_bar[s], (it / stages) & 1)) {
+          failed = 1;
+          break;
+        }
+        fence_after();
+        const Tile ti = tile_of(blockIdx.x + it * gridDim.x, N, Np, per_plane);
+        const uint32_t sa = a0 + (uint32_t)(s * gm.stage_bytes);
+        const uint32_t goff = (uint32_t)(conv_at(N, ti.b, ti.zh, 0, ti.s0) & 7);
+        const uint64_t dg = smem_desc_lin(sa + g_off, 128, G_BYTES) + goff;
+        const uint64_t dx0 = smem_desc_lin(sa, 128, gm.box_bytes);
+        for (int dy = 0; dy < 3; dy++) {
+          // the run holding stencil row dy and the row of dx = -1 within it
+          const long long first = (long long)ti.s0 + (ny == 1 ? -Np : (dy - 1) * Np) - 1;
+          const uint32_t row = (uint32_t)(first & 7) + (ny == 1 ? (uint32_t)(dy * Np) : 0u);
+          const uint32_t run = ny == 1 ? 0u : (uint32_t)(dy * gm.row_bytes) >> 4;
+#pragma unroll
+          for (int dx = 0; dx < 3; dx++) {
+            const uint32_t acc = tmem + (uint32_t)((dy * 3 + dx) * CH);
+#pragma unroll
+            for (int ks = 0; ks < ROWS / 16; ks++)
+              mma_bf16(acc, dx0 + (uint64_t)(run + row + dx + ks * 16), dg + (uint64_t)(ks * 16), idesc,
+                       (it % DRAIN == 0 && ks == 0) ? 0u : 1u);
+          }
+        }
+        mma_commit(&empty_bar[s]);
+        if (it % DRAIN == DRAIN - 1 || it == mine - 1) mma_commit(&acc_full);
+      }
+      mma_commit(&done_bar);
+      if (!mbar_wait(&done_bar, 0)) failed = 1;
+    }
+  } else if (warp == 2) {
+    for (int it = 0; it < mine; it++) {
+      const int s = it % stages;
+      int ok = 1;
+      if (lane == 0) ok = mbar_wait(&full_bar[s], (it / stages) & 1) ? 1 : 0;
+      ok = __shfl_sync(0xffffffffu, ok, 0);
+      if (!ok) {
+        if (lane == 0) failed = 1;
+        break;
+      }
+      const Tile ti = tile_of(blockIdx.x + it * gridDim.x, N, Np, per_plane);
+      const int goff = (int)(conv_at(N, ti.b, ti.zh, 0, ti.s0) & 7);
+      uint8_t *g = base + s * gm.stage_bytes + g_off;
+      for (int i = lane; i < ROWS; i += 32) {
+        const int slot = ti.s0 + i, yh = slot / Np, xh = slot - yh * Np;
+        if (yh < 1 || yh > N || xh < 1 || xh > N)
+          for (int k = 0; k < 4; k++) *reinterpret_cast<uint4 *>(g + k * G_BYTES + (goff + i) * 16) = make_uint4(0, 0, 0, 0);
+      }
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&ready_bar[s]);
+      if (__any_sync(0xffffffffu, *(volatile int *)&failed != 0)) break;
+    }
+  } else {
+    // D row 32 q + lane = (dz = q, ci = lane), row 96 the sums of g; column co
+    const int q = warp & 3, t0 = ((warp - 3) >> 2) * TAPS_PER_WARP;
+    float sum[TAPS_PER_WARP][CH] = {};
+    const int groups = (mine + DRAIN - 1) / DRAIN;
+    bool good = true;
+    for (int grp = 0; grp < groups; grp++) {
+      int ok = 1;
+      if (lane == 0) ok = mbar_wait(&acc_full, grp & 1) ? 1 : 0;
+      ok = __shfl_sync(0xffffffffu, ok, 0);
+      if (!ok) {
+        if (lane == 0) failed = 1;
+        good = false;
+        break;
+      }
+      fence_after();
+#pragma unroll
+      for (int t = 0; t < TAPS_PER_WARP; t++) {
+        uint32_t r[32];
+        tmem_ld32_async(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)((t0 + t) * CH), r);
+        tmem_wait_ld();
+#pragma unroll
+        for (int c = 0; c < CH; c++) sum[t][c] += __uint_as_float(r[c]);
+      }
+      fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&acc_empty);
+    }
+    if (good) {
+#pragma unroll
+      for (int t = 0; t < TAPS_PER_WARP; t++) {
+        const int tap2 = t0 + t;
+        if (q < 3) {
+          float *d = dw + ((long long)(q * TAPS2 + tap2) * CH) * CH + lane;
+#pragma unroll
+          for (int c = 0; c < CH; c++) atomicAdd(d + c * CH, sum[t][c]);
+        } else if (tap2 == 4 && lane == 0 && db) {
+#pragma unroll
+          for (int c = 0; c < CH; c++) atomicAdd(db + c, sum[t][c]);
+        }
+      }
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x == 0 && failed) atomicExch(err, 1);
+  if (warp == 1) {
+    fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(WG_TMEM) : "memory");
+  }
+}
+
+}  // namespace wg
+}  // namespace conv
+
+cudaError_t launch_conv_wgrad(const __nv_bfloat16 *in, const __nv_bfloat16 *g, int N, int batch, float *dw, float *db,
+                              int *err, cudaStream_t s) {
+  using namespace conv;
+  constexpr int MAXDEV = 64;
+  static std::mutex mu;
+  static int sms_of[MAXDEV] = {0};
+  int dev = 0, sms = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  if (dev < 0 || dev >= MAXDEV) return cudaErrorInvalidDevice;
+  {
+    std::lock_guard<std::mutex> lock(mu);
+    if (!sms_of[dev]) {
+      e = cudaFuncSetAttribute(wg::wgrad_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_LIMIT);
+      if (e != cudaSuccess) return e;
+      e = cudaDeviceGetAttribute(&sms_of[dev], cudaDevAttrMultiProcessorCount, dev);
+      if (e != cudaSuccess) return e;
+    }
+    sms = sms_of[dev];
+  }
+  const wg::Geom a = wg::geom_for(N, 1), b = wg::geom_for(N, 3);
+  const int forced = conv_runs();
+  // one run per plane while it is the smaller load and two stages fit
+  const bool planes = forced == 1 ? a.stages >= 1 : forced == 3 ? false : a.stages >= 2;
+  const wg::Geom gm = planes ? a : b;
+  if (N < 2 || batch < 1 || gm.stages < 1 || gm.box_rows > 256) return cudaErrorInvalidValue;
+  const long long lines = conv_units(N, batch) / 8;
+  if (lines >= 0x7fffffffLL) return cudaErrorInvalidValue;
+  CUtensorMap mx, mg;
+  if ((e = make_map_lines(&mx, in, lines, gm.box_rows)) != cudaSuccess) return e;
+  if ((e = make_map_lines(&mg, g, lines, wg::G_ROWS)) != cudaSuccess) return e;
+  const long long tiles = (long long)batch * N * (((long long)N * (N + 2) + ROWS - 1) / ROWS);
+  const int grid = (int)(tiles < sms ? tiles : sms);
+  wg::wgrad_tc_kernel<<<grid, wg::WG_THREADS, gm.smem, s>>>(mx, mg, N, batch, dw, db, err, gm);
+  launch_counter()++;
+  return cudaGetLastError();
+}
+
+}  // namespace sclet

@@ -53,6 +53,7 @@ cudaError_t launch_conv(const __nv_bfloat16 *in, const __nv_bfloat16 *w, const C
 // Input runs per tile of launch_conv (sclet_net_set_conv_runs); returns the
 // previous setting, -1 for an invalid one.
 int conv_set_runs(int runs_per_plane);
+int conv_runs();  // the current setting
 
 // Periodic halo of batch haloed blocks, in place.
 cudaError_t launch_conv_halo(__nv_bfloat16 *a, int N, int batch, cudaStream_t s);
@@ -64,9 +65,10 @@ cudaError_t launch_conv_pack(const float *in, int cin, int N, int batch, __nv_bf
 cudaError_t launch_conv_pack_grad(const float *g, int cout, float scale, int N, int batch, __nv_bfloat16 *a,
                                   cudaStream_t s);
 // dW[t][co][ci] += sum over owned cells of g[cell][co] x in[cell + off(t)][ci];
-// db[co] += sum of g[cell][co] (FP32 accumulators).
+// db[co] += sum of g[cell][co] (FP32 accumulators); db may be null.  err is set
+// to 1 when a bounded wait gives up.
 cudaError_t launch_conv_wgrad(const __nv_bfloat16 *in, const __nv_bfloat16 *g, int N, int batch, float *dw, float *db,
-                              cudaStream_t s);
+                              int *err, cudaStream_t s);
 // FP32 master weights [layers][TAPS][CH][CH] -> BF16 forward copies (same layout)
 // and adjoint copies (taps flipped, co and ci swapped).
 cudaError_t launch_conv_weights(const float *w, int layers, __nv_bfloat16 *wf, __nv_bfloat16 *wt, cudaStream_t s);

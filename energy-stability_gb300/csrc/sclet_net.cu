@@ -168,18 +168,18 @@ int backward(sclet_net *net, int N, int batch, const float *target, double *loss
   NK(launch_conv_pack_grad(net->resid, SCLET_NET_OUT, (float)(2.0 / (double)count) * net->out_scale, N, batch,
                            net->gy, s));
   const int L = LAYERS - 1;
-  NK(launch_conv_wgrad(net->h[SCLET_NET_BLOCKS], net->gy, N, batch, wof(net->g, L), bof(net->g, L), s));
+  NK(launch_conv_wgrad(net->h[SCLET_NET_BLOCKS], net->gy, N, batch, wof(net->g, L), bof(net->g, L), net->dev_err, s));
   __nv_bfloat16 *gcur = net->gh[0], *gnext = net->gh[1];
   NK(launch_conv(net->gy, wl(net->wt, L), conv_args(net, N, batch, CONV_LINEAR, -1, nullptr, gcur), s));
   NK(launch_conv_halo(gcur, N, batch, s));
   for (int k = SCLET_NET_BLOCKS - 1; k >= 0; k--) {
     const int l1 = 2 * k + 1, l2 = 2 * k + 2;
     // h_{k+1} = h_k + conv_l2 r_k: gradient of conv_l2's weights, then of r_k
-    NK(launch_conv_wgrad(net->r[k], gcur, N, batch, wof(net->g, l2), bof(net->g, l2), s));
+    NK(launch_conv_wgrad(net->r[k], gcur, N, batch, wof(net->g, l2), bof(net->g, l2), net->dev_err, s));
     NK(launch_conv(gcur, wl(net->wt, l2), conv_args(net, N, batch, CONV_MASK, -1, net->r[k], net->ga), s));
     NK(launch_conv_halo(net->ga, N, batch, s));
     // r_k = relu(conv_l1 h_k): weights of conv_l1, then h_k (plus the skip path)
-    NK(launch_conv_wgrad(net->h[k], net->ga, N, batch, wof(net->g, l1), bof(net->g, l1), s));
+    NK(launch_conv_wgrad(net->h[k], net->ga, N, batch, wof(net->g, l1), bof(net->g, l1), net->dev_err, s));
     NK(launch_conv(net->ga, wl(net->wt, l1), conv_args(net, N, batch, CONV_RESIDUAL, -1, gcur, gnext), s));
     NK(launch_conv_halo(gnext, N, batch, s));
     __nv_bfloat16 *t = gcur;
@@ -188,7 +188,7 @@ int backward(sclet_net *net, int N, int batch, const float *target, double *loss
   }
   // h0 = relu(conv0 x)
   NK(launch_conv_relu_mask(gcur, net->h[0], N, batch, s));
-  NK(launch_conv_wgrad(net->x, gcur, N, batch, wof(net->g, 0), bof(net->g, 0), s));
+  NK(launch_conv_wgrad(net->x, gcur, N, batch, wof(net->g, 0), bof(net->g, 0), net->dev_err, s));
   NK(cudaStreamSynchronize(s));
   double acc = 0.0;
   for (int i = 0; i < NPARTS; i++) acc += net->part_host[i];

@@ -100,6 +100,58 @@ def test_gradients_match_oracle(learned):
     net.close()
 
 
+@pytest.mark.parametrize("N,B,runs", [(4, 1, 1), (5, 3, 1), (13, 1, 3), (15, 2, 0)])
+def test_weight_gradient_ragged_tiles(N, B, runs, learned, sclet_lib):
+    """The tensor-core weight gradient where a plane is less than one tile,
+    where the last tile of a plane is partial and its slots start off a
+    128-byte line, and with both run tilings; bounds as in
+    test_gradients_match_oracle."""
+    torch = _torch()
+    rng = np.random.default_rng(40 + N)
+    p = co.random_params(12 + N).astype(np.float32)
+    inp = co.bf16(rng.random((B, co.NIN, N, N, N)) - 0.5).astype(np.float32)
+    tgt = (0.2 * rng.standard_normal((B, co.NOUT, N, N, N))).astype(np.float32)
+    L = sclet_lib.lib()
+    assert L.sclet_net_set_conv_runs(runs) in (0, 1, 3)
+    try:
+        net = learned.Net(seed=1, out_scale=0.5)
+        net.set_params(p)
+        _, g = net.gradient(torch.from_numpy(inp).cuda(), torch.from_numpy(tgt).cuda())
+        net.close()
+    finally:
+        L.sclet_net_set_conv_runs(0)
+    _, want = co.loss_and_grad(p.astype(np.float64), inp.astype(np.float64), tgt.astype(np.float64), 0.5,
+                               bf16_round=True)
+    gW, gb = co.unpack(g.astype(np.float64))
+    wW, wb = co.unpack(want)
+    for layer in range(co.LAYERS):
+        assert rel(gW[layer], wW[layer]) <= (5e-2 if layer == 0 else 1e-2), (layer, rel(gW[layer], wW[layer]))
+        assert rel(gb[layer], wb[layer]) <= 1e-2, (layer, rel(gb[layer], wb[layer]))
+
+
+def test_weight_gradient_sums_over_many_tiles(learned):
+    """A batch's gradient is the mean of its samples' gradients.  At 4 x 48^3 a
+    CTA sums two dozen tiles through several drains of its accumulators, at
+    1 x 48^3 six through one; the sample count is a power of two, so the
+    stored BF16 values agree and only the FP32 sums differ: at most 64
+    accumulator roundings of 2^-24 each side, and round-to-nearest adds."""
+    torch = _torch()
+    rng = np.random.default_rng(77)
+    N, B = 48, 4
+    x = torch.from_numpy((rng.random((B, co.NIN, N, N, N)) - 0.5).astype(np.float32)).cuda()
+    y = torch.from_numpy((0.2 * rng.standard_normal((B, co.NOUT, N, N, N))).astype(np.float32)).cuda()
+    net = learned.Net(seed=1, out_scale=0.5)
+    net.set_params(co.random_params(5).astype(np.float32))
+    _, g = net.gradient(x, y)
+    one = sum(net.gradient(x[b:b + 1].contiguous(), y[b:b + 1].contiguous())[1].astype(np.float64) for b in range(B))
+    net.close()
+    gW, gb = co.unpack(g.astype(np.float64))
+    oW, ob = co.unpack(one / B)
+    for layer in range(co.LAYERS):
+        assert rel(gW[layer], oW[layer]) <= 1e-5, (layer, rel(gW[layer], oW[layer]))
+        assert rel(gb[layer], ob[layer]) <= 1e-5, (layer, rel(gb[layer], ob[layer]))
+
+
 def _omega(seed, N=32):
     return cases.Case(big_n=N, nac=4, nch=0, dt=0.01, steps=1000, epn2=0.5, elastic=1, seed=seed, suffix="lc")
 
