@@ -21,8 +21,7 @@
 
 namespace sclet {
 
-constexpr int ZC = 32;  // default z-planes per CTA of the Allen-Cahn kernel
-constexpr int PZ = 16;  // z-planes per CTA of the one-cell-per-thread CH kernels
+constexpr int PZ = 16;  // z-planes per CTA of the variable-mobility kernels
 
 template <typename T>
 struct P {
@@ -31,7 +30,7 @@ struct P {
   T ih2x, ih2y, ih2z;   // 1 / h^2 per axis
   T i2hx, i2hy, i2hz;   // 1 / (2 h) per axis
   T K[16];              // plugin constants (reference composition shifted by cshift)
-  int zc, runs;         // z-planes per CTA (AC kernel); runs side by side
+  int zc, runs;         // z-planes per CTA; runs side by side
   const double *krun;   // per-run plugin constant 0, or null
   // anisotropic term folded: kan[m][3 r + c] = epn2 LE (1/2h_r) lam_m[r][c] (1/2h_c),
   // the flux row r differenced along axis r
@@ -49,7 +48,7 @@ static P<T> to_p(const Phys &ph) {
   p.i2hx = (T)(0.5 / ph.h[0]); p.i2hy = (T)(0.5 / ph.h[1]); p.i2hz = (T)(0.5 / ph.h[2]);
   p.LE = (T)ph.LE; p.KE = (T)ph.KE; p.LCI = (T)ph.LCI; p.KCI = (T)ph.KCI; p.es = (T)ph.elastic_scale;
   for (int k = 0; k < 16; k++) p.K[k] = (T)ph.K[k];
-  p.zc = ph.rhs_zc > 0 ? ph.rhs_zc : ZC;
+  p.zc = ph.rhs_zc;
   p.runs = ph.runs > 0 ? ph.runs : 1;
   p.krun = ph.krun;
   const double i2h[3] = {0.5 / ph.h[0], 0.5 / ph.h[1], 0.5 / ph.h[2]};
@@ -86,20 +85,186 @@ __device__ __forceinline__ T ch_f(const P<T> &p, const T *e, T c) {
 
 __device__ inline long long L3(int n, int z, int y, int x) { return ((long long)z * n + y) * n + x; }
 
-// One cell per thread on a 3-D launch: threadIdx.x along x (coalesced),
-// blockIdx.z = z; no index division.
+// img() for v in -1 .. n: one wrap, no division
+__device__ __forceinline__ int img1(int n, int v) {
+  const int N = n - 4;
+  int r = v - 2;
+  r += r < 0 ? N : 0;
+  r -= r >= N ? N : 0;
+  return 2 + r;
+}
+
+// The cells on the block's six faces, z faces first: s in 0 .. face_cells(n) - 1.
+__host__ __device__ inline int face_cells(int n) { return 2 * n * n + 2 * n * (n - 2) + 2 * (n - 2) * (n - 2); }
+__device__ __forceinline__ void face_cell(int n, int s, int &z, int &y, int &x) {
+  const int nn = n * n, i = n - 2;
+  if (s < 2 * nn) {
+    z = s < nn ? 0 : n - 1;
+    const int r = s < nn ? s : s - nn;
+    y = r / n;
+    x = r - y * n;
+    return;
+  }
+  s -= 2 * nn;
+  if (s < 2 * n * i) {
+    const int q = s / n;  // row: z, then the two y faces
+    x = s - q * n;
+    z = 1 + (q >> 1);
+    y = (q & 1) ? n - 1 : 0;
+    return;
+  }
+  s -= 2 * n * i;
+  const int q = s >> 1;
+  x = (s & 1) ? n - 1 : 0;
+  z = 1 + q / i;
+  y = 1 + q % i;
+}
+
+// threadIdx.x along x (coalesced), threadIdx.y along y
 constexpr int RX = 32, RY = 8;
 
-// Allen-Cahn right-hand side, 2.5-D: a CTA owns a 32 x 8 (x, y) tile and
-// marches over p.zc planes in z (ZC by default), keeping for every order parameter a ring of five
+// ---- Allen-Cahn, no stencil or a diagonal one ------------------------------
+// Without the anisotropic term a cell needs its own values only; with a
+// diagonal lambda (the usual case: diag(kk) - diag file) it needs the cells two
+// away along each axis.  Either way no plane has to be shared: a thread owns an
+// (x, y) column, keeps the five z-values of each order parameter in registers
+// as it marches, and takes x +- 2 and y +- 2 through L1.  The face cells, whose
+// boundary lifting reads far images and would stall whole warps of the march,
+// are computed apart by the launch's last CTAs (one cell per thread).
+// Bound by the FP32 issue and L1 (FP64: the FP64 pipe).  Before, every case
+// took the five-plane shared-memory ring below with the lifting inside; all
+// right-hand sides of a step, then and now: 4 fields of 36^3, FP32, no tensor
+// 103 -> 8 us; 4 + 1 fields of 196^3, diagonal tensors 525 -> 257 us, of 516^3
+// 5.74 -> 3.69 ms; 4 fields of 68^3 in FP64 303 -> 61 us.
+template <typename PL, typename T, int NAC, bool DIAG>
+__global__ void __launch_bounds__(RX * RY, sizeof(T) == 4 ? 3 : 2)
+    rhs_ac_diag_kernel(P<T> p0, const T *__restrict__ u, const T *__restrict__ felas, T *__restrict__ out, int zblocks) {
+  const int n = p0.n;
+  const size_t nn = (size_t)n * n, n3 = nn * n;
+  P<T> p = p0;
+  const bool el = p.elastic == 1, has_c = p.nch > 0;
+  if ((int)blockIdx.z < zblocks) {
+    const int zchunks = (n + p.zc - 1) / p.zc;
+    const int run = blockIdx.z / zchunks, zci = blockIdx.z - run * zchunks;
+    if (p0.krun) p.K[0] = (T)p0.krun[run];
+    u += (size_t)run * p.F * n3;
+    felas += (size_t)run * NAC * n3;
+    out += (size_t)run * p.F * n3;
+    const int x = blockIdx.x * RX + threadIdx.x, y = blockIdx.y * RY + threadIdx.y;
+    if (x < 1 || x > n - 2 || y < 1 || y > n - 2) return;
+    const int z0 = max(1, zci * p.zc), z1 = min(n - 1, (zci + 1) * p.zc);
+    if (z0 >= z1) return;
+    size_t l = (size_t)z0 * nn + (size_t)y * n + x;
+    T w[NAC][5];  // planes z - 2 .. z + 2
+    if (DIAG) {
+#pragma unroll
+      for (int m = 0; m < NAC; m++) {
+        const T *um = u + m * n3 + l;
+        w[m][1] = z0 > 1 ? um[-2 * (long long)nn] : (T)0;
+        w[m][2] = um[-(long long)nn];
+        w[m][3] = um[0];
+        w[m][4] = um[nn];
+      }
+    }
+    for (int z = z0; z < z1; z++, l += nn) {
+      T e[NAC], xm[NAC], xp[NAC], ym[NAC], yp[NAC], fe[NAC];
+#pragma unroll
+      for (int m = 0; m < NAC; m++) {
+        const T *um = u + m * n3 + l;
+        if (DIAG) {
+#pragma unroll
+          for (int k = 0; k < 4; k++) w[m][k] = w[m][k + 1];
+          w[m][4] = z < n - 2 ? um[2 * nn] : (T)0;
+          e[m] = w[m][2];
+          xm[m] = x > 1 ? um[-2] : (T)0;
+          xp[m] = x < n - 2 ? um[2] : (T)0;
+          ym[m] = y > 1 ? um[-2 * n] : (T)0;
+          yp[m] = y < n - 2 ? um[2 * n] : (T)0;
+        } else {
+          e[m] = um[0];
+        }
+        fe[m] = el ? felas[m * n3 + l] : (T)0;
+      }
+      const T c = has_c ? u[NAC * n3 + l] : (T)0;
+#pragma unroll
+      for (int m = 0; m < NAC; m++) {
+        T v = p.LE * p.KE * e[m];
+        v -= p.LE * ac_f_n<PL, T, NAC>(p, e, c, m);
+        if (DIAG) {
+          const T *k = p.kan[m];
+          const T ar = k[0] * (xp[m] - e[m]), al = k[0] * (e[m] - xm[m]);
+          const T at = k[4] * (ym[m] - e[m]), ab = k[4] * (e[m] - yp[m]);
+          const T af = k[8] * (w[m][0] - e[m]), ak = k[8] * (e[m] - w[m][4]);
+          v -= ((ar - al) + (at - ab)) + (af - ak);
+        }
+        if (el) v -= p.LE * p.es * fe[m];
+        out[m * n3 + l] = v;
+      }
+    }
+    return;
+  }
+  // face cells of every run
+  const int per = face_cells(n), total = per * p.runs;
+  const int stride = (int)(gridDim.z - zblocks) * gridDim.y * gridDim.x * (RX * RY);
+  int i = (((int)blockIdx.z - zblocks) * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
+  for (i = i * (RX * RY) + threadIdx.y * RX + threadIdx.x; i < total; i += stride) {
+    const int run = i / per;
+    int z, y, x;
+    face_cell(n, i - run * per, z, y, x);
+    if (p0.krun) p.K[0] = (T)p0.krun[run];
+    const T *ur = u + (size_t)run * p.F * n3;
+    const size_t l = (size_t)z * nn + (size_t)y * n + x;
+    const int iz = img1(n, z), iy = img1(n, y), ix = img1(n, x), lo = img1(n, -1), hi = img1(n, n);
+    T e[NAC], lift[NAC];
+#pragma unroll
+    for (int m = 0; m < NAC; m++) {
+      e[m] = ur[m * n3 + l];
+      lift[m] = (T)0;
+    }
+    const T c = has_c ? ur[NAC * n3 + l] : (T)0;
+    // per face the cell lies on: the cell beyond it, at its periodic image
+    auto add = [&](size_t q, T ih2) {
+#pragma unroll
+      for (int m = 0; m < NAC; m++) lift[m] += p.LE * p.epn2 * ur[m * n3 + q] * ih2;
+    };
+    if (x == 0) add(L3(n, iz, iy, lo), p.ih2x);
+    if (x == n - 1) add(L3(n, iz, iy, hi), p.ih2x);
+    if (y == 0) add(L3(n, iz, lo, ix), p.ih2y);
+    if (y == n - 1) add(L3(n, iz, hi, ix), p.ih2y);
+    if (z == 0) add(L3(n, lo, iy, ix), p.ih2z);
+    if (z == n - 1) add(L3(n, hi, iy, ix), p.ih2z);
+#pragma unroll
+    for (int m = 0; m < NAC; m++) {
+      T v = p.LE * p.KE * e[m];
+      v -= p.LE * ac_f_n<PL, T, NAC>(p, e, c, m);
+      v += lift[m];
+      if (DIAG) {
+        const T *um = ur + m * n3 + l, *k = p.kan[m];
+        // a flux is zero outside the block, a value outside it too
+        const T ar = x < n - 1 ? k[0] * ((x < n - 2 ? um[2] : (T)0) - e[m]) : (T)0;
+        const T al = x > 0 ? k[0] * (e[m] - (x > 1 ? um[-2] : (T)0)) : (T)0;
+        const T at = y > 0 ? k[4] * ((y > 1 ? um[-2 * n] : (T)0) - e[m]) : (T)0;
+        const T ab = y < n - 1 ? k[4] * (e[m] - (y < n - 2 ? um[2 * n] : (T)0)) : (T)0;
+        const T af = z > 0 ? k[8] * ((z > 1 ? um[-2 * (long long)nn] : (T)0) - e[m]) : (T)0;
+        const T ak = z < n - 1 ? k[8] * (e[m] - (z < n - 2 ? um[2 * nn] : (T)0)) : (T)0;
+        v -= ((ar - al) + (at - ab)) + (af - ak);
+      }
+      if (el) v -= p.LE * p.es * felas[((size_t)run * NAC + m) * n3 + l];
+      out[((size_t)run * p.F + m) * n3 + l] = v;
+    }
+  }
+}
+
+// ---- Allen-Cahn, full gradient tensors ---------------------------------------
+// 2.5-D: a CTA owns a 32 x 8 (x, y) tile and
+// marches over p.zc planes in z, keeping for every order parameter a ring of five
 // planes (z-2 .. z+2) with a two-cell halo in x and y in shared memory (zero
 // outside the block, as ac_calc_F2 reads it).  Each value comes from global
 // memory about once per CTA instead of once per stencil tap.
-// (ZC, the default planes per CTA, is defined at the top of the file)
 constexpr int HX = RX + 4, HY = RY + 4;
 constexpr int PLANE = HX * HY;     // one haloed plane
 
-template <typename PL, typename T, int NAC, bool ANISO>
+template <typename PL, typename T, int NAC>
 __global__ void __launch_bounds__(RX * RY, sizeof(T) == 4 ? 3 : 1) rhs_ac_kernel(P<T> p0, const T *__restrict__ u, const T *__restrict__ felas,
                                                          T *__restrict__ out) {
   extern __shared__ unsigned char smem_raw[];
@@ -180,7 +345,7 @@ __global__ void __launch_bounds__(RX * RY, sizeof(T) == 4 ? 3 : 1) rhs_ac_kernel
         T v = p.LE * p.KE * e[m];
         v -= p.LE * ac_f_n<PL, T, NAC>(p, e, c, m);
         if (face) {
-          const int iz = img(n, z), iy = img(n, y), ix = img(n, x), lo = img(n, -1), hi = img(n, n);
+          const int iz = img1(n, z), iy = img1(n, y), ix = img1(n, x), lo = img1(n, -1), hi = img1(n, n);
           const T w = p.LE * p.epn2;
           if (x == 0) v += w * um[L3(n, iz, iy, lo)] * p.ih2x;
           if (x == n - 1) v += w * um[L3(n, iz, iy, hi)] * p.ih2x;
@@ -189,7 +354,7 @@ __global__ void __launch_bounds__(RX * RY, sizeof(T) == 4 ? 3 : 1) rhs_ac_kernel
           if (z == 0) v += w * um[L3(n, lo, iy, ix)] * p.ih2z;
           if (z == n - 1) v += w * um[L3(n, hi, iy, ix)] * p.ih2z;
         }
-        if (ANISO) {
+        {
           // div(lambda grad eta), ac_calc_F2 (anisotropic.c:164-628): the flux
           // component c at a neighbour q is lam[c] . (central differences at q),
           // zero when q is outside the block; y and z differences are
@@ -219,44 +384,6 @@ __global__ void __launch_bounds__(RX * RY, sizeof(T) == 4 ? 3 : 1) rhs_ac_kernel
   }
 }
 
-// t = -LCI KCI c + LCI CH_f, minus the face liftings (first part of
-// ch_calc_FU_ConstantMobility).
-template <typename PL, typename T>
-__global__ void __launch_bounds__(RX * RY) rhs_ch_t_kernel(P<T> p0, const T *__restrict__ u, T *__restrict__ t) {
-  const int n = p0.n;
-  const int zch = (n + PZ - 1) / PZ;  // blockIdx.z = run x chunk of PZ planes
-  const int run = blockIdx.z / zch, z0 = (blockIdx.z - run * zch) * PZ, z1 = z0 + PZ < n ? z0 + PZ : n;
-  const int x = blockIdx.x * RX + threadIdx.x, y = blockIdx.y * RY + threadIdx.y;
-  if (x >= n || y >= n) return;
-  const size_t n3 = (size_t)n * n * n;
-  P<T> p = p0;
-  if (p0.krun) p.K[0] = (T)p0.krun[run];
-  u += (size_t)run * p.F * n3;
-  t += (size_t)run * n3;
-  for (int z = z0; z < z1; z++) {
-    const size_t l = ((size_t)z * n + y) * n + x;
-    const T *cf = u + p.nac * n3;
-    T e[4] = {(T)0, (T)0, (T)0, (T)0};
-#pragma unroll
-    for (int m = 0; m < 4; m++)
-      if (m < p.nac) e[m] = u[m * n3 + l];
-    const T c = cf[l];
-    T v = -p.LCI * p.KCI * c;
-    v += p.LCI * ch_f<PL>(p, e, c);
-    if (x == 0 || x == n - 1 || y == 0 || y == n - 1 || z == 0 || z == n - 1) {
-      const int iz = img(n, z), iy = img(n, y), ix = img(n, x), lo = img(n, -1), hi = img(n, n);
-      const T w = p.LCI * p.epn2;
-      if (x == 0) v -= w * cf[L3(n, iz, iy, lo)] * p.ih2x;
-      if (x == n - 1) v -= w * cf[L3(n, iz, iy, hi)] * p.ih2x;
-      if (y == 0) v -= w * cf[L3(n, iz, lo, ix)] * p.ih2y;
-      if (y == n - 1) v -= w * cf[L3(n, iz, hi, ix)] * p.ih2y;
-      if (z == 0) v -= w * cf[L3(n, lo, iy, ix)] * p.ih2z;
-      if (z == n - 1) v -= w * cf[L3(n, hi, iy, ix)] * p.ih2z;
-    }
-    t[l] = v;
-  }
-}
-
 // Boundary chemical potential at periodic image cell (z,y,x) (ch_mu).
 template <typename PL, typename T>
 __device__ inline T ch_mu_at(const P<T> &p, const T *__restrict__ u, int z, int y, int x) {
@@ -264,9 +391,9 @@ __device__ inline T ch_mu_at(const P<T> &p, const T *__restrict__ u, int z, int 
   long long n3 = (long long)n * n * n;
   const T *cf = u + p.nac * n3;
   T cv = cf[L3(n, z, y, x)];
-  T lap = (cf[L3(n, z, y, img(n, x - 1))] + (T)(-2.0) * cv + cf[L3(n, z, y, img(n, x + 1))]) * p.ih2x;
-  lap += (cf[L3(n, z, img(n, y - 1), x)] + (T)(-2.0) * cv + cf[L3(n, z, img(n, y + 1), x)]) * p.ih2y;
-  lap += (cf[L3(n, img(n, z - 1), y, x)] + (T)(-2.0) * cv + cf[L3(n, img(n, z + 1), y, x)]) * p.ih2z;
+  T lap = (cf[L3(n, z, y, img1(n, x - 1))] + (T)(-2.0) * cv + cf[L3(n, z, y, img1(n, x + 1))]) * p.ih2x;
+  lap += (cf[L3(n, z, img1(n, y - 1), x)] + (T)(-2.0) * cv + cf[L3(n, z, img1(n, y + 1), x)]) * p.ih2y;
+  lap += (cf[L3(n, img1(n, z - 1), y, x)] + (T)(-2.0) * cv + cf[L3(n, img1(n, z + 1), y, x)]) * p.ih2z;
   T e[4] = {(T)0, (T)0, (T)0, (T)0};
   for (int m = 0; m < p.nac; m++) e[m] = u[m * n3 + L3(n, z, y, x)];
   T mu = p.LCI * p.epn2 * lap;
@@ -274,43 +401,122 @@ __device__ inline T ch_mu_at(const P<T> &p, const T *__restrict__ u, int z, int 
   return mu;
 }
 
+// The two constant-mobility kernels: p.zc planes per CTA away from the faces,
+// the face cells (whose lifting reads far images) one per thread in the
+// launch's last CTAs, so that no warp of the march waits on them.
+
+// t = -LCI KCI c + LCI CH_f, minus the face liftings (first part of
+// ch_calc_FU_ConstantMobility).
+template <typename PL, typename T>
+__global__ void __launch_bounds__(RX * RY) rhs_ch_t_kernel(P<T> p0, const T *__restrict__ u, T *__restrict__ t,
+                                                           int zblocks) {
+  const int n = p0.n;
+  const size_t nn = (size_t)n * n, n3 = nn * n;
+  P<T> p = p0;
+  auto value = [&](const T *ur, size_t l) {
+    T e[4] = {(T)0, (T)0, (T)0, (T)0};
+#pragma unroll
+    for (int m = 0; m < 4; m++)
+      if (m < p.nac) e[m] = ur[m * n3 + l];
+    const T c = ur[p.nac * n3 + l];
+    T v = -p.LCI * p.KCI * c;
+    v += p.LCI * ch_f<PL>(p, e, c);
+    return v;
+  };
+  if ((int)blockIdx.z < zblocks) {
+    const int zch = (n + p.zc - 1) / p.zc;
+    const int run = blockIdx.z / zch, zci = blockIdx.z - run * zch;
+    const int x = blockIdx.x * RX + threadIdx.x, y = blockIdx.y * RY + threadIdx.y;
+    if (x < 1 || x > n - 2 || y < 1 || y > n - 2) return;
+    if (p0.krun) p.K[0] = (T)p0.krun[run];
+    u += (size_t)run * p.F * n3;
+    t += (size_t)run * n3;
+    const int z0 = max(1, zci * p.zc), z1 = min(n - 1, (zci + 1) * p.zc);
+#pragma unroll 2
+    for (int z = z0; z < z1; z++) {
+      const size_t l = (size_t)z * nn + (size_t)y * n + x;
+      t[l] = value(u, l);
+    }
+    return;
+  }
+  const int per = face_cells(n), total = per * p.runs;
+  const int stride = (int)(gridDim.z - zblocks) * gridDim.y * gridDim.x * (RX * RY);
+  int i = (((int)blockIdx.z - zblocks) * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
+  for (i = i * (RX * RY) + threadIdx.y * RX + threadIdx.x; i < total; i += stride) {
+    const int run = i / per;
+    int z, y, x;
+    face_cell(n, i - run * per, z, y, x);
+    if (p0.krun) p.K[0] = (T)p0.krun[run];
+    const T *ur = u + (size_t)run * p.F * n3, *cf = ur + p.nac * n3;
+    const size_t l = (size_t)z * nn + (size_t)y * n + x;
+    T v = value(ur, l);
+    const int iz = img1(n, z), iy = img1(n, y), ix = img1(n, x), lo = img1(n, -1), hi = img1(n, n);
+    const T w = p.LCI * p.epn2;
+    if (x == 0) v -= w * cf[L3(n, iz, iy, lo)] * p.ih2x;
+    if (x == n - 1) v -= w * cf[L3(n, iz, iy, hi)] * p.ih2x;
+    if (y == 0) v -= w * cf[L3(n, iz, lo, ix)] * p.ih2y;
+    if (y == n - 1) v -= w * cf[L3(n, iz, hi, ix)] * p.ih2y;
+    if (z == 0) v -= w * cf[L3(n, lo, iy, ix)] * p.ih2z;
+    if (z == n - 1) v -= w * cf[L3(n, hi, iy, ix)] * p.ih2z;
+    t[(size_t)run * n3 + l] = v;
+  }
+}
+
 // N_c = lap(t) (zero outside), minus mu(outside)/h^2 on faces.
 template <typename PL, typename T>
 __global__ void __launch_bounds__(RX * RY) rhs_ch_lap_kernel(P<T> p0, const T *__restrict__ u, const T *__restrict__ t,
-                                                             T *__restrict__ out) {
+                                                             T *__restrict__ out, int zblocks) {
   const int n = p0.n;
-  const int zch = (n + PZ - 1) / PZ;  // blockIdx.z = run x chunk of PZ planes
-  const int run = blockIdx.z / zch, z0 = (blockIdx.z - run * zch) * PZ, z1 = z0 + PZ < n ? z0 + PZ : n;
-  const int x = blockIdx.x * RX + threadIdx.x, y = blockIdx.y * RY + threadIdx.y;
-  if (x >= n || y >= n) return;
+  const size_t nn = (size_t)n * n, n3 = nn * n;
   P<T> p = p0;
-  if (p0.krun) p.K[0] = (T)p0.krun[run];
-  {
-    const size_t n3 = (size_t)n * n * n;
-    u += (size_t)run * p.F * n3;
+  if ((int)blockIdx.z < zblocks) {
+    const int zch = (n + p.zc - 1) / p.zc;
+    const int run = blockIdx.z / zch, zci = blockIdx.z - run * zch;
+    const int x = blockIdx.x * RX + threadIdx.x, y = blockIdx.y * RY + threadIdx.y;
+    if (x < 1 || x > n - 2 || y < 1 || y > n - 2) return;
     t += (size_t)run * n3;
     out += (size_t)run * p.F * n3;
+    const int z0 = max(1, zci * p.zc), z1 = min(n - 1, (zci + 1) * p.zc);
+    if (z0 >= z1) return;
+    size_t l = (size_t)z0 * nn + (size_t)y * n + x;
+    T tm = t[l - nn], tc = t[l];  // planes z - 1 and z
+#pragma unroll 2
+    for (int z = z0; z < z1; z++, l += nn) {
+      const T tp = t[l + nn];
+      T v = (t[l - 1] + t[l + 1] - (T)2 * tc) * p.ih2x;
+      v += (t[l - n] + t[l + n] - (T)2 * tc) * p.ih2y;
+      v += (tm + tp - (T)2 * tc) * p.ih2z;
+      out[l] = v;
+      tm = tc;
+      tc = tp;
+    }
+    return;
   }
-  const size_t nn = (size_t)n * n;
-  for (int z = z0; z < z1; z++) {
+  const int per = face_cells(n), total = per * p.runs;
+  const int stride = (int)(gridDim.z - zblocks) * gridDim.y * gridDim.x * (RX * RY);
+  int i = (((int)blockIdx.z - zblocks) * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
+  for (i = i * (RX * RY) + threadIdx.y * RX + threadIdx.x; i < total; i += stride) {
+    const int run = i / per;
+    int z, y, x;
+    face_cell(n, i - run * per, z, y, x);
+    if (p0.krun) p.K[0] = (T)p0.krun[run];
+    const T *ur = u + (size_t)run * p.F * n3, *tr = t + (size_t)run * n3;
     const size_t l = (size_t)z * nn + (size_t)y * n + x;
-    const T tc = t[l];
-    const T fl = x > 0 ? t[l - 1] : (T)0, fr = x < n - 1 ? t[l + 1] : (T)0;
-    const T ft = y > 0 ? t[l - n] : (T)0, fb = y < n - 1 ? t[l + n] : (T)0;
-    const T ff = z > 0 ? t[l - nn] : (T)0, fk = z < n - 1 ? t[l + nn] : (T)0;
+    const T tc = tr[l];
+    const T fl = x > 0 ? tr[l - 1] : (T)0, fr = x < n - 1 ? tr[l + 1] : (T)0;
+    const T ft = y > 0 ? tr[l - n] : (T)0, fb = y < n - 1 ? tr[l + n] : (T)0;
+    const T ff = z > 0 ? tr[l - nn] : (T)0, fk = z < n - 1 ? tr[l + nn] : (T)0;
     T v = (fl + fr - (T)2 * tc) * p.ih2x;
     v += (ft + fb - (T)2 * tc) * p.ih2y;
     v += (ff + fk - (T)2 * tc) * p.ih2z;
-    if (x == 0 || x == n - 1 || y == 0 || y == n - 1 || z == 0 || z == n - 1) {
-      const int iz = img(n, z), iy = img(n, y), ix = img(n, x), lo = img(n, -1), hi = img(n, n);
-      if (x == 0) v -= ch_mu_at<PL>(p, u, iz, iy, lo) * p.ih2x;
-      if (x == n - 1) v -= ch_mu_at<PL>(p, u, iz, iy, hi) * p.ih2x;
-      if (y == 0) v -= ch_mu_at<PL>(p, u, iz, lo, ix) * p.ih2y;
-      if (y == n - 1) v -= ch_mu_at<PL>(p, u, iz, hi, ix) * p.ih2y;
-      if (z == 0) v -= ch_mu_at<PL>(p, u, lo, iy, ix) * p.ih2z;
-      if (z == n - 1) v -= ch_mu_at<PL>(p, u, hi, iy, ix) * p.ih2z;
-    }
-    out[l] = v;
+    const int iz = img1(n, z), iy = img1(n, y), ix = img1(n, x), lo = img1(n, -1), hi = img1(n, n);
+    if (x == 0) v -= ch_mu_at<PL>(p, ur, iz, iy, lo) * p.ih2x;
+    if (x == n - 1) v -= ch_mu_at<PL>(p, ur, iz, iy, hi) * p.ih2x;
+    if (y == 0) v -= ch_mu_at<PL>(p, ur, iz, lo, ix) * p.ih2y;
+    if (y == n - 1) v -= ch_mu_at<PL>(p, ur, iz, hi, ix) * p.ih2y;
+    if (z == 0) v -= ch_mu_at<PL>(p, ur, lo, iy, ix) * p.ih2z;
+    if (z == n - 1) v -= ch_mu_at<PL>(p, ur, hi, iy, ix) * p.ih2z;
+    out[(size_t)run * p.F * n3 + l] = v;
   }
 }
 
@@ -401,7 +607,7 @@ __global__ void __launch_bounds__(RX * RY) mob_t_kernel(P<T> p0, const T *__rest
     T a = -f0 + p.KCI * c;
     T b = p.epn2 * la - f0;
     if (x == 0 || x == n - 1 || y == 0 || y == n - 1 || z == 0 || z == n - 1) {
-      const int iz = img(n, z), iy = img(n, y), ix = img(n, x), lo = img(n, -1), hi = img(n, n);
+      const int iz = img1(n, z), iy = img1(n, y), ix = img1(n, x), lo = img1(n, -1), hi = img1(n, n);
       T w;
       if (x == 0) { w = p.epn2 * cf[L3(n, iz, iy, lo)] * p.ih2x; a += w; b += w; }
       if (x == n - 1) { w = p.epn2 * cf[L3(n, iz, iy, hi)] * p.ih2x; a += w; b += w; }
@@ -443,7 +649,7 @@ __global__ void __launch_bounds__(RX * RY) mob_n_kernel(P<T> p0, const T *__rest
     la += (af + ak - (T)2 * tc) * p.ih2z;
     T f1 = -C * la;
     if (x == 0 || x == n - 1 || y == 0 || y == n - 1 || z == 0 || z == n - 1) {
-      const int iz = img(n, z), iy = img(n, y), ix = img(n, x), lo = img(n, -1), hi = img(n, n);
+      const int iz = img1(n, z), iy = img1(n, y), ix = img1(n, x), lo = img1(n, -1), hi = img1(n, n);
       if (x == 0) f1 -= C * ch_mu_at<PL>(p, u, iz, iy, lo) * p.ih2x;
       if (x == n - 1) f1 -= C * ch_mu_at<PL>(p, u, iz, iy, hi) * p.ih2x;
       if (y == 0) f1 -= C * ch_mu_at<PL>(p, u, iz, lo, ix) * p.ih2y;
@@ -476,24 +682,47 @@ __global__ void __launch_bounds__(RX * RY) mob_n_kernel(P<T> p0, const T *__rest
   }
 }
 
+// z-planes per CTA: the tuned value if any, else the most of `zmax`, zmax / 2,
+// .. 2 that still gives every SM four CTAs (a small block marched 32 planes a
+// CTA left 20 CTAs on 152 SMs: 121 us at 36^3).
+static int planes_per_cta(const Phys &ph, int tuned, int zmax, int runs) {
+  if (tuned > 0) return tuned;
+  const long long tiles = (long long)((ph.n + RX - 1) / RX) * ((ph.n + RY - 1) / RY) * runs;
+  int zc = zmax;
+  while (zc > 2 && tiles * ((ph.n + zc - 1) / zc) < 4 * 152) zc /= 2;
+  return zc;
+}
+
 template <typename PL, typename T>
 static cudaError_t launch_rhs_pl(const Phys &ph, const T *u, const T *felas, T *out, T *scratch, cudaStream_t s) {
   P<T> p = to_p<T>(ph);
   long long n3 = (long long)ph.n * ph.n * ph.n;
-  const dim3 blk(RX, RY), grd((ph.n + RX - 1) / RX, (ph.n + RY - 1) / RY, ((ph.n + PZ - 1) / PZ) * p.runs);
+  const int gx = (ph.n + RX - 1) / RX, gy = (ph.n + RY - 1) / RY;
+  const dim3 blk(RX, RY), grd(gx, gy, ((ph.n + PZ - 1) / PZ) * p.runs);
+  // CTAs (in z) for the face cells of the kernels that take them apart
+  const int zface = (int)(((long long)face_cells(ph.n) * p.runs + RX * RY * gx * gy - 1) / ((long long)RX * RY * gx * gy));
   if (ph.nac > 0) {
+    bool diag = true;  // every gradient tensor diagonal
+    for (int m = 0; m < ph.nac; m++)
+      for (int k = 0; k < 9; k++) diag = diag && (k % 4 == 0 || p.kan[m][k] == (T)0);
+    const bool ring = ph.anisotropic && !diag;
+    p.zc = planes_per_cta(ph, ph.rhs_zc, ph.anisotropic ? 32 : 8, p.runs);
+    const int zblocks = ((ph.n + p.zc - 1) / p.zc) * p.runs;
     const size_t smem = sizeof(T) * ph.nac * 5 * PLANE;
-    const dim3 gac((ph.n + RX - 1) / RX, (ph.n + RY - 1) / RY, ((ph.n + p.zc - 1) / p.zc) * p.runs);
     cudaError_t e = cudaSuccess;
-    switch (ph.nac * 2 + (ph.anisotropic ? 1 : 0)) {
-#define SCLET_RHS_AC(NAC, AN)                                                                                  \
-  case NAC * 2 + AN:                                                                                           \
-    e = cudaFuncSetAttribute(rhs_ac_kernel<PL, T, NAC, AN>, cudaFuncAttributeMaxDynamicSharedMemorySize,        \
-                             (int)smem);                                                                       \
-    if (e == cudaSuccess) rhs_ac_kernel<PL, T, NAC, AN><<<gac, blk, smem, s>>>(p, u, felas, out);               \
+    switch (ph.nac * 3 + (ring ? 2 : ph.anisotropic ? 1 : 0)) {
+#define SCLET_RHS_AC(NAC)                                                                                         \
+  case NAC * 3:                                                                                                   \
+    rhs_ac_diag_kernel<PL, T, NAC, false><<<dim3(gx, gy, zblocks + zface), blk, 0, s>>>(p, u, felas, out, zblocks); \
+    break;                                                                                                        \
+  case NAC * 3 + 1:                                                                                               \
+    rhs_ac_diag_kernel<PL, T, NAC, true><<<dim3(gx, gy, zblocks + zface), blk, 0, s>>>(p, u, felas, out, zblocks);  \
+    break;                                                                                                        \
+  case NAC * 3 + 2:                                                                                               \
+    e = cudaFuncSetAttribute(rhs_ac_kernel<PL, T, NAC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);   \
+    if (e == cudaSuccess) rhs_ac_kernel<PL, T, NAC><<<dim3(gx, gy, zblocks), blk, smem, s>>>(p, u, felas, out);     \
     break;
-      SCLET_RHS_AC(1, 0) SCLET_RHS_AC(1, 1) SCLET_RHS_AC(2, 0) SCLET_RHS_AC(2, 1)
-      SCLET_RHS_AC(3, 0) SCLET_RHS_AC(3, 1) SCLET_RHS_AC(4, 0) SCLET_RHS_AC(4, 1)
+      SCLET_RHS_AC(1) SCLET_RHS_AC(2) SCLET_RHS_AC(3) SCLET_RHS_AC(4)
 #undef SCLET_RHS_AC
       default: e = cudaErrorInvalidValue;
     }
@@ -512,8 +741,11 @@ static cudaError_t launch_rhs_pl(const Phys &ph, const T *u, const T *felas, T *
   } else if (PL::max_nch > 0) {
     for (int m = 0; m < ph.nch; m++) {
       // one conserved field (the plugins' CH_f is defined for c_0 only)
-      rhs_ch_t_kernel<PL, T><<<grd, blk, 0, s>>>(p, u, scratch);
-      rhs_ch_lap_kernel<PL, T><<<grd, blk, 0, s>>>(p, u, scratch, out + (long long)ph.nac * n3);  // per run: + r F n^3
+      p.zc = planes_per_cta(ph, 0, 16, p.runs);
+      const int zblocks = ((ph.n + p.zc - 1) / p.zc) * p.runs;
+      const dim3 gch(gx, gy, zblocks + zface);
+      rhs_ch_t_kernel<PL, T><<<gch, blk, 0, s>>>(p, u, scratch, zblocks);
+      rhs_ch_lap_kernel<PL, T><<<gch, blk, 0, s>>>(p, u, scratch, out + (long long)ph.nac * n3, zblocks);  // per run: + r F n^3
       launch_counter() += 2;
     }
   }
