@@ -682,6 +682,40 @@ __global__ void __launch_bounds__(RX * RY) mob_n_kernel(P<T> p0, const T *__rest
   }
 }
 
+// r = N - H u = N + LE (epn2 sum_a kk_a T_a u - KE u) of the Allen-Cahn fields,
+// T_a the second difference along axis a with zero values outside the block
+// (the operator the eigenbasis diagonalises).  A thread marches an (x, y)
+// column; differences are taken first, so a smooth field loses no digits.
+// blockIdx.z = (run, field) x chunk of planes.  Bound by HBM (u and N read, r
+// written).
+template <typename T>
+__global__ void __launch_bounds__(RX * RY) increment_rhs_kernel(P<T> p, const T *__restrict__ u,
+                                                                const T *__restrict__ rhs, T *__restrict__ r, T cx, T cy,
+                                                                T cz) {
+  const int n = p.n;
+  const size_t nn = (size_t)n * n, n3 = nn * n;
+  const int zch = (n + p.zc - 1) / p.zc;
+  const int t = blockIdx.z / zch, zci = blockIdx.z - t * zch;  // t = run nac + m
+  const int x = blockIdx.x * RX + threadIdx.x, y = blockIdx.y * RY + threadIdx.y;
+  if (x >= n || y >= n) return;
+  const size_t f = (size_t)(t / p.nac) * p.F + t % p.nac;
+  const int z0 = zci * p.zc, z1 = min(n, z0 + p.zc);
+  size_t l = (size_t)z0 * nn + (size_t)y * n + x;
+  const T *uf = u + f * n3, *nf = rhs + f * n3;
+  T *rf = r + (size_t)t * n3;
+  T um = z0 > 0 ? uf[l - nn] : (T)0, uc = uf[l];
+#pragma unroll 2
+  for (int z = z0; z < z1; z++, l += nn) {
+    const T up = z < n - 1 ? uf[l + nn] : (T)0;
+    const T xm = x > 0 ? uf[l - 1] : (T)0, xp = x < n - 1 ? uf[l + 1] : (T)0;
+    const T ym = y > 0 ? uf[l - n] : (T)0, yp = y < n - 1 ? uf[l + n] : (T)0;
+    const T lx = (xm - uc) + (xp - uc), ly = (ym - uc) + (yp - uc), lz = (um - uc) + (up - uc);
+    rf[l] = (nf[l] - p.LE * p.KE * uc) + (cx * lx + cy * ly + cz * lz);
+    um = uc;
+    uc = up;
+  }
+}
+
 // z-planes per CTA: the tuned value if any, else the most of `zmax`, zmax / 2,
 // .. 2 that still gives every SM four CTAs (a small block marched 32 planes a
 // CTA left 20 CTAs on 152 SMs: 121 us at 36^3).
@@ -692,6 +726,21 @@ static int planes_per_cta(const Phys &ph, int tuned, int zmax, int runs) {
   while (zc > 2 && tiles * ((ph.n + zc - 1) / zc) < 4 * 152) zc /= 2;
   return zc;
 }
+
+template <typename T>
+cudaError_t launch_increment_rhs(const Phys &ph, const T *u, const T *rhs, T *r, cudaStream_t s) {
+  P<T> p = to_p<T>(ph);
+  const int gx = (ph.n + RX - 1) / RX, gy = (ph.n + RY - 1) / RY, count = p.runs * ph.nac;
+  p.zc = planes_per_cta(ph, 0, 16, count);
+  T c[3];
+  for (int a = 0; a < 3; a++) c[a] = (T)(ph.LE * ph.epn2 * ph.kk[a] / (ph.h[a] * ph.h[a]));
+  increment_rhs_kernel<T><<<dim3(gx, gy, ((ph.n + p.zc - 1) / p.zc) * count), dim3(RX, RY), 0, s>>>(p, u, rhs, r, c[0],
+                                                                                                  c[1], c[2]);
+  launch_counter()++;
+  return cudaGetLastError();
+}
+template cudaError_t launch_increment_rhs<double>(const Phys &, const double *, const double *, double *, cudaStream_t);
+template cudaError_t launch_increment_rhs<float>(const Phys &, const float *, const float *, float *, cudaStream_t);
 
 template <typename PL, typename T>
 static cudaError_t launch_rhs_pl(const Phys &ph, const T *u, const T *felas, T *out, T *scratch, cudaStream_t s) {

@@ -21,10 +21,6 @@
 #include "sclet_physics.cuh"
 #include "sclet_tc.cuh"
 
-namespace sclet {
-void set_phi_tables(const double *phi1_ac, const double *phi1_ch, const double *phi2_ac, const double *phi2_ch);
-}
-
 using namespace sclet;
 
 struct StageEv {
@@ -60,6 +56,11 @@ struct sclet_ctx {
   double *felas = nullptr, *scratch = nullptr, *shell = nullptr;
   double *V[3] = {nullptr, nullptr, nullptr}, *Vi[3] = {nullptr, nullptr, nullptr};
   double *phi1[2] = {nullptr, nullptr}, *phi2[2] = {nullptr, nullptr};
+  // the basis is the block's own Dirichlet one (sclet_basis.cu): folded
+  // products foldVi, foldV; the order parameters advance by increments (see
+  // increments_allowed)
+  bool dirichlet = false, increments = false;
+  double *foldVi = nullptr, *foldV = nullptr;
   // MIXED form: fstate2 = [u (F) | rhs1 (F)] in FP32; FP32 work tensors W1, W2
   // (2F blocks each); slice planes P of up to 2F tensors with their row scales
   // scaleP; sliced matrices with row scales
@@ -208,8 +209,29 @@ int mass_weights_setup(sclet_ctx *ctx, const double *v, const double *vi);
 int queue_diagnostics(sclet_ctx *ctx, int energy_form);
 int read_diagnostics(sclet_ctx *ctx, sclet_diag *out);
 
+// Whether the order parameters may advance as u' = u + V phi1 V^-1 (N - H u)
+// instead of u' = V (e V^-1 u + phi1 V^-1 N): the same in exact arithmetic
+// where V diag(d) V^-1 is the stencil's operator, with three products per
+// field less.  Two conditions keep it as accurate: no mode whose H the scheme
+// takes as zero (|H| <= 1e-8, vars.c:302-359), and no mode damped so far in
+// one step that u' is small beside u (dt H <= 4: the increment's rounding is
+// relative to u, at most the rounding the three saved products leave).
+bool increments_allowed(const sclet_ctx *ctx, const double *d) {
+  const sclet_params &p = ctx->p;
+  const double kk[3] = {p.kkx, p.kky, p.kkz}, L = ctx->ph.LE, K = ctx->ph.KE;
+  if (!ctx->dirichlet || ctx->nac < 1) return false;
+  double top = K;
+  for (int a = 0; a < 3; a++) {
+    if (!(kk[a] * p.epn2 >= 0.0)) return false;
+    top += p.epn2 * kk[a] * fabs(d[0]) / (ctx->ph.h[a] * ctx->ph.h[a]);  // d ascending: d[0] the largest in size
+  }
+  return L > 0.0 && K > 0.0 && L * K > 1.0e-7 && p.dt * L * top <= 4.0;
+}
+
 int upload_eigen(sclet_ctx *ctx, const double *d, const double *v, const double *vi) {
   const int n = ctx->n;
+  ctx->dirichlet = !mixed(ctx) && basis_is_dirichlet(n, d, v, vi);
+  ctx->increments = increments_allowed(ctx, d);
   std::vector<double> ds(n);
   for (int ax = 0; ax < 3; ax++) {
     double h = ctx->ph.h[ax];
@@ -240,6 +262,12 @@ int upload_eigen(sclet_ctx *ctx, const double *d, const double *v, const double 
   for (int ax = 0; ax < 3; ax++) {
     CK(cudaMemcpyAsync(ctx->V[ax], v, sizeof(double) * n * n, cudaMemcpyHostToDevice, ctx->stream));
     CK(cudaMemcpyAsync(ctx->Vi[ax], vi, sizeof(double) * n * n, cudaMemcpyHostToDevice, ctx->stream));
+  }
+  if (ctx->dirichlet) {
+    const std::vector<double> fi = fold_matrix(n, vi, false), fv = fold_matrix(n, v, true);
+    CK(cudaMemcpyAsync(ctx->foldVi, fi.data(), sizeof(double) * fi.size(), cudaMemcpyHostToDevice, ctx->stream));
+    CK(cudaMemcpyAsync(ctx->foldV, fv.data(), sizeof(double) * fv.size(), cudaMemcpyHostToDevice, ctx->stream));
+    CK(cudaStreamSynchronize(ctx->stream));
   }
   const sclet_params &p = ctx->p;
   const Phys &ph = ctx->ph;  // LE, KE, LCI, KCI from the plugin's init_KL
@@ -444,7 +472,8 @@ void sclet_destroy(sclet_ctx *ctx) {
                   ctx->fstate2, ctx->frhs2, ctx->ffelas, ctx->fscratch, ctx->fshell, ctx->W1, ctx->W2, ctx->P,
                   ctx->scaleP, ctx->rsV, ctx->rsVi, ctx->matV, ctx->matVi, ctx->stage64,
                   ctx->coef[0], ctx->coef[1], ctx->coef2[0], ctx->coef2[1], ctx->massW, ctx->massPart,
-                  ctx->massRes, ctx->in_stage, ctx->out_stage, ctx->krun, ctx->mob_t, ctx->mob_part};
+                  ctx->massRes, ctx->in_stage, ctx->out_stage, ctx->krun, ctx->mob_t, ctx->mob_part, ctx->foldVi,
+                  ctx->foldV};
   for (void *b : bufs) cudaFree(b);
   if (ctx->diag_host) cudaFreeHost(ctx->diag_host);
   for (int a = 0; a < 3; a++) {
@@ -589,6 +618,11 @@ int sclet_create_runs(const sclet_params *p, int runs, const double *krun, int p
     for (int a = 0; a < 3; a++) {
       CC(cudaMalloc(&ctx->V[a], sizeof(double) * n * n));
       CC(cudaMalloc(&ctx->Vi[a], sizeof(double) * n * n));
+    }
+    {
+      const size_t fb = sizeof(double) * 2 * fold_half(n) * fold_half(n);
+      CC(cudaMalloc(&ctx->foldVi, fb));
+      CC(cudaMalloc(&ctx->foldV, fb));
     }
     for (int k = 0; k < 2; k++) {
       CC(cudaMalloc(&ctx->phi1[k], blk));
@@ -960,6 +994,30 @@ static int etd2_correct_mixed(sclet_ctx *ctx) {
   return SCLET_OK;
 }
 
+// The FP64 transforms on the folded products.  Tensors, in order: the nI order
+// parameters that advance by increments (their r), then u, then N of the nF
+// other fields.
+static int etd_update_fold64(sclet_ctx *ctx) {
+  const int F = ctx->F, n = ctx->n, nI = ctx->increments ? ctx->nac : 0, nF = F - nI;
+  const long long n3 = ctx->n3;
+  const EtdCoef ec = etd_coef(ctx);
+  cudaStream_t s = ctx->stream;
+  const FoldEpi plain = {{nullptr, nullptr}, 0, 0, 0, 0};
+  FoldEpi scaled = {{ctx->phi1[0], ctx->phi1[1]}, nI, 0, 0, 0}, etd = {{ctx->phi1[0], ctx->phi1[1]}, 0, 1, nI, 0};
+  if (nI) CK(launch_increment_rhs<double>(ctx->ph, u_of(ctx), rhs1_of(ctx), ctx->A, s));
+  const TensorList<double> in = {{ctx->A, u_of(ctx) + nI * n3, rhs1_of(ctx) + nI * n3}, {0, nI, nI + nF}};
+  CK(launch_fold_fwd_f64(ctx->foldVi, in, nullptr, ctx->B, nI + 2 * nF, n, plain, ec, s));
+  CK(launch_fold_fwd_f64(ctx->foldVi, tensor_list<double>(ctx->B), nullptr, ctx->A, nI + 2 * nF, n, plain, ec, s));
+  CK(launch_fold_fwd_f64(ctx->foldVi, tensor_list<double>(ctx->A), nullptr, ctx->B, F, n, scaled, ec, s));
+  if (nF)
+    CK(launch_fold_fwd_f64(ctx->foldVi, tensor_list<double>(ctx->A + F * n3), nullptr, ctx->B + nI * n3, nF, n, etd, ec,
+                           s));
+  CK(launch_fold_inv_f64(ctx->foldV, ctx->B, ctx->A, F, n, F, 0, s));
+  CK(launch_fold_inv_f64(ctx->foldV, ctx->A, ctx->B, F, n, F, 0, s));
+  CK(launch_fold_inv_f64(ctx->foldV, ctx->B, u_of(ctx), F, n, F, nI, s));
+  return SCLET_OK;
+}
+
 int sclet_etd_update(sclet_ctx *ctx) {
   StageEv ev;
   long long l0 = launch_counter();
@@ -970,17 +1028,23 @@ int sclet_etd_update(sclet_ctx *ctx) {
     stage_end(ctx, ev, l0);
     return SCLET_OK;
   }
+  if (ctx->dirichlet) {
+    int rc = etd_update_fold64(ctx);
+    if (rc != SCLET_OK) return rc;
+    stage_end(ctx, ev, l0);
+    return SCLET_OK;
+  }
   const int F = ctx->F;
   const long long n3 = ctx->n3;
   EtdCoef ec = etd_coef(ctx);
-  set_phi_tables(ctx->phi1[0], ctx->phi1[1], ctx->phi2[0], ctx->phi2[1]);
   cudaStream_t s = ctx->stream;
   // V^-1 along x, y for u and N1 together; along z for u, then for N1 with
   // the ETD1 update fused (uhat in A[0..F) is updated in place).
   CK(launch_modeprod_f64(ctx->Vi[0], ctx->state2, nullptr, ctx->A, nullptr, 2 * F, ctx->n, 0, ec, n3, n3, s));
   CK(launch_modeprod_f64(ctx->Vi[1], ctx->A, nullptr, ctx->B, nullptr, 2 * F, ctx->n, 0, ec, n3, n3, s));
   CK(launch_modeprod_f64(ctx->Vi[2], ctx->B, nullptr, ctx->A, nullptr, F, ctx->n, 0, ec, n3, n3, s));
-  CK(launch_modeprod_f64(ctx->Vi[2], ctx->B + F * n3, nullptr, ctx->A, ctx->A, F, ctx->n, 1, ec, n3, n3, s));
+  CK(launch_modeprod_f64(ctx->Vi[2], ctx->B + F * n3, nullptr, ctx->A, ctx->A, F, ctx->n, 1, ec, n3, n3, s,
+                         ctx->phi1));
   // V along x, y, z back to physical space
   CK(launch_modeprod_f64(ctx->V[0], ctx->A, nullptr, ctx->B, nullptr, F, ctx->n, 0, ec, n3, n3, s));
   CK(launch_modeprod_f64(ctx->V[1], ctx->B, nullptr, ctx->A, nullptr, F, ctx->n, 0, ec, n3, n3, s));
@@ -1003,11 +1067,21 @@ int sclet_etd2_correct(sclet_ctx *ctx) {
   const int F = ctx->F;
   const long long n3 = ctx->n3;
   EtdCoef ec = etd_coef(ctx);
-  set_phi_tables(ctx->phi1[0], ctx->phi1[1], ctx->phi2[0], ctx->phi2[1]);
   cudaStream_t s = ctx->stream;
+  if (ctx->dirichlet) {
+    const FoldEpi plain = {{nullptr, nullptr}, 0, 0, 0, 0}, scaled = {{ctx->phi2[0], ctx->phi2[1]}, F, 0, 0, 0};
+    CK(launch_fold_fwd_f64(ctx->foldVi, tensor_list<double>(ctx->rhs2), rhs1_of(ctx), ctx->A, F, ctx->n, plain, ec, s));
+    CK(launch_fold_fwd_f64(ctx->foldVi, tensor_list<double>(ctx->A), nullptr, ctx->B, F, ctx->n, plain, ec, s));
+    CK(launch_fold_fwd_f64(ctx->foldVi, tensor_list<double>(ctx->B), nullptr, ctx->A, F, ctx->n, scaled, ec, s));
+    CK(launch_fold_inv_f64(ctx->foldV, ctx->A, ctx->B, F, ctx->n, F, 0, s));
+    CK(launch_fold_inv_f64(ctx->foldV, ctx->B, ctx->A, F, ctx->n, F, 0, s));
+    CK(launch_fold_inv_f64(ctx->foldV, ctx->A, u_of(ctx), F, ctx->n, F, F, s));
+    stage_end(ctx, ev, l0);
+    return SCLET_OK;
+  }
   CK(launch_modeprod_f64(ctx->Vi[0], ctx->rhs2, rhs1_of(ctx), ctx->A, nullptr, F, ctx->n, 0, ec, n3, n3, s));
   CK(launch_modeprod_f64(ctx->Vi[1], ctx->A, nullptr, ctx->B, nullptr, F, ctx->n, 0, ec, n3, n3, s));
-  CK(launch_modeprod_f64(ctx->Vi[2], ctx->B, nullptr, ctx->A, nullptr, F, ctx->n, 2, ec, n3, n3, s));
+  CK(launch_modeprod_f64(ctx->Vi[2], ctx->B, nullptr, ctx->A, nullptr, F, ctx->n, 2, ec, n3, n3, s, ctx->phi2));
   CK(launch_modeprod_f64(ctx->V[0], ctx->A, nullptr, ctx->B, nullptr, F, ctx->n, 0, ec, n3, n3, s));
   CK(launch_modeprod_f64(ctx->V[1], ctx->B, nullptr, ctx->A, nullptr, F, ctx->n, 0, ec, n3, n3, s));
   CK(launch_modeprod_f64(ctx->V[2], ctx->A, nullptr, u_of(ctx), nullptr, F, ctx->n, 3, ec, n3, n3, s));
@@ -1106,8 +1180,14 @@ int sclet_mode_product(sclet_ctx *ctx, int inverse, const double *in, double *ou
   }
   EtdCoef ec = etd_coef(ctx);
   CK(cudaMemcpyAsync(ctx->A, in, sizeof(double) * n3, cudaMemcpyHostToDevice, ctx->stream));
-  CK(launch_modeprod_f64(inverse ? ctx->V[0] : ctx->Vi[0], ctx->A, nullptr, ctx->B, nullptr, 1, ctx->n, 0, ec, n3, n3,
-                         ctx->stream));
+  if (ctx->dirichlet && inverse)
+    CK(launch_fold_inv_f64(ctx->foldV, ctx->A, ctx->B, 1, ctx->n, 1, 0, ctx->stream));
+  else if (ctx->dirichlet)
+    CK(launch_fold_fwd_f64(ctx->foldVi, tensor_list<double>(ctx->A), nullptr, ctx->B, 1, ctx->n,
+                           FoldEpi{{nullptr, nullptr}, 0, 0, 0, 0}, ec, ctx->stream));
+  else
+    CK(launch_modeprod_f64(inverse ? ctx->V[0] : ctx->Vi[0], ctx->A, nullptr, ctx->B, nullptr, 1, ctx->n, 0, ec, n3,
+                           n3, ctx->stream));
   CK(cudaMemcpyAsync(out, ctx->B, sizeof(double) * n3, cudaMemcpyDeviceToHost, ctx->stream));
   CK(cudaStreamSynchronize(ctx->stream));
   return SCLET_OK;

@@ -4,6 +4,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <vector>
+
 #include "sclet_gb300.h"
 
 namespace sclet {
@@ -127,15 +129,64 @@ cudaError_t launch_rhs(const Phys &ph, const T *u, const T *felas, T *out, T *sc
 // Epilogues: 0 store; 1 ETD1 update out = (1 - phi H) uhat + phi * acc with
 // uhat = aux_t (read) ; 2 out = phi2 * acc ; 3 out += acc.  Prologue `sub`:
 // in_t - sub_t.  kinds: per-tensor field kind selector (t % F >= nac -> CH).
+// phi: the tables of the two field kinds (phi1 for epilogue 1, phi2 for 2).
 struct EtdCoef {
   const double *dd[3];   // eigenvalues / h^2 per axis (device)
   double kk[3];
   double epn2, dt, LE, KE, LCI, KCI;
   int nac, F;
 };
+// ---- folded transforms (sclet_basis.cu) -----------------------------------
+// half edge of a folded product, and the first mode of each parity
+// (part 0 even, part 1 odd about the block's centre; mode k is even when
+// n - k is odd)
+__host__ __device__ inline int fold_half(int n) { return (n + 1) / 2; }
+__host__ __device__ inline int fold_mode0(int n, int part) { return part == 0 ? (n + 1) % 2 : n % 2; }
+bool basis_is_dirichlet(int n, const double *d, const double *v, const double *vi);
+std::vector<double> fold_matrix(int n, const double *m, bool inverse);
+
+// Blocks of a batch that do not lie in one run of memory: tensor t is the
+// block t - first of the last segment with first <= t (blocks n^3 apart).
+template <typename T>
+struct TensorList {
+  const T *base[3];
+  int first[3];
+  __host__ __device__ const T *at(int t, long long n3) const {
+    const int s = t >= first[2] ? 2 : (t >= first[1] ? 1 : 0);
+    return base[s] + (t - first[s]) * n3;
+  }
+};
+template <typename T>
+inline TensorList<T> tensor_list(const T *a) {  // one run of blocks
+  return TensorList<T>{{a, a, a}, {0, 0x7fffffff, 0x7fffffff}};
+}
+
+// Right-hand side of the increment form of the Allen-Cahn fields (m < nac of
+// every run): r = N - H u with H the step's linear operator applied as a
+// stencil (zero outside the block), so that u' = u + V phi1 V^-1 r.
+// u, rhs: F blocks per run; r: nac blocks per run.
+template <typename T>
+cudaError_t launch_increment_rhs(const Phys &ph, const T *u, const T *rhs, T *r, cudaStream_t s);
+
+// Folded FP64 products of `count` tensors (layout rotation as in
+// launch_modeprod_f64).  W: fold_matrix of V^-1 (forward) or V (inverse).
+// Forward epilogue: phi[kind] (n^3, may be null: plain store) times the value
+// for tensors t < scaled, a plain store for the others; etd: tensor t is N^ of
+// field t + t0 and out holds its u^, updated in place (1 - phi1 H) u^ + phi1 N^.
+// Inverse: out += for tensors with t % F < acc, a store for the others.
+struct FoldEpi {
+  const double *phi[2];
+  int scaled, etd, t0, acc;
+};
+cudaError_t launch_fold_fwd_f64(const double *W, const TensorList<double> &in, const double *sub, double *out, int count,
+                                int n, const FoldEpi &ep, const EtdCoef &ec, cudaStream_t s);
+cudaError_t launch_fold_inv_f64(const double *W, const double *in, double *out, int count, int n, int F, int acc,
+                                cudaStream_t s);
+
 cudaError_t launch_modeprod_f64(const double *M, const double *in, const double *sub, double *out,
                                 const double *aux, int count, int n, int epilogue, const EtdCoef &ec,
-                                long long in_stride, long long out_stride, cudaStream_t s);
+                                long long in_stride, long long out_stride, cudaStream_t s,
+                                const double *const *phi = nullptr);
 
 // Elastic force (FFT based) -- see k_fft.cu.
 struct ElasticPlan;

@@ -1,0 +1,89 @@
+"""The parity-folded transforms and the increment form of the step against the
+general path.  A basis with two modes swapped is the same basis to the scheme
+but not in ascending order, so it takes the general path."""
+import numpy as np
+import pytest
+
+import cases
+
+pytestmark = pytest.mark.gpu
+
+
+def _params(sg, N, nac, nch, etd2=0, dt=0.005, kk=(1.0, 1.0, 1.0)):
+    p = sg.default_params()
+    p.nx = p.ny = p.nz = N + 4
+    p.xmax, p.ymax, p.zmax = 0.5 * N, 0.45 * N, 0.55 * N
+    p.nac, p.nch, p.elastic, p.etd2, p.dt = nac, nch, 0, etd2, dt
+    p.kkx, p.kky, p.kkz = kk
+    return p
+
+
+def _swapped(n):
+    d, v, vi = cases.eigen_variant(n, 3)
+    q = np.arange(n)
+    q[:2] = 1, 0
+    return d[q], np.ascontiguousarray(v[:, q]), np.ascontiguousarray(vi[q])
+
+
+def _rel(a, b):
+    return np.linalg.norm(a - b) / np.linalg.norm(b)
+
+
+# half edges: 4, 5 (odd block), 18 and 19 (one inverse tile and two), 36 and 37
+# (one forward tile and two), 66
+EDGES = [4, 5, 31, 33, 68, 70, 128]
+
+
+@pytest.mark.parametrize("N", EDGES)
+def test_fp64_folded_products(N, sclet_lib):
+    """One folded product each way against the dense sum in numpy: sums of n
+    terms in another order, n 2^-53 at most, about sqrt(n) 2^-53 as they fall."""
+    sg = sclet_lib
+    s = sg.Solver(_params(sg, N, 1, 0), sg.FP64)
+    n = s.n
+    a = np.random.default_rng(N).standard_normal((n, n, n))
+    _, v, vi = cases.eigen_variant(n, 3)
+    for inverse, m in ((False, vi), (True, v)):
+        got = s.mode_product(a, inverse)
+        # the library's own basis is built like the oracle's, sines of arguments up to n pi: 1e-13
+        assert _rel(got, np.einsum("pa,cba->pcb", m, a)) <= 1e-12, inverse
+    s.close()
+
+
+@pytest.mark.parametrize("N,nac,nch,etd2", [(4, 1, 0, 0), (5, 2, 1, 1), (31, 4, 1, 0), (33, 3, 0, 1), (68, 1, 1, 0),
+                                            (70, 2, 0, 0)])
+def test_fp64_steps_match_the_general_path(N, nac, nch, etd2, sclet_lib):
+    sg = sclet_lib
+    p = _params(sg, N, nac, nch, etd2, kk=(1.0, 0.7, 0.4))
+    n = N + 4
+    rng = np.random.default_rng(N)
+    u0 = rng.uniform(-0.5, 0.5, size=(nac + nch, n, n, n))
+    out = []
+    for basis in (cases.eigen_variant(n, 3), _swapped(n)):
+        s = sg.Solver(p, sg.FP64)
+        s.set_eigen(*basis)
+        s.set_fields(u0)
+        s.step(3)
+        out.append(s.get_fields())
+        s.close()
+    for f in range(nac + nch):
+        assert _rel(out[0][f], out[1][f]) <= 1e-12, f
+
+
+@pytest.mark.parametrize("dt", [0.05, 5.0])
+def test_strong_damping_takes_the_full_form(dt, sclet_lib):
+    """dt H reaches 1.7 and 170 on the finest modes: below 4 the increment form
+    runs, above it the full one; both match the general path."""
+    sg = sclet_lib
+    p = _params(sg, 20, 2, 0, dt=dt)
+    u0 = np.random.default_rng(3).uniform(-0.1, 0.1, size=(2, 24, 24, 24))
+    out = []
+    for basis in (cases.eigen_variant(24, 3), _swapped(24)):
+        s = sg.Solver(p, sg.FP64)
+        s.set_eigen(*basis)
+        s.set_fields(u0)
+        s.step(2)
+        out.append(s.get_fields())
+        s.close()
+    for f in range(2):
+        assert _rel(out[0][f], out[1][f]) <= 1e-12, f
