@@ -198,7 +198,7 @@ __global__ void to_pairs_kernel(double *w, long long count) {
 int mass_partials() { return 152 * 16; }
 
 cudaError_t mass_weight(double *w, double *tmp, const double *g, const double *viT, int n, int which, const EtdCoef &ec,
-                        cudaStream_t s) {
+                        cudaStream_t s, bool folded) {
   const long long n3 = (long long)n * n * n;
   long long b = (n3 + 255) / 256;
   seed_kernel<<<(int)(b > 152 * 16 ? 152 * 16 : b), 256, 0, s>>>(w, g, n, which, ec.dd[0], ec.dd[1], ec.dd[2], ec.epn2,
@@ -207,9 +207,13 @@ cudaError_t mass_weight(double *w, double *tmp, const double *g, const double *v
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   // three products with V^-T return to the [k][j][i] layout
-  if ((e = launch_modeprod_f64(viT, w, nullptr, tmp, nullptr, 1, n, 0, ec, n3, n3, s)) != cudaSuccess) return e;
-  if ((e = launch_modeprod_f64(viT, tmp, nullptr, w, nullptr, 1, n, 0, ec, n3, n3, s)) != cudaSuccess) return e;
-  if ((e = launch_modeprod_f64(viT, w, nullptr, tmp, nullptr, 1, n, 0, ec, n3, n3, s)) != cudaSuccess) return e;
+  auto product = [&](const double *in, double *out) {
+    return folded ? launch_fold_inv_f64(viT, in, out, 1, n, 1, 0, s)
+                  : launch_modeprod_f64(viT, in, nullptr, out, nullptr, 1, n, 0, ec, n3, n3, s);
+  };
+  if ((e = product(w, tmp)) != cudaSuccess) return e;
+  if ((e = product(tmp, w)) != cudaSuccess) return e;
+  if ((e = product(w, tmp)) != cudaSuccess) return e;
   if ((e = cudaMemcpyAsync(w, tmp, sizeof(double) * n3, cudaMemcpyDeviceToDevice, s)) != cudaSuccess) return e;
   to_pairs_kernel<<<(int)(b > 152 * 16 ? 152 * 16 : b), 256, 0, s>>>(w, n3);
   launch_counter()++;

@@ -46,6 +46,11 @@
 // (128 a' rows x 32 k), both K-major, in a three-stage mbarrier pipeline
 // that runs ahead across tiles; a stage is refilled once the MMAs that read
 // it have completed.
+// The folded forms (the default basis) halve the MMAs of a product and, with
+// the increment form, a field needs six products instead of nine.  Kernel time
+// of a step, dense and nine products before, now: 4 + 1 fields of 516^3
+// 52.8 -> 28.0 ms, of 196^3 1.64 -> 1.05 ms, 4 fields of 68^3 124 -> 85 us; the
+// step's error against 64 bits fell from 2.2e-7 to 0.6e-7 (196^3, ten steps).
 // Warp 0 issues TMA, warp 1 issues MMAs (one elected thread each) and owns the
 // tensor memory (4 classes x 128 columns).  Warps 2-5 run the epilogue (TMEM
 // lane quadrant warp % 4): the four classes of the tile are combined into
@@ -72,9 +77,24 @@ namespace sclet {
 
 namespace tc {
 
-template <int EPI, int OUT>
+// FORM 0: any basis.  FORM 1, 2: the parity-folded forward and inverse products
+// of the Dirichlet basis (sclet_basis.cu): the sliced lines and the matrix come
+// in two parts (even, odd modes) of h = ceil(n / 2) columns, a group's tiles run
+// over a'-tiles of h with the part fastest.  The forward epilogue interleaves
+// the parts' modes; the inverse one keeps the even part's tile E in registers
+// until the odd part's O is there and stores E + O and E - O.
+// EPI 0 store, 1 ETD1 update, 2 phi scaling (FORM 0; the folded transforms apply
+// them where the lines are sliced for the inverse, slice_fold_kernel).
+// OUT 1 store, 2 accumulate (FORM 2: of fields below g.acc, the others store;
+// as reductions at the L2, so that no epilogue warp waits for the old values).
+// BN: a'-tile width.  128 columns of the four classes fill tensor memory; with
+// 64, for halves up to 64, two accumulator sets alternate.
+template <int FORM, int EPI, int OUT, int BN>
 __global__ void __launch_bounds__(THREADS, 1)
     modeprod_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, TcArgs g) {
+  using G = TileGeom<BN>;
+  constexpr int STAGES = G::STAGES, STAGE_BYTES = G::STAGE_BYTES, PLANE_B = G::PLANE_B, NBUF = G::NBUF;
+  constexpr int ACC_COLS = G::ACC_COLS, TMEM_COLS = G::TMEM_COLS, CPW = G::CPW;
   extern __shared__ uint8_t smem_raw[];
   __shared__ __align__(8) uint64_t full_bar[STAGES];
   __shared__ __align__(8) uint64_t empty_bar[STAGES];
@@ -87,11 +107,14 @@ __global__ void __launch_bounds__(THREADS, 1)
   uint8_t *base = (uint8_t *)(((uintptr_t)smem_raw + SMEM_ALIGN - 1) & ~(uintptr_t)(SMEM_ALIGN - 1));
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const long long rows = (long long)g.n * g.n;
-  const int a_tiles = (g.n + BN - 1) / BN;
+  constexpr int PARTS = FORM == 0 ? 1 : 2;
+  const int h = FORM == 0 ? g.n : fold_half(g.n);  // outputs of one part
+  const int a_tiles = (h + BN - 1) / BN;
+  const int units = a_tiles * PARTS;
   const int r_tiles = (int)((rows + BM - 1) / BM);
   // whole groups (every a'-tile of one input tile) per CTA, round robin
   const int groups = r_tiles * g.count;
-  const int mine = (int)blockIdx.x < groups ? a_tiles * ((groups - 1 - (int)blockIdx.x) / (int)gridDim.x + 1) : 0;
+  const int mine = (int)blockIdx.x < groups ? units * ((groups - 1 - (int)blockIdx.x) / (int)gridDim.x + 1) : 0;
   const int nkb = g.kblocks;
 
   if (threadIdx.x == 0) {
@@ -126,7 +149,7 @@ __global__ void __launch_bounds__(THREADS, 1)
       int it = 0;
       // the self-test leaves every barrier without arrivals (no copy is issued)
       for (int u = g.idle ? mine : 0; u < mine; u++) {
-        const TileIdx ti = cta_tile(u, a_tiles, g.count, blockIdx.x, gridDim.x);
+        const TileIdx ti = cta_tile<PARTS>(u, a_tiles, g.count, blockIdx.x, gridDim.x);
         for (int kb = 0; kb < nkb; kb++, it++) {
           const int s = it % STAGES;
           if (it >= STAGES && !mbar_wait(&empty_bar[s], ((it / STAGES) & 1) ^ 1)) {
@@ -138,9 +161,11 @@ __global__ void __launch_bounds__(THREADS, 1)
           mbar_expect_tx(&full_bar[s], STAGE_BYTES);
           // k-block kb of plane z is the contiguous block z * nkb + kb
           for (int p = 0; p < NP; p++)
-            tma_load_3d(st + p * PLANE_A, &tmA, 0, ti.r_tile * BM, (ti.t * NP + p) * nkb + kb, &full_bar[s]);
+            tma_load_3d(st + p * PLANE_A, &tmA, 0, ti.r_tile * BM, ((ti.t * PARTS + ti.part) * NP + p) * nkb + kb,
+                        &full_bar[s]);
           for (int p = 0; p < NPM; p++)
-            tma_load_3d(st + NP * PLANE_A + p * PLANE_B, &tmB, 0, ti.a_tile * BN, p * nkb + kb, &full_bar[s]);
+            tma_load_3d(st + NP * PLANE_A + p * PLANE_B, &tmB, 0, ti.a_tile * BN, (ti.part * NPM + p) * nkb + kb,
+                        &full_bar[s]);
         }
         if (*(volatile int *)&failed) break;
       }
@@ -155,13 +180,13 @@ __global__ void __launch_bounds__(THREADS, 1)
       // slice, matrix slice, class) grouped by class, small classes first; the
       // first term of each class at a tile's first k-step starts its
       // accumulator.  The last a'-tile runs N = its rows rounded up to 16.
-      const int last_cols = g.n - (a_tiles - 1) * BN;
+      const int last_cols = h - (a_tiles - 1) * BN;
       const uint32_t idesc_full = idesc_bf16(BM, BN);
       const uint32_t idesc_last = idesc_bf16(BM, (last_cols + 15) / 16 * 16);
       const int pairA[11] = {0, 3, 2, 1, 0, 2, 1, 0, 1, 0, 0};  // input slice
       const int pairB[11] = {4, 0, 1, 2, 3, 0, 1, 2, 0, 1, 0};  // matrix slice
       const int cls[11] = {3, 3, 3, 3, 3, 2, 2, 2, 1, 1, 0};
-      const bool last_two = g.n - (nkb - 1) * BK > 16;  // the last k-block needs both k-steps
+      const bool last_two = h - (nkb - 1) * BK > 16;  // the last k-block needs both k-steps
       int it = 0, j = 0;
       for (int u = 0; u < mine && !*(volatile int *)&failed; u++, j++) {
         const int b = j % NBUF;
@@ -172,7 +197,7 @@ __global__ void __launch_bounds__(THREADS, 1)
         }
         fence_after();
         const uint32_t acc = tmem + (uint32_t)(b * ACC_COLS);
-        const uint32_t idesc = u % a_tiles == a_tiles - 1 ? idesc_last : idesc_full;
+        const uint32_t idesc = (u % units) / PARTS == a_tiles - 1 ? idesc_last : idesc_full;
         bool ok = true;
         for (int kb = 0; kb < nkb; kb++, it++) {
           const int s = it % STAGES;
@@ -228,8 +253,23 @@ __global__ void __launch_bounds__(THREADS, 1)
     const float wt[NACC] = {ldexpf(1.0f, -2 * g.bits), ldexpf(1.0f, -3 * g.bits), ldexpf(1.0f, -4 * g.bits),
                             ldexpf(1.0f, -5 * g.bits)};
     int j = 0;
+    float even[FORM == 2 ? CPW : 1][32];  // the even part's tile of an inverse product
     for (int u = 0; u < mine; u++, j++) {
       const int b = j % NBUF;
+      const TileIdx ti = cta_tile<PARTS>(u, a_tiles, g.count, blockIdx.x, gridDim.x);
+      const int at0 = ti.a_tile * BN;
+      const int nch = (min(BN, h - at0) + 31) / 32;  // 32-column chunks holding live a'
+      const long long r = (long long)ti.r_tile * BM + q * 32 + lane;
+      const bool live = r < rows;
+      // the scales come while the tile's MMAs run: the input row's, and per
+      // chunk the 32 matrix rows', one per lane, broadcast below
+      const float si = live ? g.in_scale[((long long)ti.t * PARTS + ti.part) * rows + r] : 0.0f;
+      float rsv[CPW];
+#pragma unroll
+      for (int cl = 0; cl < CPW; cl++) {
+        const int a = at0 + (c_first + cl) * 32 + lane;
+        rsv[cl] = a < h ? g.row_scale[ti.part * h + a] : 0.0f;
+      }
       // one lane waits, the warp follows its verdict (tcgen05.ld below needs
       // the whole warp converged)
       int ok = 1;
@@ -240,9 +280,6 @@ __global__ void __launch_bounds__(THREADS, 1)
         break;
       }
       fence_after();
-      const TileIdx ti = cta_tile(u, a_tiles, g.count, blockIdx.x, gridDim.x);
-      const int at0 = ti.a_tile * BN;
-      const int nch = (min(BN, g.n - at0) + 31) / 32;  // 32-column chunks holding live a'
       const uint32_t ta = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(b * ACC_COLS);
       // per live chunk two classes in flight at a time
       float acc[CPW][32];
@@ -268,14 +305,12 @@ __global__ void __launch_bounds__(THREADS, 1)
       fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&tempty_bar[b]);
-      const long long r = (long long)ti.r_tile * BM + q * 32 + lane;
-      const bool live = r < rows;
-      const bool ch = (ti.t % g.F) >= g.nac;  // field kind: Cahn-Hilliard
+      const bool ch = ti.t % g.F >= g.nac;  // field kind: Cahn-Hilliard
+      const bool add = OUT == 2 && (FORM != 2 || ti.t % g.F < g.acc);
       const float4 *cf = ch ? g.coef[1] : g.coef[0];
       const float2 *cf2 = ch ? g.coef2[1] : g.coef2[0];
       const long long tb = (long long)ti.t * g.n * rows;
       float *outT = g.out + tb;
-      const float si = live ? g.in_scale[(long long)ti.t * rows + r] : 0.0f;
       // offsets within one tensor stay below n^3 < 2^32 (n <= 1088)
       const uint32_t urows = (uint32_t)rows;
 #pragma unroll
@@ -283,14 +318,43 @@ __global__ void __launch_bounds__(THREADS, 1)
         const int c = c_first + cl;
         if (c < nch) {
           const int a0 = at0 + c * 32;
-          const int lim = min(32, g.n - a0);  // live a' in the chunk
-          // the chunk's 32 matrix-row scales, one per lane, broadcast below
-          const float rs = lane < lim ? g.row_scale[a0 + lane] : 0.0f;
-          const uint32_t o0 = (uint32_t)a0 * urows + (uint32_t)(live ? r : 0);  // eigen-mode [k][j][i] of a z-contraction
+          const int lim = min(32, h - a0);  // live a' in the chunk
+          const float rs = rsv[cl];
+          if (FORM == 2) {
+            if (ti.part == 0) {
+#pragma unroll
+              for (int jj = 0; jj < 32; jj++) even[cl][jj] = acc[cl][jj] * (si * __shfl_sync(0xffffffffu, rs, jj));
+              continue;
+            }
+            const uint32_t o0 = (uint32_t)a0 * urows + (uint32_t)(live ? r : 0);
+            const uint32_t q0 = (uint32_t)(g.n - 1 - a0) * urows + (uint32_t)(live ? r : 0);  // mirrored position
+#pragma unroll
+            for (int jj = 0; jj < 32; jj++) {
+              const float od = acc[cl][jj] * (si * __shfl_sync(0xffffffffu, rs, jj));
+              if (jj < lim && live) {
+                const float y = even[cl][jj] + od, z = even[cl][jj] - od;
+                float *oy = outT + (o0 + (uint32_t)jj * urows), *oz = outT + (q0 - (uint32_t)jj * urows);
+                const bool mirror = a0 + jj < g.n / 2;  // an odd block's middle cell has none
+                if (add) {
+                  atomicAdd(oy, y);
+                  if (mirror) atomicAdd(oz, z);
+                } else {
+                  *oy = y;
+                  if (mirror) *oz = z;
+                }
+              }
+            }
+            continue;
+          }
+          // output row of column jj: a0 + jj, or mode 2 (a0 + jj) + the part's first
+          const int live_o = FORM == 0 ? lim : min(lim, (ti.part == 0 ? h : g.n / 2) - a0);
+          const uint32_t ostep = FORM == 0 ? urows : 2 * urows;
+          const uint32_t o0 = (FORM == 0 ? (uint32_t)a0 : (uint32_t)(2 * a0 + fold_mode0(g.n, ti.part))) * urows +
+                              (uint32_t)(live ? r : 0);  // eigen-mode [k][j][i] of a z-contraction
           // batches of columns: every load of a batch is issued before its
           // first store (aux and the coefficient tables are read-only here:
           // the ETD update never runs in place)
-          constexpr int NB = EPI == 0 ? 8 : 4;
+          constexpr int NB = EPI == 1 ? 4 : 8;
 #pragma unroll
           for (int j0 = 0; j0 < 32; j0 += NB) {
             float uh[NB], old[NB];
@@ -298,8 +362,8 @@ __global__ void __launch_bounds__(THREADS, 1)
             float2 c2[NB];
 #pragma unroll
             for (int jj = 0; jj < NB; jj++) {
-              const uint32_t o = o0 + (uint32_t)(j0 + jj) * urows;
-              if (j0 + jj < lim && live) {
+              const uint32_t o = o0 + (uint32_t)(j0 + jj) * ostep;
+              if (j0 + jj < live_o && live) {
                 if (EPI == 1) {
                   uh[jj] = __ldg(g.aux + tb + o);
                   c1[jj] = __ldg(cf + o);
@@ -311,9 +375,9 @@ __global__ void __launch_bounds__(THREADS, 1)
             }
 #pragma unroll
             for (int jj = 0; jj < NB; jj++) {
-              const uint32_t o = o0 + (uint32_t)(j0 + jj) * urows;
+              const uint32_t o = o0 + (uint32_t)(j0 + jj) * ostep;
               const float sc = si * __shfl_sync(0xffffffffu, rs, j0 + jj);
-              if (j0 + jj < lim && live) {
+              if (j0 + jj < live_o && live) {
                 float y = acc[cl][j0 + jj] * sc;
                 if (EPI == 1) {
                   const float4 cc = c1[jj];  // (e_hi, e_lo, phi1_hi, phi1_lo)
@@ -419,6 +483,229 @@ __global__ void __launch_bounds__(256) slice_fields_kernel(const float *__restri
   }
 }
 
+// Power-of-two scale S > m (as pow2_scale) and 1 / S from m's exponent bits.
+__device__ __forceinline__ void scale_of(float m, float &S, float &inv) {
+  const uint32_t e = __float_as_uint(m) >> 23;
+  if (e >= 1 && e <= 252) {
+    S = __uint_as_float((e + 1) << 23);
+    inv = __uint_as_float((253 - e) << 23);
+  } else {  // zero, subnormal, huge, not finite
+    S = pow2_scale(m);
+    inv = 1.0f / S;
+  }
+}
+
+// The four digits of y (|y| < 1) plus a remainder e far below it: y's
+// nearest multiples of 1 / step level by level (adding and subtracting
+// 1.5 2^23 rounds to the nearest integer; every residual is exact), e joining
+// the last one.
+__device__ __forceinline__ void digits(float y, float e, float step, float step4, float (&d)[TC_PLANES]) {
+  constexpr float M = 12582912.0f;
+#pragma unroll
+  for (int p = 0; p < TC_PLANES - 1; p++) {
+    d[p] = __fadd_rn(__fmaf_rn(y, step, M), -M);
+    y = __fmaf_rn(y, step, -d[p]);
+  }
+  d[TC_PLANES - 1] = __fadd_rn(__fadd_rn(__fmaf_rn(e, step4, y * step), M), -M);
+}
+// integers of at most 8 bits: their BF16 is the upper half of the FP32
+__device__ __forceinline__ uint32_t bf16_pair(float lo, float hi) {
+  return __byte_perm(__float_as_uint(lo), __float_as_uint(hi), 0x7632);
+}
+
+// Lines -> the slices of their two parity parts, [t][part][p][kb][r][32] with a
+// scale per line and part, one line per half-warp as above.
+//   MODE 0 (forward): even x[k] + x[n-1-k], odd x[k] - x[n-1-k], k < h, formed
+//        as exact pairs (TwoSum) whose low half joins the last slice, so
+//        folding rounds nothing above the slices' own 28 bits; an odd block's
+//        middle cell counts once.  x - sub where sub is given.
+//   MODE 1 (inverse): the even and the odd modes of the line, interleaved in x
+//   MODE 2: the same after the step's update of the eigen-modes: phi x for
+//        tensors t < sp.nI, e u^ + phi1 N^ for the others (u^ the block t, N^
+//        the block t + count - nI)
+// A CTA takes SLICE_ROWS lines of one tensor, the tensors of the same lines in
+// neighbouring CTAs (the coefficients of MODE 2 come from HBM about once).
+// 4 B read and 8 B written per element: HBM is the bound once the
+// instructions per element are few (about 30: digits by FMA and add instead of
+// a conversion, BF16 by byte permute, scales from exponent bits, no division).
+constexpr int SLICE_ROWS = 64;
+
+template <int C, int MODE>
+__global__ void __launch_bounds__(256) slice_fold_kernel(TensorList<float> xs, const float *__restrict__ sub,
+                                                         float *__restrict__ scale, __nv_bfloat16 *__restrict__ out,
+                                                         int n, int kp, int count, int bits, SpecUpdate sp) {
+  const float step = ldexpf(1.0f, bits), step4 = ldexpf(1.0f, 4 * bits);
+  const int rows = n * n;
+  const long long n3 = (long long)rows * n;
+  const int lane = threadIdx.x & 31, hw = lane >> 4, kl = 2 * (lane & 15);
+  const int h = fold_half(n), odd0 = fold_mode0(n, 1);
+  const int align = n % 4 == 0 ? 4 : n % 2 == 0 ? 2 : 1;  // values per aligned load of a line
+  const int t = blockIdx.x % count, rb = blockIdx.x / count;
+  const float *xt = xs.at(t, n3);
+  const float *st = sub ? sub + t * n3 : nullptr;
+  const uint32_t plane = (uint32_t)rows * (uint32_t)kp, chunk = (uint32_t)rows * BK;
+  __nv_bfloat16 *ot = out + 2LL * t * TC_PLANES * plane;
+  // MODE 2
+  const bool etd = MODE == 2 && t >= sp.nI;
+  const float4 *ce = MODE == 2 ? sp.etd[t % sp.F >= sp.nac ? 1 : 0] : nullptr;
+  const float2 *cp = MODE == 2 ? sp.phi[t % sp.F >= sp.nac ? 1 : 0] : nullptr;
+  const long long nhat = (long long)(count - sp.nI) * n3;  // from u^ to N^
+  const int row_end = min(rows, (rb + 1) * SLICE_ROWS);
+  for (int row0 = rb * SLICE_ROWS + (threadIdx.x >> 5) * 2; row0 < row_end; row0 += 16) {
+    const int row = row0 + hw;
+    const bool live = row < row_end;
+    const long long l0 = (long long)(live ? row : row0) * n;
+    const float *x = xt + l0;
+    // MODE 0: a = x[k], x[k+1], b = their mirrors; else a = the even part's
+    // two modes, b = the odd part's
+    float a0[C], a1[C], b0[C], b1[C];
+    float me = 0.0f, mo = 0.0f;
+#pragma unroll
+    for (int c = 0; c < C; c++) {
+      const int k = kl + BK * c;
+      a0[c] = a1[c] = b0[c] = b1[c] = 0.0f;
+      if (k >= h) continue;
+      if (MODE == 0) {
+        const int q = n - 1 - k;
+        if (align >= 2) {  // n even: pairs and their mirrors aligned, no middle cell
+          float2 a = *reinterpret_cast<const float2 *>(x + k), b = *reinterpret_cast<const float2 *>(x + q - 1);
+          if (st) {
+            const float2 sa = *reinterpret_cast<const float2 *>(st + l0 + k);
+            const float2 s2 = *reinterpret_cast<const float2 *>(st + l0 + q - 1);
+            a.x -= sa.x;
+            a.y -= sa.y;
+            b.x -= s2.x;
+            b.y -= s2.y;
+          }
+          a0[c] = a.x;
+          b0[c] = b.y;
+          if (k + 1 < h) {
+            a1[c] = a.y;
+            b1[c] = b.x;
+          }
+        } else {
+          auto one = [&](int i) { return st ? x[i] - st[l0 + i] : x[i]; };
+          a0[c] = one(k);
+          if (q != k) b0[c] = one(q);
+          if (k + 1 < h) {
+            a1[c] = one(k + 1);
+            if (q - 1 != k + 1) b1[c] = one(q - 1);
+          }
+        }
+        me = fmaxf(me, fmaxf(fabsf(a0[c] + b0[c]), fabsf(a1[c] + b1[c])));
+        mo = fmaxf(mo, fmaxf(fabsf(a0[c] - b0[c]), fabsf(a1[c] - b1[c])));
+      } else {
+        const int k2 = 2 * k;
+        float v[4];
+        auto load = [&](const float *p, float (&w)[4]) {
+          if (align == 4) {  // then k2 + 3 < n
+            const float4 f = *reinterpret_cast<const float4 *>(p + k2);
+            w[0] = f.x, w[1] = f.y, w[2] = f.z, w[3] = f.w;
+          } else if (align == 2 && k2 + 3 < n) {
+            const float2 f = *reinterpret_cast<const float2 *>(p + k2), g = *reinterpret_cast<const float2 *>(p + k2 + 2);
+            w[0] = f.x, w[1] = f.y, w[2] = g.x, w[3] = g.y;
+          } else {
+#pragma unroll
+            for (int i = 0; i < 4; i++) w[i] = k2 + i < n ? p[k2 + i] : 0.0f;
+          }
+        };
+        load(x, v);
+        if (MODE == 2) {
+          if (etd) {
+            float nh[4];
+            load(x + nhat, nh);
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+              if (k2 + i < n) {
+                const float4 f = __ldg(ce + l0 + k2 + i);  // (e_hi, e_lo, phi1_hi, phi1_lo)
+                v[i] = fmaf(f.x, v[i], fmaf(f.y, v[i], fmaf(f.z, nh[i], f.w * nh[i])));
+              }
+          } else {
+            float2 f[4];
+            if (align >= 2 && k2 + 3 < n) {
+              const float4 p = __ldg(reinterpret_cast<const float4 *>(cp + l0 + k2));
+              const float4 q = __ldg(reinterpret_cast<const float4 *>(cp + l0 + k2 + 2));
+              f[0] = make_float2(p.x, p.y), f[1] = make_float2(p.z, p.w);
+              f[2] = make_float2(q.x, q.y), f[3] = make_float2(q.z, q.w);
+            } else {
+#pragma unroll
+              for (int i = 0; i < 4; i++) f[i] = k2 + i < n ? __ldg(cp + l0 + k2 + i) : make_float2(0.0f, 0.0f);
+            }
+#pragma unroll
+            for (int i = 0; i < 4; i++) v[i] = fmaf(f[i].x, v[i], f[i].y * v[i]);  // (phi_hi, phi_lo)
+          }
+        }
+        a0[c] = odd0 ? v[0] : v[1];
+        a1[c] = odd0 ? v[2] : v[3];
+        b0[c] = odd0 ? v[1] : v[0];
+        b1[c] = odd0 ? v[3] : v[2];
+        me = fmaxf(me, fmaxf(fabsf(a0[c]), fabsf(a1[c])));
+        mo = fmaxf(mo, fmaxf(fabsf(b0[c]), fabsf(b1[c])));
+      }
+    }
+    // an odd block's middle cell is in the even part only: its difference with
+    // the missing mirror must not enter the odd one
+    const int mid = MODE == 0 && align == 1 ? h - 1 : -1;
+    if (mid >= 0 && (mid & ~1) % BK == kl) {
+      mo = 0.0f;
+#pragma unroll
+      for (int c = 0; c < C; c++) {
+        const int k = kl + BK * c;
+        if (k != mid) mo = fmaxf(mo, fabsf(a0[c] - b0[c]));
+        if (k + 1 != mid) mo = fmaxf(mo, fabsf(a1[c] - b1[c]));
+      }
+    }
+#pragma unroll
+    for (int off = 8; off > 0; off >>= 1) {
+      me = fmaxf(me, __shfl_xor_sync(0xffffffffu, me, off));
+      mo = fmaxf(mo, __shfl_xor_sync(0xffffffffu, mo, off));
+    }
+    if (!live) continue;
+    float Se, So, ie, io;
+    scale_of(me, Se, ie);
+    scale_of(mo, So, io);
+    if (kl == 0) {
+      scale[2LL * t * rows + row] = Se;
+      scale[(2LL * t + 1) * rows + row] = So;
+    }
+    // 32-bit offsets within a part (4 n^2 kp < 2^32)
+    uint32_t o = (uint32_t)row * BK + kl;
+#pragma unroll
+    for (int c = 0; c < C; c++, o += chunk) {
+      const int k = kl + BK * c;
+      if (k >= h) continue;
+      float d0[TC_PLANES], d1[TC_PLANES];
+      auto put = [&](__nv_bfloat16 *base) {
+#pragma unroll
+        for (int p = 0; p < TC_PLANES; p++)
+          *reinterpret_cast<uint32_t *>(base + (o + (uint32_t)p * plane)) = bf16_pair(d0[p], d1[p]);
+      };
+      __nv_bfloat16 *oo = ot + (long long)TC_PLANES * plane;
+      if (MODE == 0) {
+        // TwoSum (Knuth) of the pair and its difference
+        auto fold = [&](float a, float b, float inv, float (&d)[TC_PLANES]) {
+          const float s = __fadd_rn(a, b), bp = __fadd_rn(s, -a);
+          const float e = __fadd_rn(__fadd_rn(a, -__fadd_rn(s, -bp)), __fadd_rn(b, -bp));
+          digits(s * inv, e * inv, step, step4, d);
+        };
+        fold(a0[c], b0[c], ie, d0);
+        fold(a1[c], b1[c], ie, d1);
+        put(ot);
+        fold(k == mid ? 0.0f : a0[c], k == mid ? 0.0f : -b0[c], io, d0);
+        fold(k + 1 == mid ? 0.0f : a1[c], k + 1 == mid ? 0.0f : -b1[c], io, d1);
+        put(oo);
+      } else {
+        digits(a0[c] * ie, 0.0f, step, step4, d0);
+        digits(a1[c] * ie, 0.0f, step, step4, d1);
+        put(ot);
+        digits(b0[c] * io, 0.0f, step, step4, d0);
+        digits(b1[c] * io, 0.0f, step, step4, d1);
+        put(oo);
+      }
+    }
+  }
+}
+
 // FP64 matrix rows -> slices with a power-of-two scale per row.
 __global__ void slice_matrix_kernel(const double *__restrict__ m, __nv_bfloat16 *__restrict__ out,
                                     float *__restrict__ row_scale, int n, int kp, int bits) {
@@ -457,7 +744,7 @@ __global__ void slice_matrix_kernel(const double *__restrict__ m, __nv_bfloat16 
 
 // ETD coefficients in FP64 (the plain form's ac_init_phi / ch_init_phi and
 // ac_updateU_new / ch_updateU_new arithmetic), stored as FP32 hi + lo.
-__global__ void coef_kernel(float4 *coef, float2 *coef2, int n, int kind, const double *dx, const double *dy,
+__global__ void coef_kernel(float4 *coef, float2 *phi1, float2 *coef2, int n, int kind, const double *dx, const double *dy,
                             const double *dz, double kkx, double kky, double kkz, double epn2, double dt, double L,
                             double K) {
   const long long n3 = (long long)n * n * n;
@@ -486,7 +773,8 @@ __global__ void coef_kernel(float4 *coef, float2 *coef2, int n, int kind, const 
     c.y = (float)(e - (double)c.x);
     c.z = (float)p1;
     c.w = (float)(p1 - (double)c.z);
-    coef[o] = c;
+    if (coef) coef[o] = c;
+    if (phi1) phi1[o] = make_float2(c.z, c.w);
     if (coef2) {
       float2 c2;
       c2.x = (float)p2;
@@ -530,29 +818,68 @@ cudaError_t tc_slice_fields(const float *x, const float *sub, float *scale, __nv
   return cudaGetLastError();
 }
 
-cudaError_t tc_make_coefs(float4 *coef, float2 *coef2, int n, int kind, const double *dx, const double *dy,
+template <int MODE>
+static void run_slice_fold(int chunks, int g, const TensorList<float> &x, const float *sub, float *scale,
+                           __nv_bfloat16 *planes, int n, int count, const SpecUpdate &sp, cudaStream_t s) {
+  const int h = fold_half(n), kp = tc_kp(h), bits = tc_slice_bits(h);
+#define SCLET_SLICE(C) tc::slice_fold_kernel<C, MODE><<<g, 256, 0, s>>>(x, sub, scale, planes, n, kp, count, bits, sp)
+  if (chunks <= 1) SCLET_SLICE(1);
+  else if (chunks <= 2) SCLET_SLICE(2);
+  else if (chunks <= 4) SCLET_SLICE(4);
+  else if (chunks <= 5) SCLET_SLICE(5);
+  else if (chunks <= 9) SCLET_SLICE(9);
+  else SCLET_SLICE(17);
+#undef SCLET_SLICE
+}
+
+cudaError_t tc_slice_fold(bool forward, const TensorList<float> &x, const float *sub, const SpecUpdate *sp, float *scale,
+                          __nv_bfloat16 *planes, int n, int count, cudaStream_t s) {
+  const int chunks = (fold_half(n) + tc::BK - 1) / tc::BK;
+  if (chunks > 17) return cudaErrorInvalidValue;
+  const long long g = ((long long)n * n + tc::SLICE_ROWS - 1) / tc::SLICE_ROWS * count;
+  if (g > 0x7fffffffLL) return cudaErrorInvalidValue;
+  if (forward) run_slice_fold<0>(chunks, (int)g, x, sub, scale, planes, n, count, SpecUpdate(), s);
+  else if (!sp) run_slice_fold<1>(chunks, (int)g, x, nullptr, scale, planes, n, count, SpecUpdate(), s);
+  else run_slice_fold<2>(chunks, (int)g, x, nullptr, scale, planes, n, count, *sp, s);
+  launch_counter()++;
+  return cudaGetLastError();
+}
+
+cudaError_t tc_make_coefs(float4 *coef, float2 *phi1, float2 *coef2, int n, int kind, const double *dx, const double *dy,
                           const double *dz, const double *kk, double epn2, double dt, double L, double K,
                           cudaStream_t s) {
   long long n3 = (long long)n * n * n;
   long long b = (n3 + 255) / 256;
-  tc::coef_kernel<<<(int)(b > 152 * 16 ? 152 * 16 : b), 256, 0, s>>>(coef, coef2, n, kind, dx, dy, dz, kk[0], kk[1],
+  tc::coef_kernel<<<(int)(b > 152 * 16 ? 152 * 16 : b), 256, 0, s>>>(coef, phi1, coef2, n, kind, dx, dy, dz, kk[0], kk[1],
                                                                      kk[2], epn2, dt, L, K);
   launch_counter()++;
   return cudaGetLastError();
 }
 
-// The kernel's instances (fused update, output): (none, store), (none,
-// accumulate), (ETD1, store), (phi2, store) -- the combinations the step uses.
+// The kernel's instances, the combinations the step uses: any basis (none,
+// store), (none, accumulate), (ETD1, store), (phi2, store); folded forward
+// (store) and inverse (store, accumulate), each for halves beyond 64 and up to
+// 64.
 using TcKernel = void (*)(const CUtensorMap, const CUtensorMap, TcArgs);
-constexpr int TC_INSTANCES = 4;
-static TcKernel tc_instance(int i) {
-  static const TcKernel k[TC_INSTANCES] = {tc::modeprod_tc_kernel<0, 1>, tc::modeprod_tc_kernel<0, 2>,
-                                           tc::modeprod_tc_kernel<1, 1>, tc::modeprod_tc_kernel<2, 1>};
+struct TcInstance {
+  int form, epi, out, bn, smem;
+  TcKernel kern;
+};
+constexpr int TC_INSTANCES = 10;
+static const TcInstance &tc_instance(int i) {
+#define SCLET_TC(F, E, O, B) {F, E, O, B, tc::TileGeom<B>::SMEM_BYTES, tc::modeprod_tc_kernel<F, E, O, B>}
+  static const TcInstance k[TC_INSTANCES] = {
+      SCLET_TC(0, 0, 1, 128), SCLET_TC(0, 0, 2, 128), SCLET_TC(0, 1, 1, 128), SCLET_TC(0, 2, 1, 128),
+      SCLET_TC(1, 0, 1, 128), SCLET_TC(2, 0, 1, 128), SCLET_TC(2, 0, 2, 128),
+      SCLET_TC(1, 0, 1, 64),  SCLET_TC(2, 0, 1, 64),  SCLET_TC(2, 0, 2, 64)};
+#undef SCLET_TC
   return k[i];
 }
-static TcKernel tc_kernel(int epi, int outmode) {
-  if (outmode == 1 && epi >= 0 && epi <= 2) return tc_instance(epi == 0 ? 0 : epi + 1);
-  if (outmode == 2 && epi == 0) return tc_instance(1);
+static const TcInstance *tc_kernel(int form, int epi, int outmode, int bn) {
+  for (int i = 0; i < TC_INSTANCES; i++) {
+    const TcInstance &k = tc_instance(i);
+    if (k.form == form && k.epi == epi && k.out == outmode && k.bn == bn) return &k;
+  }
   return nullptr;
 }
 
@@ -571,13 +898,13 @@ static int tc_setup(int *ctas) {
   if (!resident[dev]) {
     for (int i = 0; i < TC_INSTANCES; i++) {
       // all of the unified L1/shared capacity as shared memory
-      e = cudaFuncSetAttribute(tc_instance(i), cudaFuncAttributeMaxDynamicSharedMemorySize, tc::SMEM_BYTES);
+      e = cudaFuncSetAttribute(tc_instance(i).kern, cudaFuncAttributeMaxDynamicSharedMemorySize, tc_instance(i).smem);
       if (e != cudaSuccess) return e;
-      e = cudaFuncSetAttribute(tc_instance(i), cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+      e = cudaFuncSetAttribute(tc_instance(i).kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
       if (e != cudaSuccess) return e;
     }
     int per_sm = 0, sms = 0;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, tc_kernel(0, 1), tc::THREADS, tc::SMEM_BYTES);
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, tc_instance(0).kern, tc::THREADS, tc_instance(0).smem);
     if (e != cudaSuccess) return e;
     e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (e != cudaSuccess) return e;
@@ -593,25 +920,27 @@ cudaError_t launch_modeprod_tc(const __nv_bfloat16 *mat, const __nv_bfloat16 *pl
   int ctas = 0;
   cudaError_t e = (cudaError_t)tc_setup(&ctas);
   if (e != cudaSuccess) return e;
-  const TcKernel kern = tc_kernel(args.epi, args.outmode);
-  if (!kern) return cudaErrorInvalidValue;
-  const int n = args.n, kp = tc_kp(n);
-  const int bits = tc_slice_bits(n);
-  if ((long long)tc::BK * ((n + tc::BK - 1) / tc::BK) > (1LL << (24 - 2 * bits))) return cudaErrorInvalidValue;
+  // contraction length and outputs of one part
+  const int n = args.n, parts = args.form == 0 ? 1 : 2, h = parts == 1 ? n : fold_half(n), kp = tc_kp(h);
+  const int bn = args.form != 0 && h <= 64 ? 64 : 128;
+  const TcInstance *inst = tc_kernel(args.form, args.epi, args.outmode, bn);
+  if (!inst) return cudaErrorInvalidValue;
+  const int bits = tc_slice_bits(h);
+  if ((long long)kp > (1LL << (24 - 2 * bits))) return cudaErrorInvalidValue;
   if ((long long)n * n * n > 0xffffffffLL) return cudaErrorInvalidValue;  // 32-bit offsets within a tensor
   CUtensorMap ma, mb;
-  if ((e = make_map(&ma, planes, kp, (long long)n * n, TC_PLANES * count, tc::BM)) != cudaSuccess) return e;
-  if ((e = make_map(&mb, mat, kp, n, TC_PLANES_M, tc::BN)) != cudaSuccess) return e;
+  if ((e = make_map(&ma, planes, kp, (long long)n * n, TC_PLANES * parts * count, tc::BM)) != cudaSuccess) return e;
+  if ((e = make_map(&mb, mat, kp, h, TC_PLANES_M * parts, bn)) != cudaSuccess) return e;
   TcArgs g = args;
   g.kp = kp;
-  g.kblocks = (n + tc::BK - 1) / tc::BK;
+  g.kblocks = kp / tc::BK;
   g.bits = bits;
   const long long groups = (((long long)n * n + tc::BM - 1) / tc::BM) * count;  // input tiles
-  if (groups * ((n + tc::BN - 1) / tc::BN) > 0x7fffffffLL) return cudaErrorInvalidValue;
+  if (groups * parts * ((h + bn - 1) / bn) > 0x7fffffffLL) return cudaErrorInvalidValue;
   // persistent: as many CTAs as can be resident at once (or the tuned count)
   if (args.max_ctas > 0 && args.max_ctas < ctas) ctas = args.max_ctas;
   const int grid = (int)(groups < ctas ? groups : ctas);
-  kern<<<grid, tc::THREADS, tc::SMEM_BYTES, s>>>(ma, mb, g);
+  inst->kern<<<grid, tc::THREADS, inst->smem, s>>>(ma, mb, g);
   launch_counter()++;
   return cudaGetLastError();
 }

@@ -67,8 +67,10 @@ struct sclet_ctx {
   float *fstate2 = nullptr, *frhs2 = nullptr, *ffelas = nullptr, *fscratch = nullptr, *fshell = nullptr;
   float *W1 = nullptr, *W2 = nullptr, *scaleP = nullptr, *rsV = nullptr, *rsVi = nullptr;
   __nv_bfloat16 *P = nullptr, *matV = nullptr, *matVi = nullptr;
-  float4 *coef[2] = {nullptr, nullptr};   // ETD1 coefficient pairs per field kind
+  float4 *coef[2] = {nullptr, nullptr};   // ETD1 coefficient pairs per field kind (full form)
+  float2 *coef1[2] = {nullptr, nullptr};  // phi1 pairs per field kind (increment form)
   float2 *coef2[2] = {nullptr, nullptr};  // ETD2 phi2 pairs per field kind
+  int plane_form = -1;                    // layout the slice planes' zero pads are set for: 0 dense, 1 folded
   double *stage64 = nullptr;  // n^3 FP64 staging block for host transfers
   // variable-mobility CH: two scratch blocks per run in the state's type and
   // the block maxima of the mobility (Phys::mob_t, Phys::mob_part)
@@ -209,6 +211,15 @@ int mass_weights_setup(sclet_ctx *ctx, const double *v, const double *vi);
 int queue_diagnostics(sclet_ctx *ctx, int energy_form);
 int read_diagnostics(sclet_ctx *ctx, sclet_diag *out);
 
+// Elements of one sliced tensor: TC_PLANES planes of n*n rows of kp, or two
+// parts of them over half the columns
+long long dense_elems(int n) { return (long long)TC_PLANES * n * n * tc_kp(n); }
+long long fold_elems(int n) { return 2LL * TC_PLANES * n * n * tc_kp(fold_half(n)); }
+long long tc_plane_elems(const sclet_ctx *ctx) {  // as allocated: room for either
+  const long long a = dense_elems(ctx->n), b = fold_elems(ctx->n);
+  return a > b ? a : b;
+}
+
 // Whether the order parameters may advance as u' = u + V phi1 V^-1 (N - H u)
 // instead of u' = V (e V^-1 u + phi1 V^-1 N): the same in exact arithmetic
 // where V diag(d) V^-1 is the stencil's operator, with three products per
@@ -230,7 +241,7 @@ bool increments_allowed(const sclet_ctx *ctx, const double *d) {
 
 int upload_eigen(sclet_ctx *ctx, const double *d, const double *v, const double *vi) {
   const int n = ctx->n;
-  ctx->dirichlet = !mixed(ctx) && basis_is_dirichlet(n, d, v, vi);
+  ctx->dirichlet = basis_is_dirichlet(n, d, v, vi);
   ctx->increments = increments_allowed(ctx, d);
   std::vector<double> ds(n);
   for (int ax = 0; ax < 3; ax++) {
@@ -244,17 +255,46 @@ int upload_eigen(sclet_ctx *ctx, const double *d, const double *v, const double 
   }
   if (mixed(ctx)) {
     // the stage block holds the FP64 matrices while they are split
-    CK(cudaMemcpyAsync(ctx->stage64, vi, sizeof(double) * n * n, cudaMemcpyHostToDevice, ctx->stream));
-    CK(tc_slice_matrix(ctx->stage64, ctx->matVi, ctx->rsVi, n, ctx->stream));
-    CK(cudaStreamSynchronize(ctx->stream));
-    CK(cudaMemcpyAsync(ctx->stage64, v, sizeof(double) * n * n, cudaMemcpyHostToDevice, ctx->stream));
-    CK(tc_slice_matrix(ctx->stage64, ctx->matV, ctx->rsV, n, ctx->stream));
+    const int form = ctx->dirichlet ? 1 : 0;
+    if (ctx->plane_form != form) {
+      // pad columns of the slice planes are never written and must be zero
+      CK(cudaMemsetAsync(ctx->P, 0, sizeof(__nv_bfloat16) * tc_plane_elems(ctx) * 2 * ctx->FT, ctx->stream));
+      ctx->plane_form = form;
+    }
+    for (int inv = 0; inv < 2; inv++) {
+      __nv_bfloat16 *mat = inv ? ctx->matV : ctx->matVi;
+      float *rs = inv ? ctx->rsV : ctx->rsVi;
+      const double *src = inv ? v : vi;
+      if (!ctx->dirichlet) {
+        CK(cudaMemcpyAsync(ctx->stage64, src, sizeof(double) * n * n, cudaMemcpyHostToDevice, ctx->stream));
+        CK(tc_slice_matrix(ctx->stage64, mat, rs, n, ctx->stream));
+        CK(cudaStreamSynchronize(ctx->stream));
+        continue;
+      }
+      const int h = fold_half(n);
+      const std::vector<double> w = fold_matrix(n, src, inv != 0);  // [part][k][o]
+      std::vector<double> m(w.size());                              // [part][o][k]
+      for (int part = 0; part < 2; part++)
+        for (int k = 0; k < h; k++)
+          for (int o = 0; o < h; o++) m[((size_t)part * h + o) * h + k] = w[((size_t)part * h + k) * h + o];
+      CK(cudaMemcpyAsync(ctx->stage64, m.data(), sizeof(double) * m.size(), cudaMemcpyHostToDevice, ctx->stream));
+      for (int part = 0; part < 2; part++)
+        CK(tc_slice_matrix(ctx->stage64 + (size_t)part * h * h, mat + (size_t)part * TC_PLANES_M * h * tc_kp(h),
+                           rs + part * h, h, ctx->stream));
+      CK(cudaStreamSynchronize(ctx->stream));
+    }
     const sclet_params &p = ctx->p;
     const double kk[3] = {p.kkx, p.kky, p.kkz};
-    for (int kind = 0; kind < 2; kind++)
-      CK(tc_make_coefs(ctx->coef[kind], ctx->coef2[kind], n, kind, ctx->dd[0], ctx->dd[1], ctx->dd[2], kk, p.epn2,
-                       p.dt, kind == 0 ? ctx->ph.LE : ctx->ph.LCI, kind == 0 ? ctx->ph.KE : ctx->ph.KCI,
-                       ctx->stream));
+    for (int kind = 0; kind < 2; kind++) {
+      if ((kind == 0 ? ctx->nac : ctx->nch) == 0) continue;
+      // the full form's (e, phi1) pairs, or phi1 alone for increments
+      const bool inc = kind == 0 && ctx->increments;
+      if (!inc && !ctx->coef[kind]) CK(cudaMalloc(&ctx->coef[kind], sizeof(float4) * ctx->n3));
+      if (inc && !ctx->coef1[kind]) CK(cudaMalloc(&ctx->coef1[kind], sizeof(float2) * ctx->n3));
+      CK(tc_make_coefs(inc ? nullptr : ctx->coef[kind], inc ? ctx->coef1[kind] : nullptr, ctx->coef2[kind], n, kind,
+                       ctx->dd[0], ctx->dd[1], ctx->dd[2], kk, p.epn2, p.dt, kind == 0 ? ctx->ph.LE : ctx->ph.LCI,
+                       kind == 0 ? ctx->ph.KE : ctx->ph.KCI, ctx->stream));
+    }
     CK(cudaStreamSynchronize(ctx->stream));
     if (ctx->nch > 0) return mass_weights_setup(ctx, v, vi);
     return SCLET_OK;
@@ -287,20 +327,23 @@ EtdCoef etd_coef(sclet_ctx *ctx);
 // g = column sums of V over the owned rows, V^-T as a row-major matrix.
 int mass_weights_setup(sclet_ctx *ctx, const double *v, const double *vi) {
   const int n = ctx->n;
-  std::vector<double> g(n, 0.0), viT((size_t)n * n);
+  std::vector<double> g(n, 0.0), viT((size_t)n * n), fold;
   for (int i = 2; i < n - 2; i++)
     for (int q = 0; q < n; q++) g[q] += v[(size_t)i * n + q];
   for (int i = 0; i < n; i++)
     for (int q = 0; q < n; q++) viT[(size_t)i * n + q] = vi[(size_t)q * n + i];
+  // V^-T maps modes to positions as V does: folded like an inverse product
+  if (ctx->dirichlet) fold = fold_matrix(n, viT.data(), true);
+  const std::vector<double> &w = ctx->dirichlet ? fold : viT;
   double *dg = nullptr, *dm = nullptr;
   cudaError_t e = cudaMalloc(&dg, sizeof(double) * n);
-  if (e == cudaSuccess) e = cudaMalloc(&dm, sizeof(double) * n * n);
+  if (e == cudaSuccess) e = cudaMalloc(&dm, sizeof(double) * w.size());
   if (e == cudaSuccess) e = cudaMemcpyAsync(dg, g.data(), sizeof(double) * n, cudaMemcpyHostToDevice, ctx->stream);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(dm, viT.data(), sizeof(double) * n * n, cudaMemcpyHostToDevice, ctx->stream);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(dm, w.data(), sizeof(double) * w.size(), cudaMemcpyHostToDevice, ctx->stream);
   const EtdCoef ec = etd_coef(ctx);
   const int nw = ctx->p.etd2 ? 3 : 2;
-  for (int w = 0; w < nw && e == cudaSuccess; w++)
-    e = mass_weight(ctx->massW + w * ctx->n3, ctx->stage64, dg, dm, n, w, ec, ctx->stream);
+  for (int k = 0; k < nw && e == cudaSuccess; k++)
+    e = mass_weight(ctx->massW + k * ctx->n3, ctx->stage64, dg, dm, n, k, ec, ctx->stream, ctx->dirichlet);
   if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
   cudaFree(dg);
   cudaFree(dm);
@@ -325,8 +368,6 @@ EtdCoef etd_coef(sclet_ctx *ctx) {
   return ec;
 }
 
-// Elements of one sliced tensor (TC_PLANES planes of n*n rows of kp)
-long long plane_stride(const sclet_ctx *ctx) { return (long long)TC_PLANES * ctx->n * ctx->n * tc_kp(ctx->n); }
 
 void stage_begin(sclet_ctx *ctx, int cls, StageEv &ev) {
   if (!ctx->profiling) return;
@@ -471,7 +512,8 @@ void sclet_destroy(sclet_ctx *ctx) {
                   ctx->partials, ctx->phi1[0], ctx->phi1[1], ctx->phi2[0], ctx->phi2[1], ctx->dev_err,
                   ctx->fstate2, ctx->frhs2, ctx->ffelas, ctx->fscratch, ctx->fshell, ctx->W1, ctx->W2, ctx->P,
                   ctx->scaleP, ctx->rsV, ctx->rsVi, ctx->matV, ctx->matVi, ctx->stage64,
-                  ctx->coef[0], ctx->coef[1], ctx->coef2[0], ctx->coef2[1], ctx->massW, ctx->massPart,
+                  ctx->coef[0], ctx->coef[1], ctx->coef1[0], ctx->coef1[1], ctx->coef2[0],
+                  ctx->coef2[1], ctx->massW, ctx->massPart,
                   ctx->massRes, ctx->in_stage, ctx->out_stage, ctx->krun, ctx->mob_t, ctx->mob_part, ctx->foldVi,
                   ctx->foldV};
   for (void *b : bufs) cudaFree(b);
@@ -641,22 +683,19 @@ int sclet_create_runs(const sclet_params *p, int runs, const double *krun, int p
     CC(cudaMalloc(&ctx->fshell, sizeof(float) * FT * shell_count(n)));
     CC(cudaMalloc(&ctx->W1, 2 * FT * blk));
     CC(cudaMalloc(&ctx->W2, 2 * FT * blk));
+    CC(cudaMalloc(&ctx->P, sizeof(__nv_bfloat16) * tc_plane_elems(ctx) * 2 * FT));
+    CC(cudaMalloc(&ctx->scaleP, sizeof(float) * 2 * 2 * FT * n * n));
     {
-      const size_t pbytes = sizeof(__nv_bfloat16) * plane_stride(ctx) * 2 * FT;
-      // pad columns of the slice planes are never written and must stay zero
-      CC(cudaMalloc(&ctx->P, pbytes));
-      CC(cudaMemsetAsync(ctx->P, 0, pbytes, s));
-      CC(cudaMalloc(&ctx->scaleP, sizeof(float) * 2 * FT * n * n));
+      // dense n x n or two folded h x h matrices
+      const size_t h = fold_half(n), md = (size_t)n * tc_kp(n), mf = 2 * h * tc_kp((int)h), m = md > mf ? md : mf;
+      CC(cudaMalloc(&ctx->matV, sizeof(__nv_bfloat16) * TC_PLANES_M * m));
+      CC(cudaMalloc(&ctx->matVi, sizeof(__nv_bfloat16) * TC_PLANES_M * m));
+      CC(cudaMalloc(&ctx->rsV, sizeof(float) * 2 * h));
+      CC(cudaMalloc(&ctx->rsVi, sizeof(float) * 2 * h));
     }
-    CC(cudaMalloc(&ctx->matV, sizeof(__nv_bfloat16) * TC_PLANES_M * n * tc_kp(n)));
-    CC(cudaMalloc(&ctx->matVi, sizeof(__nv_bfloat16) * TC_PLANES_M * n * tc_kp(n)));
-    CC(cudaMalloc(&ctx->rsV, sizeof(float) * n));
-    CC(cudaMalloc(&ctx->rsVi, sizeof(float) * n));
     CC(cudaMalloc(&ctx->stage64, sizeof(double) * ctx->n3));
-    for (int k = 0; k < 2; k++) {
-      CC(cudaMalloc(&ctx->coef[k], sizeof(float4) * ctx->n3));
+    for (int k = 0; k < 2; k++)
       if (p->etd2) CC(cudaMalloc(&ctx->coef2[k], sizeof(float2) * ctx->n3));
-    }
     if (ctx->nch > 0) {
       CC(cudaMalloc(&ctx->massW, sizeof(double) * ctx->n3 * (p->etd2 ? 3 : 2)));
       CC(cudaMalloc(&ctx->massPart, sizeof(double) * 4 * mass_partials()));
@@ -899,8 +938,10 @@ static TcArgs tc_args(sclet_ctx *ctx, bool inverse, int count, float *out, int e
   memset(&g, 0, sizeof g);
   g.n = ctx->n;
   g.count = count;
+  g.form = ctx->dirichlet ? (inverse ? 2 : 1) : 0;
   g.epi = epi;
   g.outmode = outmode;
+  g.acc = ctx->F;
   g.aux = aux;
   g.out = out;
   g.row_scale = inverse ? ctx->rsV : ctx->rsVi;
@@ -918,13 +959,25 @@ static TcArgs tc_args(sclet_ctx *ctx, bool inverse, int count, float *out, int e
 // One fixed-point tensor-core product of `count` sliced tensors (planes at
 // `planes`, row scales at `scale`) into FP32 `out`.
 static cudaError_t tc_prod(sclet_ctx *ctx, bool inverse, const __nv_bfloat16 *planes, const float *scale, int count,
-                           float *out, int epi, const float *aux, int outmode) {
+                           float *out, int epi, const float *aux, int outmode, int acc = -1) {
   StageEv ev;
   long long l0 = launch_counter();
   stage_begin(ctx, 5, ev);
   TcArgs g = tc_args(ctx, inverse, count, out, epi, aux, outmode);
   g.in_scale = scale;
+  if (acc >= 0) g.acc = acc;  // fields the folded inverse accumulates
   cudaError_t e = launch_modeprod_tc(inverse ? ctx->matV : ctx->matVi, planes, count, g, ctx->stream);
+  stage_end(ctx, ev, l0);
+  return e;
+}
+
+// the lines of x, for a folded product
+static cudaError_t tc_slice_parts(sclet_ctx *ctx, bool forward, const TensorList<float> &x, const float *sub, int count,
+                                  const SpecUpdate *sp = nullptr) {
+  StageEv ev;
+  long long l0 = launch_counter();
+  stage_begin(ctx, 6, ev);
+  cudaError_t e = tc_slice_fold(forward, x, sub, sp, ctx->scaleP, ctx->P, ctx->n, count, ctx->stream);
   stage_end(ctx, ev, l0);
   return e;
 }
@@ -939,30 +992,68 @@ static cudaError_t tc_slice(sclet_ctx *ctx, const float *x, const float *sub, in
   return e;
 }
 
+// Mixed form of the transforms on the folded products.  Tensors, in order: the
+// nI order parameters that advance by increments (their r), then u, then N of
+// the nF other fields.
+static int etd_update_fold(sclet_ctx *ctx) {
+  // several runs side by side hold order parameters only: all of one sort
+  const int F = ctx->FT, nI = ctx->increments ? ctx->nac * ctx->runs : 0, nF = F - nI, T = nI + 2 * nF;
+  const long long n3 = ctx->n3;
+  const float *u = fu_of(ctx), *N1 = frhs1_of(ctx);
+  auto list = [](const float *a) { return tensor_list<float>(a); };
+  if (nI) CK(launch_increment_rhs<float>(ctx->ph, u, N1, ctx->W2, ctx->stream));
+  CK(tc_slice_parts(ctx, true, TensorList<float>{{ctx->W2, u + nI * n3, N1 + nI * n3}, {0, nI, nI + nF}}, nullptr, T));
+  CK(tc_prod(ctx, false, ctx->P, ctx->scaleP, T, ctx->W1, 0, nullptr, 1));
+  CK(tc_slice_parts(ctx, true, list(ctx->W1), nullptr, T));
+  CK(tc_prod(ctx, false, ctx->P, ctx->scaleP, T, ctx->W2, 0, nullptr, 1));
+  CK(tc_slice_parts(ctx, true, list(ctx->W2), nullptr, T));
+  CK(tc_prod(ctx, false, ctx->P, ctx->scaleP, T, ctx->W1, 0, nullptr, 1));
+  SpecUpdate sp;
+  for (int k = 0; k < 2; k++) {
+    sp.phi[k] = ctx->coef1[k];
+    sp.etd[k] = ctx->coef[k];
+  }
+  sp.nI = nI;
+  sp.F = ctx->F;
+  sp.nac = ctx->nac;
+  CK(tc_slice_parts(ctx, false, list(ctx->W1), nullptr, F, &sp));
+  CK(tc_prod(ctx, true, ctx->P, ctx->scaleP, F, ctx->W1, 0, nullptr, 1));
+  CK(tc_slice_parts(ctx, false, list(ctx->W1), nullptr, F));
+  CK(tc_prod(ctx, true, ctx->P, ctx->scaleP, F, ctx->W2, 0, nullptr, 1));
+  CK(tc_slice_parts(ctx, false, list(ctx->W2), nullptr, F));
+  CK(tc_prod(ctx, true, ctx->P, ctx->scaleP, F, fu_of(ctx), 0, nullptr, nI ? 2 : 1, nI ? ctx->nac : 0));
+  return SCLET_OK;
+}
+
 // Mixed form of the transforms (ScLETD.c:105-142): V^-1 along x and y for u
 // and N1 together, along z for u, then for N1 with the ETD update fused; V
 // along x, y, z back to the FP32 state.
 static int etd_update_mixed(sclet_ctx *ctx) {
   const int F = ctx->FT;  // every run's fields
-  const long long ps = plane_stride(ctx), rows = (long long)ctx->n * ctx->n, n3 = ctx->n3;
+  const long long ps = dense_elems(ctx->n), rows = (long long)ctx->n * ctx->n, n3 = ctx->n3;
   if (ctx->nch > 0)  // target mass of the conserved field from (u, N1)
     CK(mass_target(fu_of(ctx) + ctx->nac * n3, ctx->massW, frhs1_of(ctx) + ctx->nac * n3, nullptr, ctx->massW + n3,
                    ctx->n, ctx->massPart, ctx->stream));
-  CK(tc_slice(ctx, ctx->fstate2, nullptr, 2 * F));
-  CK(tc_prod(ctx, false, ctx->P, ctx->scaleP, 2 * F, ctx->W1, 0, nullptr, 1));
-  CK(tc_slice(ctx, ctx->W1, nullptr, 2 * F));
-  CK(tc_prod(ctx, false, ctx->P, ctx->scaleP, 2 * F, ctx->W2, 0, nullptr, 1));
-  CK(tc_slice(ctx, ctx->W2, nullptr, 2 * F));
-  // uhat into W2 (free once sliced), so that the fused update reads it from a
-  // buffer it does not write
-  CK(tc_prod(ctx, false, ctx->P, ctx->scaleP, F, ctx->W2, 0, nullptr, 1));
-  CK(tc_prod(ctx, false, ctx->P + F * ps, ctx->scaleP + F * rows, F, ctx->W1, 1, ctx->W2, 1));
-  CK(tc_slice(ctx, ctx->W1, nullptr, F));
-  CK(tc_prod(ctx, true, ctx->P, ctx->scaleP, F, ctx->W2, 0, nullptr, 1));
-  CK(tc_slice(ctx, ctx->W2, nullptr, F));
-  CK(tc_prod(ctx, true, ctx->P, ctx->scaleP, F, ctx->W1, 0, nullptr, 1));
-  CK(tc_slice(ctx, ctx->W1, nullptr, F));
-  CK(tc_prod(ctx, true, ctx->P, ctx->scaleP, F, fu_of(ctx), 0, nullptr, 1));
+  if (ctx->dirichlet) {
+    int rc = etd_update_fold(ctx);
+    if (rc != SCLET_OK) return rc;
+  } else {
+    CK(tc_slice(ctx, ctx->fstate2, nullptr, 2 * F));
+    CK(tc_prod(ctx, false, ctx->P, ctx->scaleP, 2 * F, ctx->W1, 0, nullptr, 1));
+    CK(tc_slice(ctx, ctx->W1, nullptr, 2 * F));
+    CK(tc_prod(ctx, false, ctx->P, ctx->scaleP, 2 * F, ctx->W2, 0, nullptr, 1));
+    CK(tc_slice(ctx, ctx->W2, nullptr, 2 * F));
+    // uhat into W2 (free once sliced), so that the fused update reads it from a
+    // buffer it does not write
+    CK(tc_prod(ctx, false, ctx->P, ctx->scaleP, F, ctx->W2, 0, nullptr, 1));
+    CK(tc_prod(ctx, false, ctx->P + F * ps, ctx->scaleP + F * rows, F, ctx->W1, 1, ctx->W2, 1));
+    CK(tc_slice(ctx, ctx->W1, nullptr, F));
+    CK(tc_prod(ctx, true, ctx->P, ctx->scaleP, F, ctx->W2, 0, nullptr, 1));
+    CK(tc_slice(ctx, ctx->W2, nullptr, F));
+    CK(tc_prod(ctx, true, ctx->P, ctx->scaleP, F, ctx->W1, 0, nullptr, 1));
+    CK(tc_slice(ctx, ctx->W1, nullptr, F));
+    CK(tc_prod(ctx, true, ctx->P, ctx->scaleP, F, fu_of(ctx), 0, nullptr, 1));
+  }
   if (ctx->nch > 0)
     CK(mass_fix(fu_of(ctx) + ctx->nac * n3, ctx->n, ctx->massPart, ctx->massPart + 2 * mass_partials(), ctx->massRes,
                 ctx->stream));
@@ -976,17 +1067,27 @@ static int etd2_correct_mixed(sclet_ctx *ctx) {
   if (ctx->nch > 0)  // target: current mass plus <w2, N2 - N1>
     CK(mass_target(fu_of(ctx) + off, nullptr, ctx->frhs2 + off, frhs1_of(ctx) + off, ctx->massW + 2 * n3, ctx->n,
                    ctx->massPart, ctx->stream));
-  CK(tc_slice(ctx, ctx->frhs2, frhs1_of(ctx), F));
+  const bool fold = ctx->dirichlet;
+  SpecUpdate sp;  // the folded form scales the modes by phi2 where it slices them
+  for (int k = 0; k < 2; k++) sp.phi[k] = ctx->coef2[k];
+  sp.nI = F;
+  sp.F = ctx->F;
+  sp.nac = ctx->nac;
+  auto slice = [&](bool fwd, const float *x, const float *sub, bool update = false) {
+    return fold ? tc_slice_parts(ctx, fwd, tensor_list<float>(x), sub, F, update ? &sp : nullptr)
+                : tc_slice(ctx, x, sub, F);
+  };
+  CK(slice(true, ctx->frhs2, frhs1_of(ctx)));
   CK(tc_prod(ctx, false, ctx->P, ctx->scaleP, F, ctx->W1, 0, nullptr, 1));
-  CK(tc_slice(ctx, ctx->W1, nullptr, F));
+  CK(slice(true, ctx->W1, nullptr));
   CK(tc_prod(ctx, false, ctx->P, ctx->scaleP, F, ctx->W2, 0, nullptr, 1));
-  CK(tc_slice(ctx, ctx->W2, nullptr, F));
-  CK(tc_prod(ctx, false, ctx->P, ctx->scaleP, F, ctx->W1, 2, nullptr, 1));
-  CK(tc_slice(ctx, ctx->W1, nullptr, F));
+  CK(slice(true, ctx->W2, nullptr));
+  CK(tc_prod(ctx, false, ctx->P, ctx->scaleP, F, ctx->W1, fold ? 0 : 2, nullptr, 1));
+  CK(slice(false, ctx->W1, nullptr, true));
   CK(tc_prod(ctx, true, ctx->P, ctx->scaleP, F, ctx->W2, 0, nullptr, 1));
-  CK(tc_slice(ctx, ctx->W2, nullptr, F));
+  CK(slice(false, ctx->W2, nullptr));
   CK(tc_prod(ctx, true, ctx->P, ctx->scaleP, F, ctx->W1, 0, nullptr, 1));
-  CK(tc_slice(ctx, ctx->W1, nullptr, F));
+  CK(slice(false, ctx->W1, nullptr));
   CK(tc_prod(ctx, true, ctx->P, ctx->scaleP, F, fu_of(ctx), 0, nullptr, 2));
   if (ctx->nch > 0)
     CK(mass_fix(fu_of(ctx) + off, ctx->n, ctx->massPart, ctx->massPart + 2 * mass_partials(), ctx->massRes,
@@ -1170,7 +1271,8 @@ int sclet_mode_product(sclet_ctx *ctx, int inverse, const double *in, double *ou
     f64_to_f32<<<grid_of(n3), 256, 0, ctx->stream>>>(ctx->stage64, tmp, n3, 0.0);
     launch_counter()++;
     CK(cudaGetLastError());
-    CK(tc_slice(ctx, tmp, nullptr, 1));
+    if (ctx->dirichlet) CK(tc_slice_parts(ctx, inverse == 0, tensor_list<float>(tmp), nullptr, 1));
+    else CK(tc_slice(ctx, tmp, nullptr, 1));
     CK(tc_prod(ctx, inverse != 0, ctx->P, ctx->scaleP, 1, tmp + n3, 0, nullptr, 1));
     f32_to_f64<<<grid_of(n3), 256, 0, ctx->stream>>>(tmp + n3, ctx->stage64, n3, 0.0);
     launch_counter()++;

@@ -4,6 +4,8 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include "sclet_internal.cuh"
+
 namespace sclet {
 
 constexpr int TC_PLANES = 4;    // fixed-point slices per data operand (tc_slice_bits each)
@@ -13,12 +15,14 @@ constexpr int TC_PLANES_M = 5;  // slices per matrix: four 6-bit slices and a fi
 struct TcArgs {
   int n, kp, kblocks, count;
   int bits;                 // slice width (set by launch_modeprod_tc)
-  int epi;                  // 0 none, 1 ETD1 update (aux = uhat), 2 phi2 scaling
+  int form;                 // 0 any basis, 1 folded forward, 2 folded inverse product
+  int epi;                  // 0 none, 1 ETD1 update (aux = uhat), 2 phi scaling
   int outmode;              // 1 FP32 store, 2 FP32 accumulate
+  int acc;                  // form 2, outmode 2: fields t % F < acc accumulate, the others store
   const float *aux;         // [count][n^3] FP32 uhat, same layout as out
   float *out;               // [count][n^3] FP32, rotated layout
-  const float *in_scale;    // [count][n*n] power-of-two scale of each input row's slices
-  const float *row_scale;   // [n] power-of-two scale of each matrix row's slices
+  const float *in_scale;    // [count][n*n] power-of-two scale of each input row's slices ([count][2][n*n] folded)
+  const float *row_scale;   // [n] power-of-two scale of each matrix row's slices ([2][h] folded)
   // per field kind (0 AC, 1 CH), per eigen-mode [k][j][i]: ETD1
   // (e = 1 - phi1 H, phi1) and ETD2 (phi2) coefficients computed in FP64
   // (ac_init_phi / ch_init_phi, vars.c:302-359) as hi + lo FP32 pairs
@@ -42,8 +46,23 @@ cudaError_t tc_slice_matrix(const double *m, __nv_bfloat16 *planes, float *row_s
 // scale[count][n*n]; the pad columns are never written (zero from allocation).
 cudaError_t tc_slice_fields(const float *x, const float *sub, float *scale, __nv_bfloat16 *planes, int n, int count,
                             cudaStream_t s);
-// ETD coefficient tables of one field kind (see TcArgs::coef)
-cudaError_t tc_make_coefs(float4 *coef, float2 *coef2, int n, int kind, const double *dx, const double *dy,
+// The update of the eigen-modes done where they are sliced for the inverse
+// transform: tensors t < nI are multiplied by phi (hi, lo pairs of their
+// field kind); the others are u^ and become e u^ + phi1 N^, their N^ the block
+// count - nI blocks on (etd: (e, phi1) pairs as TcArgs::coef).
+struct SpecUpdate {
+  const float2 *phi[2] = {nullptr, nullptr};
+  const float4 *etd[2] = {nullptr, nullptr};
+  int nI = 0, F = 1, nac = 0;
+};
+// Lines -> the slices of their parity parts (see slice_fold_kernel), planes
+// [count][2][p][kp / 32][n*n][32], kp = tc_kp(fold_half(n)), scales
+// [count][2][n*n]; forward: x - sub folded (sub may be null), else split by
+// mode after the update sp (may be null)
+cudaError_t tc_slice_fold(bool forward, const TensorList<float> &x, const float *sub, const SpecUpdate *sp, float *scale,
+                          __nv_bfloat16 *planes, int n, int count, cudaStream_t s);
+// ETD coefficient tables of one field kind (see TcArgs::coef); null ones are left out
+cudaError_t tc_make_coefs(float4 *coef, float2 *phi1, float2 *coef2, int n, int kind, const double *dx, const double *dy,
                           const double *dz, const double *kk, double epn2, double dt, double L, double K,
                           cudaStream_t s);
 // out[t] = mat x in[t] (contracting the row axis, rotating), count tensors

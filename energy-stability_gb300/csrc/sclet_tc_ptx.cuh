@@ -14,22 +14,27 @@ namespace sclet {
 namespace tc {
 
 
-constexpr int BM = 128, BN = 128, BK = 32, STAGES = 3, NP = TC_PLANES, NPM = TC_PLANES_M;
+constexpr int BM = 128, BK = 32, NP = TC_PLANES, NPM = TC_PLANES_M;
 constexpr int PLANE_A = BM * BK * 2;  // 8 KB: one input slice (M side, 128 input rows)
-constexpr int PLANE_B = BN * BK * 2;  // 8 KB: one matrix slice (N side, 128 a' rows)
-constexpr int STAGE_BYTES = NP * PLANE_A + NPM * PLANE_B;
 constexpr int SMEM_ALIGN = 512;  // period of the 64-byte swizzle pattern
-constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + SMEM_ALIGN;
 constexpr int NACC = 4;               // weight classes w = 0..3
-constexpr int ACC_COLS = NACC * BN;   // one accumulator set
-constexpr int NBUF = 512 / ACC_COLS;   // accumulator sets in tensor memory (1 or 2)
-constexpr int TMEM_COLS = NBUF * ACC_COLS;
 constexpr int EPI_WARPS = 8;          // two per TMEM lane quadrant, each half of the columns
-constexpr int CPW = BN / 32 / 2;      // 32-column chunks per epilogue warp
 constexpr int THREADS = 64 + 32 * EPI_WARPS;  // producer, MMA, epilogue warps
 constexpr long long WAIT_LIMIT = 1LL << 22;  // polls (with backoff) before giving up
-static_assert(TMEM_COLS <= 512, "tensor memory holds 512 columns");
-static_assert(SMEM_BYTES <= 227 * 1024, "shared memory per CTA");
+
+// what follows from the a'-tile width BN (N side)
+template <int BN>
+struct TileGeom {
+  static constexpr int PLANE_B = BN * BK * 2;  // one matrix slice
+  static constexpr int STAGE_BYTES = NP * PLANE_A + NPM * PLANE_B;
+  static constexpr int STAGES = BN == 128 ? 3 : 4;
+  static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + SMEM_ALIGN;
+  static constexpr int ACC_COLS = NACC * BN;      // one accumulator set
+  static constexpr int NBUF = 512 / ACC_COLS;     // accumulator sets in tensor memory (1 or 2)
+  static constexpr int TMEM_COLS = NBUF * ACC_COLS;
+  static constexpr int CPW = BN / 32 / 2;         // 32-column chunks per epilogue warp
+  static_assert(SMEM_BYTES <= 227 * 1024, "shared memory per CTA");
+};
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
@@ -129,7 +134,7 @@ __device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
 }
 
 struct TileIdx {
-  int a_tile, r_tile, t;
+  int a_tile, r_tile, t, part;
 };
 // power-of-two scale S >= m (S = 1 for m = 0)
 __device__ __forceinline__ float pow2_scale(float m) {
@@ -147,10 +152,13 @@ __device__ __forceinline__ float pow2_scale(float m) {
 // a'-tiles; and the tensors of one input tile run side by side on
 // neighbouring CTAs, so the fused update's coefficient tables (one per field
 // kind) come from HBM about once per input tile.
+// PARTS parts per a'-tile, the part fastest.
+template <int PARTS>
 __device__ __forceinline__ TileIdx cta_tile(int u, int a_tiles, int count, int cta, int grid) {
   TileIdx x;
-  const int grp = cta + (u / a_tiles) * grid;
-  x.a_tile = u % a_tiles;
+  const int units = a_tiles * PARTS, grp = cta + (u / units) * grid, ug = u % units;
+  x.a_tile = ug / PARTS;
+  x.part = ug % PARTS;
   x.t = grp % count;
   x.r_tile = grp / count;
   return x;

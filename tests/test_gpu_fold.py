@@ -87,3 +87,71 @@ def test_strong_damping_takes_the_full_form(dt, sclet_lib):
         s.close()
     for f in range(2):
         assert _rel(out[0][f], out[1][f]) <= 1e-12, f
+
+
+# as EDGES, and halves of 64 and 65 (one epilogue column group full, one live
+# column more), 128 and 130 (one a'-tile full, a second of two live columns),
+# odd blocks, and block edges that are 0, 2 and odd modulo 4
+MIXED_EDGES = [4, 5, 6, 31, 68, 75, 124, 126, 252, 253, 256]
+
+
+@pytest.mark.parametrize("N", MIXED_EDGES)
+def test_mixed_folded_products(N, sclet_lib):
+    """One folded tensor-core product each way against FP64 sums of the
+    FP32-rounded input, at the bound the dense product is held to."""
+    sg = sclet_lib
+    s = sg.Solver(_params(sg, N, 1, 0), sg.MIXED)
+    n = s.n
+    a = np.random.default_rng(N).standard_normal((n, n, n)).astype(np.float32).astype(np.float64)
+    _, v, vi = cases.eigen_variant(n, 3)
+    for inverse, m in ((False, vi), (True, v)):
+        want = (a.reshape(-1, n) @ m.T).T.reshape(n, n, n)  # out[a', c, b]
+        assert _rel(s.mode_product(a, inverse), want) <= 2e-7, inverse
+    s.sync()
+    s.close()
+
+
+@pytest.mark.parametrize("N,nac,nch,etd2,dt", [(5, 2, 1, 1, 0.005), (31, 4, 1, 0, 0.005), (33, 3, 0, 1, 0.02),
+                                               (68, 1, 1, 0, 0.005), (126, 1, 0, 0, 0.005), (20, 2, 1, 0, 5.0)])
+def test_mixed_steps_are_no_further_from_fp64_than_the_general_path(N, nac, nch, etd2, dt, sclet_lib):
+    sg = sclet_lib
+    p = _params(sg, N, nac, nch, etd2, dt=dt, kk=(1.0, 0.7, 0.4))
+    n = N + 4
+    u0 = np.random.default_rng(N).uniform(-0.3, 0.3, size=(nac + nch, n, n, n))
+    u0[nac:] = 0.5 + 0.1 * u0[nac:]
+
+    def run(prec, basis):
+        s = sg.Solver(p, prec)
+        s.set_eigen(*basis)
+        s.set_fields(u0)
+        s.step(3)
+        u = s.get_fields()
+        s.sync()
+        s.close()
+        return u
+
+    exact = run(sg.FP64, cases.eigen_variant(n, 3))
+    fold, general = run(sg.MIXED, cases.eigen_variant(n, 3)), run(sg.MIXED, _swapped(n))
+    for f in range(nac + nch):
+        ef, eg = _rel(fold[f], exact[f]), _rel(general[f], exact[f])
+        # the two differ by chance where both are a few roundings of 2^-24
+        assert ef <= 1.5 * eg + 3e-8, (f, ef, eg)
+
+
+def test_basis_can_change_back_and_forth(sclet_lib):
+    """set_eigen switches the layout of the slice planes; nothing of one layout
+    may be left in the other's zero columns."""
+    sg = sclet_lib
+    p = _params(sg, 31, 2, 0)
+    u0 = np.random.default_rng(1).uniform(-0.3, 0.3, size=(2, 35, 35, 35))
+    out = []
+    s = sg.Solver(p, sg.MIXED)
+    for basis in (cases.eigen_variant(35, 3), _swapped(35), cases.eigen_variant(35, 3), _swapped(35)):
+        s.set_eigen(*basis)
+        s.set_fields(u0)
+        s.step(2)
+        out.append(s.get_fields())
+    s.sync()
+    s.close()
+    np.testing.assert_array_equal(out[0], out[2])
+    np.testing.assert_array_equal(out[1], out[3])
