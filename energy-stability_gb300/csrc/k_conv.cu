@@ -45,8 +45,9 @@ using tc::mbar_arrive;
 using tc::mbar_expect_tx;
 using tc::mbar_init;
 using tc::mbar_wait;
-using tc::mma_bf16;
-using tc::mma_commit;
+using tc::elect_one;
+using tc::mma_bf16_from;
+using tc::mma_commit_from;
 using tc::smem_desc;
 using tc::smem_u32;
 using tc::tmem_ld32;
@@ -107,7 +108,7 @@ __global__ void __launch_bounds__(THREADS, 1)
   uint8_t *wsm = base;                    // 27 tap tiles of weights
   uint8_t *asm_ = base + TAPS * WTILE;    // stages x 12 ny input runs
   const int stage_bytes = 12 * ny * box_bytes;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int N = g.N, Np = N + 2;
   const int per_plane = (N * Np + ROWS - 1) / ROWS;
   const int total = g.batch * N * per_plane;
@@ -170,59 +171,56 @@ __global__ void __launch_bounds__(THREADS, 1)
       mbar_wait(&w_bar, 0);
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      const uint32_t idesc = tc::idesc_bf16(ROWS, CH);
-      bool ok = mbar_wait(&w_bar, 0);
-      if (!ok) failed = 1;
+    // the warp runs the loop together, one lane issues (mma_bf16_from)
+    const bool issue = elect_one();
+    const uint32_t idesc = tc::idesc_bf16(ROWS, CH);
+    bool ok = __all_sync(0xffffffffu, mbar_wait(&w_bar, 0));
+    fence_after();
+    int it = 0;
+    // descriptors: constant high words; a tap adds its run and row offsets
+    // (16-byte units) to the low word's address field
+    const uint64_t da0 = smem_desc_lin(smem_u32(asm_), box_bytes, 128), dw0 = smem_desc(smem_u32(wsm));
+    const uint32_t a_hi = (uint32_t)(da0 >> 32), w_hi = (uint32_t)(dw0 >> 32), w_lo = (uint32_t)dw0;
+    const uint32_t run16 = (uint32_t)box_bytes >> 4;
+    for (int tile = blockIdx.x; ok && tile < total; tile += gridDim.x, it++) {
+      const int b = it % NACC, s = it % stages;
+      if (it >= NACC) ok = mbar_wait(&tempty_bar[b], ((it / NACC) & 1) ^ 1);
+      ok = __all_sync(0xffffffffu, ok && mbar_wait(&full_bar[s], (it / stages) & 1));
+      if (!ok) break;
       fence_after();
-      int it = 0;
-      const uint32_t w0 = smem_u32(wsm), a0 = smem_u32(asm_);
-      for (int tile = blockIdx.x; ok && tile < total && !*(volatile int *)&failed; tile += gridDim.x, it++) {
-        const int b = it % NACC;
-        if (it >= NACC && !mbar_wait(&tempty_bar[b], ((it / NACC) & 1) ^ 1)) {
-          failed = 1;
-          break;
-        }
-        const int s = it % stages;
-        if (!mbar_wait(&full_bar[s], (it / stages) & 1)) {
-          failed = 1;
-          break;
-        }
-        fence_after();
-        const uint32_t acc = tmem + (uint32_t)(b * CH);
-        const Tile ti = tile_of(tile, N, Np, per_plane);
-        // per stencil row dy: the run holding it (its offset in runs from the
-        // plane's first) and the row of the tap dx = -1 within that run
-        uint32_t rrun[3], rrow[3];
+      const uint32_t acc = tmem + (uint32_t)(b * CH);
+      const Tile ti = tile_of(tile, N, Np, per_plane);
+      const uint32_t a_lo = (uint32_t)da0 + (uint32_t)(s * stage_bytes >> 4);
+      // per stencil row dy: the run holding it (its offset in runs from the
+      // plane's first) and the row of the tap dx = -1 within that run
+      uint32_t rofs[3];
+#pragma unroll
+      for (int dy = 0; dy < 3; dy++) {
+        const uint32_t first = (uint32_t)(ti.s0 + (ny == 1 ? -Np : (dy - 1) * Np) - 1);
+        rofs[dy] = a_lo + (ny == 1 ? 0u : (uint32_t)(dy * 4) * run16) + (first & 7) + (ny == 1 ? (uint32_t)(dy * Np) : 0u);
+      }
+#pragma unroll
+      for (int dz = 0; dz < 3; dz++) {
+        const uint32_t pz = (uint32_t)(dz * ny * 4) * run16;
 #pragma unroll
         for (int dy = 0; dy < 3; dy++) {
-          const long long first = (long long)ti.s0 + (ny == 1 ? -Np : (dy - 1) * Np) - 1;
-          rrun[dy] = ny == 1 ? 0u : (uint32_t)(dy * 4);
-          rrow[dy] = (uint32_t)(first & 7) + (ny == 1 ? (uint32_t)(dy * Np) : 0u);
-        }
-        // descriptors of the stage's first run and of the first weight tile;
-        // a tap adds its run and row offsets (16-byte units) to the address
-        // field, which stays below 2^14 inside the shared memory
-        const uint64_t dab = smem_desc_lin(a0 + (uint32_t)(s * stage_bytes), box_bytes, 128);
-        const uint64_t dwb = smem_desc(w0);
-        const uint32_t run16 = (uint32_t)box_bytes >> 4;
 #pragma unroll
-        for (int tap = 0; tap < TAPS; tap++) {
-          const int dz = tap / 9, dy = (tap / 3) % 3, dx = tap % 3;  // each 0..2
+          for (int dx = 0; dx < 3; dx++) {
+            const int tap = dz * 9 + dy * 3 + dx;
 #pragma unroll
-          for (int ks = 0; ks < 2; ks++) {
-            const uint64_t da =
-                dab + (uint64_t)(((uint32_t)(dz * ny * 4 + 2 * ks) + rrun[dy]) * run16 + rrow[dy] + (uint32_t)dx);
-            const uint64_t dw = dwb + (uint64_t)((tap * WTILE + ks * 32) >> 4);
-            mma_bf16(acc, da, dw, idesc, (tap == 0 && ks == 0) ? 0u : 1u);
+            for (int ks = 0; ks < 2; ks++)
+              mma_bf16_from(issue, acc, rofs[dy] + pz + (uint32_t)(2 * ks) * run16 + (uint32_t)dx, a_hi,
+                            w_lo + (uint32_t)((tap * WTILE + ks * 32) >> 4), w_hi, idesc, (tap == 0 && ks == 0) ? 0u : 1u);
           }
         }
-        mma_commit(&empty_bar[s]);
-        mma_commit(&tfull_bar[b]);
       }
-      mma_commit(&done_bar);
-      if (!mbar_wait(&done_bar, 0)) failed = 1;
+      mma_commit_from(issue, &empty_bar[s]);
+      mma_commit_from(issue, &tfull_bar[b]);
+      ok = !__any_sync(0xffffffffu, *(volatile int *)&failed);
     }
+    if (!ok && lane == 0) failed = 1;
+    mma_commit_from(issue, &done_bar);
+    if (!mbar_wait(&done_bar, 0) && lane == 0) failed = 1;
   } else {
     const int q = warp & 3;
     const int row = q * 32 + lane;

@@ -105,7 +105,7 @@ __global__ void __launch_bounds__(THREADS, 1)
   __shared__ int failed;
 
   uint8_t *base = (uint8_t *)(((uintptr_t)smem_raw + SMEM_ALIGN - 1) & ~(uintptr_t)(SMEM_ALIGN - 1));
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const long long rows = (long long)g.n * g.n;
   constexpr int PARTS = FORM == 0 ? 1 : 2;
   const int h = FORM == 0 ? g.n : fold_half(g.n);  // outputs of one part
@@ -175,68 +175,62 @@ __global__ void __launch_bounds__(THREADS, 1)
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      // MMA issuer: 2 k-steps of 16 per stage, eleven terms each; (input
-      // slice, matrix slice, class) grouped by class, small classes first; the
-      // first term of each class at a tile's first k-step starts its
-      // accumulator.  The last a'-tile runs N = its rows rounded up to 16.
-      const int last_cols = h - (a_tiles - 1) * BN;
-      const uint32_t idesc_full = idesc_bf16(BM, BN);
-      const uint32_t idesc_last = idesc_bf16(BM, (last_cols + 15) / 16 * 16);
-      const int pairA[11] = {0, 3, 2, 1, 0, 2, 1, 0, 1, 0, 0};  // input slice
-      const int pairB[11] = {4, 0, 1, 2, 3, 0, 1, 2, 0, 1, 0};  // matrix slice
-      const int cls[11] = {3, 3, 3, 3, 3, 2, 2, 2, 1, 1, 0};
-      const bool last_two = h - (nkb - 1) * BK > 16;  // the last k-block needs both k-steps
-      int it = 0, j = 0;
-      for (int u = 0; u < mine && !*(volatile int *)&failed; u++, j++) {
-        const int b = j % NBUF;
-        // accumulator set b was last used by tile j - NBUF
-        if (j >= NBUF && !mbar_wait(&tempty_bar[b], ((j / NBUF) & 1) ^ 1)) {
-          failed = 1;
-          break;
-        }
+    // MMA issuer: 2 k-steps of 16 per stage, eleven terms each; (input slice,
+    // matrix slice, class) grouped by class, small classes first; the first
+    // term of each class at a tile's first k-step starts its accumulator.  The
+    // last a'-tile runs N = its rows rounded up to 16.  The warp runs the loop
+    // together, one lane issues (mma_bf16_from).
+    const bool issue = elect_one();
+    const int last_cols = h - (a_tiles - 1) * BN;
+    const uint32_t idesc_full = idesc_bf16(BM, BN);
+    const uint32_t idesc_last = idesc_bf16(BM, (last_cols + 15) / 16 * 16);
+    constexpr int pairA[11] = {0, 3, 2, 1, 0, 2, 1, 0, 1, 0, 0};  // input slice
+    constexpr int pairB[11] = {4, 0, 1, 2, 3, 0, 1, 2, 0, 1, 0};  // matrix slice
+    constexpr int cls[11] = {3, 3, 3, 3, 3, 2, 2, 2, 1, 1, 0};
+    const bool last_two = h - (nkb - 1) * BK > 16;  // the last k-block needs both k-steps
+    // descriptors: the high word is constant, the low word's address field
+    // (16-byte units) takes the stage, slice and k-step offsets
+    const uint64_t d0 = smem_desc(smem_u32(base));
+    const uint32_t hi = (uint32_t)(d0 >> 32), lo0 = (uint32_t)d0;
+    int it = 0;
+    bool ok = true;
+    for (int u = 0; u < mine && ok; u++) {
+      const int b = u % NBUF;
+      // accumulator set b was last used by tile u - NBUF
+      if (u >= NBUF) ok = __all_sync(0xffffffffu, mbar_wait(&tempty_bar[b], ((u / NBUF) & 1) ^ 1));
+      if (!ok) break;
+      fence_after();
+      const uint32_t acc = tmem + (uint32_t)(b * ACC_COLS);
+      const uint32_t idesc = (u % units) / PARTS == a_tiles - 1 ? idesc_last : idesc_full;
+      for (int kb = 0; kb < nkb; kb++, it++) {
+        const int s = it % STAGES;
+        ok = __all_sync(0xffffffffu, mbar_wait(&full_bar[s], (it / STAGES) & 1));
+        if (!ok) break;
         fence_after();
-        const uint32_t acc = tmem + (uint32_t)(b * ACC_COLS);
-        const uint32_t idesc = (u % units) / PARTS == a_tiles - 1 ? idesc_last : idesc_full;
-        bool ok = true;
-        for (int kb = 0; kb < nkb; kb++, it++) {
-          const int s = it % STAGES;
-          if (!mbar_wait(&full_bar[s], (it / STAGES) & 1)) {
-            ok = false;
-            break;
-          }
-          fence_after();
-          const uint32_t sa = smem_u32(base + s * STAGE_BYTES);
-          const uint32_t sb = sa + NP * PLANE_A;
+        const uint32_t la = lo0 + (uint32_t)(s * STAGE_BYTES >> 4), lb = la + (uint32_t)(NP * PLANE_A >> 4);
 #pragma unroll
-          for (int ks = 0; ks < BK / 16; ks++) {
-            // the last k-block's second k-step holds only zero columns when
-            // n mod 32 is in 1..16: skipped (adding zero products changes no
-            // accumulator)
-            if (ks > 0 && kb == nkb - 1 && !last_two) continue;
-            const uint32_t koff = ks * 32;
-            const bool first = (kb == 0 && ks == 0);
+        for (int ks = 0; ks < BK / 16; ks++) {
+          // the last k-block's second k-step holds only zero columns when
+          // h mod 32 is in 1..16: skipped (adding zero products changes no
+          // accumulator)
+          if (ks > 0 && kb == nkb - 1 && !last_two) continue;
+          const uint32_t first = (kb == 0 && ks == 0) ? 0u : 1u;
 #pragma unroll
-            for (int q = 0; q < 11; q++) {
-              const int pa = pairA[q], pb = pairB[q], w = cls[q];
-              const bool start = first && (q == 0 || q == 5 || q == 8 || q == 10);
-              uint64_t da = smem_desc(sa + pa * PLANE_A + koff);
-              uint64_t db = smem_desc(sb + pb * PLANE_B + koff);
-              mma_bf16(acc + (uint32_t)(w * BN), da, db, idesc, start ? 0u : 1u);
-            }
+          for (int q = 0; q < 11; q++) {
+            const bool start = q == 0 || q == 5 || q == 8 || q == 10;
+            mma_bf16_from(issue, acc + (uint32_t)(cls[q] * BN), la + (uint32_t)((pairA[q] * PLANE_A + ks * 32) >> 4), hi,
+                          lb + (uint32_t)((pairB[q] * PLANE_B + ks * 32) >> 4), hi, idesc, start ? first : 1u);
           }
-          mma_commit(&empty_bar[s]);
         }
-        if (!ok) {
-          failed = 1;
-          break;
-        }
-        mma_commit(&tfull_bar[b]);
+        mma_commit_from(issue, &empty_bar[s]);
       }
-      // every MMA issued so far must complete before the memory is freed
-      mma_commit(&done_bar);
-      if (!mbar_wait(&done_bar, 0)) failed = 1;
+      if (ok) mma_commit_from(issue, &tfull_bar[b]);
+      ok = ok && !__any_sync(0xffffffffu, *(volatile int *)&failed);
     }
+    if (!ok && lane == 0) failed = 1;
+    // every MMA issued so far must complete before the memory is freed
+    mma_commit_from(issue, &done_bar);
+    if (!mbar_wait(&done_bar, 0) && lane == 0) failed = 1;
   } else {
     // epilogue warps 2-9: TMEM lane quadrant q = warp % 4 holds input rows
     // q*32 .. q*32+31 of the tile, one per lane; the columns are the tile's

@@ -77,7 +77,7 @@ __global__ void __launch_bounds__(WG_THREADS, 1)
   __shared__ int failed;
 
   uint8_t *base = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int Np = N + 2, ny = gm.ny, stages = gm.stages;
   const int per_plane = (N * Np + ROWS - 1) / ROWS;
   const int total = batch * N * per_plane;
@@ -149,46 +149,44 @@ __global__ void __launch_bounds__(WG_THREADS, 1)
         for (int i = it - stages < 0 ? 0 : it - stages; i < it; i++) mbar_wait(&full_bar[i % stages], (i / stages) & 1);
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      const uint32_t idesc = idesc_bf16(ROWS, CH) | (1u << 15) | (1u << 16);  // both operands MN-major
-      const uint32_t a0 = smem_u32(base);
-      for (int it = 0; it < mine && !*(volatile int *)&failed; it++) {
-        const int grp = it / DRAIN;
-        if (it % DRAIN == 0 && grp > 0 && !mbar_wait(&acc_empty, (grp - 1) & 1)) {
-          failed = 1;
-          break;
-        }
-        const int s = it % stages;
-        if (!mbar_wait(&ready_bar[s], (it / stages) & 1)) {
-          failed = 1;
-          break;
-        }
-        fence_after();
-        const Tile ti = tile_of(blockIdx.x + it * gridDim.x, N, Np, per_plane);
-        const uint32_t sa = a0 + (uint32_t)(s * gm.stage_bytes);
-        const uint32_t goff = (uint32_t)(conv_at(N, ti.b, ti.zh, 0, ti.s0) & 7);
-        const uint64_t dg = smem_desc_lin(sa + g_off, 128, G_BYTES) + goff;
-        const uint64_t dx0 = smem_desc_lin(sa, 128, gm.box_bytes);
-        for (int dy = 0; dy < 3; dy++) {
-          // the run holding stencil row dy and the row of dx = -1 within it
-          const long long first = (long long)ti.s0 + (ny == 1 ? -Np : (dy - 1) * Np) - 1;
-          const uint32_t row = (uint32_t)(first & 7) + (ny == 1 ? (uint32_t)(dy * Np) : 0u);
-          const uint32_t run = ny == 1 ? 0u : (uint32_t)(dy * gm.row_bytes) >> 4;
+    // the warp runs the loop together, one lane issues (mma_bf16_from)
+    const bool issue = elect_one();
+    const uint32_t idesc = idesc_bf16(ROWS, CH) | (1u << 15) | (1u << 16);  // both operands MN-major
+    const uint64_t dg0 = smem_desc_lin(smem_u32(base) + g_off, 128, G_BYTES);
+    const uint64_t dx0 = smem_desc_lin(smem_u32(base), 128, gm.box_bytes);
+    const uint32_t g_hi = (uint32_t)(dg0 >> 32), x_hi = (uint32_t)(dx0 >> 32);
+    bool ok = true;
+    for (int it = 0; it < mine && ok; it++) {
+      const int grp = it / DRAIN, s = it % stages;
+      if (it % DRAIN == 0 && grp > 0) ok = mbar_wait(&acc_empty, (grp - 1) & 1);
+      ok = __all_sync(0xffffffffu, ok && mbar_wait(&ready_bar[s], (it / stages) & 1));
+      if (!ok) break;
+      fence_after();
+      const Tile ti = tile_of(blockIdx.x + it * gridDim.x, N, Np, per_plane);
+      const uint32_t st = (uint32_t)(s * gm.stage_bytes >> 4);
+      const uint32_t g_lo = (uint32_t)dg0 + st + (uint32_t)(conv_at(N, ti.b, ti.zh, 0, ti.s0) & 7);
+      const uint32_t first_tile = it % DRAIN == 0 ? 0u : 1u;
 #pragma unroll
-          for (int dx = 0; dx < 3; dx++) {
-            const uint32_t acc = tmem + (uint32_t)((dy * 3 + dx) * CH);
+      for (int dy = 0; dy < 3; dy++) {
+        // the run holding stencil row dy and the row of dx = -1 within it
+        const uint32_t first = (uint32_t)(ti.s0 + (ny == 1 ? -Np : (dy - 1) * Np) - 1);
+        const uint32_t x_lo = (uint32_t)dx0 + st + (ny == 1 ? 0u : (uint32_t)(dy * gm.row_bytes) >> 4) + (first & 7) +
+                              (ny == 1 ? (uint32_t)(dy * Np) : 0u);
 #pragma unroll
-            for (int ks = 0; ks < ROWS / 16; ks++)
-              mma_bf16(acc, dx0 + (uint64_t)(run + row + dx + ks * 16), dg + (uint64_t)(ks * 16), idesc,
-                       (it % DRAIN == 0 && ks == 0) ? 0u : 1u);
-          }
+        for (int dx = 0; dx < 3; dx++) {
+#pragma unroll
+          for (int ks = 0; ks < ROWS / 16; ks++)
+            mma_bf16_from(issue, tmem + (uint32_t)((dy * 3 + dx) * CH), x_lo + (uint32_t)(dx + ks * 16), x_hi,
+                          g_lo + (uint32_t)(ks * 16), g_hi, idesc, ks == 0 ? first_tile : 1u);
         }
-        mma_commit(&empty_bar[s]);
-        if (it % DRAIN == DRAIN - 1 || it == mine - 1) mma_commit(&acc_full);
       }
-      mma_commit(&done_bar);
-      if (!mbar_wait(&done_bar, 0)) failed = 1;
+      mma_commit_from(issue, &empty_bar[s]);
+      if (it % DRAIN == DRAIN - 1 || it == mine - 1) mma_commit_from(issue, &acc_full);
+      ok = !__any_sync(0xffffffffu, *(volatile int *)&failed);
     }
+    if (!ok && lane == 0) failed = 1;
+    mma_commit_from(issue, &done_bar);
+    if (!mbar_wait(&done_bar, 0) && lane == 0) failed = 1;
   } else if (warp == 2) {
     for (int it = 0; it < mine; it++) {
       const int s = it % stages;
