@@ -49,7 +49,7 @@
 // The folded forms (the default basis) halve the MMAs of a product and, with
 // the increment form, a field needs six products instead of nine.  Kernel time
 // of a step, dense and nine products before, now: 4 + 1 fields of 516^3
-// 52.8 -> 28.0 ms, of 196^3 1.64 -> 1.05 ms, 4 fields of 68^3 124 -> 85 us; the
+// 52.8 -> 24.6 ms, of 196^3 1.64 -> 0.96 ms, 4 fields of 68^3 124 -> 78 us; the
 // step's error against 64 bits fell from 2.2e-7 to 0.6e-7 (196^3, ten steps).
 // Warp 0 issues TMA, warp 1 issues MMAs (one elected thread each) and owns the
 // tensor memory (4 classes x 128 columns).  Warps 2-5 run the epilogue (TMEM
@@ -175,18 +175,16 @@ __global__ void __launch_bounds__(THREADS, 1)
       }
     }
   } else if (warp == 1) {
-    // MMA issuer: 2 k-steps of 16 per stage, eleven terms each; (input slice,
-    // matrix slice, class) grouped by class, small classes first; the first
-    // term of each class at a tile's first k-step starts its accumulator.  The
+    // MMA issuer: 2 k-steps of 16 per stage, eleven terms each, grouped by input
+    // slice so that each is read from shared memory once (the A collector): the
+    // operand reads, not the multiplications, bound MMAs of this shape.  The
+    // first term of each class at a tile's first k-step starts its accumulator.  The
     // last a'-tile runs N = its rows rounded up to 16.  The warp runs the loop
     // together, one lane issues (mma_bf16_from).
     const bool issue = elect_one();
     const int last_cols = h - (a_tiles - 1) * BN;
     const uint32_t idesc_full = idesc_bf16(BM, BN);
     const uint32_t idesc_last = idesc_bf16(BM, (last_cols + 15) / 16 * 16);
-    constexpr int pairA[11] = {0, 3, 2, 1, 0, 2, 1, 0, 1, 0, 0};  // input slice
-    constexpr int pairB[11] = {4, 0, 1, 2, 3, 0, 1, 2, 0, 1, 0};  // matrix slice
-    constexpr int cls[11] = {3, 3, 3, 3, 3, 2, 2, 2, 1, 1, 0};
     const bool last_two = h - (nkb - 1) * BK > 16;  // the last k-block needs both k-steps
     // descriptors: the high word is constant, the low word's address field
     // (16-byte units) takes the stage, slice and k-step offsets
@@ -215,12 +213,23 @@ __global__ void __launch_bounds__(THREADS, 1)
           // accumulator)
           if (ks > 0 && kb == nkb - 1 && !last_two) continue;
           const uint32_t first = (kb == 0 && ks == 0) ? 0u : 1u;
-#pragma unroll
-          for (int q = 0; q < 11; q++) {
-            const bool start = q == 0 || q == 5 || q == 8 || q == 10;
-            mma_bf16_from(issue, acc + (uint32_t)(cls[q] * BN), la + (uint32_t)((pairA[q] * PLANE_A + ks * 32) >> 4), hi,
-                          lb + (uint32_t)((pairB[q] * PLANE_B + ks * 32) >> 4), hi, idesc, start ? first : 1u);
-          }
+          auto term = [&](auto c, int pa, int pb, int cls, uint32_t keep) {
+            mma_bf16_from<decltype(c)::value>(issue, acc + (uint32_t)(cls * BN),
+                                              la + (uint32_t)((pa * PLANE_A + ks * 32) >> 4), hi,
+                                              lb + (uint32_t)((pb * PLANE_B + ks * 32) >> 4), hi, idesc, keep);
+          };
+          // (input slice, matrix slice, class)
+          term(Keep<A_FILL>(), 0, 4, 3, first);
+          term(Keep<A_USE>(), 0, 3, 3, 1u);
+          term(Keep<A_USE>(), 0, 2, 2, first);
+          term(Keep<A_USE>(), 0, 1, 1, first);
+          term(Keep<A_LAST>(), 0, 0, 0, first);
+          term(Keep<A_FILL>(), 1, 2, 3, 1u);
+          term(Keep<A_USE>(), 1, 1, 2, 1u);
+          term(Keep<A_LAST>(), 1, 0, 1, 1u);
+          term(Keep<A_FILL>(), 2, 1, 3, 1u);
+          term(Keep<A_LAST>(), 2, 0, 2, 1u);
+          term(Keep<A_DROP>(), 3, 0, 3, 1u);
         }
         mma_commit_from(issue, &empty_bar[s]);
       }

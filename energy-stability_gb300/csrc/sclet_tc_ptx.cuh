@@ -99,14 +99,29 @@ __device__ __forceinline__ bool elect_one() {
   asm volatile("{\n .reg .pred q;\n elect.sync _|q, 0xffffffff;\n selp.u32 %0, 1, 0, q;\n}\n" : "=r"(ok));
   return ok != 0;
 }
+// What becomes of the A operand: read and dropped, read and kept in the
+// collector, taken from the collector, taken from it for the last time.
+// Consecutive MMAs of one A operand read it from shared memory once.
+enum Collect { A_DROP, A_FILL, A_USE, A_LAST };
+template <Collect C>
+struct Keep {
+  static constexpr Collect value = C;
+};
+template <Collect C = A_DROP>
 __device__ __forceinline__ void mma_bf16_from(bool issue, uint32_t dtmem, uint32_t a_lo, uint32_t a_hi, uint32_t b_lo,
                                               uint32_t b_hi, uint32_t idesc, uint32_t acc) {
-  asm volatile(
-      "{\n .reg .pred p, q;\n .reg .b64 a, b;\n mov.b64 a, {%1, %2};\n mov.b64 b, {%3, %4};\n"
-      " setp.ne.b32 p, %6, 0;\n setp.ne.b32 q, %7, 0;\n"
-      " @q tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %5, p;\n}\n" ::"r"(dtmem),
-      "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(acc), "r"((uint32_t)issue)
-      : "memory");
+#define SCLET_MMA(MOD)                                                                                     \
+  asm volatile(                                                                                            \
+      "{\n .reg .pred p, q;\n .reg .b64 a, b;\n mov.b64 a, {%1, %2};\n mov.b64 b, {%3, %4};\n"            \
+      " setp.ne.b32 p, %6, 0;\n setp.ne.b32 q, %7, 0;\n"                                                   \
+      " @q tcgen05.mma.cta_group::1.kind::f16.collector::a::" MOD " [%0], a, b, %5, p;\n}\n" ::"r"(dtmem),  \
+      "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(acc), "r"((uint32_t)issue)               \
+      : "memory")
+  if (C == A_DROP) SCLET_MMA("discard");
+  else if (C == A_FILL) SCLET_MMA("fill");
+  else if (C == A_USE) SCLET_MMA("use");
+  else SCLET_MMA("lastuse");
+#undef SCLET_MMA
 }
 __device__ __forceinline__ void mma_commit_from(bool issue, uint64_t *bar) {
   asm volatile(
