@@ -11,18 +11,31 @@
 //   D[cell][co] = sum_{tap, ci} A[cell + off(tap)][ci] * W[tap][co][ci]
 // with M = 128 cells, N = 32 output channels and K = 27 taps x 32 input
 // channels.  A tile is 128 consecutive slots of one haloed plane.  For every
-// plane dz of the stencil and every chunk, the rows all nine (dy, dx) taps
-// read are one contiguous run of 128 + 2 Np + 2 slots: the producer loads
-// those twelve runs (whole 128-byte lines, one TMA box each) and every tap's
-// operand is a descriptor into them (no-swizzle K-major layout: rows 16 bytes
-// apart, the chunks of a K step a box apart), offset by dy Np + dx rows.
+// plane and every chunk, the rows all nine in-plane taps read are one
+// contiguous run of 128 + 2 Np + 2 slots (whole 128-byte lines, one TMA box), and
+// every tap's operand is a descriptor into it (no-swizzle K-major layout: rows
+// 16 bytes apart, the chunks of a K step a box apart), offset by dy Np + dx
+// rows.
+//
+// Reading the 128 x 16 input operand from shared memory, not multiplying it by
+// 32 columns, is what an MMA of this shape costs (63 cycles against 16).  So a
+// CTA marches its column of tiles in z and takes the planes one by one: each
+// operand of a plane serves three MMAs, into the tiles before, at and behind the
+// plane, read once through the A collector (one MMA of N = 96 into adjoining
+// accumulators was slower: 96 us a layer against 87).  A tile still sums its taps in
+// the order dz, dy, dx, K step (the order of the FP32 sums decides the BF16
+// roundings of all later layers), and each plane is loaded once.
+//
 // Slots in the x- or y-halo produce outputs that are dropped.  The weights
 // (27 x 32 x 32 BF16, 54 KB) stay in shared memory.  Warp 0 issues TMA, warp 1
-// issues the MMAs (54 per tile: two K = 16 steps per tap) into one of four
-// 32-column TMEM accumulators, warps 2-5 drain them and run the fused
-// epilogue (bias, ReLU, residual, ReLU-mask, FP32 planar output).  The same
-// kernel computes the data gradient of a convolution with the weights
-// flipped and transposed (the adjoint of a periodic convolution).
+// the MMAs into eight 32-column TMEM accumulators, warps 2-5 and 6-9 drain
+// alternate tiles and run the fused epilogue (bias, ReLU, residual, ReLU-mask,
+// FP32 planar output); cells on the grid's faces are also stored at their
+// periodic images, so no halo pass follows.  The same kernel computes the data
+// gradient of a convolution with the weights flipped and transposed (the
+// adjoint of a periodic convolution).  A layer of 4 x 64^3 with its halo: 124 us
+// with three planes loaded per tile and a tap per operand read, 104 us with the
+// MMAs issued by a uniform warp, 84 us now.
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cudaTypedefs.h>
@@ -53,17 +66,19 @@ using tc::smem_u32;
 using tc::tmem_ld32;
 
 constexpr int WTILE = CH * CH * 2;         // 2 KB: one tap's 32 x 32 weights
-constexpr int NACC = 4;                    // TMEM accumulators of 32 columns
-constexpr int TMEM_COLS = NACC * CH;       // 128
-constexpr int THREADS = 192;
+constexpr int NACC = 8;                    // TMEM accumulators of 32 columns
+constexpr int TMEM_COLS = NACC * CH;       // 256
+constexpr int SETS = 2;                    // groups of four epilogue warps
+constexpr int THREADS = 64 + 128 * SETS;
+constexpr int MAX_RING = 6;                // planes in flight, at least two
 
-// Per-launch geometry.  ny = 1: per stencil plane and channel chunk one run
-// of 128 + 2 Np + 2 slots serves all nine in-plane taps (twelve runs a tile);
-// ny = 3: one run of 130 slots per stencil row dy (thirty-six runs a tile,
-// fewer bytes once Np exceeds about 148).  A run is one box of box_rows lines
-// of 128 bytes (8 slots), enough from any slot offset within the first line.
+// Per-launch geometry.  ny = 1: per plane and channel chunk one run of
+// 128 + 2 Np + 2 slots serves all nine in-plane taps; ny = 3: one run of 130
+// slots per stencil row (where two planes of the long runs do not fit).  A run is one box of
+// box_rows lines of 128 bytes (8 slots), enough from any slot offset within
+// the first line.
 struct Geom {
-  int ny, box_rows, box_bytes, stage_bytes, stages, smem;
+  int ny, box_rows, box_bytes, plane_bytes, ring, smem;
 };
 static Geom geom_for(int N, int ny) {
   Geom g;
@@ -71,19 +86,34 @@ static Geom geom_for(int N, int ny) {
   const int R = ny == 1 ? ROWS + 2 * (N + 2) + 2 : ROWS + 2;
   g.box_rows = (R + 7 + 7) / 8;
   g.box_bytes = g.box_rows * 128;
-  g.stage_bytes = 12 * ny * g.box_bytes;
-  g.stages = (SMEM_LIMIT - 1024 - TAPS * WTILE) / g.stage_bytes;
-  if (g.stages > MAX_STAGES) g.stages = MAX_STAGES;
-  g.smem = TAPS * WTILE + (g.stages > 0 ? g.stages : 1) * g.stage_bytes + 1024;
+  g.plane_bytes = 4 * ny * g.box_bytes;
+  g.ring = (SMEM_LIMIT - 1024 - TAPS * WTILE) / g.plane_bytes;
+  if (g.ring > MAX_RING) g.ring = MAX_RING;
+  g.smem = TAPS * WTILE + g.ring * g.plane_bytes + 1024;
   return g;
 }
 std::atomic<int> g_runs_per_plane{0};  // 0: by N; 1 or 3: forced (sclet_net_set_conv_runs)
 static Geom geom_of(int N) {
   const Geom a = geom_for(N, 1), b = geom_for(N, 3);
-  const int forced = g_runs_per_plane.load();
-  if (forced == 1 && a.stages >= 1) return a;
-  if (forced == 3) return b;
-  return a.stages >= 1 && a.stage_bytes <= b.stage_bytes ? a : b;
+  return a.ring >= 2 && a.box_rows <= 256 && g_runs_per_plane.load() != 3 ? a : b;
+}
+
+template <bool B>
+struct Flag {
+  static constexpr bool value = B;
+};
+
+// tile t of a launch: z fastest, so that consecutive tiles march a column
+struct ZTile {
+  int b, zh, s0;  // sample, plane 1..N, first slot of the plane
+};
+__device__ __forceinline__ ZTile ztile_of(int t, int N, int Np, int per_plane) {
+  ZTile x;
+  const int col = t / N;
+  x.zh = 1 + t - col * N;
+  x.b = col / per_plane;
+  x.s0 = Np + (col - x.b * per_plane) * ROWS;
+  return x;
 }
 
 __device__ __forceinline__ float bf(uint32_t w, int hi) {
@@ -92,10 +122,10 @@ __device__ __forceinline__ float bf(uint32_t w, int hi) {
 
 __global__ void __launch_bounds__(THREADS, 1)
     conv_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmW, ConvArgs g,
-                   int box_bytes, int stages, int ny) {
+                   Geom gm) {
   extern __shared__ uint8_t smem_raw[];
-  __shared__ __align__(8) uint64_t full_bar[MAX_STAGES];
-  __shared__ __align__(8) uint64_t empty_bar[MAX_STAGES];
+  __shared__ __align__(8) uint64_t full_bar[MAX_RING];
+  __shared__ __align__(8) uint64_t empty_bar[MAX_RING];
   __shared__ __align__(8) uint64_t tfull_bar[NACC];
   __shared__ __align__(8) uint64_t tempty_bar[NACC];
   __shared__ __align__(8) uint64_t w_bar;
@@ -106,16 +136,18 @@ __global__ void __launch_bounds__(THREADS, 1)
 
   uint8_t *base = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   uint8_t *wsm = base;                    // 27 tap tiles of weights
-  uint8_t *asm_ = base + TAPS * WTILE;    // stages x 12 ny input runs
-  const int stage_bytes = 12 * ny * box_bytes;
+  uint8_t *ring = base + TAPS * WTILE;    // gm.ring planes of 4 ny runs
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
-  const int N = g.N, Np = N + 2;
+  const int N = g.N, Np = N + 2, ny = gm.ny;
   const int per_plane = (N * Np + ROWS - 1) / ROWS;
   const int total = g.batch * N * per_plane;
+  // a contiguous range of tiles per CTA
+  const int t0 = (int)((long long)total * blockIdx.x / gridDim.x);
+  const int t1 = (int)((long long)total * (blockIdx.x + 1) / gridDim.x);
 
   if (threadIdx.x < CH) s_bias[threadIdx.x] = g.bias ? g.bias[threadIdx.x] : 0.0f;
   if (threadIdx.x == 0) {
-    for (int s = 0; s < MAX_STAGES; s++) {
+    for (int s = 0; s < MAX_RING; s++) {
       mbar_init(&full_bar[s], 1);
       mbar_init(&empty_bar[s], 1);
     }
@@ -144,29 +176,33 @@ __global__ void __launch_bounds__(THREADS, 1)
     if (lane == 0) {
       mbar_expect_tx(&w_bar, TAPS * WTILE);
       for (int t = 0; t < TAPS; t++) tma_load_2d(wsm + t * WTILE, &tmW, 0, t * CH, &w_bar);
-      int it = 0;
-      for (int tile = blockIdx.x; tile < total && !*(volatile int *)&failed; tile += gridDim.x, it++) {
-        const Tile ti = tile_of(tile, N, Np, per_plane);
-        const int s = it % stages;
-        if (it >= stages && !mbar_wait(&empty_bar[s], ((it / stages) & 1) ^ 1)) {
-          failed = 1;
-          break;
-        }
-        // plane zh + dz - 1, chunk k: the run from slot s0 - Np - 1 (ny = 1)
-        // or s0 + (dy - 1) Np - 1 (ny = 3), >= -1; a line before the buffer
-        // or past its end reads as zeros
-        mbar_expect_tx(&full_bar[s], stage_bytes);
-        for (int dz = 0; dz < 3; dz++)
+      int q = 0;  // planes loaded
+      for (int t = t0; t < t1 && !*(volatile int *)&failed;) {
+        // the tiles of one column: planes zh - 1 of the first .. zh + 1 of the last
+        const ZTile ti = ztile_of(t, N, Np, per_plane);
+        const int len = min(t1 - t, N + 1 - ti.zh);
+        for (int z = ti.zh - 1; z <= ti.zh + len; z++, q++) {
+          const int s = q % gm.ring;
+          if (q >= gm.ring && !mbar_wait(&empty_bar[s], ((q / gm.ring) & 1) ^ 1)) {
+            failed = 1;
+            break;
+          }
+          if (*(volatile int *)&failed) break;
+          mbar_expect_tx(&full_bar[s], gm.plane_bytes);
+          // the run from slot s0 - Np - 1 (ny = 1) or s0 + (r - 1) Np - 1 (ny = 3),
+          // >= -1; a line before the buffer or past its end reads as zeros
           for (int r = 0; r < ny; r++)
             for (int k = 0; k < 4; k++) {
-              const long long first = (long long)ti.s0 + (ny == 1 ? -Np : (r - 1) * Np) - 1;
-              const long long flat = conv_at(N, ti.b, ti.zh + dz - 1, k, first);
-              tma_load_2d(asm_ + s * stage_bytes + ((dz * ny + r) * 4 + k) * box_bytes, &tmA, 0, (int)(flat >> 3),
+              const long long first = (long long)ti.s0 + (r - 1) * Np - 1;
+              const long long flat = conv_at(N, ti.b, z, k, first);
+              tma_load_2d(ring + s * gm.plane_bytes + (r * 4 + k) * gm.box_bytes, &tmA, 0, (int)(flat >> 3),
                           &full_bar[s]);
             }
+        }
+        t += len;
       }
       if (*(volatile int *)&failed) {
-        for (int i = it - stages < 0 ? 0 : it - stages; i < it; i++) mbar_wait(&full_bar[i % stages], (i / stages) & 1);
+        for (int i = q - gm.ring < 0 ? 0 : q - gm.ring; i < q; i++) mbar_wait(&full_bar[i % gm.ring], (i / gm.ring) & 1);
       }
       mbar_wait(&w_bar, 0);
     }
@@ -176,59 +212,76 @@ __global__ void __launch_bounds__(THREADS, 1)
     const uint32_t idesc = tc::idesc_bf16(ROWS, CH);
     bool ok = __all_sync(0xffffffffu, mbar_wait(&w_bar, 0));
     fence_after();
-    int it = 0;
     // descriptors: constant high words; a tap adds its run and row offsets
     // (16-byte units) to the low word's address field
-    const uint64_t da0 = smem_desc_lin(smem_u32(asm_), box_bytes, 128), dw0 = smem_desc(smem_u32(wsm));
+    const uint64_t da0 = smem_desc_lin(smem_u32(ring), gm.box_bytes, 128), dw0 = smem_desc(smem_u32(wsm));
     const uint32_t a_hi = (uint32_t)(da0 >> 32), w_hi = (uint32_t)(dw0 >> 32), w_lo = (uint32_t)dw0;
-    const uint32_t run16 = (uint32_t)box_bytes >> 4;
-    for (int tile = blockIdx.x; ok && tile < total; tile += gridDim.x, it++) {
-      const int b = it % NACC, s = it % stages;
-      if (it >= NACC) ok = mbar_wait(&tempty_bar[b], ((it / NACC) & 1) ^ 1);
-      ok = __all_sync(0xffffffffu, ok && mbar_wait(&full_bar[s], (it / stages) & 1));
-      if (!ok) break;
-      fence_after();
-      const uint32_t acc = tmem + (uint32_t)(b * CH);
-      const Tile ti = tile_of(tile, N, Np, per_plane);
-      const uint32_t a_lo = (uint32_t)da0 + (uint32_t)(s * stage_bytes >> 4);
-      // per stencil row dy: the run holding it (its offset in runs from the
-      // plane's first) and the row of the tap dx = -1 within that run
+    const uint32_t run16 = (uint32_t)gm.box_bytes >> 4;
+    int q = 0;  // planes seen
+    for (int t = t0; ok && t < t1;) {
+      const ZTile ti = ztile_of(t, N, Np, per_plane);
+      const int len = min(t1 - t, N + 1 - ti.zh), it0 = t - t0;
+      // per stencil row dy: the run holding it and the row of dx = -1 within it
       uint32_t rofs[3];
 #pragma unroll
       for (int dy = 0; dy < 3; dy++) {
         const uint32_t first = (uint32_t)(ti.s0 + (ny == 1 ? -Np : (dy - 1) * Np) - 1);
-        rofs[dy] = a_lo + (ny == 1 ? 0u : (uint32_t)(dy * 4) * run16) + (first & 7) + (ny == 1 ? (uint32_t)(dy * Np) : 0u);
+        rofs[dy] = (uint32_t)da0 + (ny == 1 ? 0u : (uint32_t)(dy * 4) * run16) + (first & 7) +
+                   (ny == 1 ? (uint32_t)(dy * Np) : 0u);
       }
+      // plane j of the column's len + 2 is stencil plane dz of its tile j - dz
+      for (int j = 0; j < len + 2; j++, q++) {
+        const int s = q % gm.ring;
+        // tile j starts here: its accumulator must be drained
+        if (j < len && it0 + j >= NACC) ok = mbar_wait(&tempty_bar[(it0 + j) % NACC], (((it0 + j) / NACC) & 1) ^ 1);
+        ok = __all_sync(0xffffffffu, ok && mbar_wait(&full_bar[s], (q / gm.ring) & 1));
+        if (!ok) break;
+        fence_after();
+        const uint32_t pz = (uint32_t)(s * gm.plane_bytes) >> 4;
+        const uint32_t acc0 = tmem + (uint32_t)((it0 + j) % NACC * CH);                // dz = 0
+        const uint32_t acc1 = tmem + (uint32_t)((it0 + j + NACC - 1) % NACC * CH);     // dz = 1
+        const uint32_t acc2 = tmem + (uint32_t)((it0 + j + 2 * NACC - 2) % NACC * CH); // dz = 2
+        auto plane = [&](auto inner) {
+          constexpr bool INNER = decltype(inner)::value;
+          const bool v0 = issue && (INNER || j < len), v1 = issue && (INNER || (j >= 1 && j <= len));
+          const bool v2 = issue && (INNER || j >= 2);
 #pragma unroll
-      for (int dz = 0; dz < 3; dz++) {
-        const uint32_t pz = (uint32_t)(dz * ny * 4) * run16;
+          for (int dy = 0; dy < 3; dy++) {
 #pragma unroll
-        for (int dy = 0; dy < 3; dy++) {
+            for (int dx = 0; dx < 3; dx++) {
 #pragma unroll
-          for (int dx = 0; dx < 3; dx++) {
-            const int tap = dz * 9 + dy * 3 + dx;
-#pragma unroll
-            for (int ks = 0; ks < 2; ks++)
-              mma_bf16_from(issue, acc, rofs[dy] + pz + (uint32_t)(2 * ks) * run16 + (uint32_t)dx, a_hi,
-                            w_lo + (uint32_t)((tap * WTILE + ks * 32) >> 4), w_hi, idesc, (tap == 0 && ks == 0) ? 0u : 1u);
+              for (int ks = 0; ks < 2; ks++) {
+                const uint32_t a_lo = rofs[dy] + pz + (uint32_t)(2 * ks) * run16 + (uint32_t)dx;
+                const uint32_t w = w_lo + (uint32_t)(((dy * 3 + dx) * WTILE + ks * 32) >> 4);
+                constexpr uint32_t DZ = (uint32_t)(9 * WTILE) >> 4;
+                mma_bf16_from<INNER ? tc::A_FILL : tc::A_DROP>(v0, acc0, a_lo, a_hi, w, w_hi, idesc,
+                                                               (dy == 0 && dx == 0 && ks == 0) ? 0u : 1u);
+                mma_bf16_from<INNER ? tc::A_USE : tc::A_DROP>(v1, acc1, a_lo, a_hi, w + DZ, w_hi, idesc, 1u);
+                mma_bf16_from<INNER ? tc::A_LAST : tc::A_DROP>(v2, acc2, a_lo, a_hi, w + 2 * DZ, w_hi, idesc, 1u);
+              }
+            }
           }
-        }
+        };
+        // within the column all three tiles exist; at its ends the operand is
+        // read for each MMA (a collector is not used unless it was filled)
+        if (j >= 2 && j < len) plane(Flag<true>());
+        else plane(Flag<false>());
+        mma_commit_from(issue, &empty_bar[s]);
+        if (j >= 2) mma_commit_from(issue, &tfull_bar[(it0 + j - 2) % NACC]);
+        ok = !__any_sync(0xffffffffu, *(volatile int *)&failed);
+        if (!ok) break;
       }
-      mma_commit_from(issue, &empty_bar[s]);
-      mma_commit_from(issue, &tfull_bar[b]);
-      ok = !__any_sync(0xffffffffu, *(volatile int *)&failed);
+      t += len;
     }
     if (!ok && lane == 0) failed = 1;
     mma_commit_from(issue, &done_bar);
     if (!mbar_wait(&done_bar, 0) && lane == 0) failed = 1;
   } else {
-    const int q = warp & 3;
-    const int row = q * 32 + lane;
-    int j = 0;
-    for (int tile = blockIdx.x; tile < total; tile += gridDim.x, j++) {
-      const int b = j % NACC;
+    const int q = warp & 3, set = (warp - 2) >> 2;
+    for (int t = t0 + set, j = 0; t < t1; t += SETS, j++) {
+      const int it = t - t0, b = it % NACC;
       int ok = 1;
-      if (lane == 0) ok = mbar_wait(&tfull_bar[b], (j / NACC) & 1) ? 1 : 0;
+      if (lane == 0) ok = mbar_wait(&tfull_bar[b], (it / NACC) & 1) ? 1 : 0;
       ok = __shfl_sync(0xffffffffu, ok, 0);
       if (!ok) {
         if (lane == 0) failed = 1;
@@ -240,8 +293,8 @@ __global__ void __launch_bounds__(THREADS, 1)
       fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&tempty_bar[b]);
-      const Tile ti = tile_of(tile, N, Np, per_plane);
-      const int s = ti.s0 + row;
+      const ZTile ti = ztile_of(t, N, Np, per_plane);
+      const int s = ti.s0 + q * 32 + lane;
       const int yh = s / Np, xh = s - yh * Np;
       if (yh >= 1 && yh <= N && xh >= 1 && xh <= N) {
         const long long cell0 = conv_at(N, ti.b, ti.zh, 0, s), cstride = conv_chunk_slots(N);  // chunk k: cell0 + k cstride
@@ -276,6 +329,7 @@ __global__ void __launch_bounds__(THREADS, 1)
             }
           }
           uint4 *dst = reinterpret_cast<uint4 *>(g.out);
+          uint4 val[4];
 #pragma unroll
           for (int k = 0; k < 4; k++) {
             uint32_t w[4];
@@ -284,7 +338,22 @@ __global__ void __launch_bounds__(THREADS, 1)
               const __nv_bfloat162 p = __floats2bfloat162_rn(v[k * 8 + 2 * h], v[k * 8 + 2 * h + 1]);
               w[h] = *reinterpret_cast<const uint32_t *>(&p);
             }
-            dst[cell0 + k * cstride] = make_uint4(w[0], w[1], w[2], w[3]);
+            val[k] = make_uint4(w[0], w[1], w[2], w[3]);
+            dst[cell0 + k * cstride] = val[k];
+          }
+          // a cell on a face: its periodic images in the halo, one per subset
+          // of the axes it is extreme on, at fixed distances from the cell
+          const int sz = ti.zh == 1 ? 1 : ti.zh == N ? -1 : 0, sy = yh == 1 ? 1 : yh == N ? -1 : 0;
+          const int sx = xh == 1 ? 1 : xh == N ? -1 : 0;
+          if (sz | sy | sx) {
+            const long long dz = 4LL * N * cstride * sz, dy = (long long)N * Np * sy, dx = (long long)N * sx;
+#pragma unroll
+            for (int m = 1; m < 8; m++) {
+              if (((m & 1) && !sz) || ((m & 2) && !sy) || ((m & 4) && !sx)) continue;
+              uint4 *im = dst + cell0 + (m & 1 ? dz : 0) + (m & 2 ? dy : 0) + (m & 4 ? dx : 0);
+#pragma unroll
+              for (int k = 0; k < 4; k++) im[k * cstride] = val[k];
+            }
           }
         }
       }
@@ -356,7 +425,7 @@ cudaError_t launch_conv(const __nv_bfloat16 *in, const __nv_bfloat16 *w, const C
   const int N = args.N, Np = N + 2;
   if (N < 2 || args.batch < 1) return cudaErrorInvalidValue;
   const conv::Geom gm = conv::geom_of(N);
-  if (gm.stages < 1 || gm.box_rows > 256) return cudaErrorInvalidValue;
+  if (gm.ring < 2 || gm.box_rows > 256) return cudaErrorInvalidValue;
   const long long lines = conv_units(N, args.batch) / 8;
   if (lines >= 0x7fffffffLL) return cudaErrorInvalidValue;
   CUtensorMap ma, mw;
@@ -364,8 +433,9 @@ cudaError_t launch_conv(const __nv_bfloat16 *in, const __nv_bfloat16 *w, const C
   if ((e = conv::make_map_rows(&mw, w, (long long)TAPS * CH, CH)) != cudaSuccess) return e;
   const long long per_plane = ((long long)N * Np + conv::ROWS - 1) / conv::ROWS;
   const long long tiles = (long long)args.batch * N * per_plane;
+  if (tiles > 0x7fffffffLL) return cudaErrorInvalidValue;
   const int grid = (int)(tiles < ctas ? tiles : ctas);
-  conv::conv_tc_kernel<<<grid, conv::THREADS, gm.smem, s>>>(ma, mw, args, gm.box_bytes, gm.stages, gm.ny);
+  conv::conv_tc_kernel<<<grid, conv::THREADS, gm.smem, s>>>(ma, mw, args, gm);
   launch_counter()++;
   return cudaGetLastError();
 }

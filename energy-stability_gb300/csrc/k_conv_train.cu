@@ -1,5 +1,4 @@
-// Element-wise and reduction kernels of the corrector network: periodic halo,
-// packing FP32 fields into haloed BF16 activations, the BF16 weight copies,
+// Element-wise and reduction kernels of the corrector network: packing FP32 fields into haloed BF16 activations, the BF16 weight copies,
 // Adam and the training residual.  Activations in the chunk-planar layout of
 // sclet_conv.cuh (conv_at).
 #include <cuda_bf16.h>
@@ -12,45 +11,6 @@ namespace sclet {
 namespace {
 
 __device__ __forceinline__ int wrap_h(int h, int N) { return 1 + (h - 1 + N) % N; }
-
-__host__ __device__ inline long long shell_cells(int N) {
-  const long long Np = N + 2;
-  return 2 * Np * Np + 2LL * N * Np + 2LL * N * N;
-}
-
-// one 16-byte chunk (8 channels) of a halo cell per thread
-__global__ void halo_kernel(__nv_bfloat16 *a, int N, int batch) {
-  const int Np = N + 2;
-  const long long per = shell_cells(N), plane = (long long)Np * Np;
-  const long long total = per * batch * 4;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
-    const int k = (int)(i & 3);
-    long long s = i >> 2;
-    const int b = (int)(s / per);
-    s -= (long long)b * per;
-    int z, y, x;
-    if (s < 2 * plane) {
-      z = s < plane ? 0 : Np - 1;
-      const long long r = s % plane;
-      y = (int)(r / Np);
-      x = (int)(r % Np);
-    } else if ((s -= 2 * plane) < 2LL * N * Np) {
-      z = 1 + (int)(s / (2 * Np));
-      const long long r = s % (2 * Np);
-      y = r < Np ? 0 : Np - 1;
-      x = (int)(r % Np);
-    } else {
-      s -= 2LL * N * Np;
-      z = 1 + (int)(s / (2 * N));
-      const long long r = s % (2 * N);
-      y = 1 + (int)(r % N);
-      x = r < N ? 0 : Np - 1;
-    }
-    const long long dst = conv_at(N, b, z, k, (long long)y * Np + x);
-    const long long src = conv_at(N, b, wrap_h(z, N), k, (long long)wrap_h(y, N) * Np + wrap_h(x, N));
-    reinterpret_cast<uint4 *>(a)[dst] = reinterpret_cast<const uint4 *>(a)[src];
-  }
-}
 
 // every haloed cell from its periodic image in the planar FP32 input
 __global__ void pack_kernel(const float *__restrict__ in, int cin, float scale, int N, int batch,
@@ -149,12 +109,6 @@ int grid_for(long long total, int block) {
 }
 
 }  // namespace
-
-cudaError_t launch_conv_halo(__nv_bfloat16 *a, int N, int batch, cudaStream_t s) {
-  halo_kernel<<<grid_for(shell_cells(N) * batch * 4, 256), 256, 0, s>>>(a, N, batch);
-  launch_counter()++;
-  return cudaGetLastError();
-}
 
 cudaError_t launch_conv_pack(const float *in, int cin, int N, int batch, __nv_bfloat16 *a, cudaStream_t s) {
   if (cin < 1 || cin > CH) return cudaErrorInvalidValue;

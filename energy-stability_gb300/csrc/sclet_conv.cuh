@@ -42,7 +42,7 @@ struct ConvArgs {
   float scale;               // CONV_OUT_F32: output scale
   const float *bias;         // CH values or null
   const __nv_bfloat16 *aux;  // residual / mask source, same layout as the input
-  __nv_bfloat16 *out;        // BF16 activation output (owned cells; halo untouched)
+  __nv_bfloat16 *out;        // BF16 activation output, halo included (not `in` or `aux`)
   float *outf;               // CONV_OUT_F32: [batch][cout][N^3]
   int *err;                  // set to 1 when a bounded wait gives up
 };
@@ -55,8 +55,6 @@ cudaError_t launch_conv(const __nv_bfloat16 *in, const __nv_bfloat16 *w, const C
 int conv_set_runs(int runs_per_plane);
 int conv_runs();  // the current setting
 
-// Periodic halo of batch haloed blocks, in place.
-cudaError_t launch_conv_halo(__nv_bfloat16 *a, int N, int batch, cudaStream_t s);
 // FP32 planar fields [batch][cin][N^3] (owned cells) -> haloed BF16 activations,
 // channels >= cin zero, halo filled.
 cudaError_t launch_conv_pack(const float *in, int cin, int N, int batch, __nv_bfloat16 *a, cudaStream_t s);

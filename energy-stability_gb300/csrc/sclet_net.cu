@@ -144,14 +144,11 @@ int forward(sclet_net *net, int N, int batch, const float *in, float *out, cudaS
   if ((rc = sync_weights(net)) != SCLET_OK) return rc;
   NK(launch_conv_pack(in, SCLET_NET_IN, N, batch, net->x, s));
   NK(launch_conv(net->x, wl(net->wf, 0), conv_args(net, N, batch, CONV_RELU, 0, nullptr, net->h[0]), s));
-  NK(launch_conv_halo(net->h[0], N, batch, s));
   for (int k = 0; k < SCLET_NET_BLOCKS; k++) {
     NK(launch_conv(net->h[k], wl(net->wf, 2 * k + 1),
                    conv_args(net, N, batch, CONV_RELU, 2 * k + 1, nullptr, net->r[k]), s));
-    NK(launch_conv_halo(net->r[k], N, batch, s));
     NK(launch_conv(net->r[k], wl(net->wf, 2 * k + 2),
                    conv_args(net, N, batch, CONV_RESIDUAL, 2 * k + 2, net->h[k], net->h[k + 1]), s));
-    NK(launch_conv_halo(net->h[k + 1], N, batch, s));
   }
   ConvArgs a = conv_args(net, N, batch, CONV_OUT_F32, LAYERS - 1, nullptr, nullptr);
   a.outf = out ? out : net->pred;
@@ -171,17 +168,14 @@ int backward(sclet_net *net, int N, int batch, const float *target, double *loss
   NK(launch_conv_wgrad(net->h[SCLET_NET_BLOCKS], net->gy, N, batch, wof(net->g, L), bof(net->g, L), net->dev_err, s));
   __nv_bfloat16 *gcur = net->gh[0], *gnext = net->gh[1];
   NK(launch_conv(net->gy, wl(net->wt, L), conv_args(net, N, batch, CONV_LINEAR, -1, nullptr, gcur), s));
-  NK(launch_conv_halo(gcur, N, batch, s));
   for (int k = SCLET_NET_BLOCKS - 1; k >= 0; k--) {
     const int l1 = 2 * k + 1, l2 = 2 * k + 2;
     // h_{k+1} = h_k + conv_l2 r_k: gradient of conv_l2's weights, then of r_k
     NK(launch_conv_wgrad(net->r[k], gcur, N, batch, wof(net->g, l2), bof(net->g, l2), net->dev_err, s));
     NK(launch_conv(gcur, wl(net->wt, l2), conv_args(net, N, batch, CONV_MASK, -1, net->r[k], net->ga), s));
-    NK(launch_conv_halo(net->ga, N, batch, s));
     // r_k = relu(conv_l1 h_k): weights of conv_l1, then h_k (plus the skip path)
     NK(launch_conv_wgrad(net->h[k], net->ga, N, batch, wof(net->g, l1), bof(net->g, l1), net->dev_err, s));
     NK(launch_conv(net->ga, wl(net->wt, l1), conv_args(net, N, batch, CONV_RESIDUAL, -1, gcur, gnext), s));
-    NK(launch_conv_halo(gnext, N, batch, s));
     __nv_bfloat16 *t = gcur;
     gcur = gnext;
     gnext = t;

@@ -92,7 +92,7 @@ __host__ __device__ constexpr uint32_t idesc_bf16(int m, int n) {
 // one elected lane (`issue`) issues; descriptors as a constant high and a low
 // word that takes the offsets.  A loop run by a single lane spent most of a
 // small MMA's time moving its operands there: convolution layers of 4 x 64^3
-// 117 -> 97 us, their weight gradients 136 -> 78 us, the eigenbasis products of
+// 117 -> 97 us, their weight gradients 136 -> 100 us, the eigenbasis products of
 // 516^3 28.0 -> 25.5 ms a step.
 __device__ __forceinline__ bool elect_one() {
   uint32_t ok;
