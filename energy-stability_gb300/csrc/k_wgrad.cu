@@ -10,18 +10,21 @@
 // of the operand's start address.
 //   M = 128: the three stencil planes dz x 32 input channels (twelve runs, a
 //       run apart), then one run of ones, whose row sums g: the bias gradient
-//   N = 32 output channels, K = the tile's 128 cells in steps of 16
-// The nine in-plane taps (dy, dx) have one 32-column accumulator each in
-// tensor memory, kept across tiles, and are drained into FP32 registers every
-// DRAIN tiles with round-to-nearest adds (the accumulator's own rounding then
-// acts on at most 8 DRAIN sums); each CTA adds its sums to the gradient once,
-// at the end.  Warp 0 issues TMA, warp 1 the 72 MMAs of a tile, warp 2 clears
-// the gradient's slots outside the owned cells (the halo holds periodic
-// images, which the data gradient needs), warps 3-14 drain.
+//   N = 32 output channels, from one of three copies of the gradient, shifted by
+//       the dx taps; K = the tile's 128 slots in steps of 16
+// (dx moved to the gradient: sum_c g[c] x[c + dx] = sum_c' g[c' - dx] x[c'].)
+// What such MMAs cost is reading their operands from shared memory: the three dx
+// of one input operand read it once, through the A collector.  The nine in-plane
+// taps have 32 accumulator columns each in tensor memory, kept across tiles, and are
+// drained into FP32 registers every DRAIN tiles with round-to-nearest adds (the
+// accumulator's own rounding then acts on at most 8 DRAIN sums); each CTA adds
+// its sums to the gradient once, at the end.  Warp 0 issues TMA, warp 1 the
+// MMAs, warps 2-3 write the gradient's shifted copies with the slots outside the
+// owned cells cleared (the halo holds periodic images, which the data gradient
+// needs), warps 4-15 drain.
 //
-// Bound by the L2 -> shared-memory ingest of the three planes (61 KB a tile
-// at 64^3): 0.14 ms a layer on 4 x 64^3, where the FP32-issue kernel it
-// replaces took 2.22 ms.
+// A layer on 4 x 64^3: 2.22 ms as an FP32-issue kernel, 0.10 ms with an operand
+// read per tap, 0.09 ms now.
 #include <mutex>
 
 #include "sclet_conv_tc.cuh"
@@ -33,31 +36,34 @@ namespace wg {
 
 using namespace tc;
 
-constexpr int TAPS2 = 9;                    // in-plane taps, one accumulator each
-constexpr int G_ROWS = (ROWS + 7 + 7) / 8;  // 128-byte lines of one gradient run
+constexpr int TAPS2 = 9;                    // in-plane taps, 32 accumulator columns each
+constexpr int G_ROWS = (ROWS + 2 + 7 + 7) / 8;  // 128-byte lines of one gradient run (130 slots)
 constexpr int G_BYTES = G_ROWS * 128;
+constexpr int S_BYTES = ROWS * 16;          // one chunk of a shifted copy
+constexpr int SHIFTERS = 2;                 // warps writing the shifted copies
 constexpr int EPI = 12;                     // draining warps, three per TMEM lane quadrant
 constexpr int TAPS_PER_WARP = TAPS2 / 3;
-constexpr int WG_THREADS = 32 * (3 + EPI);
+constexpr int WG_THREADS = 32 * (2 + SHIFTERS + EPI);
 constexpr int WG_TMEM = 512;                // 288 columns used; allocations are powers of two
 constexpr int DRAIN = 8;                    // tiles per drain
 
-// Runs of the input per stage as in k_conv.cu's ny: 1 one run of 128 + 2 Np + 2
-// slots per plane and chunk, 3 one run of 130 slots per stencil row.  A stage:
-// for each of ny rows the twelve runs (dz, chunk), the ones run, three run
-// lengths that rows 104..127 of M read and drop (they overlay what follows),
-// and the four gradient runs at the end.
+// Runs of the input per stage as in k_conv.cu's ny: 1 one run of 128 + 2 Np
+// slots per plane and chunk, 3 one run of 128 slots per stencil row.  A stage:
+// for each of ny rows the twelve runs (dz, chunk) and the ones run (three run
+// lengths more are read as rows 104..127 of M and dropped: they overlay what
+// follows), the four gradient runs as they lie, and their twelve shifted
+// copies.
 struct Geom {
   int ny, box_rows, box_bytes, row_bytes, stage_bytes, stages, smem;
 };
 static Geom geom_for(int N, int ny) {
   Geom g;
   g.ny = ny;
-  const int R = ny == 1 ? ROWS + 2 * (N + 2) + 2 : ROWS + 2;
+  const int R = ny == 1 ? ROWS + 2 * (N + 2) : ROWS;
   g.box_rows = (R + 7 + 7) / 8;
   g.box_bytes = g.box_rows * 128;
   g.row_bytes = 13 * g.box_bytes;
-  g.stage_bytes = ny * g.row_bytes + 4 * G_BYTES;
+  g.stage_bytes = ny * g.row_bytes + 4 * G_BYTES + 12 * S_BYTES;
   const int tail = 3 * g.box_bytes + 128;  // the dropped rows' reads past the last stage
   g.stages = (SMEM_LIMIT - 1024 - tail) / g.stage_bytes;
   if (g.stages > MAX_STAGES) g.stages = MAX_STAGES;
@@ -70,7 +76,7 @@ __global__ void __launch_bounds__(WG_THREADS, 1)
                     float *__restrict__ dw, float *__restrict__ db, int *err, Geom gm) {
   extern __shared__ uint8_t smem_raw[];
   __shared__ __align__(8) uint64_t full_bar[MAX_STAGES];
-  __shared__ __align__(8) uint64_t ready_bar[MAX_STAGES];  // gradient slots outside the owned cells cleared
+  __shared__ __align__(8) uint64_t ready_bar[MAX_STAGES];  // shifted copies written
   __shared__ __align__(8) uint64_t empty_bar[MAX_STAGES];
   __shared__ __align__(8) uint64_t acc_full, acc_empty, done_bar;
   __shared__ uint32_t tmem_slot;
@@ -82,7 +88,7 @@ __global__ void __launch_bounds__(WG_THREADS, 1)
   const int per_plane = (N * Np + ROWS - 1) / ROWS;
   const int total = batch * N * per_plane;
   const int mine = (int)blockIdx.x < total ? (total - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
-  const int g_off = ny * gm.row_bytes;  // gradient runs within a stage
+  const int g_off = ny * gm.row_bytes, s_off = g_off + 4 * G_BYTES;  // gradient runs and shifted copies of a stage
 
   // shared memory starts as zeros, the ones runs as ones: what the dropped
   // rows read is initialised too
@@ -102,7 +108,7 @@ __global__ void __launch_bounds__(WG_THREADS, 1)
   if (threadIdx.x == 0) {
     for (int s = 0; s < MAX_STAGES; s++) {
       mbar_init(&full_bar[s], 1);
-      mbar_init(&ready_bar[s], 1);
+      mbar_init(&ready_bar[s], SHIFTERS);
       mbar_init(&empty_bar[s], 1);
     }
     mbar_init(&acc_full, 1);
@@ -138,12 +144,12 @@ __global__ void __launch_bounds__(WG_THREADS, 1)
         for (int r = 0; r < ny; r++)
           for (int dz = 0; dz < 3; dz++)
             for (int k = 0; k < 4; k++) {
-              const long long first = (long long)ti.s0 + (ny == 1 ? -Np : (r - 1) * Np) - 1;
+              const long long first = (long long)ti.s0 + (ny == 1 ? -Np : (r - 1) * Np);
               const long long flat = conv_at(N, ti.b, ti.zh + dz - 1, k, first);
               tma_load_2d(st + r * gm.row_bytes + (dz * 4 + k) * gm.box_bytes, &tmX, 0, (int)(flat >> 3), &full_bar[s]);
             }
         for (int k = 0; k < 4; k++)
-          tma_load_2d(st + g_off + k * G_BYTES, &tmG, 0, (int)(conv_at(N, ti.b, ti.zh, k, ti.s0) >> 3), &full_bar[s]);
+          tma_load_2d(st + g_off + k * G_BYTES, &tmG, 0, (int)(conv_at(N, ti.b, ti.zh, k, ti.s0 - 1) >> 3), &full_bar[s]);
       }
       if (*(volatile int *)&failed)  // drain (bounded) the copies still in flight
         for (int i = it - stages < 0 ? 0 : it - stages; i < it; i++) mbar_wait(&full_bar[i % stages], (i / stages) & 1);
@@ -152,7 +158,7 @@ __global__ void __launch_bounds__(WG_THREADS, 1)
     // the warp runs the loop together, one lane issues (mma_bf16_from)
     const bool issue = elect_one();
     const uint32_t idesc = idesc_bf16(ROWS, CH) | (1u << 15) | (1u << 16);  // both operands MN-major
-    const uint64_t dg0 = smem_desc_lin(smem_u32(base) + g_off, 128, G_BYTES);
+    const uint64_t dg0 = smem_desc_lin(smem_u32(base) + s_off, 128, S_BYTES);
     const uint64_t dx0 = smem_desc_lin(smem_u32(base), 128, gm.box_bytes);
     const uint32_t g_hi = (uint32_t)(dg0 >> 32), x_hi = (uint32_t)(dx0 >> 32);
     bool ok = true;
@@ -164,20 +170,22 @@ __global__ void __launch_bounds__(WG_THREADS, 1)
       fence_after();
       const Tile ti = tile_of(blockIdx.x + it * gridDim.x, N, Np, per_plane);
       const uint32_t st = (uint32_t)(s * gm.stage_bytes >> 4);
-      const uint32_t g_lo = (uint32_t)dg0 + st + (uint32_t)(conv_at(N, ti.b, ti.zh, 0, ti.s0) & 7);
       const uint32_t first_tile = it % DRAIN == 0 ? 0u : 1u;
 #pragma unroll
       for (int dy = 0; dy < 3; dy++) {
-        // the run holding stencil row dy and the row of dx = -1 within it
-        const uint32_t first = (uint32_t)(ti.s0 + (ny == 1 ? -Np : (dy - 1) * Np) - 1);
+        // the run holding stencil row dy and its first slot within it
+        const uint32_t first = (uint32_t)(ti.s0 + (ny == 1 ? -Np : (dy - 1) * Np));
         const uint32_t x_lo = (uint32_t)dx0 + st + (ny == 1 ? 0u : (uint32_t)(dy * gm.row_bytes) >> 4) + (first & 7) +
                               (ny == 1 ? (uint32_t)(dy * Np) : 0u);
 #pragma unroll
-        for (int dx = 0; dx < 3; dx++) {
-#pragma unroll
-          for (int ks = 0; ks < ROWS / 16; ks++)
-            mma_bf16_from(issue, tmem + (uint32_t)((dy * 3 + dx) * CH), x_lo + (uint32_t)(dx + ks * 16), x_hi,
-                          g_lo + (uint32_t)(ks * 16), g_hi, idesc, ks == 0 ? first_tile : 1u);
+        for (int ks = 0; ks < ROWS / 16; ks++) {
+          // one input operand, the three dx
+          const uint32_t acc = tmem + (uint32_t)(dy * 3 * CH), x = x_lo + (uint32_t)(ks * 16);
+          const uint32_t g = (uint32_t)dg0 + st + (uint32_t)(ks * 16), on = ks == 0 ? first_tile : 1u;
+          constexpr uint32_t DX = (uint32_t)(4 * S_BYTES) >> 4;
+          mma_bf16_from<A_FILL>(issue, acc, x, x_hi, g, g_hi, idesc, on);
+          mma_bf16_from<A_USE>(issue, acc + CH, x, x_hi, g + DX, g_hi, idesc, on);
+          mma_bf16_from<A_LAST>(issue, acc + 2 * CH, x, x_hi, g + 2 * DX, g_hi, idesc, on);
         }
       }
       mma_commit_from(issue, &empty_bar[s]);
@@ -187,7 +195,9 @@ __global__ void __launch_bounds__(WG_THREADS, 1)
     if (!ok && lane == 0) failed = 1;
     mma_commit_from(issue, &done_bar);
     if (!mbar_wait(&done_bar, 0) && lane == 0) failed = 1;
-  } else if (warp == 2) {
+  } else if (warp < 2 + SHIFTERS) {
+    // copy [dx][chunk]: slot i = the gradient at s0 + i - (dx - 1), zero outside
+    // the owned cells; the raw runs start at slot s0 - 1
     for (int it = 0; it < mine; it++) {
       const int s = it % stages;
       int ok = 1;
@@ -198,12 +208,21 @@ __global__ void __launch_bounds__(WG_THREADS, 1)
         break;
       }
       const Tile ti = tile_of(blockIdx.x + it * gridDim.x, N, Np, per_plane);
-      const int goff = (int)(conv_at(N, ti.b, ti.zh, 0, ti.s0) & 7);
-      uint8_t *g = base + s * gm.stage_bytes + g_off;
-      for (int i = lane; i < ROWS; i += 32) {
-        const int slot = ti.s0 + i, yh = slot / Np, xh = slot - yh * Np;
-        if (yh < 1 || yh > N || xh < 1 || xh > N)
-          for (int k = 0; k < 4; k++) *reinterpret_cast<uint4 *>(g + k * G_BYTES + (goff + i) * 16) = make_uint4(0, 0, 0, 0);
+      const int goff = (int)(conv_at(N, ti.b, ti.zh, 0, ti.s0 - 1) & 7);
+      uint8_t *st = base + s * gm.stage_bytes;
+      for (int i = (warp - 2) * 32 + lane; i < ROWS + 2; i += 32 * SHIFTERS) {
+        const int slot = ti.s0 - 1 + i, yh = slot / Np, xh = slot - yh * Np;
+        const bool own = yh >= 1 && yh <= N && xh >= 1 && xh <= N;
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+          uint4 v = make_uint4(0, 0, 0, 0);
+          if (own) v = *reinterpret_cast<const uint4 *>(st + g_off + k * G_BYTES + (goff + i) * 16);
+#pragma unroll
+          for (int dx = 0; dx < 3; dx++) {
+            const int at = i - 1 + dx - 1;  // slot of copy dx that takes it
+            if (at >= 0 && at < ROWS) *reinterpret_cast<uint4 *>(st + s_off + (dx * 4 + k) * S_BYTES + at * 16) = v;
+          }
+        }
       }
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       __syncwarp();
@@ -212,7 +231,7 @@ __global__ void __launch_bounds__(WG_THREADS, 1)
     }
   } else {
     // D row 32 q + lane = (dz = q, ci = lane), row 96 the sums of g; column co
-    const int q = warp & 3, t0 = ((warp - 3) >> 2) * TAPS_PER_WARP;
+    const int q = warp & 3, t0 = ((warp - 2 - SHIFTERS) >> 2) * TAPS_PER_WARP;
     float sum[TAPS_PER_WARP][CH] = {};
     const int groups = (mine + DRAIN - 1) / DRAIN;
     bool good = true;
