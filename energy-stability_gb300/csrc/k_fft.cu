@@ -84,7 +84,7 @@ static Radices factor(int n) {
 // One batch of line FFTs over one or two grids (blockIdx.y selects data0 /
 // data1).  axis 0: lines along x (contiguous); 1: along y; 2: along z.  sign
 // -1 forward, +1 backward (unscaled).  tw[j] = exp(-2 pi i j / N).  A CTA
-// keeps 2^ltile lines in shared memory; element-to-line maps use shifts, and
+// keeps up to 2^ltile lines in shared memory; element-to-line maps use shifts, and
 // the per-stage quotients use a float reciprocal, exact for these ranges (a
 // quotient's fractional part stays >= 0.5 / divisor away from the next
 // integer, far above float rounding at operands below 2^16).
@@ -94,16 +94,20 @@ struct StageDiv {
 
 __device__ __forceinline__ int fdiv(int e, float inv) { return __float2int_rd(((float)e + 0.5f) * inv); }
 
-// One Stockham stage of radix R over all lines of the tile (src -> dst).
-template <int R, typename C>
-__device__ __forceinline__ void fft_stage(const C *__restrict__ src, C *__restrict__ dst, int tile, int N, int Ns,
+// One Stockham stage of radix R over all lines of the tile (src -> dst), lines
+// ls apart.  Radices 3 and 5 use the symmetric sums and differences of their
+// inputs (real coefficients: 12 and 32 additions and multiplications per
+// butterfly against 36 and 120 of the plain sums; FP64 operations are what the
+// FP64 plan's passes cost).
+template <int R, typename T, typename C>
+__device__ __forceinline__ void fft_stage(const C *__restrict__ src, C *__restrict__ dst, int tile, int N, int ls, int Ns,
                                           float inv_nb, float inv_ns, const C *__restrict__ tw, int sign) {
   const int nb = N / R;
   for (int e = threadIdx.x; e < tile * nb; e += blockDim.x) {
     const int line = fdiv(e, inv_nb), j = e - line * nb;
     const int jq = fdiv(j, inv_ns), k = j - jq * Ns;
-    const C *s = src + line * N;
-    C *d = dst + line * N;
+    const C *s = src + line * ls;
+    C *d = dst + line * ls;
     C v[R];
     // twiddle r k N / (Ns R) < N: no reduction needed
     const int tstep = k * (N / (Ns * R));
@@ -117,32 +121,57 @@ __device__ __forceinline__ void fft_stage(const C *__restrict__ src, C *__restri
       }
     }
     C o[R];
+    // multiply by -i (forward) or +i (backward)
+    auto turn = [&](C a) {
+      C b;
+      b.x = sign < 0 ? a.y : -a.y;
+      b.y = sign < 0 ? -a.x : a.x;
+      return b;
+    };
     if (R == 2) {
       o[0] = cadd(v[0], v[1]);
       o[1] = csub(v[0], v[1]);
     } else if (R == 4) {
       C a = cadd(v[0], v[2]), b = csub(v[0], v[2]);
-      C c = cadd(v[1], v[3 % R]), d2 = csub(v[1], v[3 % R]);
-      // multiply d2 by -i (forward) or +i (backward)
-      C dj;
-      if (sign < 0) { dj.x = d2.y; dj.y = -d2.x; }
-      else { dj.x = -d2.y; dj.y = d2.x; }
+      C c = cadd(v[1], v[3 % R]), dj = turn(csub(v[1], v[3 % R]));
       o[0] = cadd(a, c);
       o[2 % R] = csub(a, c);
       o[1] = cadd(b, dj);
       o[3 % R] = csub(b, dj);
+    } else if (R == 3) {
+      const T s3 = (T)0.86602540378443864676;  // sin(2 pi / 3)
+      const C t = cadd(v[1], v[2 % R]);
+      C m, q = csub(v[1], v[2 % R]);
+      m.x = v[0].x - (T)0.5 * t.x;
+      m.y = v[0].y - (T)0.5 * t.y;
+      q.x *= s3;
+      q.y *= s3;
+      q = turn(q);
+      o[0] = cadd(v[0], t);
+      o[1] = cadd(m, q);
+      o[2 % R] = csub(m, q);
     } else {
-#pragma unroll
-      for (int q = 0; q < R; q++) {
-        C acc = v[0];
-#pragma unroll
-        for (int r = 1; r < R; r++) {
-          C w = tw[((r * q) % R) * nb];
-          if (sign > 0) w.y = -w.y;
-          acc = cadd(acc, cmul(v[r], w));
-        }
-        o[q] = acc;
-      }
+      // cos and sin of 2 pi / 5 and 4 pi / 5
+      const T c1 = (T)0.30901699437494742410, c2 = (T)-0.80901699437494742410;
+      const T s1 = (T)0.95105651629515357212, s2 = (T)0.58778525229247312917;
+      const C t1 = cadd(v[1], v[4 % R]), t2 = cadd(v[2 % R], v[3 % R]);
+      const C d1 = csub(v[1], v[4 % R]), d2 = csub(v[2 % R], v[3 % R]);
+      C m1, m2, q1, q2;
+      m1.x = v[0].x + (c1 * t1.x + c2 * t2.x);
+      m1.y = v[0].y + (c1 * t1.y + c2 * t2.y);
+      m2.x = v[0].x + (c2 * t1.x + c1 * t2.x);
+      m2.y = v[0].y + (c2 * t1.y + c1 * t2.y);
+      q1.x = s1 * d1.x + s2 * d2.x;
+      q1.y = s1 * d1.y + s2 * d2.y;
+      q2.x = s2 * d1.x - s1 * d2.x;
+      q2.y = s2 * d1.y - s1 * d2.y;
+      q1 = turn(q1);
+      q2 = turn(q2);
+      o[0] = cadd(v[0], cadd(t1, t2));
+      o[1] = cadd(m1, q1);
+      o[4 % R] = csub(m1, q1);
+      o[2 % R] = cadd(m2, q2);
+      o[3 % R] = csub(m2, q2);
     }
     const int idxD = jq * Ns * R + k;
 #pragma unroll
@@ -150,37 +179,46 @@ __device__ __forceinline__ void fft_stage(const C *__restrict__ src, C *__restri
   }
 }
 
+// A CTA takes 2^ltile lines; the last tile of a row (axes 1, 2) or of the grid
+// (axis 0) may be partial: an edge without a power of two still moves runs of
+// adjacent x (a tile that divides an odd N is one line, 16 bytes per access).
+// Elastic stage of 75^3 in FP64 2.00 -> 0.68 ms a second-order step, of 100^3 in
+// FP32 1.02 -> 0.46 ms, with the radix-3 and 5 butterflies above.
 template <typename T>
 __global__ void __launch_bounds__(256) fft_lines_kernel(typename Cx<T>::t *data0, typename Cx<T>::t *data1, int N,
                                                         int axis, int ltile, const typename Cx<T>::t *__restrict__ tw,
                                                         int sign, Radices rad, StageDiv sd) {
   typedef typename Cx<T>::t C;
   extern __shared__ unsigned char smem_raw[];
-  const int tile = 1 << ltile;
+  const int tile = 1 << ltile, ls = N + 1;
   C *buf0 = reinterpret_cast<C *>(smem_raw);
-  C *buf1 = buf0 + (size_t)tile * N;
+  C *buf1 = buf0 + (size_t)tile * ls;
   C *data = blockIdx.y == 0 ? data0 : data1;
   const long long NN = (long long)N * N;
   // Line set of this CTA
-  long long base, stride, lstride;
+  long long base, stride;
+  int lines;
   if (axis == 0) {
     base = (long long)blockIdx.x * tile * N;  // lines indexed by (z*N + y)
     stride = 1;
-    lstride = N;
+    lines = (int)min((long long)tile, NN - (long long)blockIdx.x * tile);
   } else {
-    const int ntx = N >> ltile;
+    const int ntx = (N + tile - 1) >> ltile;
     const int xt = blockIdx.x % ntx, w = blockIdx.x / ntx;  // w = z (axis 1) or y (axis 2)
     base = (axis == 1 ? (long long)w * NN : (long long)w * N) + (long long)xt * tile;
     stride = axis == 1 ? N : NN;
-    lstride = 1;
+    lines = min(tile, N - xt * tile);
   }
-  const int total = tile * N;
   if (axis == 0) {
-    for (int e = threadIdx.x; e < total; e += blockDim.x) buf0[e] = data[base + e];
+    const float inv_n = 1.0f / (float)N;
+    for (int e = threadIdx.x; e < lines * N; e += blockDim.x) {
+      const int line = fdiv(e, inv_n);
+      buf0[line * ls + (e - line * N)] = data[base + e];
+    }
   } else {
-    for (int e = threadIdx.x; e < total; e += blockDim.x) {
+    for (int e = threadIdx.x; e < tile * N; e += blockDim.x) {
       const int line = e & (tile - 1), pos = e >> ltile;
-      buf0[line * N + pos] = data[base + line * lstride + (long long)pos * stride];
+      if (line < lines) buf0[line * ls + pos] = data[base + line + (long long)pos * stride];
     }
   }
   __syncthreads();
@@ -190,10 +228,10 @@ __global__ void __launch_bounds__(256) fft_lines_kernel(typename Cx<T>::t *data0
     const int R = rad.r[st];
     const float inb = sd.inv_nb[st], ins = sd.inv_ns[st];
     switch (R) {
-      case 4: fft_stage<4, C>(src, dst, tile, N, Ns, inb, ins, tw, sign); break;
-      case 2: fft_stage<2, C>(src, dst, tile, N, Ns, inb, ins, tw, sign); break;
-      case 3: fft_stage<3, C>(src, dst, tile, N, Ns, inb, ins, tw, sign); break;
-      default: fft_stage<5, C>(src, dst, tile, N, Ns, inb, ins, tw, sign); break;
+      case 4: fft_stage<4, T, C>(src, dst, lines, N, ls, Ns, inb, ins, tw, sign); break;
+      case 2: fft_stage<2, T, C>(src, dst, lines, N, ls, Ns, inb, ins, tw, sign); break;
+      case 3: fft_stage<3, T, C>(src, dst, lines, N, ls, Ns, inb, ins, tw, sign); break;
+      default: fft_stage<5, T, C>(src, dst, lines, N, ls, Ns, inb, ins, tw, sign); break;
     }
     __syncthreads();
     C *t = src;
@@ -202,11 +240,15 @@ __global__ void __launch_bounds__(256) fft_lines_kernel(typename Cx<T>::t *data0
     Ns *= R;
   }
   if (axis == 0) {
-    for (int e = threadIdx.x; e < total; e += blockDim.x) data[base + e] = src[e];
+    const float inv_n = 1.0f / (float)N;
+    for (int e = threadIdx.x; e < lines * N; e += blockDim.x) {
+      const int line = fdiv(e, inv_n);
+      data[base + e] = src[line * ls + (e - line * N)];
+    }
   } else {
-    for (int e = threadIdx.x; e < total; e += blockDim.x) {
+    for (int e = threadIdx.x; e < tile * N; e += blockDim.x) {
       const int line = e & (tile - 1), pos = e >> ltile;
-      data[base + line * lstride + (long long)pos * stride] = src[line * N + pos];
+      if (line < lines) data[base + line + (long long)pos * stride] = src[line * ls + pos];
     }
   }
 }
@@ -610,6 +652,7 @@ __global__ void contract_kernel(typename Cx<T>::t *z01, typename Cx<T>::t *z23, 
   // blockIdx.y = run: its grids at run N^3
   z01 += blockIdx.y * N3;
   if (z23) z23 += blockIdx.y * N3;
+  auto mid = [&](int v) { return v == N / 2 || N - v == N / 2; };
   for (int row = blockIdx.x; row < N * N; row += gridDim.x) {
   const int z = row / N, y = row - z * N;
   const int ym = y == 0 ? 0 : N - y, zm = z == 0 ? 0 : N - z;
@@ -619,6 +662,9 @@ __global__ void contract_kernel(typename Cx<T>::t *z01, typename Cx<T>::t *z23, 
     const int xm = x == 0 ? 0 : N - x;
     const long long g = (long long)row * N + x, gm = (long long)rowm * N + xm;
     if (gm < g) continue;  // the pair is handled by its lower index
+    // B(-k) has B(k)'s bits where no component's wave number is its own or its
+    // neighbour's mirror (N / 2, or the two middle ones of an odd N): one read
+    const bool even = !(mid(z) || mid(y) || mid(x));
     C H[4], Hm[4];
     C a = z01[g], am = z01[gm];
     C b, bm;
@@ -629,19 +675,26 @@ __global__ void contract_kernel(typename Cx<T>::t *z01, typename Cx<T>::t *z23, 
     H[1].x = (T)0.5 * (a.y + am.y); H[1].y = (T)0.5 * (am.x - a.x);
     H[2].x = (T)0.5 * (b.x + bm.x); H[2].y = (T)0.5 * (b.y - bm.y);
     H[3].x = (T)0.5 * (b.y + bm.y); H[3].y = (T)0.5 * (bm.x - b.x);
+#pragma unroll
     for (int q = 0; q < 4; q++) {
       if (q >= nac) { H[q].x = 0; H[q].y = 0; }
       Hm[q] = cconj(H[q]);
     }
+    T bk[10], bkm[10];
+#pragma unroll
+    for (int i = 0; i < 10; i++) bk[i] = (T)bn[i * N3 + g];
+#pragma unroll
+    for (int i = 0; i < 10; i++) bkm[i] = even ? bk[i] : (T)bn[i * N3 + gm];
     C G[4];
+#pragma unroll
     for (int p = 0; p < 4; p++) {
       C f, fm;
       f.x = 0; f.y = 0; fm = f;
+#pragma unroll
       for (int q = 0; q < 4; q++) {
-        T bk = (T)bn[(long long)pq_slot(p, q) * N3 + g];
-        T bkm = (T)bn[(long long)pq_slot(p, q) * N3 + gm];
-        f.x += bk * H[q].x; f.y += bk * H[q].y;
-        fm.x += bkm * Hm[q].x; fm.y += bkm * Hm[q].y;
+        const T c = bk[pq_slot(p, q)], cm = bkm[pq_slot(p, q)];
+        f.x += c * H[q].x; f.y += c * H[q].y;
+        fm.x += cm * Hm[q].x; fm.y += cm * Hm[q].y;
       }
       // Hermitian part: its inverse transform is Re(IFFT(F_p))
       G[p].x = (T)0.5 * (f.x + fm.x);
@@ -779,14 +832,13 @@ cudaError_t elastic_plan_create(ElasticPlan **out, int N, int nac, const double 
     if ((e = cudaGetLastError()) != cudaSuccess) goto fail;
   }
   {
-    // tile of lines per CTA: two ping-pong buffers within ~96 KB
+    // tile of lines per CTA: two ping-pong buffers within ~72 KB (three CTAs an SM)
     int tile = 16;
-    while (tile > 1 && 2 * (size_t)tile * N * csz > 96 * 1024) tile /= 2;
-    while (N % tile) tile /= 2;
+    while (tile > 1 && 2 * (size_t)tile * (N + 1) * csz > 72 * 1024) tile /= 2;
     p->tile = tile;
     p->ltile = 0;
     while ((1 << p->ltile) < tile) p->ltile++;
-    p->smem = 2 * (size_t)tile * N * csz;
+    p->smem = 2 * (size_t)tile * (N + 1) * csz;
     int ns = 1;
     for (int st = 0; st < p->rad.count; st++) {
       p->sd.inv_nb[st] = 1.0f / (float)(N / p->rad.r[st]);
@@ -832,11 +884,12 @@ static cudaError_t fft3d(ElasticPlan *p, typename Cx<T>::t *z0, typename Cx<T>::
       attr_set[dev][which] = true;
     }
   }
-  const dim3 grid((unsigned)((long long)N * N / p->tile), z1 ? 2u : 1u);
+  const long long across = (long long)N * ((N + p->tile - 1) / p->tile), along = ((long long)N * N + p->tile - 1) / p->tile;
   const typename Cx<T>::t *tw = (const typename Cx<T>::t *)p->tw;
   int order[3] = {0, 1, 2};
   if (sign > 0) { order[0] = 2; order[2] = 0; }
   for (int k = 0; k < 3; k++) {
+    const dim3 grid((unsigned)(order[k] == 0 ? along : across), z1 ? 2u : 1u);
     fft_lines_kernel<T><<<grid, 256, p->smem, s>>>(z0, z1, N, order[k], p->ltile, tw, sign, p->rad, p->sd);
     launch_counter()++;
   }
@@ -892,23 +945,9 @@ cudaError_t elastic_compute(ElasticPlan *p, const T *u, T *felas, int n, T *shel
     unpack_kernel<T><<<rows_grid(N), rows_block(N), 0, s>>>(z01, z23, felas, N, p->nac);
     launch_counter()++;
   }
-  // ghost cells: the shared-scratch semantics, field by field in order (all
-  // runs of a field in one launch)
-  const long long fstride = (long long)p->nac * n3;
-  for (int q = 0; q < p->nac; q++) {
-    const T *prev = felas + (long long)((q + p->nac - 1) % p->nac) * n3;
-    long long pstride = fstride;
-    T *gbuf = shell;
-    if (p->first && q == 0) {
-      // before the first call the scratch block is all zero
-      cudaMemsetAsync(shell, 0, sizeof(T) * n3, s);
-      prev = shell;
-      pstride = 0;
-      gbuf = shell + n3;
-    }
-    cudaError_t e = launch_elastic_shell<T>(felas + q * n3, prev, n, gbuf, s, p->runs, fstride, pstride);
-    if (e != cudaSuccess) return e;
-  }
+  // ghost cells: the shared-scratch semantics
+  cudaError_t e = launch_elastic_shell<T>(felas, p->nac, n, shell, s, p->runs, p->first);
+  if (e != cudaSuccess) return e;
   p->first = false;
   return cudaGetLastError();
 }

@@ -67,62 +67,73 @@ cudaError_t launch_ghost_fill(T *u, int count, int n, T *shell, cudaStream_t s) 
   return cudaGetLastError();
 }
 
-// The elastic force is written into one shared scratch block per field p
-// (elastic_calculate_ElasDri, elastic.c:617-687): interior = the field's
+// The elastic force is written into one shared scratch block per field p in
+// order (elastic_calculate_ElasDri, elastic.c:617-687): interior = the field's
 // result, ghosts = the exchange of that block, whose stale ghost cells still
-// hold the previously exchanged field.  felas_p already carries its interior;
-// `prev` is the previously exchanged block.  A ghost's source is either an
-// interior cell (this field's value) or a ghost cell (prev's value).
+// hold the previously exchanged field.  A ghost of field p whose one-axis image
+// is an owned cell takes this field's value there; one whose image is itself a
+// ghost takes field p - 1's value at the image, which is found the same way, and
+// before field 0 comes the last field of the previous call (zero before the
+// first).  Each hop removes one ghost axis, so two or three hops resolve a cell:
+// all fields in one gather and one scatter, where a fill per field took two
+// launches each.  felas: runs x nac blocks, `per` CTAs each.
 template <typename T>
-__global__ void elastic_shell_gather(const T *__restrict__ fp, const T *__restrict__ prev, T *__restrict__ shell, int n,
-                                     long long ns, long long fstride, long long pstride) {
-  // blockIdx.y = run
-  fp += blockIdx.y * fstride;
-  prev += blockIdx.y * pstride;
-  shell += blockIdx.y * ns;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < ns; i += (long long)gridDim.x * blockDim.x) {
+__global__ void elastic_shell_gather(const T *__restrict__ felas, T *__restrict__ shell, int n, long long ns, int nac,
+                                     int first, int per) {
+  const long long n3 = (long long)n * n * n;
+  const int b = blockIdx.x / per, p = b % nac;
+  const T *run = felas + (b - p) * n3;  // the run's blocks
+  shell += b * ns;
+  for (long long i = (blockIdx.x - b * per) * (long long)blockDim.x + threadIdx.x; i < ns; i += (long long)per * blockDim.x) {
     int z, y, x;
     shell_cell(n, i, z, y, x);
-    bool gz = z < 2 || z >= n - 2, gy = y < 2 || y >= n - 2;
-    if (gz) z = wrap1(n, z);
-    else if (gy) y = wrap1(n, y);
-    else x = wrap1(n, x);
-    bool inner = z >= 2 && z < n - 2 && y >= 2 && y < n - 2 && x >= 2 && x < n - 2;
-    long long l = ((long long)z * n + y) * n + x;
-    shell[i] = inner ? fp[l] : prev[l];
+    T v = (T)0;
+    for (int q = p;; q--) {
+      const bool gz = z < 2 || z >= n - 2, gy = y < 2 || y >= n - 2;
+      if (gz) z = wrap1(n, z);
+      else if (gy) y = wrap1(n, y);
+      else x = wrap1(n, x);
+      const bool inner = z >= 2 && z < n - 2 && y >= 2 && y < n - 2 && x >= 2 && x < n - 2;
+      const long long l = ((long long)z * n + y) * n + x;
+      if (inner) {
+        v = run[q * n3 + l];
+        break;
+      }
+      if (q == 0) {  // the last field as the previous call left it
+        if (!first) v = run[(nac - 1) * n3 + l];
+        break;
+      }
+    }
+    shell[i] = v;
   }
 }
 
-// one scatter of the shell of blockIdx.y's run (stride between runs' blocks)
 template <typename T>
-__global__ void shell_scatter_runs(T *__restrict__ u, const T *__restrict__ shell, int n, long long ns,
-                                   long long stride) {
-  u += blockIdx.y * stride;
-  shell += blockIdx.y * ns;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < ns; i += (long long)gridDim.x * blockDim.x) {
+__global__ void elastic_shell_scatter(T *__restrict__ felas, const T *__restrict__ shell, int n, long long ns, int per) {
+  const int b = blockIdx.x / per;
+  felas += b * (long long)n * n * n;
+  shell += b * ns;
+  for (long long i = (blockIdx.x - b * per) * (long long)blockDim.x + threadIdx.x; i < ns; i += (long long)per * blockDim.x) {
     int z, y, x;
     shell_cell(n, i, z, y, x);
-    u[((long long)z * n + y) * n + x] = shell[i];
+    felas[((long long)z * n + y) * n + x] = shell[i];
   }
 }
 
 template <typename T>
-cudaError_t launch_elastic_shell(T *felas_p, const T *prev, int n, T *shell, cudaStream_t s, int runs,
-                                 long long fstride, long long pstride) {
-  long long ns = shell_count(n);
-  const dim3 g(grid_for(ns), runs > 0 ? runs : 1);
-  elastic_shell_gather<T><<<g, 256, 0, s>>>(felas_p, prev, shell, n, ns, fstride, pstride);
-  shell_scatter_runs<T><<<g, 256, 0, s>>>(felas_p, shell, n, ns, fstride);
+cudaError_t launch_elastic_shell(T *felas, int nac, int n, T *shell, cudaStream_t s, int runs, bool first) {
+  const long long ns = shell_count(n);
+  const int per = grid_for(ns), g = per * nac * (runs > 0 ? runs : 1);
+  elastic_shell_gather<T><<<g, 256, 0, s>>>(felas, shell, n, ns, nac, first ? 1 : 0, per);
+  elastic_shell_scatter<T><<<g, 256, 0, s>>>(felas, shell, n, ns, per);
   launch_counter() += 2;
   return cudaGetLastError();
 }
 
 template cudaError_t launch_ghost_fill<double>(double *, int, int, double *, cudaStream_t);
 template cudaError_t launch_ghost_fill<float>(float *, int, int, float *, cudaStream_t);
-template cudaError_t launch_elastic_shell<double>(double *, const double *, int, double *, cudaStream_t, int,
-                                                  long long, long long);
-template cudaError_t launch_elastic_shell<float>(float *, const float *, int, float *, cudaStream_t, int, long long,
-                                                 long long);
+template cudaError_t launch_elastic_shell<double>(double *, int, int, double *, cudaStream_t, int, bool);
+template cudaError_t launch_elastic_shell<float>(float *, int, int, float *, cudaStream_t, int, bool);
 
 long long &launch_counter() {
   static long long c = 0;

@@ -12,6 +12,7 @@
 #include <stdlib.h>
 #include <string.h>
 
+#include <algorithm>
 #include <string>
 #include <vector>
 #include <sys/stat.h>
@@ -655,7 +656,8 @@ int sclet_create_runs(const sclet_params *p, int runs, const double *krun, int p
     CC(cudaMalloc(&ctx->B, 2 * F * blk));
     CC(cudaMalloc(&ctx->felas, nfel * blk));
     CC(cudaMemsetAsync(ctx->felas, 0, nfel * blk, s));
-    CC(cudaMalloc(&ctx->scratch, 2 * blk));
+    // CH scratch of the right-hand side, or the elastic ghost shells of all fields
+    CC(cudaMalloc(&ctx->scratch, std::max(2 * blk, sizeof(double) * nfel * (size_t)shell_count(n))));
     CC(cudaMalloc(&ctx->shell, sizeof(double) * F * shell_count(n)));
     for (int a = 0; a < 3; a++) {
       CC(cudaMalloc(&ctx->V[a], sizeof(double) * n * n));
@@ -677,9 +679,8 @@ int sclet_create_runs(const sclet_params *p, int runs, const double *krun, int p
     if (p->etd2) CC(cudaMalloc(&ctx->frhs2, FT * blk));
     CC(cudaMalloc(&ctx->ffelas, nfel * runs * blk));
     CC(cudaMemsetAsync(ctx->ffelas, 0, nfel * runs * blk, s));
-    // elastic ghost shells of every run (and the zero block of the first
-    // call) or the CH scratch of every run
-    CC(cudaMalloc(&ctx->fscratch, (runs + 1) * blk));
+    // elastic ghost shells of every run's fields or the CH scratch of every run
+    CC(cudaMalloc(&ctx->fscratch, std::max((runs + 1) * blk, sizeof(float) * nfel * runs * (size_t)shell_count(n))));
     CC(cudaMalloc(&ctx->fshell, sizeof(float) * FT * shell_count(n)));
     CC(cudaMalloc(&ctx->W1, 2 * FT * blk));
     CC(cudaMalloc(&ctx->W2, 2 * FT * blk));

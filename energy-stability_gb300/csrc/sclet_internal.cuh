@@ -111,14 +111,11 @@ __device__ inline void shell_cell(int n, long long s, int &z, int &y, int &x) {
 // count * shell_count(n) elements.
 template <typename T>
 cudaError_t launch_ghost_fill(T *u, int count, int n, T *shell, cudaStream_t s);
-// Elastic scratch semantics: felas_p (p in order) gets its ghost cells from
-// the fill of the shared scratch block (see k_halo.cu).  `prev` is the block
-// that was last filled (felas_{p-1}, or the last field of the previous call).
-// runs: blocks side by side, felas_p's at fstride and prev's at pstride
-// apart (0: one prev for all); shell holds runs * shell_count(n) values.
+// Ghost cells of the elastic force of every field and run (nac blocks per run
+// side by side) by the shared-scratch semantics, see k_halo.cu.  shell holds
+// nac * runs * shell_count(n) values; first: no previous call.
 template <typename T>
-cudaError_t launch_elastic_shell(T *felas_p, const T *prev, int n, T *shell, cudaStream_t s, int runs = 1,
-                                 long long fstride = 0, long long pstride = 0);
+cudaError_t launch_elastic_shell(T *felas, int nac, int n, T *shell, cudaStream_t s, int runs, bool first);
 
 // Right-hand sides of all fields into out (F blocks).  felas: nac blocks.
 template <typename T>
@@ -195,7 +192,7 @@ cudaError_t elastic_plan_create(ElasticPlan **plan, int big_n, int nac, const do
 void elastic_plan_destroy(ElasticPlan *plan);
 // felas (nac blocks of n^3) from the AC fields u (first nac blocks).
 // runs (the plan's): run r's order parameters at u + r ustride, its force at
-// felas + r nac n^3; shell holds n^3 + runs * shell_count(n) values
+// felas + r nac n^3; shell holds nac * runs * shell_count(n) values
 template <typename T>
 cudaError_t elastic_compute(ElasticPlan *plan, const T *u, T *felas, int n, T *shell, cudaStream_t s,
                             long long ustride = 0);
