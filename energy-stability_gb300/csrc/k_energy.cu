@@ -87,197 +87,6 @@ __device__ __forceinline__ KS shfl_ks(KS v, int off) {
   return ks_merge(v, o);
 }
 
-// Lane 0 of every warp holds its warp's values: the block's record.
-__device__ __forceinline__ void block_record_from_warps(const double (&mxd)[MAXF], const double (&mnd)[MAXF],
-                                                        const KS (&vol)[MAXF], KS eac, KS ech, int F,
-                                                        double *__restrict__ part) {
-  const int tid = threadIdx.y * blockDim.x + threadIdx.x;
-  const int lane = tid & 31, wid = tid >> 5;
-  constexpr int NW = EB / 32;
-  __shared__ double wrec[NW][4 * MAXF + 4];
-  if (lane == 0) {
-    for (int f = 0; f < F; f++) {
-      wrec[wid][4 * f] = mxd[f];
-      wrec[wid][4 * f + 1] = mnd[f];
-      wrec[wid][4 * f + 2] = vol[f].s;
-      wrec[wid][4 * f + 3] = vol[f].c;
-    }
-    wrec[wid][4 * F] = eac.s;
-    wrec[wid][4 * F + 1] = eac.c;
-    wrec[wid][4 * F + 2] = ech.s;
-    wrec[wid][4 * F + 3] = ech.c;
-  }
-  __syncthreads();
-  if (wid == 0) {
-    const int src = lane < NW ? lane : 0;  // lanes beyond the warp count repeat warp 0 (idempotent for max/min)
-    double *dst = part + (long long)blockIdx.x * rec_len(F);
-    for (int f = 0; f < F; f++) {
-      double a = wrec[src][4 * f], b = wrec[src][4 * f + 1];
-      KS v = {lane < NW ? wrec[src][4 * f + 2] : 0.0, lane < NW ? wrec[src][4 * f + 3] : 0.0};
-#pragma unroll
-      for (int off = NW / 2; off > 0; off >>= 1) {
-        a = fmax(a, __shfl_xor_sync(0xffffffffu, a, off));
-        b = fmin(b, __shfl_xor_sync(0xffffffffu, b, off));
-        v = shfl_ks(v, off);
-      }
-      if (lane == 0) {
-        dst[4 * f] = a;
-        dst[4 * f + 1] = b;
-        dst[4 * f + 2] = v.s;
-        dst[4 * f + 3] = v.c;
-      }
-    }
-    KS ea = {lane < NW ? wrec[src][4 * F] : 0.0, lane < NW ? wrec[src][4 * F + 1] : 0.0};
-    KS eb = {lane < NW ? wrec[src][4 * F + 2] : 0.0, lane < NW ? wrec[src][4 * F + 3] : 0.0};
-#pragma unroll
-    for (int off = NW / 2; off > 0; off >>= 1) {
-      ea = shfl_ks(ea, off);
-      eb = shfl_ks(eb, off);
-    }
-    if (lane == 0) {
-      dst[4 * F] = ea.s;
-      dst[4 * F + 1] = ea.c;
-      dst[4 * F + 2] = eb.s;
-      dst[4 * F + 3] = eb.c;
-    }
-  }
-}
-
-__device__ __forceinline__ void block_record(double (&mxd)[MAXF], double (&mnd)[MAXF], KS (&vol)[MAXF], KS eac, KS ech,
-                                             int F, double *__restrict__ part) {
-#pragma unroll
-  for (int off = 16; off > 0; off >>= 1) {
-#pragma unroll
-    for (int f = 0; f < MAXF; f++) {
-      mxd[f] = fmax(mxd[f], __shfl_xor_sync(0xffffffffu, mxd[f], off));
-      mnd[f] = fmin(mnd[f], __shfl_xor_sync(0xffffffffu, mnd[f], off));
-      vol[f] = shfl_ks(vol[f], off);
-    }
-    eac = shfl_ks(eac, off);
-    ech = shfl_ks(ech, off);
-  }
-  block_record_from_warps(mxd, mnd, vol, eac, ech, F, part);
-}
-
-
-template <typename PL, typename T>
-__global__ void __launch_bounds__(EB) energy_partial_kernel(Phys ph, const T *__restrict__ u, const double *__restrict__ elam,
-                                                            int form, double *__restrict__ part) {
-  // Per-cell arithmetic in the state's precision T: the cell terms of an FP32
-  // state carry FP32 rounding, which is unbiased and averages out over the
-  // sum; every sum (per thread, per block, over blocks) is FP64, and the
-  // volume integrals add the FP32 values exactly.
-  const int n = ph.n, N = n - 4, F = ph.F, nac = ph.nac;
-  const long long n3 = (long long)n * n * n;
-  const T i4hx = (T)(0.25 / ph.h[0]), i4hy = (T)(0.25 / ph.h[1]), i4hz = (T)(0.25 / ph.h[2]);
-  const T half_epn2 = (T)(0.5 * ph.epn2);
-  const double cshift = ph.cshift;
-  T L[4][9];
-  for (int m = 0; m < 4; m++)
-    for (int k = 0; k < 9; k++) L[m][k] = (T)elam[9 * m + k];
-  T Kt[16];  // plugin constants
-#pragma unroll
-  for (int k = 0; k < 16; k++) Kt[k] = (T)ph.K[k];
-  T mx[MAXF], mn[MAXF];
-  Acc<T> vsum[MAXF], eac_p, ech_p;
-  long long cnt = 0;
-#pragma unroll
-  for (int f = 0; f < MAXF; f++) {
-    mx[f] = (T)-1.0e30;
-    mn[f] = (T)1.0e30;
-  }
-  // rows (j, k) of owned cells over the grid, x across the block: no index division per cell
-  for (int row = blockIdx.x; row < N * N; row += gridDim.x) {
-  const int j = 2 + row % N, k = 2 + row / N;
-  for (int i = 2 + threadIdx.x; i < n - 2; i += blockDim.x) {
-    const long long l = ((long long)k * n + j) * n + i;
-    cnt++;
-#pragma unroll
-    for (int f = 0; f < MAXF; f++) {
-      if (f >= F) break;
-      const T t = u[f * n3 + l];
-      mx[f] = t > mx[f] ? t : mx[f];
-      mn[f] = t < mn[f] ? t : mn[f];
-      vsum[f].add(t);
-    }
-    if (i >= n - 3 || j >= n - 3 || k >= n - 3) continue;
-    T avg[MAXF];
-    double cbar = 0.0;  // true concentration average, exact sum of the 8 values
-    double cst = 0.0;   // the same of the stored values (c - cshift)
-    T e_ac = (T)0, e_ch = (T)0;
-#pragma unroll
-    for (int f = 0; f < MAXF; f++) {
-      if (f >= F) break;
-      const T *q = u + f * n3;
-      const T v0 = q[l], v1 = q[l + 1], v2 = q[l + n], v3 = q[l + n + 1];
-      const T v4 = q[l + n * n], v5 = q[l + n * n + 1], v6 = q[l + n * n + n], v7 = q[l + n * n + n + 1];
-      avg[f] = (v0 + v1 + v2 + v3 + v4 + v5 + v6 + v7) * (T)0.125;
-      const T ux = ((v1 - v0) + (v3 - v2) + (v5 - v4) + (v7 - v6)) * i4hx;
-      const T uy = ((v2 - v0) + (v3 - v1) + (v6 - v4) + (v7 - v5)) * i4hy;
-      const T uz = ((v4 - v0) + (v5 - v1) + (v6 - v2) + (v7 - v3)) * i4hz;
-      if (f < nac) {
-        const T *Lm = L[f];
-        const T fx = ux * Lm[0] + uy * Lm[3] + uz * Lm[6];
-        const T fy = ux * Lm[1] + uy * Lm[4] + uz * Lm[7];
-        const T fz = ux * Lm[2] + uy * Lm[5] + uz * Lm[8];
-        e_ac += half_epn2 * (fx * ux + fy * uy + fz * uz);
-      } else {
-        const T gr = half_epn2 * (ux * ux + uy * uy + uz * uz);
-        if (form == 0) e_ch += gr; else e_ac += gr;
-        Acc<T> cs;
-        cs.add(v0);
-        cs.add(v1);
-        cs.add(v2);
-        cs.add(v3);
-        cs.add(v4);
-        cs.add(v5);
-        cs.add(v6);
-        cs.add(v7);
-        cst = cs.value() * 0.125;
-        cbar = cst + cshift;
-      }
-    }
-    if (form == 0) {
-      T e[4] = {0, 0, 0, 0};
-#pragma unroll
-      for (int f = 0; f < 4; f++)
-        if (f < nac) e[f] = avg[f];
-      const T s2 = e[0] * e[0] + e[1] * e[1] + e[2] * e[2] + e[3] * e[3];
-      const T s3 = e[0] * e[0] * e[0] + e[1] * e[1] * e[1] + e[2] * e[2] * e[2] + e[3] * e[3] * e[3];
-      if (nac > 0)
-        e_ac += (T)(2376.0 / 2372.0 / 2.0) * s2 - (T)((7128.0 + 12.0 * 2372.0) / 2372.0 / 3.0) * s3 +
-                (T)((4752.0 + 12.0 * 2372.0) / 2372.0 / 4.0) * s2 * s2;
-      if (ph.nch > 0) {
-        const T c = (T)cbar;
-        e_ch += (c * c - (T)1) * (c * c - (T)1) * (T)0.25;
-      }
-    } else {
-      sclet_acv<T> ac[4];
-      sclet_chv<T> ch[1];
-#pragma unroll
-      for (int m = 0; m < 4; m++) ac[m].u = m < nac ? avg[m] : (T)0;
-      ch[0].c = (T)cst;
-      e_ac += PL::template f_bulk<T>(ac, ch, nac, ph.nch, Kt);
-    }
-    eac_p.add(e_ac);
-    ech_p.add(e_ch);
-  }
-  }
-  double mxd[MAXF], mnd[MAXF];
-  KS vol[MAXF], eac = {eac_p.value(), 0.0}, ech = {ech_p.value(), 0.0};
-#pragma unroll
-  for (int f = 0; f < MAXF; f++) {
-    const double sh = f >= nac ? cshift : 0.0;
-    mxd[f] = (double)mx[f] + sh;
-    mnd[f] = (double)mn[f] + sh;
-    // sum of (value + 1) over this thread's cells, the constant part exact
-    vol[f].s = vsum[f].value();
-    vol[f].c = 0.0;
-    ks_add(vol[f], (double)cnt * (sh + 1.0));
-  }
-  block_record(mxd, mnd, vol, eac, ech, F, part);
-}
-
 // ---- FP32 states: z-marching form of the same reduction --------------------
 //
 // A CTA of 32 x 8 threads owns 32 x 8 owned (x, y) columns of one unit and
@@ -286,7 +95,10 @@ __global__ void __launch_bounds__(EB) energy_partial_kernel(Phys ph, const T *__
 // neighbours from the next lane, so a cell costs two loads per field instead
 // of eight.  The conserved field's corner average is an exact FP32 pair sum
 // finished in pair arithmetic (no FP64 instructions per cell).  Blocks loop
-// over units; one partial record per block, the same layout as above.
+// over units; one partial record per block (rec_len).  Bound by FP32 issue:
+// diagnostics of a 4-field 36^3 block 31 -> 19 us, of a 196^3 block with five
+// fields 191 -> 160 us, since a plane's sums are shared by the cubes on both of
+// its sides and no reduction runs through FP64.
 constexpr int EZ = 8;  // planes per unit
 
 __host__ __device__ inline int energy_units(int N) { return ((N + 31) / 32) * ((N + 7) / 8) * ((N + EZ - 1) / EZ); }
@@ -336,6 +148,46 @@ static EConst econst(const Phys &ph) {
   return c;
 }
 
+// (a + b) + c of pairs, rounded to float
+__device__ __forceinline__ Pair pair_merge(Pair a, Pair b) {
+  const float t = a.s + b.s, bp = t - a.s;
+  return Pair{t, (a.e + b.e) + ((a.s - (t - bp)) + (b.s - bp))};
+}
+
+// A plane's share of the cubes above and below it, computed once: the corner
+// sum, and the sums of the x- and y-differences (differences are formed before
+// sums, so a smooth field loses no digits).
+template <typename T>
+struct Face4 {
+  T v0, v1, v2, v3;  // (i, j) (i+1, j) (i, j+1) (i+1, j+1)
+  T s, dx, dy;
+  __device__ __forceinline__ void set(T a, T b, T c, T d) {
+    v0 = a, v1 = b, v2 = c, v3 = d;
+    s = (v0 + v1) + (v2 + v3);
+    dx = (v1 - v0) + (v3 - v2);
+    dy = (v2 - v0) + (v3 - v1);
+  }
+};
+
+// Half epn2 times the symmetrised gradient tensors, the four-fold spacings
+// folded in: xx yy zz xy xz yz (m < 4), then the conserved field's (4).
+template <typename T>
+__device__ __forceinline__ void energy_tensors(const Phys &ph, const double *elam, T (*q6)[6]) {
+  if (threadIdx.x < 5 * 6 && threadIdx.y == 0) {
+    const int m = threadIdx.x / 6, c = threadIdx.x % 6;
+    const double i4[3] = {0.25 / ph.h[0], 0.25 / ph.h[1], 0.25 / ph.h[2]};
+    const int r[6] = {0, 1, 2, 0, 0, 1}, k[6] = {0, 1, 2, 1, 2, 2};
+    double v = c < 3 ? 1.0 : 0.0;
+    if (m < 4) v = c < 3 ? elam[9 * m + 4 * c] : elam[9 * m + 3 * r[c] + k[c]] + elam[9 * m + 3 * k[c] + r[c]];
+    q6[m][c] = (T)(0.5 * ph.epn2 * v * i4[r[c]] * i4[k[c]]);
+  }
+  __syncthreads();
+}
+template <typename T>
+__device__ __forceinline__ T gradient_energy(const T *q, T ux, T uy, T uz) {
+  return ux * (q[0] * ux + q[3] * uy + q[4] * uz) + uy * (q[1] * uy + q[5] * uz) + q[2] * uz * uz;
+}
+
 template <typename PL, int NAC, int NCH>
 __global__ void __launch_bounds__(256, 2) energy_partial_f32(Phys ph, EConst ec, const float *__restrict__ u,
                                                              const double *__restrict__ elam, int form,
@@ -343,15 +195,8 @@ __global__ void __launch_bounds__(256, 2) energy_partial_f32(Phys ph, EConst ec,
   constexpr int F = NAC + NCH;
   const int n = ph.n, N = n - 4;
   const long long n3 = (long long)n * n * n;
-  __shared__ float q6[4][6];  // half epn2 times the symmetrised gradient tensors: xx yy zz xy xz yz
-  if (threadIdx.x < 4 * 6 && threadIdx.y == 0) {
-    const int m = threadIdx.x / 6, c = threadIdx.x % 6;
-    const double *L = elam + 9 * m;
-    const double v = c == 0 ? L[0] : c == 1 ? L[4] : c == 2 ? L[8] : c == 3 ? L[1] + L[3] : c == 4 ? L[2] + L[6] : L[5] + L[7];
-    q6[m][c] = (float)(0.5 * ph.epn2 * v);
-  }
-  __syncthreads();
-  const float i4hx = ec.i4hx, i4hy = ec.i4hy, i4hz = ec.i4hz, half_epn2 = ec.half_epn2;
+  __shared__ float q6[5][6];
+  energy_tensors<float>(ph, elam, q6);
   float Kt[16];
 #pragma unroll
   for (int k = 0; k < 16; k++) Kt[k] = ec.K[k];
@@ -360,7 +205,6 @@ __global__ void __launch_bounds__(256, 2) energy_partial_f32(Phys ph, EConst ec,
   u += (long long)blockIdx.y * F * n3;
   part += (long long)blockIdx.y * gridDim.x * rec_len(F);
   const float p2 = ec.p2, p3 = ec.p3, p4 = ec.p4;
-  const Pair kdp = ec.kdp, kcp = ec.kcp;
   float mx[F], mn[F];
   Acc<float> vsum[F], eac_p, ech_p;
   int cnt = 0;
@@ -377,42 +221,53 @@ __global__ void __launch_bounds__(256, 2) energy_partial_f32(Phys ph, EConst ec,
     const bool own = i <= n - 3 && j <= n - 3, inner = i <= n - 4 && j <= n - 4;
     const int ic = i < n - 2 ? i : n - 2, jc = j < n - 2 ? j : n - 2;  // clamped: loads stay inside the block
     const int k0 = 2 + zc * EZ, k1 = k0 + EZ < n - 2 ? k0 + EZ : n - 2;
-    float a0[F], a1[F], a2[F], a3[F];  // plane k: (i, j) (i+1, j) (i, j+1) (i+1, j+1)
-    const long long row0 = ((long long)k0 * n + jc) * n + ic;
-#pragma unroll
-    for (int f = 0; f < F; f++) {
-      const float *q = u + f * n3 + row0;
-      a0[f] = q[0];
-      a2[f] = q[n];
-      a1[f] = __shfl_down_sync(0xffffffffu, a0[f], 1);
-      a3[f] = __shfl_down_sync(0xffffffffu, a2[f], 1);
-      if (tx == 31) {
-        a1[f] = q[1];
-        a3[f] = q[n + 1];
-      }
-    }
-    for (int k = k0; k < k1; k++) {
-      float b0[F], b1[F], b2[F], b3[F];  // plane k + 1
-      const long long row = ((long long)(k + 1) * n + jc) * n + ic;
+    const float *row = u + ((long long)k0 * n + jc) * n + ic;
+    Face4<float> a[F];
+    Pair ca = {0.0f, 0.0f};  // the conserved field's exact corner sum of plane k
+    float nx[F][2], ne[F][2];  // plane in flight: (i, j), (i, j+1); the last lane's (i+1, j), (i+1, j+1)
+    auto fetch = [&](const float *q) {
 #pragma unroll
       for (int f = 0; f < F; f++) {
-        const float *q = u + f * n3 + row;
-        b0[f] = q[0];
-        b2[f] = q[n];
-        b1[f] = __shfl_down_sync(0xffffffffu, b0[f], 1);
-        b3[f] = __shfl_down_sync(0xffffffffu, b2[f], 1);
-        if (tx == 31) {
-          b1[f] = q[1];
-          b3[f] = q[n + 1];
-        }
+        const float *p = q + f * n3;
+        nx[f][0] = p[0];
+        nx[f][1] = p[n];
+        ne[f][0] = tx == 31 ? p[1] : 0.0f;
+        ne[f][1] = tx == 31 ? p[n + 1] : 0.0f;
       }
+    };
+    auto take = [&](int f, Face4<float> &b) {
+      float r0 = __shfl_down_sync(0xffffffffu, nx[f][0], 1), r1 = __shfl_down_sync(0xffffffffu, nx[f][1], 1);
+      if (tx == 31) r0 = ne[f][0], r1 = ne[f][1];
+      b.set(nx[f][0], r0, nx[f][1], r1);
+    };
+    auto corner_pair = [&](const Face4<float> &b) {
+      Pair c = {b.v0, 0.0f};
+      pair_add(c, b.v1);
+      pair_add(c, b.v2);
+      pair_add(c, b.v3);
+      return c;
+    };
+    fetch(row);
+#pragma unroll
+    for (int f = 0; f < F; f++) take(f, a[f]);
+    if (NCH > 0) ca = corner_pair(a[F - 1]);
+    row += (long long)n * n;
+    fetch(row);
+    for (int k = k0; k < k1; k++) {
+      Face4<float> b[F];  // plane k + 1
+#pragma unroll
+      for (int f = 0; f < F; f++) take(f, b[f]);
+      row += (long long)n * n;
+      if (k + 1 < k1) fetch(row);  // plane k + 2 while this one is worked on
+      Pair cb = {0.0f, 0.0f};
+      if (NCH > 0) cb = corner_pair(b[F - 1]);
       if (own) {
         cnt++;
 #pragma unroll
         for (int f = 0; f < F; f++) {
-          mx[f] = fmaxf(mx[f], a0[f]);
-          mn[f] = fminf(mn[f], a0[f]);
-          vsum[f].add(a0[f]);
+          mx[f] = fmaxf(mx[f], a[f].v0);
+          mn[f] = fminf(mn[f], a[f].v0);
+          vsum[f].add(a[f].v0);
         }
       }
       if (inner && k <= n - 4) {
@@ -420,33 +275,20 @@ __global__ void __launch_bounds__(256, 2) energy_partial_f32(Phys ph, EConst ec,
         float e_ac = 0.0f, e_ch = 0.0f, cd = 0.0f, cval = 0.0f;
 #pragma unroll
         for (int f = 0; f < F; f++) {
-          const float v0 = a0[f], v1 = a1[f], v2 = a2[f], v3 = a3[f], v4 = b0[f], v5 = b1[f], v6 = b2[f], v7 = b3[f];
-          avg[f] = (((v0 + v1) + (v2 + v3)) + ((v4 + v5) + (v6 + v7))) * 0.125f;
-          const float ux = ((v1 - v0) + (v3 - v2) + (v5 - v4) + (v7 - v6)) * i4hx;
-          const float uy = ((v2 - v0) + (v3 - v1) + (v6 - v4) + (v7 - v5)) * i4hy;
-          const float uz = ((v4 - v0) + (v5 - v1) + (v6 - v2) + (v7 - v3)) * i4hz;
-          if (f < NAC) {
-            const float *qm = q6[f];
-            e_ac += qm[0] * ux * ux + qm[1] * uy * uy + qm[2] * uz * uz + qm[3] * ux * uy + qm[4] * ux * uz +
-                    qm[5] * uy * uz;
-          } else {
-            const float gr = half_epn2 * (ux * ux + uy * uy + uz * uz);
-            if (form == 0) e_ch += gr;
-            else e_ac += gr;
-            // exact corner sum, then (sum / 8 + cshift - c0) and (sum / 8 + cshift)
-            Pair cs = {v0, 0.0f};
-            pair_add(cs, v1);
-            pair_add(cs, v2);
-            pair_add(cs, v3);
-            pair_add(cs, v4);
-            pair_add(cs, v5);
-            pair_add(cs, v6);
-            pair_add(cs, v7);
-            cs.s *= 0.125f;
-            cs.e *= 0.125f;
-            cd = pair_sum(cs, kdp);
-            cval = pair_sum(cs, kcp);
-          }
+          avg[f] = (a[f].s + b[f].s) * 0.125f;
+          const float ux = a[f].dx + b[f].dx, uy = a[f].dy + b[f].dy;
+          const float uz = ((b[f].v0 - a[f].v0) + (b[f].v1 - a[f].v1)) + ((b[f].v2 - a[f].v2) + (b[f].v3 - a[f].v3));
+          const float gr = gradient_energy(q6[f < NAC ? f : 4], ux, uy, uz);
+          if (f < NAC || form != 0) e_ac += gr;
+          else e_ch += gr;
+        }
+        if (NCH > 0) {
+          // exact corner sum, then (sum / 8 + cshift - c0) and (sum / 8 + cshift)
+          Pair cs = pair_merge(ca, cb);
+          cs.s *= 0.125f;
+          cs.e *= 0.125f;
+          cd = pair_sum(cs, ec.kdp);
+          cval = pair_sum(cs, ec.kcp);
         }
         if (form == 0) {
           if (NAC > 0) {
@@ -468,19 +310,17 @@ __global__ void __launch_bounds__(256, 2) energy_partial_f32(Phys ph, EConst ec,
           e_ac += PL::template f_bulk<float>(ac, ch, NAC, NCH, Kt);
         }
         eac_p.add(e_ac);
-        ech_p.add(e_ch);
+        if (form == 0) ech_p.add(e_ch);
       }
 #pragma unroll
-      for (int f = 0; f < F; f++) {
-        a0[f] = b0[f];
-        a1[f] = b1[f];
-        a2[f] = b2[f];
-        a3[f] = b3[f];
-      }
+      for (int f = 0; f < F; f++) a[f] = b[f];
+      ca = cb;
     }
   }
-  // warp butterflies in FP32 (max, min) and exact-pair arithmetic (sums),
-  // then the warps' values in FP64 as in energy_partial_kernel
+  // warp butterflies, then the warps' values by one warp, in FP32 (max, min) and
+  // exact-pair arithmetic (sums); only the record is FP64, a lane per field (an
+  // FP64 warp instruction is 64 cycles of its scheduler: the block's merges in
+  // FP64, one field after the other, took longer than a small block's cells)
 #pragma unroll
   for (int off = 16; off > 0; off >>= 1) {
 #pragma unroll
@@ -493,56 +333,96 @@ __global__ void __launch_bounds__(256, 2) energy_partial_f32(Phys ph, EConst ec,
     ech_p.merge_lane(off);
     cnt += __shfl_xor_sync(0xffffffffu, cnt, off);
   }
-  double mxd[MAXF], mnd[MAXF];
-  KS vol[MAXF], eac = {0.0, 0.0}, ech = {0.0, 0.0};
-  if ((threadIdx.x & 31) == 0) {
-    eac = KS{(double)eac_p.s, (double)eac_p.e};
-    ech = KS{(double)ech_p.s, (double)ech_p.e};
+  constexpr int NW = EB / 32;
+  __shared__ float wv[4 * F + 4][NW];
+  __shared__ int wc[NW];
+  const int lane = tx, wid = ty;
+  if (lane == 0) {
 #pragma unroll
-    for (int f = 0; f < MAXF; f++) {
-      const double sh = f >= NAC ? ph.cshift : 0.0;
-      mxd[f] = f < F ? (double)mx[f < F ? f : 0] + sh : -1.0e30;
-      mnd[f] = f < F ? (double)mn[f < F ? f : 0] + sh : 1.0e30;
-      vol[f] = f < F ? KS{(double)vsum[f < F ? f : 0].s, (double)vsum[f < F ? f : 0].e} : KS{0.0, 0.0};
-      ks_add(vol[f], (double)cnt * (sh + 1.0));
+    for (int f = 0; f < F; f++) {
+      wv[4 * f][wid] = mx[f];
+      wv[4 * f + 1][wid] = mn[f];
+      wv[4 * f + 2][wid] = vsum[f].s;
+      wv[4 * f + 3][wid] = vsum[f].e;
+    }
+    wv[4 * F][wid] = eac_p.s;
+    wv[4 * F + 1][wid] = eac_p.e;
+    wv[4 * F + 2][wid] = ech_p.s;
+    wv[4 * F + 3][wid] = ech_p.e;
+    wc[wid] = cnt;
+  }
+  __syncthreads();
+  if (wid == 0 && lane < F + 2) {
+    // lane f: field f; lanes F and F + 1: the two energies
+    double *dst = part + (long long)blockIdx.x * rec_len(F);
+    const int at = lane < F ? 4 * lane + 2 : 4 * F + 2 * (lane - F);
+    Acc<float> s;
+    float top = -1.0e30f, low = 1.0e30f;
+    int count = 0;
+    for (int w = 0; w < NW; w++) {
+      s.add(wv[at][w]);
+      s.e += wv[at + 1][w];
+      if (lane < F) {
+        top = fmaxf(top, wv[4 * lane][w]);
+        low = fminf(low, wv[4 * lane + 1][w]);
+        count += wc[w];
+      }
+    }
+    if (lane < F) {
+      const double sh = lane >= NAC ? ph.cshift : 0.0;
+      KS v = {(double)s.s, (double)s.e};
+      ks_add(v, (double)count * (sh + 1.0));  // sum of (value + 1)
+      dst[4 * lane] = (double)top + sh;
+      dst[4 * lane + 1] = (double)low + sh;
+      dst[4 * lane + 2] = v.s;
+      dst[4 * lane + 3] = v.c;
+    } else {
+      dst[at] = (double)s.s;
+      dst[at + 1] = (double)s.e;
     }
   }
-  block_record_from_warps(mxd, mnd, vol, eac, ech, F, part);
 }
 
 // ---- FP64 states: the same z-marching form in FP64 -------------------------
 //
 // The column tile and the plane walk of energy_partial_f32, with FP64 values
-// and compensated FP64 (TwoSum) running sums.  Two loads per field and cell
-// instead of eight.
+// and compensated FP64 (TwoSum) running sums.  Bound by FP64 instructions:
+// diagnostics of 4 fields of 68^3 205 -> 146 us, of 4 + 1 fields of 132^3 1.54 ->
+// 1.12 ms with about 270 of them per cell instead of 370.
+// The largest (smallest) of doubles without FP64 instructions: a key that orders
+// as the values do; NaN never wins.
+__device__ __forceinline__ long long order_key(double v) {
+  const long long b = __double_as_longlong(v);
+  return b ^ ((b >> 63) & 0x7fffffffffffffffLL);
+}
+__device__ __forceinline__ double key_value(long long k) {
+  return __longlong_as_double(k ^ ((k >> 63) & 0x7fffffffffffffffLL));
+}
+__device__ __forceinline__ bool is_nan_bits(double v) {
+  return (__double_as_longlong(v) & 0x7fffffffffffffffLL) > 0x7ff0000000000000LL;
+}
+
 template <typename PL, int NAC, int NCH>
 __global__ void __launch_bounds__(256, 1) energy_partial_f64z(Phys ph, const double *__restrict__ u,
                                                               const double *__restrict__ elam, int form,
                                                               double *__restrict__ part) {
-  constexpr int F = NAC + NCH;
+  constexpr int F = NAC + NCH, Q = F + 2;  // sums of a block: one per field, two energies
   const int n = ph.n, N = n - 4;
   const long long n3 = (long long)n * n * n;
-  __shared__ double q6[4][6];  // half epn2 times the symmetrised gradient tensors: xx yy zz xy xz yz
-  if (threadIdx.x < 4 * 6 && threadIdx.y == 0) {
-    const int m = threadIdx.x / 6, c = threadIdx.x % 6;
-    const double *L = elam + 9 * m;
-    const double v = c == 0 ? L[0] : c == 1 ? L[4] : c == 2 ? L[8] : c == 3 ? L[1] + L[3] : c == 4 ? L[2] + L[6] : L[5] + L[7];
-    q6[m][c] = 0.5 * ph.epn2 * v;
-  }
-  __syncthreads();
-  const double i4hx = 0.25 / ph.h[0], i4hy = 0.25 / ph.h[1], i4hz = 0.25 / ph.h[2], half_epn2 = 0.5 * ph.epn2;
+  __shared__ double q6[5][6];
+  energy_tensors<double>(ph, elam, q6);
   double Kt[16];
 #pragma unroll
   for (int k = 0; k < 16; k++) Kt[k] = ph.K[k];
   const double p2 = 2376.0 / 2372.0 / 2.0, p3 = (7128.0 + 12.0 * 2372.0) / 2372.0 / 3.0,
                p4 = (4752.0 + 12.0 * 2372.0) / 2372.0 / 4.0;
-  double mx[F], mn[F];
+  long long mx[F], mn[F];  // order keys
   KS vsum[F], eac = {0.0, 0.0}, ech = {0.0, 0.0};
-  long long cnt = 0;
+  int cnt = 0;
 #pragma unroll
   for (int f = 0; f < F; f++) {
-    mx[f] = -1.0e30;
-    mn[f] = 1.0e30;
+    mx[f] = order_key(-1.0e30);
+    mn[f] = order_key(1.0e30);
     vsum[f] = KS{0.0, 0.0};
   }
   const int tx = threadIdx.x, ty = threadIdx.y;
@@ -553,65 +433,44 @@ __global__ void __launch_bounds__(256, 1) energy_partial_f64z(Phys ph, const dou
     const bool own = i <= n - 3 && j <= n - 3, inner = i <= n - 4 && j <= n - 4;
     const int ic = i < n - 2 ? i : n - 2, jc = j < n - 2 ? j : n - 2;
     const int k0 = 2 + zc * EZ, k1 = k0 + EZ < n - 2 ? k0 + EZ : n - 2;
-    double a0[F], a1[F], a2[F], a3[F];
-    const long long row0 = ((long long)k0 * n + jc) * n + ic;
+    const double *row = u + ((long long)k0 * n + jc) * n + ic;
+    Face4<double> a[F];
+    auto take = [&](const double *q, Face4<double> &b) {
+      const double v0 = q[0], v2 = q[n];
+      double v1 = __shfl_down_sync(0xffffffffu, v0, 1), v3 = __shfl_down_sync(0xffffffffu, v2, 1);
+      if (tx == 31) v1 = q[1], v3 = q[n + 1];
+      b.set(v0, v1, v2, v3);
+    };
 #pragma unroll
-    for (int f = 0; f < F; f++) {
-      const double *q = u + f * n3 + row0;
-      a0[f] = q[0];
-      a2[f] = q[n];
-      a1[f] = __shfl_down_sync(0xffffffffu, a0[f], 1);
-      a3[f] = __shfl_down_sync(0xffffffffu, a2[f], 1);
-      if (tx == 31) {
-        a1[f] = q[1];
-        a3[f] = q[n + 1];
-      }
-    }
+    for (int f = 0; f < F; f++) take(row + f * n3, a[f]);
     for (int k = k0; k < k1; k++) {
-      double b0[F], b1[F], b2[F], b3[F];
-      const long long row = ((long long)(k + 1) * n + jc) * n + ic;
+      row += (long long)n * n;
+      Face4<double> b[F];  // plane k + 1
 #pragma unroll
-      for (int f = 0; f < F; f++) {
-        const double *q = u + f * n3 + row;
-        b0[f] = q[0];
-        b2[f] = q[n];
-        b1[f] = __shfl_down_sync(0xffffffffu, b0[f], 1);
-        b3[f] = __shfl_down_sync(0xffffffffu, b2[f], 1);
-        if (tx == 31) {
-          b1[f] = q[1];
-          b3[f] = q[n + 1];
-        }
-      }
+      for (int f = 0; f < F; f++) take(row + f * n3, b[f]);
       if (own) {
         cnt++;
 #pragma unroll
         for (int f = 0; f < F; f++) {
-          mx[f] = fmax(mx[f], a0[f]);
-          mn[f] = fmin(mn[f], a0[f]);
-          ks_add(vsum[f], a0[f]);
+          const long long key = order_key(a[f].v0);
+          if (!is_nan_bits(a[f].v0)) {
+            mx[f] = key > mx[f] ? key : mx[f];
+            mn[f] = key < mn[f] ? key : mn[f];
+          }
+          ks_add(vsum[f], a[f].v0);
         }
       }
       if (inner && k <= n - 4) {
         double avg[F > 0 ? F : 1];
-        double e_ac = 0.0, e_ch = 0.0, cbar = 0.0;
+        double e_ac = 0.0, e_ch = 0.0;
 #pragma unroll
         for (int f = 0; f < F; f++) {
-          const double v0 = a0[f], v1 = a1[f], v2 = a2[f], v3 = a3[f], v4 = b0[f], v5 = b1[f], v6 = b2[f],
-                       v7 = b3[f];
-          avg[f] = (v0 + v1 + v2 + v3 + v4 + v5 + v6 + v7) * 0.125;
-          const double ux = ((v1 - v0) + (v3 - v2) + (v5 - v4) + (v7 - v6)) * i4hx;
-          const double uy = ((v2 - v0) + (v3 - v1) + (v6 - v4) + (v7 - v5)) * i4hy;
-          const double uz = ((v4 - v0) + (v5 - v1) + (v6 - v2) + (v7 - v3)) * i4hz;
-          if (f < NAC) {
-            const double *qm = q6[f];
-            e_ac += qm[0] * ux * ux + qm[1] * uy * uy + qm[2] * uz * uz + qm[3] * ux * uy + qm[4] * ux * uz +
-                    qm[5] * uy * uz;
-          } else {
-            const double gr = half_epn2 * (ux * ux + uy * uy + uz * uz);
-            if (form == 0) e_ch += gr;
-            else e_ac += gr;
-            cbar = avg[f];
-          }
+          avg[f] = (a[f].s + b[f].s) * 0.125;
+          const double ux = a[f].dx + b[f].dx, uy = a[f].dy + b[f].dy;
+          const double uz = ((b[f].v0 - a[f].v0) + (b[f].v1 - a[f].v1)) + ((b[f].v2 - a[f].v2) + (b[f].v3 - a[f].v3));
+          const double gr = gradient_energy(q6[f < NAC ? f : 4], ux, uy, uz);
+          if (f < NAC || form != 0) e_ac += gr;
+          else e_ch += gr;
         }
         if (form == 0) {
           if (NAC > 0) {
@@ -623,80 +482,142 @@ __global__ void __launch_bounds__(256, 1) energy_partial_f64z(Phys ph, const dou
             }
             e_ac += p2 * s2 - p3 * s3 + p4 * s2 * s2;
           }
-          if (NCH > 0) e_ch += (cbar * cbar - 1.0) * (cbar * cbar - 1.0) * 0.25;
+          if (NCH > 0) e_ch += (avg[F - 1] * avg[F - 1] - 1.0) * (avg[F - 1] * avg[F - 1] - 1.0) * 0.25;
         } else {
           sclet_acv<double> ac[NAC > 0 ? NAC : 1];
           sclet_chv<double> ch[1];
 #pragma unroll
           for (int m = 0; m < NAC; m++) ac[m].u = avg[m];
-          ch[0].c = cbar;
+          ch[0].c = NCH > 0 ? avg[F - 1] : 0.0;
           e_ac += PL::template f_bulk<double>(ac, ch, NAC, NCH, Kt);
         }
         ks_add(eac, e_ac);
-        ks_add(ech, e_ch);
+        if (form == 0) ks_add(ech, e_ch);
       }
 #pragma unroll
-      for (int f = 0; f < F; f++) {
-        a0[f] = b0[f];
-        a1[f] = b1[f];
-        a2[f] = b2[f];
-        a3[f] = b3[f];
-      }
+      for (int f = 0; f < F; f++) a[f] = b[f];
     }
   }
-  double mxd[MAXF], mnd[MAXF];
-  KS vol[MAXF];
+  // The block's sums: every thread's pairs through shared memory, one warp per
+  // quantity folding eight threads per lane and then the lanes: 96 FP64 warp
+  // instructions per quantity instead of 40 per quantity in each of eight warps
+  // (an FP64 warp instruction is 64 cycles of its scheduler).
+  extern __shared__ double2 ks_of[];  // [Q][EB]
+  __shared__ long long wmx[EB / 32][F], wmn[EB / 32][F];
+  __shared__ int wcnt[EB / 32];
+  const int tid = ty * 32 + tx;
 #pragma unroll
-  for (int f = 0; f < MAXF; f++) {
-    mxd[f] = f < F ? mx[f < F ? f : 0] : -1.0e30;
-    mnd[f] = f < F ? mn[f < F ? f : 0] : 1.0e30;
-    vol[f] = f < F ? vsum[f < F ? f : 0] : KS{0.0, 0.0};
-    ks_add(vol[f], (double)cnt);  // sum of (value + 1)
+  for (int f = 0; f < F; f++) ks_of[f * EB + tid] = make_double2(vsum[f].s, vsum[f].c);
+  ks_of[F * EB + tid] = make_double2(eac.s, eac.c);
+  ks_of[(F + 1) * EB + tid] = make_double2(ech.s, ech.c);
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) {
+#pragma unroll
+    for (int f = 0; f < F; f++) {
+      const long long p = __shfl_xor_sync(0xffffffffu, mx[f], off), q = __shfl_xor_sync(0xffffffffu, mn[f], off);
+      mx[f] = p > mx[f] ? p : mx[f];
+      mn[f] = q < mn[f] ? q : mn[f];
+    }
+    cnt += __shfl_xor_sync(0xffffffffu, cnt, off);
   }
-  block_record(mxd, mnd, vol, eac, ech, F, part);
-}
-
-// Final reduction over the block records: one warp per quantity (per field
-// max, min, vol; the two energies); each lane folds a fixed strided subset of
-// the records, then a butterfly (deterministic).
-__global__ void energy_final_kernel(Phys ph, int form, const double *__restrict__ part, int npart,
-                                    double *__restrict__ out) {
-  const int F = ph.F, L = rec_len(F);
-  // blockIdx.x = run
-  part += (long long)blockIdx.x * npart * L;
-  out += (long long)blockIdx.x * 4 * F;
-  const double h3 = ph.h[0] * ph.h[1] * ph.h[2];
-  __shared__ double res[4 * MAXF + 4];
-  const int q = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int nq = 3 * F + 2;
-  if (q < nq) {
-    const int f = q < 3 * F ? q / 3 : -1, kind = q < 3 * F ? q % 3 : 3 + (q - 3 * F);
-    double m = kind == 0 ? -1.0e30 : (kind == 1 ? 1.0e30 : 0.0);
-    KS k = {0, 0};
-    for (int b = lane; b < npart; b += 32) {
-      const double *r = part + (long long)b * L;
-      if (kind == 0) m = fmax(m, r[4 * f]);
-      else if (kind == 1) m = fmin(m, r[4 * f + 1]);
-      else if (kind == 2) k = ks_merge(k, KS{r[4 * f + 2], r[4 * f + 3]});
-      else if (kind == 3) k = ks_merge(k, KS{r[4 * F], r[4 * F + 1]});
-      else k = ks_merge(k, KS{r[4 * F + 2], r[4 * F + 3]});
-    }
+  if (tx == 0) {
 #pragma unroll
-    for (int off = 16; off > 0; off >>= 1) {
-      if (kind == 0) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, off));
-      else if (kind == 1) m = fmin(m, __shfl_xor_sync(0xffffffffu, m, off));
-      else k = shfl_ks(k, off);
+    for (int f = 0; f < F; f++) {
+      wmx[ty][f] = mx[f];
+      wmn[ty][f] = mn[f];
     }
-    if (lane == 0) res[q] = kind < 2 ? m : k.s + k.c;
+    wcnt[ty] = cnt;
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    for (int f = 0; f < F; f++) {
-      out[4 * f] = res[3 * f];
-      out[4 * f + 1] = res[3 * f + 1];
-      out[4 * f + 2] = res[3 * f + 2] * h3;
-      double e = (form == 0 && f >= ph.nac) ? res[3 * F + 1] : res[3 * F];
-      out[4 * f + 3] = e * h3;
+  double *dst = part + (long long)blockIdx.x * rec_len(F);
+  for (int q = ty; q < Q; q += EB / 32) {
+    KS s = {0.0, 0.0};
+#pragma unroll
+    for (int w = 0; w < EB / 32; w++) {
+      const double2 v = ks_of[q * EB + w * 32 + tx];
+      s = w == 0 ? KS{v.x, v.y} : ks_merge(s, KS{v.x, v.y});
+    }
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) s = shfl_ks(s, off);
+    if (tx == 0) {
+      if (q < F) {
+        long long top = wmx[0][q], low = wmn[0][q];
+        int count = wcnt[0];
+        for (int w = 1; w < EB / 32; w++) {
+          top = wmx[w][q] > top ? wmx[w][q] : top;
+          low = wmn[w][q] < low ? wmn[w][q] : low;
+          count += wcnt[w];
+        }
+        ks_add(s, (double)count);  // sum of (value + 1)
+        dst[4 * q] = key_value(top);
+        dst[4 * q + 1] = key_value(low);
+      }
+      const int at = q < F ? 4 * q + 2 : 4 * F + 2 * (q - F);
+      dst[at] = s.s;
+      dst[at + 1] = s.c;
+    }
+  }
+}
+
+// Final reduction over the block records: a block per quantity (per field max
+// and min together, per field vol, the two energies; blockIdx.y = run), so that
+// every quantity's FP64 merges have an SM's FP64 pipe to themselves; each thread
+// folds a fixed strided subset of the records, then the lanes, then the warps
+// (deterministic).  One block for all quantities took 15 us.
+constexpr int FT_THREADS = 128;
+__global__ void __launch_bounds__(FT_THREADS) energy_final_kernel(Phys ph, int form, const double *__restrict__ part,
+                                                                  int npart, double *__restrict__ out) {
+  const int F = ph.F, L = rec_len(F), q = blockIdx.x;
+  part += (long long)blockIdx.y * npart * L;
+  out += (long long)blockIdx.y * 4 * F;
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  if (q < F) {  // max and min
+    __shared__ long long sx[FT_THREADS / 32], sn[FT_THREADS / 32];
+    long long mx = order_key(-1.0e30), mn = order_key(1.0e30);
+    for (int b = tid; b < npart; b += FT_THREADS) {
+      const long long x = order_key(part[(long long)b * L + 4 * q]), m = order_key(part[(long long)b * L + 4 * q + 1]);
+      mx = x > mx ? x : mx;
+      mn = m < mn ? m : mn;
+    }
+    for (int off = 16; off > 0; off >>= 1) {
+      const long long x = __shfl_xor_sync(0xffffffffu, mx, off), m = __shfl_xor_sync(0xffffffffu, mn, off);
+      mx = x > mx ? x : mx;
+      mn = m < mn ? m : mn;
+    }
+    if (lane == 0) sx[wid] = mx, sn[wid] = mn;
+    __syncthreads();
+    if (tid == 0) {
+      for (int w = 1; w < FT_THREADS / 32; w++) {
+        mx = sx[w] > mx ? sx[w] : mx;
+        mn = sn[w] < mn ? sn[w] : mn;
+      }
+      out[4 * q] = key_value(mx);
+      out[4 * q + 1] = key_value(mn);
+    }
+    return;
+  }
+  const int s = q - F;  // field s's volume, or (s >= F) an energy
+  const int at = s < F ? 4 * s + 2 : 4 * F + 2 * (s - F);
+  if (s > F && form != 0) return;  // the separate CH energy belongs to form 0
+  __shared__ double2 sk[FT_THREADS / 32];
+  KS k = {0.0, 0.0};
+  for (int b = tid; b < npart; b += FT_THREADS) {
+    const double *r = part + (long long)b * L + at;
+    k = ks_merge(k, KS{r[0], r[1]});
+  }
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) k = shfl_ks(k, off);
+  if (lane == 0) sk[wid] = make_double2(k.s, k.c);
+  __syncthreads();
+  if (tid == 0) {
+    for (int w = 1; w < FT_THREADS / 32; w++) k = ks_merge(k, KS{sk[w].x, sk[w].y});
+    const double v = (k.s + k.c) * (ph.h[0] * ph.h[1] * ph.h[2]);
+    if (s < F) {
+      out[4 * s + 2] = v;
+    } else {
+      // energy 0 goes to every field (form 0: the order parameters), 1 to the conserved ones
+      for (int f = 0; f < F; f++)
+        if ((form == 0 && f >= ph.nac) == (s > F)) out[4 * f + 3] = v;
     }
   }
 }
@@ -735,11 +656,14 @@ static cudaError_t check_soln_pl(const Phys &ph, const T *u, const double *elam,
     const dim3 g(npart), b(32, 8);
     switch (ph.nac * 2 + ph.nch) {
 #define SCLET_F64Z(NA, NC) \
-  case NA * 2 + NC: energy_partial_f64z<PL, NA, NC><<<g, b, 0, s>>>(ph, ud, elam, form, partials); break;
+  case NA * 2 + NC:                                                                                         \
+    energy_partial_f64z<PL, NA, NC>                                                                         \
+        <<<g, b, sizeof(double2) * (NA + NC + 2) * EB, s>>>(ph, ud, elam, form, partials);                  \
+    break;
       SCLET_F64Z(0, 1) SCLET_F64Z(1, 0) SCLET_F64Z(1, 1) SCLET_F64Z(2, 0) SCLET_F64Z(2, 1)
       SCLET_F64Z(3, 0) SCLET_F64Z(3, 1) SCLET_F64Z(4, 0) SCLET_F64Z(4, 1)
 #undef SCLET_F64Z
-      default: energy_partial_kernel<PL, T><<<npart, EB, 0, s>>>(ph, u, elam, form, partials);
+      default: return cudaErrorInvalidValue;
     }
   }
   return cudaGetLastError();
@@ -755,7 +679,7 @@ cudaError_t launch_check_soln(const Phys &ph, const T *u, const double *elam, in
     return check_soln_pl<PL, T>(ph, u, elam, form, partials, npart, s);
   });
   if (e != cudaSuccess) return e;
-  energy_final_kernel<<<ph.runs > 1 ? ph.runs : 1, 32 * (3 * MAXF + 2), 0, s>>>(ph, form, partials, npart, out);
+  energy_final_kernel<<<dim3(2 * ph.F + 2, ph.runs > 1 ? ph.runs : 1), FT_THREADS, 0, s>>>(ph, form, partials, npart, out);
   launch_counter() += 2;
   return cudaGetLastError();
 }

@@ -60,23 +60,27 @@ struct Fs {
   }
 };
 
-// block-wide compensated reduction; thread 0 receives the pair
-__device__ Ks block_reduce(Ks v) {
-  __shared__ double sa[MB], sb[MB];
-  sa[threadIdx.x] = v.s;
-  sb[threadIdx.x] = v.c;
-  __syncthreads();
-  for (int w = MB / 2; w > 0; w >>= 1) {
-    if (threadIdx.x < w) {
-      double s, e;
-      two_sum(sa[threadIdx.x], sa[threadIdx.x + w], s, e);
-      sa[threadIdx.x] = s;
-      sb[threadIdx.x] = sb[threadIdx.x] + sb[threadIdx.x + w] + e;
-    }
-    __syncthreads();
+// Block-wide sum of the threads' pairs: exact-pair butterflies in FP32 (a
+// merge's rounding acts on the low halves only), the warps' pairs in FP64 in
+// order; thread 0 receives the pair.  (An FP64 tree over 256 threads is 70 warp
+// instructions of 16 cycles each on this GPU, more than the block's sums.)
+__device__ Ks block_reduce(Fs v) {
+  __shared__ Fs sw[MB / 32];
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) {
+    const float os = __shfl_xor_sync(0xffffffffu, v.s, off), oe = __shfl_xor_sync(0xffffffffu, v.e, off);
+    const float t = v.s + os, bp = t - v.s;
+    v.e = (v.e + oe) + ((v.s - (t - bp)) + (os - bp));
+    v.s = t;
   }
-  Ks r = {sa[0], sb[0]};
+  if ((threadIdx.x & 31) == 0) sw[threadIdx.x >> 5] = v;
   __syncthreads();
+  Ks r = {0.0, 0.0};
+  if (threadIdx.x == 0)
+    for (int w = 0; w < MB / 32; w++) {
+      r.add((double)sw[w].s);
+      r.c += (double)sw[w].e;
+    }
   return r;
 }
 
@@ -105,82 +109,131 @@ __global__ void seed_kernel(double *X, const double *g, int n, int which, const 
 }
 
 // Partial target per block: sum of wa*a (or of a over owned cells when wa is
-// null) plus sum of wb*(b - bsub).  Rows of x (z*n + y) are spread over the
-// grid; each thread accumulates an FP32 pair, and the blocks and the final
-// fold are compensated FP64.
+// null) plus sum of wb*(b - bsub).  Each thread takes cells a grid apart, four
+// at a time (their loads are in flight together), and accumulates an FP32 pair.
 __global__ void __launch_bounds__(MB) target_kernel(const float *__restrict__ a, const float2 *__restrict__ wa,
                                                     const float *__restrict__ b, const float *__restrict__ bsub,
                                                     const float2 *__restrict__ wb, int n, double *__restrict__ part) {
-  const int nrows = n * n;
+  constexpr int U = 4;
+  const long long n3 = (long long)n * n * n, stride = (long long)gridDim.x * MB;
   Fs acc = {0.0f, 0.0f};
-  for (int row = blockIdx.x; row < nrows; row += gridDim.x) {
-    const int z = row / n, y = row - z * n;
-    const bool own_row = y >= 2 && y < n - 2 && z >= 2 && z < n - 2;
-    const size_t l0 = (size_t)row * n;
-    for (int x = threadIdx.x; x < n; x += blockDim.x) {
-      const size_t l = l0 + x;
-      if (wa) acc.add_product(wa[l], a[l]);
-      else if (own_row && x >= 2 && x < n - 2) acc.add(a[l]);
-      if (bsub) acc.add_product_diff(wb[l], b[l], bsub[l]);
-      else acc.add_product(wb[l], b[l]);
+  for (long long l0 = blockIdx.x * (long long)MB + threadIdx.x; l0 < n3; l0 += U * stride) {
+    float va[U], vb[U], vs[U];
+    float2 pa[U], pb[U];
+#pragma unroll
+    for (int k = 0; k < U; k++) {
+      const long long l = l0 + k * stride;
+      const bool in = l < n3;
+      va[k] = in ? a[l] : 0.0f;
+      vb[k] = in ? b[l] : 0.0f;
+      pb[k] = in ? wb[l] : make_float2(0.0f, 0.0f);
+      vs[k] = in && bsub ? bsub[l] : 0.0f;
+      pa[k] = in && wa ? wa[l] : make_float2(0.0f, 0.0f);
+    }
+#pragma unroll
+    for (int k = 0; k < U; k++) {
+      if (wa) {
+        acc.add_product(pa[k], va[k]);
+      } else {
+        const long long l = l0 + k * stride;
+        const int row = (int)(l / n), x = (int)(l - (long long)row * n), z = row / n, y = row - z * n;
+        if (l < n3 && x >= 2 && x < n - 2 && y >= 2 && y < n - 2 && z >= 2 && z < n - 2) acc.add(va[k]);
+      }
+      if (bsub) acc.add_product_diff(pb[k], vb[k], vs[k]);
+      else acc.add_product(pb[k], vb[k]);
     }
   }
-  Ks r = block_reduce(Ks{(double)acc.s, (double)acc.e});
+  const Ks r = block_reduce(acc);
   if (threadIdx.x == 0) {
     part[2 * blockIdx.x] = r.s;
     part[2 * blockIdx.x + 1] = r.c;
+  }
+}
+
+// f(first cell, N, lane) for every owned row (z, y), a warp each
+template <typename F>
+__device__ __forceinline__ void owned_rows(int n, F &&f) {
+  const int N = n - 4, lane = threadIdx.x & 31;
+  const int warps = gridDim.x * (MB / 32);
+  for (int row = blockIdx.x * (MB / 32) + (threadIdx.x >> 5); row < N * N; row += warps) {
+    const int zz = row / N, y = 2 + row - zz * N, z = 2 + zz;
+    f(((size_t)z * n + y) * n + 2, N, lane);
   }
 }
 
 // Partial owned-cell sum of u per block.
 __global__ void __launch_bounds__(MB) owned_sum_kernel(const float *__restrict__ u, int n, double *__restrict__ part) {
   Fs acc = {0.0f, 0.0f};
-  const int N = n - 4;
-  for (int row = blockIdx.x; row < N * N; row += gridDim.x) {
-    const int zz = row / N, y = 2 + row - zz * N, z = 2 + zz;
-    const size_t l0 = ((size_t)z * n + y) * n + 2;
-    for (int x = threadIdx.x; x < N; x += blockDim.x) acc.add(u[l0 + x]);
-  }
-  Ks r = block_reduce(Ks{(double)acc.s, (double)acc.e});
+  owned_rows(n, [&](size_t l0, int N, int lane) {
+    for (int x0 = lane; x0 < N; x0 += 128) {
+      float v[4];
+#pragma unroll
+      for (int k = 0; k < 4; k++) v[k] = x0 + 32 * k < N ? u[l0 + x0 + 32 * k] : 0.0f;
+#pragma unroll
+      for (int k = 0; k < 4; k++) acc.add(v[k]);
+    }
+  });
+  const Ks r = block_reduce(acc);
   if (threadIdx.x == 0) {
     part[2 * blockIdx.x] = r.s;
     part[2 * blockIdx.x + 1] = r.c;
   }
 }
 
-__device__ double fold(const double *part, int np) {
+// One block folds both partial sets in a fixed order, half of its warps each,
+// and records (target, before, shift) in res.  Bound by FP64 instructions (64
+// cycles of a scheduler each): few warps, a pair's low half added plainly.
+constexpr int FB = 128;  // threads per set
+__global__ void __launch_bounds__(2 * FB) fold_kernel(int n, const double *__restrict__ tpart,
+                                                      const double *__restrict__ apart, int np,
+                                                      double *__restrict__ res) {
+  __shared__ double2 sw[2 * FB / 32];
+  const int set = threadIdx.x / FB, i = threadIdx.x % FB;
+  const double2 *part = reinterpret_cast<const double2 *>(set ? apart : tpart);
   Ks acc = {0.0, 0.0};
-  for (int q = threadIdx.x; q < np; q += blockDim.x) {
-    acc.add(part[2 * q]);
-    acc.add(part[2 * q + 1]);
+  for (int q = i; q < np; q += FB) {
+    const double2 v = part[q];
+    acc.add(v.x);
+    acc.c += v.y;
   }
-  Ks r = block_reduce(acc);
-  return r.s + r.c;
-}
-
-// One block folds both partial sets in a fixed order and records (target,
-// before, shift) in res.
-__global__ void __launch_bounds__(MB) fold_kernel(int n, const double *__restrict__ tpart,
-                                                  const double *__restrict__ apart, int np, double *__restrict__ res) {
-  const double T = fold(tpart, np);
-  const double A = fold(apart, np);
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) {
+    const double os = __shfl_xor_sync(0xffffffffu, acc.s, off), oc = __shfl_xor_sync(0xffffffffu, acc.c, off);
+    acc.add(os);
+    acc.c += oc;
+  }
+  if ((threadIdx.x & 31) == 0) sw[threadIdx.x >> 5] = make_double2(acc.s, acc.c);
+  __syncthreads();
   if (threadIdx.x == 0) {
+    double v[2];
+    for (int k = 0; k < 2; k++) {
+      Ks t = {0.0, 0.0};
+      for (int w = 0; w < FB / 32; w++) {
+        t.add(sw[k * (FB / 32) + w].x);
+        t.c += sw[k * (FB / 32) + w].y;
+      }
+      v[k] = t.s + t.c;
+    }
     const double N = n - 4;
-    res[0] = T;
-    res[1] = A;
-    res[2] = (T - A) / (N * N * N);
+    res[0] = v[0];
+    res[1] = v[1];
+    res[2] = (v[0] - v[1]) / (N * N * N);
   }
 }
 
 // the uniform shift res[2] on the owned cells
 __global__ void __launch_bounds__(MB) shift_kernel(float *__restrict__ u, int n, const double *__restrict__ res) {
   const float d = (float)res[2];
-  const int N = n - 4;
-  for (int row = blockIdx.x; row < N * N; row += gridDim.x) {
-    const int zz = row / N, y = 2 + row - zz * N, z = 2 + zz;
-    const size_t l0 = ((size_t)z * n + y) * n + 2;
-    for (int x = threadIdx.x; x < N; x += blockDim.x) u[l0 + x] += d;
-  }
+  owned_rows(n, [&](size_t l0, int N, int lane) {
+    for (int x0 = lane; x0 < N; x0 += 128) {
+      float v[4];
+#pragma unroll
+      for (int k = 0; k < 4; k++) v[k] = x0 + 32 * k < N ? u[l0 + x0 + 32 * k] : 0.0f;
+#pragma unroll
+      for (int k = 0; k < 4; k++)
+        if (x0 + 32 * k < N) u[l0 + x0 + 32 * k] = v[k] + d;
+    }
+  });
 }
 
 // FP64 weights -> FP32 (hi, lo) pairs in place
@@ -194,8 +247,11 @@ __global__ void to_pairs_kernel(double *w, long long count) {
 
 }  // namespace
 
-// sixteen blocks per SM: enough loads in flight to stream the block from HBM
-int mass_partials() { return 152 * 16; }
+// Four blocks per SM, each thread with four cells in flight.  (Sixteen blocks per
+// SM spent their time in their reductions and left 2432 pairs for the one block
+// that folds them: target, sum, fold and shift of a 196^3 block 44, 37, 31 and
+// 25 us, now 31, 16, 12 and 22.)
+int mass_partials() { return 152 * 4; }
 
 cudaError_t mass_weight(double *w, double *tmp, const double *g, const double *viT, int n, int which, const EtdCoef &ec,
                         cudaStream_t s, bool folded) {
@@ -230,8 +286,8 @@ cudaError_t mass_target(const float *a, const double *wa, const float *b, const 
 
 cudaError_t mass_fix(float *u, int n, const double *tpart, double *apart, double *res, cudaStream_t s) {
   owned_sum_kernel<<<mass_partials(), MB, 0, s>>>(u, n, apart);
-  fold_kernel<<<1, MB, 0, s>>>(n, tpart, apart, mass_partials(), res);
-  shift_kernel<<<mass_partials(), MB, 0, s>>>(u, n, res);
+  fold_kernel<<<1, 2 * FB, 0, s>>>(n, tpart, apart, mass_partials(), res);
+  shift_kernel<<<mass_partials() * 2, MB, 0, s>>>(u, n, res);
   launch_counter() += 3;
   return cudaGetLastError();
 }

@@ -16,6 +16,8 @@
 //   (ch_mu, trans.c:1433-1937).
 // AC_f and CH_f come from the run's physics plugin (the drop-in form of
 // formula.c:9-56, sclet_physics.cuh), a template parameter of every kernel.
+#include <algorithm>
+
 #include "sclet_internal.cuh"
 #include "sclet_physics.cuh"
 
@@ -686,16 +688,16 @@ __global__ void __launch_bounds__(RX * RY) mob_n_kernel(P<T> p0, const T *__rest
 // T_a the second difference along axis a with zero values outside the block
 // (the operator the eigenbasis diagonalises).  A thread marches an (x, y)
 // column; differences are taken first, so a smooth field loses no digits.
-// blockIdx.z = (run, field) x chunk of planes.  Bound by HBM (u and N read, r
-// written).
+// q0 + blockIdx.z = (run, field) x chunk of planes.  Bound by HBM (u and N read,
+// r written).
 template <typename T>
 __global__ void __launch_bounds__(RX * RY) increment_rhs_kernel(P<T> p, const T *__restrict__ u,
                                                                 const T *__restrict__ rhs, T *__restrict__ r, T cx, T cy,
-                                                                T cz) {
+                                                                T cz, int q0) {
   const int n = p.n;
   const size_t nn = (size_t)n * n, n3 = nn * n;
-  const int zch = (n + p.zc - 1) / p.zc;
-  const int t = blockIdx.z / zch, zci = blockIdx.z - t * zch;  // t = run nac + m
+  const int zch = (n + p.zc - 1) / p.zc, q = q0 + blockIdx.z;
+  const int t = q / zch, zci = q - t * zch;  // t = run nac + m
   const int x = blockIdx.x * RX + threadIdx.x, y = blockIdx.y * RY + threadIdx.y;
   if (x >= n || y >= n) return;
   const size_t f = (size_t)(t / p.nac) * p.F + t % p.nac;
@@ -723,6 +725,7 @@ static int planes_per_cta(const Phys &ph, int tuned, int zmax, int runs) {
   if (tuned > 0) return tuned;
   const long long tiles = (long long)((ph.n + RX - 1) / RX) * ((ph.n + RY - 1) / RY) * runs;
   int zc = zmax;
+  if ((long long)((ph.n + zc - 1) / zc) * runs > 32767) zc = 32;  // the grid's z extent
   while (zc > 2 && tiles * ((ph.n + zc - 1) / zc) < 4 * 152) zc /= 2;
   return zc;
 }
@@ -734,9 +737,12 @@ cudaError_t launch_increment_rhs(const Phys &ph, const T *u, const T *rhs, T *r,
   p.zc = planes_per_cta(ph, 0, 16, count);
   T c[3];
   for (int a = 0; a < 3; a++) c[a] = (T)(ph.LE * ph.epn2 * ph.kk[a] / (ph.h[a] * ph.h[a]));
-  increment_rhs_kernel<T><<<dim3(gx, gy, ((ph.n + p.zc - 1) / p.zc) * count), dim3(RX, RY), 0, s>>>(p, u, rhs, r, c[0],
-                                                                                                  c[1], c[2]);
-  launch_counter()++;
+  const int total = ((ph.n + p.zc - 1) / p.zc) * count;
+  for (int q0 = 0; q0 < total; q0 += 65535) {  // the grid's z extent
+    increment_rhs_kernel<T><<<dim3(gx, gy, std::min(65535, total - q0)), dim3(RX, RY), 0, s>>>(p, u, rhs, r, c[0], c[1],
+                                                                                             c[2], q0);
+    launch_counter()++;
+  }
   return cudaGetLastError();
 }
 template cudaError_t launch_increment_rhs<double>(const Phys &, const double *, const double *, double *, cudaStream_t);
@@ -749,7 +755,7 @@ static cudaError_t launch_rhs_pl(const Phys &ph, const T *u, const T *felas, T *
   const int gx = (ph.n + RX - 1) / RX, gy = (ph.n + RY - 1) / RY;
   const dim3 blk(RX, RY), grd(gx, gy, ((ph.n + PZ - 1) / PZ) * p.runs);
   // CTAs (in z) for the face cells of the kernels that take them apart
-  const int zface = (int)(((long long)face_cells(ph.n) * p.runs + RX * RY * gx * gy - 1) / ((long long)RX * RY * gx * gy));
+  const int zfaces = (int)(((long long)face_cells(ph.n) * p.runs + RX * RY * gx * gy - 1) / ((long long)RX * RY * gx * gy));
   if (ph.nac > 0) {
     bool diag = true;  // every gradient tensor diagonal
     for (int m = 0; m < ph.nac; m++)
@@ -757,6 +763,7 @@ static cudaError_t launch_rhs_pl(const Phys &ph, const T *u, const T *felas, T *
     const bool ring = ph.anisotropic && !diag;
     p.zc = planes_per_cta(ph, ph.rhs_zc, ph.anisotropic ? 32 : 8, p.runs);
     const int zblocks = ((ph.n + p.zc - 1) / p.zc) * p.runs;
+    const int zface = std::min(zfaces, 65535 - zblocks);  // the face cells' loop covers the rest
     const size_t smem = sizeof(T) * ph.nac * 5 * PLANE;
     cudaError_t e = cudaSuccess;
     switch (ph.nac * 3 + (ring ? 2 : ph.anisotropic ? 1 : 0)) {
@@ -792,7 +799,7 @@ static cudaError_t launch_rhs_pl(const Phys &ph, const T *u, const T *felas, T *
       // one conserved field (the plugins' CH_f is defined for c_0 only)
       p.zc = planes_per_cta(ph, 0, 16, p.runs);
       const int zblocks = ((ph.n + p.zc - 1) / p.zc) * p.runs;
-      const dim3 gch(gx, gy, zblocks + zface);
+      const dim3 gch(gx, gy, zblocks + zfaces);
       rhs_ch_t_kernel<PL, T><<<gch, blk, 0, s>>>(p, u, scratch, zblocks);
       rhs_ch_lap_kernel<PL, T><<<gch, blk, 0, s>>>(p, u, scratch, out + (long long)ph.nac * n3, zblocks);  // per run: + r F n^3
       launch_counter() += 2;

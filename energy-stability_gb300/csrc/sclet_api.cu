@@ -45,10 +45,12 @@ struct sclet_ctx {
   // shared
   double *dd[3] = {nullptr, nullptr, nullptr};  // eigenvalues / h^2 (FP64)
   double *elam = nullptr, *partials = nullptr;
-  // the diagnostics record: page-locked host memory mapped into the device,
-  // written by the reduction kernel, so reading it needs no copy (a copy would
-  // queue behind large transfers on the copy engines)
-  double *diag_host = nullptr, *diag = nullptr;
+  // the diagnostics record on the device (written by every step's reduction)
+  // and page-locked host memory mapped into the device, which a kernel fills
+  // when the record is read: a reduction that writes host memory itself ends
+  // about 10 us later, every step, and a copy would queue behind large transfers
+  // on the copy engines
+  double *diag = nullptr, *diag_host = nullptr, *diag_mapped = nullptr;
   int npart = 0;
   ElasticPlan *elastic = nullptr;
   int *dev_err = nullptr;  // bounded-wait failures of device kernels
@@ -516,7 +518,7 @@ void sclet_destroy(sclet_ctx *ctx) {
                   ctx->coef[0], ctx->coef[1], ctx->coef1[0], ctx->coef1[1], ctx->coef2[0],
                   ctx->coef2[1], ctx->massW, ctx->massPart,
                   ctx->massRes, ctx->in_stage, ctx->out_stage, ctx->krun, ctx->mob_t, ctx->mob_part, ctx->foldVi,
-                  ctx->foldV};
+                  ctx->foldV, ctx->diag};
   for (void *b : bufs) cudaFree(b);
   if (ctx->diag_host) cudaFreeHost(ctx->diag_host);
   for (int a = 0; a < 3; a++) {
@@ -643,7 +645,9 @@ int sclet_create_runs(const sclet_params *p, int runs, const double *krun, int p
     CC(cudaMemcpy(ctx->krun, krun, sizeof(double) * runs, cudaMemcpyHostToDevice));
     ph.krun = ctx->krun;
   }
-  CC(cudaHostGetDevicePointer(&ctx->diag, ctx->diag_host, 0));
+  CC(cudaHostGetDevicePointer(&ctx->diag_mapped, ctx->diag_host, 0));
+  CC(cudaMalloc(&ctx->diag, sizeof(double) * 4 * FT));
+  CC(cudaMemsetAsync(ctx->diag, 0, sizeof(double) * 4 * FT, s));
   CC(cudaMalloc(&ctx->dev_err, sizeof(int)));
   CC(cudaMemsetAsync(ctx->dev_err, 0, sizeof(int), s));
   const int nfel = ctx->nac > 0 ? ctx->nac : 1;
@@ -1243,8 +1247,15 @@ int queue_diagnostics(sclet_ctx *ctx, int energy_form) {
   return SCLET_OK;
 }
 
+__global__ void record_kernel(const double *__restrict__ record, double *__restrict__ host, int count) {
+  for (int i = threadIdx.x; i < count; i += blockDim.x) host[i] = record[i];
+}
+
 // waits for the stream and copies the last diagnostics record out
 int read_diagnostics(sclet_ctx *ctx, sclet_diag *out) {
+  record_kernel<<<1, 256, 0, ctx->stream>>>(ctx->diag, ctx->diag_mapped, 4 * ctx->FT);
+  launch_counter()++;
+  CK(cudaGetLastError());
   CK(cudaStreamSynchronize(ctx->stream));
   const double *h = ctx->diag_host;
   int nonfinite = 0;
