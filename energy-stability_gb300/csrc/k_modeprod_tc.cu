@@ -527,49 +527,53 @@ __device__ __forceinline__ uint32_t bf16_pair(float lo, float hi) {
 //        tensors t < sp.nI, e u^ + phi1 N^ for the others (u^ the block t, N^
 //        the block t + count - nI)
 // A CTA takes SLICE_ROWS lines of one tensor, the tensors of the same lines in
-// neighbouring CTAs (the coefficients of MODE 2 come from HBM about once).
-// 4 B read and 8 B written per element: HBM is the bound once the
-// instructions per element are few (about 30: digits by FMA and add instead of
-// a conversion, BF16 by byte permute, scales from exponent bits, no division).
+// neighbouring CTAs (the coefficients of MODE 2 come from HBM about once).  A
+// line is held in registers, all its loads in flight at once.  (Reading it twice
+// instead, for its maxima and from L1 for its digits, let five CTAs fit an SM
+// but waited longer: 0.86 ms a step at 196^3 against 0.72.)  Bound by HBM and
+// its write pattern: 4 B read and 8 B written per element.
 constexpr int SLICE_ROWS = 64;
 
 template <int C, int MODE>
-__global__ void __launch_bounds__(256) slice_fold_kernel(TensorList<float> xs, const float *__restrict__ sub,
-                                                         float *__restrict__ scale, __nv_bfloat16 *__restrict__ out,
-                                                         int n, int kp, int count, int bits, SpecUpdate sp) {
+__global__ void __launch_bounds__(256)
+    slice_fold_kernel(TensorList<float> xs, const float *__restrict__ sub, float *__restrict__ scale,
+                      __nv_bfloat16 *__restrict__ out, int n, int kp, int count, int bits, SpecUpdate sp) {
   const float step = ldexpf(1.0f, bits), step4 = ldexpf(1.0f, 4 * bits);
   const int rows = n * n;
   const long long n3 = (long long)rows * n;
   const int lane = threadIdx.x & 31, hw = lane >> 4, kl = 2 * (lane & 15);
-  const int h = fold_half(n), odd0 = fold_mode0(n, 1);
+  const int h = fold_half(n), h16 = (h + 15) / 16 * 16, odd0 = fold_mode0(n, 1);
   const int align = n % 4 == 0 ? 4 : n % 2 == 0 ? 2 : 1;  // values per aligned load of a line
   const int t = blockIdx.x % count, rb = blockIdx.x / count;
   const float *xt = xs.at(t, n3);
   const float *st = sub ? sub + t * n3 : nullptr;
-  const uint32_t plane = (uint32_t)rows * (uint32_t)kp, chunk = (uint32_t)rows * BK;
-  __nv_bfloat16 *ot = out + 2LL * t * TC_PLANES * plane;
+  // one base per part and plane (32-bit byte offsets within a plane)
+  const long long plane = (long long)rows * kp * 2;
+  char *base[2][TC_PLANES];
+#pragma unroll
+  for (int q = 0; q < 2; q++)
+#pragma unroll
+    for (int p = 0; p < TC_PLANES; p++)
+      base[q][p] = reinterpret_cast<char *>(out) + ((2LL * t + q) * TC_PLANES + p) * plane;
+  const uint32_t chunk = (uint32_t)rows * BK * 2;
   // MODE 2
   const bool etd = MODE == 2 && t >= sp.nI;
   const float4 *ce = MODE == 2 ? sp.etd[t % sp.F >= sp.nac ? 1 : 0] : nullptr;
   const float2 *cp = MODE == 2 ? sp.phi[t % sp.F >= sp.nac ? 1 : 0] : nullptr;
   const long long nhat = (long long)(count - sp.nI) * n3;  // from u^ to N^
+  const int mid = MODE == 0 && align == 1 ? h - 1 : -1;    // an odd block's middle cell
   const int row_end = min(rows, (rb + 1) * SLICE_ROWS);
   for (int row0 = rb * SLICE_ROWS + (threadIdx.x >> 5) * 2; row0 < row_end; row0 += 16) {
     const int row = row0 + hw;
     const bool live = row < row_end;
     const long long l0 = (long long)(live ? row : row0) * n;
     const float *x = xt + l0;
-    // MODE 0: a = x[k], x[k+1], b = their mirrors; else a = the even part's
-    // two modes, b = the odd part's
-    float a0[C], a1[C], b0[C], b1[C];
-    float me = 0.0f, mo = 0.0f;
-#pragma unroll
-    for (int c = 0; c < C; c++) {
-      const int k = kl + BK * c;
-      a0[c] = a1[c] = b0[c] = b1[c] = 0.0f;
-      if (k >= h) continue;
+    // columns k, k + 1 (k < h): MODE 0: a = x[k], x[k+1], b = their mirrors; else
+    // a = the even part's two modes, b = the odd part's
+    auto load = [&](int k, float &a0, float &a1, float &b0, float &b1) {
       if (MODE == 0) {
         const int q = n - 1 - k;
+        a1 = b1 = 0.0f;
         if (align >= 2) {  // n even: pairs and their mirrors aligned, no middle cell
           float2 a = *reinterpret_cast<const float2 *>(x + k), b = *reinterpret_cast<const float2 *>(x + q - 1);
           if (st) {
@@ -580,27 +584,22 @@ __global__ void __launch_bounds__(256) slice_fold_kernel(TensorList<float> xs, c
             b.x -= s2.x;
             b.y -= s2.y;
           }
-          a0[c] = a.x;
-          b0[c] = b.y;
-          if (k + 1 < h) {
-            a1[c] = a.y;
-            b1[c] = b.x;
-          }
+          a0 = a.x;
+          b0 = b.y;
+          if (k + 1 < h) a1 = a.y, b1 = b.x;
         } else {
           auto one = [&](int i) { return st ? x[i] - st[l0 + i] : x[i]; };
-          a0[c] = one(k);
-          if (q != k) b0[c] = one(q);
+          a0 = one(k);
+          b0 = q != k ? one(q) : 0.0f;
           if (k + 1 < h) {
-            a1[c] = one(k + 1);
-            if (q - 1 != k + 1) b1[c] = one(q - 1);
+            a1 = one(k + 1);
+            if (q - 1 != k + 1) b1 = one(q - 1);
           }
         }
-        me = fmaxf(me, fmaxf(fabsf(a0[c] + b0[c]), fabsf(a1[c] + b1[c])));
-        mo = fmaxf(mo, fmaxf(fabsf(a0[c] - b0[c]), fabsf(a1[c] - b1[c])));
       } else {
         const int k2 = 2 * k;
         float v[4];
-        auto load = [&](const float *p, float (&w)[4]) {
+        auto four = [&](const float *p, float (&w)[4]) {
           if (align == 4) {  // then k2 + 3 < n
             const float4 f = *reinterpret_cast<const float4 *>(p + k2);
             w[0] = f.x, w[1] = f.y, w[2] = f.z, w[3] = f.w;
@@ -612,11 +611,11 @@ __global__ void __launch_bounds__(256) slice_fold_kernel(TensorList<float> xs, c
             for (int i = 0; i < 4; i++) w[i] = k2 + i < n ? p[k2 + i] : 0.0f;
           }
         };
-        load(x, v);
+        four(x, v);
         if (MODE == 2) {
           if (etd) {
             float nh[4];
-            load(x + nhat, nh);
+            four(x + nhat, nh);
 #pragma unroll
             for (int i = 0; i < 4; i++)
               if (k2 + i < n) {
@@ -638,24 +637,29 @@ __global__ void __launch_bounds__(256) slice_fold_kernel(TensorList<float> xs, c
             for (int i = 0; i < 4; i++) v[i] = fmaf(f[i].x, v[i], f[i].y * v[i]);  // (phi_hi, phi_lo)
           }
         }
-        a0[c] = odd0 ? v[0] : v[1];
-        a1[c] = odd0 ? v[2] : v[3];
-        b0[c] = odd0 ? v[1] : v[0];
-        b1[c] = odd0 ? v[3] : v[2];
+        a0 = odd0 ? v[0] : v[1];
+        a1 = odd0 ? v[2] : v[3];
+        b0 = odd0 ? v[1] : v[0];
+        b1 = odd0 ? v[3] : v[2];
+      }
+    };
+    float a0[C], a1[C], b0[C], b1[C];
+#pragma unroll
+    for (int c = 0; c < C; c++) {
+      a0[c] = a1[c] = b0[c] = b1[c] = 0.0f;
+      if (kl + BK * c < h) load(kl + BK * c, a0[c], a1[c], b0[c], b1[c]);
+    }
+    float me = 0.0f, mo = 0.0f;
+#pragma unroll
+    for (int c = 0; c < C; c++) {
+      const int k = kl + BK * c;
+      if (MODE == 0) {
+        me = fmaxf(me, fmaxf(fabsf(a0[c] + b0[c]), fabsf(a1[c] + b1[c])));
+        // the middle cell is in the even part only
+        mo = fmaxf(mo, fmaxf(k == mid ? 0.0f : fabsf(a0[c] - b0[c]), k + 1 == mid ? 0.0f : fabsf(a1[c] - b1[c])));
+      } else {
         me = fmaxf(me, fmaxf(fabsf(a0[c]), fabsf(a1[c])));
         mo = fmaxf(mo, fmaxf(fabsf(b0[c]), fabsf(b1[c])));
-      }
-    }
-    // an odd block's middle cell is in the even part only: its difference with
-    // the missing mirror must not enter the odd one
-    const int mid = MODE == 0 && align == 1 ? h - 1 : -1;
-    if (mid >= 0 && (mid & ~1) % BK == kl) {
-      mo = 0.0f;
-#pragma unroll
-      for (int c = 0; c < C; c++) {
-        const int k = kl + BK * c;
-        if (k != mid) mo = fmaxf(mo, fabsf(a0[c] - b0[c]));
-        if (k + 1 != mid) mo = fmaxf(mo, fabsf(a1[c] - b1[c]));
       }
     }
 #pragma unroll
@@ -671,19 +675,19 @@ __global__ void __launch_bounds__(256) slice_fold_kernel(TensorList<float> xs, c
       scale[2LL * t * rows + row] = Se;
       scale[(2LL * t + 1) * rows + row] = So;
     }
-    // 32-bit offsets within a part (4 n^2 kp < 2^32)
-    uint32_t o = (uint32_t)row * BK + kl;
+    uint32_t o = ((uint32_t)row * BK + kl) * 2;
+    // up to a multiple of 16 columns, the last ones zero: whole 32-byte sectors
+    // (a few columns' partial sectors per line and plane, as every edge of N + 4
+    // has, cost more than their line)
 #pragma unroll
     for (int c = 0; c < C; c++, o += chunk) {
       const int k = kl + BK * c;
-      if (k >= h) continue;
+      if (k >= h16) break;
       float d0[TC_PLANES], d1[TC_PLANES];
-      auto put = [&](__nv_bfloat16 *base) {
+      auto put = [&](int q) {
 #pragma unroll
-        for (int p = 0; p < TC_PLANES; p++)
-          *reinterpret_cast<uint32_t *>(base + (o + (uint32_t)p * plane)) = bf16_pair(d0[p], d1[p]);
+        for (int p = 0; p < TC_PLANES; p++) *reinterpret_cast<uint32_t *>(base[q][p] + o) = bf16_pair(d0[p], d1[p]);
       };
-      __nv_bfloat16 *oo = ot + (long long)TC_PLANES * plane;
       if (MODE == 0) {
         // TwoSum (Knuth) of the pair and its difference
         auto fold = [&](float a, float b, float inv, float (&d)[TC_PLANES]) {
@@ -693,17 +697,17 @@ __global__ void __launch_bounds__(256) slice_fold_kernel(TensorList<float> xs, c
         };
         fold(a0[c], b0[c], ie, d0);
         fold(a1[c], b1[c], ie, d1);
-        put(ot);
+        put(0);
         fold(k == mid ? 0.0f : a0[c], k == mid ? 0.0f : -b0[c], io, d0);
         fold(k + 1 == mid ? 0.0f : a1[c], k + 1 == mid ? 0.0f : -b1[c], io, d1);
-        put(oo);
+        put(1);
       } else {
         digits(a0[c] * ie, 0.0f, step, step4, d0);
         digits(a1[c] * ie, 0.0f, step, step4, d1);
-        put(ot);
+        put(0);
         digits(b0[c] * io, 0.0f, step, step4, d0);
         digits(b1[c] * io, 0.0f, step, step4, d1);
-        put(oo);
+        put(1);
       }
     }
   }
@@ -823,27 +827,31 @@ cudaError_t tc_slice_fields(const float *x, const float *sub, float *scale, __nv
 
 template <int MODE>
 static void run_slice_fold(int chunks, int g, const TensorList<float> &x, const float *sub, float *scale,
-                           __nv_bfloat16 *planes, int n, int count, const SpecUpdate &sp, cudaStream_t s) {
-  const int h = fold_half(n), kp = tc_kp(h), bits = tc_slice_bits(h);
+                           __nv_bfloat16 *planes, int n, int kp, int count, int bits, const SpecUpdate &sp,
+                           cudaStream_t s) {
 #define SCLET_SLICE(C) tc::slice_fold_kernel<C, MODE><<<g, 256, 0, s>>>(x, sub, scale, planes, n, kp, count, bits, sp)
   if (chunks <= 1) SCLET_SLICE(1);
   else if (chunks <= 2) SCLET_SLICE(2);
+  else if (chunks <= 3) SCLET_SLICE(3);
   else if (chunks <= 4) SCLET_SLICE(4);
   else if (chunks <= 5) SCLET_SLICE(5);
+  else if (chunks <= 7) SCLET_SLICE(7);
   else if (chunks <= 9) SCLET_SLICE(9);
+  else if (chunks <= 12) SCLET_SLICE(12);
   else SCLET_SLICE(17);
 #undef SCLET_SLICE
 }
 
 cudaError_t tc_slice_fold(bool forward, const TensorList<float> &x, const float *sub, const SpecUpdate *sp, float *scale,
                           __nv_bfloat16 *planes, int n, int count, cudaStream_t s) {
-  const int chunks = (fold_half(n) + tc::BK - 1) / tc::BK;
-  if (chunks > 17) return cudaErrorInvalidValue;
+  const int h = fold_half(n), kp = tc_kp(h), bits = tc_slice_bits(h);
   const long long g = ((long long)n * n + tc::SLICE_ROWS - 1) / tc::SLICE_ROWS * count;
-  if (g > 0x7fffffffLL) return cudaErrorInvalidValue;
-  if (forward) run_slice_fold<0>(chunks, (int)g, x, sub, scale, planes, n, count, SpecUpdate(), s);
-  else if (!sp) run_slice_fold<1>(chunks, (int)g, x, nullptr, scale, planes, n, count, SpecUpdate(), s);
-  else run_slice_fold<2>(chunks, (int)g, x, nullptr, scale, planes, n, count, *sp, s);
+  // 32-bit row numbers, and byte offsets within a plane
+  if (g > 0x7fffffffLL || (long long)n * n * kp * 2 > 0xffffffffLL || kp > 17 * tc::BK) return cudaErrorInvalidValue;
+  const int chunks = kp / tc::BK;
+  if (forward) run_slice_fold<0>(chunks, (int)g, x, sub, scale, planes, n, kp, count, bits, SpecUpdate(), s);
+  else if (!sp) run_slice_fold<1>(chunks, (int)g, x, nullptr, scale, planes, n, kp, count, bits, SpecUpdate(), s);
+  else run_slice_fold<2>(chunks, (int)g, x, nullptr, scale, planes, n, kp, count, bits, *sp, s);
   launch_counter()++;
   return cudaGetLastError();
 }
