@@ -25,23 +25,27 @@
 // outlier costs precision only within itself.  The scale of an output entry
 // is rank one (matrix row a' times input row r), so accumulation stays exact.
 //
-// Layout: input planes P[t][p][kb][r][32], k-blocked: rows r = 0 .. n*n-1 are
-// 1-D lines along the contracted axis, k = 32 kb + (k % 32) < kp = roundup(n,
-// 32), zero beyond n; one k-block of 128 consecutive rows is one contiguous
-// 8 KB tile, so every TMA load reads whole 128-byte lines.  Matrix slices
-// likewise [p][kb][a'][32].  Output FP32
+// Layout: input slices P[t][part][r / 128][kb][p][r % 128][32]: rows r = 0 ..
+// n*n-1 are 1-D lines along the contracted axis, k = 32 kb + (k % 32) < kp =
+// roundup(n, 32), zero beyond n.  The four slices of one k-block of a tile of
+// 128 lines are one contiguous run of 32 KB, already in the 64-byte swizzle that
+// the MMAs read, so one bulk copy brings a stage's input operand and one the
+// matrix slices (40 KB, likewise [a' / 128][kb][p][a' % 128][32]); nine tensor
+// copies of 64-byte rows kept the copy engine busy for 1600 cycles a stage, with
+// the MMAs waiting.  Output FP32
 // out[t][a' * n*n + r] for input row r = c * n + b, i.e. contracted index
 // slowest: three products return to x-fastest order.
 //
 // Kernel: persistent CTAs (one per SM) looping over output tiles D[128 r x
 // 128 a'] (input rows on the MMA's M side, eigen-modes a' on its N side, so
 // the last a'-tile runs N = its live rows rounded up to 16 rather than a full
-// 128).  A CTA takes whole groups (every a'-tile of one input tile, a'-tiles
-// fastest, groups round robin, tensor fastest), so the CTAs stay balanced,
-// the input slices come from HBM once (the group's later a'-tiles read them
-// from L2) and the tensors of one input tile share the fused update's
-// coefficient reads through L2; the matrix slices stay in L2.  Every CTA loads its own operand tiles (no
-// cluster).
+// 128).  Tiles are dealt round robin, a'-tile fastest, then tensor
+// (cta_tile): the input slices come from HBM once, the a'-tiles of one input
+// tile reading them at about the same time on neighbouring CTAs, and the
+// tensors of one input tile share the fused update's coefficient reads through
+// L2; the matrix slices stay in L2.  Every CTA loads its own operand tiles (no
+// cluster).  The order of tiles and the copies in whole runs: 4 + 1 fields of
+// 516^3 24.9 -> 20.8 ms a step, of 196^3 0.98 -> 0.84 ms.
 // A = input slices (128 r rows x 32 k, 64-byte swizzle), B = matrix slices
 // (128 a' rows x 32 k), both K-major, in a three-stage mbarrier pipeline
 // that runs ahead across tiles; a stage is refilled once the MMAs that read
@@ -49,9 +53,9 @@
 // The folded forms (the default basis) halve the MMAs of a product and, with
 // the increment form, a field needs six products instead of nine.  Kernel time
 // of a step, dense and nine products before, now: 4 + 1 fields of 516^3
-// 52.8 -> 24.6 ms, of 196^3 1.64 -> 0.96 ms, 4 fields of 68^3 124 -> 78 us; the
+// 52.8 -> 20.8 ms, of 196^3 1.64 -> 0.84 ms, 4 fields of 68^3 124 -> 72 us; the
 // step's error against 64 bits fell from 2.2e-7 to 0.6e-7 (196^3, ten steps).
-// Warp 0 issues TMA, warp 1 issues MMAs (one elected thread each) and owns the
+// Warp 0 issues the copies, warp 1 issues MMAs (one elected thread each) and owns the
 // tensor memory (4 classes x 128 columns).  Warps 2-5 run the epilogue (TMEM
 // lane quadrant warp % 4): the four classes of the tile are combined into
 // registers and the tensor memory is released at once, then the scaling, the
@@ -60,11 +64,8 @@
 // next tile's MMAs.  Every mbarrier wait is bounded: on timeout the CTA
 // records an error, drains its copies and MMAs (bounded), frees TMEM and
 // returns.
-#include <cuda.h>
 #include <cuda_bf16.h>
-#include <cudaTypedefs.h>
 #include <stdint.h>
-#include <string.h>
 
 #include <mutex>
 
@@ -79,8 +80,8 @@ namespace tc {
 
 // FORM 0: any basis.  FORM 1, 2: the parity-folded forward and inverse products
 // of the Dirichlet basis (sclet_basis.cu): the sliced lines and the matrix come
-// in two parts (even, odd modes) of h = ceil(n / 2) columns, a group's tiles run
-// over a'-tiles of h with the part fastest.  The forward epilogue interleaves
+// in two parts (even, odd modes) of h = ceil(n / 2) columns, a tile's parts one
+// after the other.  The forward epilogue interleaves
 // the parts' modes; the inverse one keeps the even part's tile E in registers
 // until the odd part's O is there and stores E + O and E - O.
 // EPI 0 store, 1 ETD1 update, 2 phi scaling (FORM 0; the folded transforms apply
@@ -91,7 +92,7 @@ namespace tc {
 // 64, for halves up to 64, two accumulator sets alternate.
 template <int FORM, int EPI, int OUT, int BN>
 __global__ void __launch_bounds__(THREADS, 1)
-    modeprod_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, TcArgs g) {
+    modeprod_tc_kernel(const char *__restrict__ planes, const char *__restrict__ mat, TcArgs g) {
   using G = TileGeom<BN>;
   constexpr int STAGES = G::STAGES, STAGE_BYTES = G::STAGE_BYTES, PLANE_B = G::PLANE_B, NBUF = G::NBUF;
   constexpr int ACC_COLS = G::ACC_COLS, TMEM_COLS = G::TMEM_COLS, CPW = G::CPW;
@@ -110,12 +111,11 @@ __global__ void __launch_bounds__(THREADS, 1)
   constexpr int PARTS = FORM == 0 ? 1 : 2;
   const int h = FORM == 0 ? g.n : fold_half(g.n);  // outputs of one part
   const int a_tiles = (h + BN - 1) / BN;
-  const int units = a_tiles * PARTS;
   const int r_tiles = (int)((rows + BM - 1) / BM);
-  // whole groups (every a'-tile of one input tile) per CTA, round robin
-  const int groups = r_tiles * g.count;
-  const int mine = (int)blockIdx.x < groups ? units * ((groups - 1 - (int)blockIdx.x) / (int)gridDim.x + 1) : 0;
+  const int tiles = r_tiles * g.count * a_tiles;  // dealt round robin (cta_tile)
+  const int mine = (int)blockIdx.x < tiles ? PARTS * ((tiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1) : 0;
   const int nkb = g.kblocks;
+  const int last_rows = (h - (a_tiles - 1) * BN + 15) / 16 * 16;  // N of the last a'-tile, at most BN
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; s++) {
@@ -158,14 +158,19 @@ __global__ void __launch_bounds__(THREADS, 1)
           }
           if (*(volatile int *)&failed) break;
           uint8_t *st = base + s * STAGE_BYTES;
-          mbar_expect_tx(&full_bar[s], STAGE_BYTES);
-          // k-block kb of plane z is the contiguous block z * nkb + kb
-          for (int p = 0; p < NP; p++)
-            tma_load_3d(st + p * PLANE_A, &tmA, 0, ti.r_tile * BM, ((ti.t * PARTS + ti.part) * NP + p) * nkb + kb,
-                        &full_bar[s]);
-          for (int p = 0; p < NPM; p++)
-            tma_load_3d(st + NP * PLANE_A + p * PLANE_B, &tmB, 0, ti.a_tile * BN, (ti.part * NPM + p) * nkb + kb,
-                        &full_bar[s]);
+          const uint32_t b_rows = ti.a_tile == a_tiles - 1 ? last_rows : BN;
+          mbar_expect_tx(&full_bar[s], NP * PLANE_A + NPM * (b_rows * BK * 2));
+          // a k-block's input slices are one run, and so are its matrix
+          // slices, of which the last a'-tile takes the rows it multiplies
+          bulk_load(st, planes + ((((long long)ti.t * PARTS + ti.part) * r_tiles + ti.r_tile) * nkb + kb) * (NP * PLANE_A),
+                    NP * PLANE_A, &full_bar[s]);
+          const char *mb = mat + (((long long)ti.part * a_tiles + ti.a_tile) * nkb + kb) * (NPM * PLANE_B);
+          if (b_rows == BN) {
+            bulk_load(st + NP * PLANE_A, mb, NPM * PLANE_B, &full_bar[s]);
+          } else {
+            for (int p = 0; p < NPM; p++)
+              bulk_load(st + NP * PLANE_A + p * PLANE_B, mb + p * PLANE_B, b_rows * BK * 2, &full_bar[s]);
+          }
         }
         if (*(volatile int *)&failed) break;
       }
@@ -182,9 +187,8 @@ __global__ void __launch_bounds__(THREADS, 1)
     // last a'-tile runs N = its rows rounded up to 16.  The warp runs the loop
     // together, one lane issues (mma_bf16_from).
     const bool issue = elect_one();
-    const int last_cols = h - (a_tiles - 1) * BN;
     const uint32_t idesc_full = idesc_bf16(BM, BN);
-    const uint32_t idesc_last = idesc_bf16(BM, (last_cols + 15) / 16 * 16);
+    const uint32_t idesc_last = idesc_bf16(BM, last_rows);
     const bool last_two = h - (nkb - 1) * BK > 16;  // the last k-block needs both k-steps
     // descriptors: the high word is constant, the low word's address field
     // (16-byte units) takes the stage, slice and k-step offsets
@@ -199,7 +203,8 @@ __global__ void __launch_bounds__(THREADS, 1)
       if (!ok) break;
       fence_after();
       const uint32_t acc = tmem + (uint32_t)(b * ACC_COLS);
-      const uint32_t idesc = (u % units) / PARTS == a_tiles - 1 ? idesc_last : idesc_full;
+      const uint32_t idesc = cta_tile<PARTS>(u, a_tiles, g.count, blockIdx.x, gridDim.x).a_tile == a_tiles - 1 ? idesc_last
+                                                                                                           : idesc_full;
       for (int kb = 0; kb < nkb; kb++, it++) {
         const int s = it % STAGES;
         ok = __all_sync(0xffffffffu, mbar_wait(&full_bar[s], (it / STAGES) & 1));
@@ -414,9 +419,9 @@ constexpr int SLICE_MAXC = 34;  // 32-column chunks per row: rows of up to 32 * 
 
 // A warp takes two adjacent rows, one per half-warp (lane l: row l / 16,
 // columns 2 (l % 16) + 32 c of chunk c, held in registers, C >= ceil(n / 32)).
-// In the k-blocked layout the two rows' k-block c is one contiguous 128-byte
-// run, so every store instruction of the warp fills whole lines.  Columns
-// load as float2 when n is even.
+// The two rows' columns of k-block c are one contiguous 128-byte run, so every
+// store instruction of the warp fills whole lines.  Columns load as float2 when
+// n is even.
 template <int C>
 __global__ void __launch_bounds__(256) slice_fields_kernel(const float *__restrict__ x, const float *__restrict__ sub,
                                                            float *__restrict__ scale, __nv_bfloat16 *__restrict__ out,
@@ -464,7 +469,8 @@ __global__ void __launch_bounds__(256) slice_fields_kernel(const float *__restri
     const long long row = wr - (long long)t * rows;
     const float S = pow2_scale(m), inv = 1.0f / S;
     if (kl == 0) scale[wr] = S;
-    const long long o0 = (long long)t * TC_PLANES * rows * kp + row * BK + kl;
+    const long long tile = ((long long)t * ((rows + BM - 1) / BM) + row / BM) * (kp / BK);
+    char *const o0 = reinterpret_cast<char *>(out) + tile * (TC_PLANES * PLANE_A) + swizzled((int)(row % BM), kl / 2);
     // stored as bf16 pairs (the pad columns n .. kp - 1 are never written:
     // they stay zero from the allocation)
 #pragma unroll
@@ -478,8 +484,7 @@ __global__ void __launch_bounds__(256) slice_fields_kernel(const float *__restri
           const float d0 = rintf(y0), d1 = rintf(y1);
           r0 = y0 - d0;
           r1 = y1 - d1;
-          *reinterpret_cast<__nv_bfloat162 *>(out + o0 + (long long)p * rows * kp + (long long)c * rows * BK) =
-              __floats2bfloat162_rn(d0, d1);
+          *reinterpret_cast<__nv_bfloat162 *>(o0 + (c * TC_PLANES + p) * PLANE_A) = __floats2bfloat162_rn(d0, d1);
         }
       }
     }
@@ -516,7 +521,7 @@ __device__ __forceinline__ uint32_t bf16_pair(float lo, float hi) {
   return __byte_perm(__float_as_uint(lo), __float_as_uint(hi), 0x7632);
 }
 
-// Lines -> the slices of their two parity parts, [t][part][p][kb][r][32] with a
+// Lines -> the slices of their two parity parts, with a
 // scale per line and part, one line per half-warp as above.
 //   MODE 0 (forward): even x[k] + x[n-1-k], odd x[k] - x[n-1-k], k < h, formed
 //        as exact pairs (TwoSum) whose low half joins the last slice, so
@@ -547,15 +552,12 @@ __global__ void __launch_bounds__(256)
   const int t = blockIdx.x % count, rb = blockIdx.x / count;
   const float *xt = xs.at(t, n3);
   const float *st = sub ? sub + t * n3 : nullptr;
-  // one base per part and plane (32-bit byte offsets within a plane)
-  const long long plane = (long long)rows * kp * 2;
-  char *base[2][TC_PLANES];
-#pragma unroll
-  for (int q = 0; q < 2; q++)
-#pragma unroll
-    for (int p = 0; p < TC_PLANES; p++)
-      base[q][p] = reinterpret_cast<char *>(out) + ((2LL * t + q) * TC_PLANES + p) * plane;
-  const uint32_t chunk = (uint32_t)rows * BK * 2;
+  // the parts' tile of these lines: SLICE_ROWS divides its height
+  static_assert(BM % SLICE_ROWS == 0, "lines of one tile");
+  const long long tile = (long long)(kp / BK) * TC_PLANES * PLANE_A;
+  const int tiles = (rows + BM - 1) / BM;
+  char *const even = reinterpret_cast<char *>(out) + (2LL * t * tiles + rb * SLICE_ROWS / BM) * tile;
+  char *const odd = even + tiles * tile;
   // MODE 2
   const bool etd = MODE == 2 && t >= sp.nI;
   const float4 *ce = MODE == 2 ? sp.etd[t % sp.F >= sp.nac ? 1 : 0] : nullptr;
@@ -675,18 +677,19 @@ __global__ void __launch_bounds__(256)
       scale[2LL * t * rows + row] = Se;
       scale[(2LL * t + 1) * rows + row] = So;
     }
-    uint32_t o = ((uint32_t)row * BK + kl) * 2;
+    const uint32_t o = swizzled(row % BM, kl / 2);
     // up to a multiple of 16 columns, the last ones zero: whole 32-byte sectors
     // (a few columns' partial sectors per line and plane, as every edge of N + 4
     // has, cost more than their line)
 #pragma unroll
-    for (int c = 0; c < C; c++, o += chunk) {
+    for (int c = 0; c < C; c++) {
       const int k = kl + BK * c;
       if (k >= h16) break;
       float d0[TC_PLANES], d1[TC_PLANES];
-      auto put = [&](int q) {
+      auto put = [&](char *part) {
 #pragma unroll
-        for (int p = 0; p < TC_PLANES; p++) *reinterpret_cast<uint32_t *>(base[q][p] + o) = bf16_pair(d0[p], d1[p]);
+        for (int p = 0; p < TC_PLANES; p++)
+          *reinterpret_cast<uint32_t *>(part + o + (c * TC_PLANES + p) * PLANE_A) = bf16_pair(d0[p], d1[p]);
       };
       if (MODE == 0) {
         // TwoSum (Knuth) of the pair and its difference
@@ -697,17 +700,17 @@ __global__ void __launch_bounds__(256)
         };
         fold(a0[c], b0[c], ie, d0);
         fold(a1[c], b1[c], ie, d1);
-        put(0);
+        put(even);
         fold(k == mid ? 0.0f : a0[c], k == mid ? 0.0f : -b0[c], io, d0);
         fold(k + 1 == mid ? 0.0f : a1[c], k + 1 == mid ? 0.0f : -b1[c], io, d1);
-        put(1);
+        put(odd);
       } else {
         digits(a0[c] * ie, 0.0f, step, step4, d0);
         digits(a1[c] * ie, 0.0f, step, step4, d1);
-        put(0);
+        put(even);
         digits(b0[c] * io, 0.0f, step, step4, d0);
         digits(b1[c] * io, 0.0f, step, step4, d1);
-        put(1);
+        put(odd);
       }
     }
   }
@@ -715,12 +718,13 @@ __global__ void __launch_bounds__(256)
 
 // FP64 matrix rows -> slices with a power-of-two scale per row.
 __global__ void slice_matrix_kernel(const double *__restrict__ m, __nv_bfloat16 *__restrict__ out,
-                                    float *__restrict__ row_scale, int n, int kp, int bits) {
+                                    float *__restrict__ row_scale, int n, int kp, int bn, int bits) {
   __shared__ double smax[128];
   const double step = ldexp(1.0, bits);
-  for (int r = blockIdx.x; r < n; r += gridDim.x) {
+  const int rows = (n + bn - 1) / bn * bn;  // whole a'-tiles, the rows beyond n zero
+  for (int r = blockIdx.x; r < rows; r += gridDim.x) {
     double mx = 0.0;
-    for (int c = threadIdx.x; c < n; c += blockDim.x) mx = fmax(mx, fabs(m[(long long)r * n + c]));
+    for (int c = threadIdx.x; r < n && c < n; c += blockDim.x) mx = fmax(mx, fabs(m[(long long)r * n + c]));
     smax[threadIdx.x] = mx;
     __syncthreads();
     for (int w = blockDim.x / 2; w > 0; w >>= 1) {
@@ -734,16 +738,17 @@ __global__ void slice_matrix_kernel(const double *__restrict__ m, __nv_bfloat16 
       S = ldexp(1.0, e);
     }
     __syncthreads();
-    if (threadIdx.x == 0) row_scale[r] = (float)S;
+    if (threadIdx.x == 0 && r < n) row_scale[r] = (float)S;
     for (int c = threadIdx.x; c < kp; c += blockDim.x) {
-      double v = c < n ? m[(long long)r * n + c] / S : 0.0;
+      double v = r < n && c < n ? m[(long long)r * n + c] / S : 0.0;
+      const long long tile = ((long long)(r / bn) * (kp / BK) + c / BK) * TC_PLANES_M * bn * BK;
       for (int p = 0; p < TC_PLANES_M; p++) {
         double y = v * step;
         double d = rint(y);
         v = y - d;
         // the fifth slice enters class 3, one factor 2^b below its own weight
         float q = p < TC_PLANES ? (float)d : (float)(d / step);
-        out[(long long)p * n * kp + (long long)(c / BK) * n * BK + r * BK + c % BK] = __float2bfloat16_rn(q);
+        out[tile + (long long)p * bn * BK + swizzled(r % bn, c % BK / 2) / 2 + c % 2] = __float2bfloat16_rn(q);
       }
     }
   }
@@ -797,6 +802,17 @@ __global__ void coef_kernel(float4 *coef, float2 *phi1, float2 *coef2, int n, in
 
 int tc_kp(int n) { return (n + tc::BK - 1) / tc::BK * tc::BK; }
 
+int tc_bn(bool folded, int h) { return folded && h <= 64 ? 64 : 128; }
+
+long long tc_plane_elems(int n, bool folded) {
+  const long long rows = ((long long)n * n + tc::BM - 1) / tc::BM * tc::BM;
+  return (folded ? 2LL * tc_kp(fold_half(n)) : tc_kp(n)) * TC_PLANES * rows;
+}
+long long tc_matrix_elems(int n, bool folded) {
+  const int h = folded ? fold_half(n) : n, bn = tc_bn(folded, h);
+  return (folded ? 2LL : 1LL) * TC_PLANES_M * ((h + bn - 1) / bn * bn) * tc_kp(h);
+}
+
 // Slice width: classes 0 and 1 stay exact while K 2^(2b) <= 2^24, K the
 // contraction length rounded up to whole k-blocks.
 int tc_slice_bits(int n) {
@@ -804,8 +820,9 @@ int tc_slice_bits(int n) {
   return K <= 1024 ? 7 : 6;
 }
 
-cudaError_t tc_slice_matrix(const double *m, __nv_bfloat16 *planes, float *row_scale, int n, cudaStream_t s) {
-  tc::slice_matrix_kernel<<<n < 1024 ? n : 1024, 128, 0, s>>>(m, planes, row_scale, n, tc_kp(n), tc_slice_bits(n));
+cudaError_t tc_slice_matrix(const double *m, __nv_bfloat16 *planes, float *row_scale, int n, int bn,
+                            cudaStream_t s) {
+  tc::slice_matrix_kernel<<<n < 1024 ? n : 1024, 128, 0, s>>>(m, planes, row_scale, n, tc_kp(n), bn, tc_slice_bits(n));
   launch_counter()++;
   return cudaGetLastError();
 }
@@ -846,8 +863,8 @@ cudaError_t tc_slice_fold(bool forward, const TensorList<float> &x, const float 
                           __nv_bfloat16 *planes, int n, int count, cudaStream_t s) {
   const int h = fold_half(n), kp = tc_kp(h), bits = tc_slice_bits(h);
   const long long g = ((long long)n * n + tc::SLICE_ROWS - 1) / tc::SLICE_ROWS * count;
-  // 32-bit row numbers, and byte offsets within a plane
-  if (g > 0x7fffffffLL || (long long)n * n * kp * 2 > 0xffffffffLL || kp > 17 * tc::BK) return cudaErrorInvalidValue;
+  // 32-bit row numbers
+  if (g > 0x7fffffffLL || kp > 17 * tc::BK) return cudaErrorInvalidValue;
   const int chunks = kp / tc::BK;
   if (forward) run_slice_fold<0>(chunks, (int)g, x, sub, scale, planes, n, kp, count, bits, SpecUpdate(), s);
   else if (!sp) run_slice_fold<1>(chunks, (int)g, x, nullptr, scale, planes, n, kp, count, bits, SpecUpdate(), s);
@@ -871,7 +888,7 @@ cudaError_t tc_make_coefs(float4 *coef, float2 *phi1, float2 *coef2, int n, int 
 // store), (none, accumulate), (ETD1, store), (phi2, store); folded forward
 // (store) and inverse (store, accumulate), each for halves beyond 64 and up to
 // 64.
-using TcKernel = void (*)(const CUtensorMap, const CUtensorMap, TcArgs);
+using TcKernel = void (*)(const char *, const char *, TcArgs);
 struct TcInstance {
   int form, epi, out, bn, smem;
   TcKernel kern;
@@ -933,25 +950,23 @@ cudaError_t launch_modeprod_tc(const __nv_bfloat16 *mat, const __nv_bfloat16 *pl
   if (e != cudaSuccess) return e;
   // contraction length and outputs of one part
   const int n = args.n, parts = args.form == 0 ? 1 : 2, h = parts == 1 ? n : fold_half(n), kp = tc_kp(h);
-  const int bn = args.form != 0 && h <= 64 ? 64 : 128;
+  const int bn = tc_bn(parts == 2, h);
   const TcInstance *inst = tc_kernel(args.form, args.epi, args.outmode, bn);
   if (!inst) return cudaErrorInvalidValue;
   const int bits = tc_slice_bits(h);
   if ((long long)kp > (1LL << (24 - 2 * bits))) return cudaErrorInvalidValue;
   if ((long long)n * n * n > 0xffffffffLL) return cudaErrorInvalidValue;  // 32-bit offsets within a tensor
-  CUtensorMap ma, mb;
-  if ((e = make_map(&ma, planes, kp, (long long)n * n, TC_PLANES * parts * count, tc::BM)) != cudaSuccess) return e;
-  if ((e = make_map(&mb, mat, kp, h, TC_PLANES_M * parts, bn)) != cudaSuccess) return e;
   TcArgs g = args;
   g.kp = kp;
   g.kblocks = kp / tc::BK;
   g.bits = bits;
-  const long long groups = (((long long)n * n + tc::BM - 1) / tc::BM) * count;  // input tiles
-  if (groups * parts * ((h + bn - 1) / bn) > 0x7fffffffLL) return cudaErrorInvalidValue;
+  const long long tiles = (((long long)n * n + tc::BM - 1) / tc::BM) * count * ((h + bn - 1) / bn);
+  if (tiles * parts > 0x7fffffffLL) return cudaErrorInvalidValue;
   // persistent: as many CTAs as can be resident at once (or the tuned count)
   if (args.max_ctas > 0 && args.max_ctas < ctas) ctas = args.max_ctas;
-  const int grid = (int)(groups < ctas ? groups : ctas);
-  inst->kern<<<grid, tc::THREADS, inst->smem, s>>>(ma, mb, g);
+  const int grid = (int)(tiles < ctas ? tiles : ctas);
+  inst->kern<<<grid, tc::THREADS, inst->smem, s>>>(reinterpret_cast<const char *>(planes),
+                                                   reinterpret_cast<const char *>(mat), g);
   launch_counter()++;
   return cudaGetLastError();
 }

@@ -214,13 +214,9 @@ int mass_weights_setup(sclet_ctx *ctx, const double *v, const double *vi);
 int queue_diagnostics(sclet_ctx *ctx, int energy_form);
 int read_diagnostics(sclet_ctx *ctx, sclet_diag *out);
 
-// Elements of one sliced tensor: TC_PLANES planes of n*n rows of kp, or two
-// parts of them over half the columns
-long long dense_elems(int n) { return (long long)TC_PLANES * n * n * tc_kp(n); }
-long long fold_elems(int n) { return 2LL * TC_PLANES * n * n * tc_kp(fold_half(n)); }
-long long tc_plane_elems(const sclet_ctx *ctx) {  // as allocated: room for either
-  const long long a = dense_elems(ctx->n), b = fold_elems(ctx->n);
-  return a > b ? a : b;
+// elements of one sliced tensor as allocated: room for either form
+long long plane_elems(const sclet_ctx *ctx) {
+  return std::max(tc_plane_elems(ctx->n, false), tc_plane_elems(ctx->n, true));
 }
 
 // Whether the order parameters may advance as u' = u + V phi1 V^-1 (N - H u)
@@ -261,7 +257,7 @@ int upload_eigen(sclet_ctx *ctx, const double *d, const double *v, const double 
     const int form = ctx->dirichlet ? 1 : 0;
     if (ctx->plane_form != form) {
       // pad columns of the slice planes are never written and must be zero
-      CK(cudaMemsetAsync(ctx->P, 0, sizeof(__nv_bfloat16) * tc_plane_elems(ctx) * 2 * ctx->FT, ctx->stream));
+      CK(cudaMemsetAsync(ctx->P, 0, sizeof(__nv_bfloat16) * plane_elems(ctx) * 2 * ctx->FT, ctx->stream));
       ctx->plane_form = form;
     }
     for (int inv = 0; inv < 2; inv++) {
@@ -270,7 +266,7 @@ int upload_eigen(sclet_ctx *ctx, const double *d, const double *v, const double 
       const double *src = inv ? v : vi;
       if (!ctx->dirichlet) {
         CK(cudaMemcpyAsync(ctx->stage64, src, sizeof(double) * n * n, cudaMemcpyHostToDevice, ctx->stream));
-        CK(tc_slice_matrix(ctx->stage64, mat, rs, n, ctx->stream));
+        CK(tc_slice_matrix(ctx->stage64, mat, rs, n, tc_bn(false, n), ctx->stream));
         CK(cudaStreamSynchronize(ctx->stream));
         continue;
       }
@@ -282,8 +278,8 @@ int upload_eigen(sclet_ctx *ctx, const double *d, const double *v, const double 
           for (int o = 0; o < h; o++) m[((size_t)part * h + o) * h + k] = w[((size_t)part * h + k) * h + o];
       CK(cudaMemcpyAsync(ctx->stage64, m.data(), sizeof(double) * m.size(), cudaMemcpyHostToDevice, ctx->stream));
       for (int part = 0; part < 2; part++)
-        CK(tc_slice_matrix(ctx->stage64 + (size_t)part * h * h, mat + (size_t)part * TC_PLANES_M * h * tc_kp(h),
-                           rs + part * h, h, ctx->stream));
+        CK(tc_slice_matrix(ctx->stage64 + (size_t)part * h * h, mat + part * tc_matrix_elems(n, true) / 2, rs + part * h,
+                           h, tc_bn(true, h), ctx->stream));
       CK(cudaStreamSynchronize(ctx->stream));
     }
     const sclet_params &p = ctx->p;
@@ -688,13 +684,13 @@ int sclet_create_runs(const sclet_params *p, int runs, const double *krun, int p
     CC(cudaMalloc(&ctx->fshell, sizeof(float) * FT * shell_count(n)));
     CC(cudaMalloc(&ctx->W1, 2 * FT * blk));
     CC(cudaMalloc(&ctx->W2, 2 * FT * blk));
-    CC(cudaMalloc(&ctx->P, sizeof(__nv_bfloat16) * tc_plane_elems(ctx) * 2 * FT));
+    CC(cudaMalloc(&ctx->P, sizeof(__nv_bfloat16) * plane_elems(ctx) * 2 * FT));
     CC(cudaMalloc(&ctx->scaleP, sizeof(float) * 2 * 2 * FT * n * n));
     {
       // dense n x n or two folded h x h matrices
-      const size_t h = fold_half(n), md = (size_t)n * tc_kp(n), mf = 2 * h * tc_kp((int)h), m = md > mf ? md : mf;
-      CC(cudaMalloc(&ctx->matV, sizeof(__nv_bfloat16) * TC_PLANES_M * m));
-      CC(cudaMalloc(&ctx->matVi, sizeof(__nv_bfloat16) * TC_PLANES_M * m));
+      const size_t h = fold_half(n), m = std::max(tc_matrix_elems(n, false), tc_matrix_elems(n, true));
+      CC(cudaMalloc(&ctx->matV, sizeof(__nv_bfloat16) * m));
+      CC(cudaMalloc(&ctx->matVi, sizeof(__nv_bfloat16) * m));
       CC(cudaMalloc(&ctx->rsV, sizeof(float) * 2 * h));
       CC(cudaMalloc(&ctx->rsVi, sizeof(float) * 2 * h));
     }
@@ -1035,7 +1031,7 @@ static int etd_update_fold(sclet_ctx *ctx) {
 // along x, y, z back to the FP32 state.
 static int etd_update_mixed(sclet_ctx *ctx) {
   const int F = ctx->FT;  // every run's fields
-  const long long ps = dense_elems(ctx->n), rows = (long long)ctx->n * ctx->n, n3 = ctx->n3;
+  const long long ps = tc_plane_elems(ctx->n, false), rows = (long long)ctx->n * ctx->n, n3 = ctx->n3;
   if (ctx->nch > 0)  // target mass of the conserved field from (u, N1)
     CK(mass_target(fu_of(ctx) + ctx->nac * n3, ctx->massW, frhs1_of(ctx) + ctx->nac * n3, nullptr, ctx->massW + n3,
                    ctx->n, ctx->massPart, ctx->stream));

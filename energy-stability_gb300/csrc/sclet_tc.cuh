@@ -11,6 +11,8 @@ namespace sclet {
 constexpr int TC_PLANES = 4;    // fixed-point slices per data operand (tc_slice_bits each)
 constexpr int TC_PLANES_M = 5;  // slices per matrix: four 6-bit slices and a fifth
                                 // stored pre-scaled by 1/64 (see k_modeprod_tc.cu)
+constexpr int TC_BM = 128;      // lines per tile of input slices
+constexpr int TC_BK = 32;       // columns per k-block
 
 struct TcArgs {
   int n, kp, kblocks, count;
@@ -34,16 +36,24 @@ struct TcArgs {
   int idle;                 // 1: the producer issues no loads (the bounded-wait self-test)
 };
 
-// kp = n rounded up to whole k-blocks of 32: the slice planes are k-blocked,
-// [p][kp / 32][rows][32], columns n .. kp - 1 zero
+// kp = n rounded up to whole k-blocks of 32.  Slices are stored in the tiles the
+// product kernel loads, each one contiguous run (see k_modeprod_tc.cu): input
+// slices [part][r / 128][kp / 32][p][128][32], matrix slices
+// [part][a' / bn][kp / 32][p][bn][32], columns n .. kp - 1 and rows beyond the
+// last one zero.
 int tc_kp(int n);
 int tc_slice_bits(int n);
-// Row-major FP64 n x n matrix -> TC_PLANES_M k-blocked slice planes
-// [p][kp / 32][n][32] (zero padded columns) and the power-of-two scale of each row.
-cudaError_t tc_slice_matrix(const double *m, __nv_bfloat16 *planes, float *row_scale, int n, cudaStream_t s);
-// FP32 blocks (x - sub; sub may be null), rows of n -> k-blocked slice planes
-// [count][p][kp / 32][n*n][32] with the power-of-two scale of each row in
-// scale[count][n*n]; the pad columns are never written (zero from allocation).
+// a'-tile width (bn) of a contraction of length h
+int tc_bn(bool folded, int h);
+// elements of one tensor's slices and of one matrix's, both parts where folded
+long long tc_plane_elems(int n, bool folded);
+long long tc_matrix_elems(int n, bool folded);
+// One part of a matrix: row-major FP64 n x n -> its TC_PLANES_M slices in
+// a'-tiles of bn and the power-of-two scale of each row.
+cudaError_t tc_slice_matrix(const double *m, __nv_bfloat16 *planes, float *row_scale, int n, int bn, cudaStream_t s);
+// FP32 blocks (x - sub; sub may be null), rows of n -> slices with the
+// power-of-two scale of each row in scale[count][n*n]; the pad columns and rows
+// are never written (zero from allocation).
 cudaError_t tc_slice_fields(const float *x, const float *sub, float *scale, __nv_bfloat16 *planes, int n, int count,
                             cudaStream_t s);
 // The update of the eigen-modes done where they are sliced for the inverse
@@ -55,9 +65,8 @@ struct SpecUpdate {
   const float4 *etd[2] = {nullptr, nullptr};
   int nI = 0, F = 1, nac = 0;
 };
-// Lines -> the slices of their parity parts (see slice_fold_kernel), planes
-// [count][2][p][kp / 32][n*n][32], kp = tc_kp(fold_half(n)), scales
-// [count][2][n*n]; forward: x - sub folded (sub may be null), else split by
+// Lines -> the slices of their two parity parts (see slice_fold_kernel), kp =
+// tc_kp(fold_half(n)), scales [count][2][n*n]; forward: x - sub folded (sub may be null), else split by
 // mode after the update sp (may be null)
 cudaError_t tc_slice_fold(bool forward, const TensorList<float> &x, const float *sub, const SpecUpdate *sp, float *scale,
                           __nv_bfloat16 *planes, int n, int count, cudaStream_t s);

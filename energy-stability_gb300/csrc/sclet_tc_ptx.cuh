@@ -14,7 +14,7 @@ namespace sclet {
 namespace tc {
 
 
-constexpr int BM = 128, BK = 32, NP = TC_PLANES, NPM = TC_PLANES_M;
+constexpr int BM = TC_BM, BK = TC_BK, NP = TC_PLANES, NPM = TC_PLANES_M;
 constexpr int PLANE_A = BM * BK * 2;  // 8 KB: one input slice (M side, 128 input rows)
 constexpr int SMEM_ALIGN = 512;  // period of the 64-byte swizzle pattern
 constexpr int NACC = 4;               // weight classes w = 0..3
@@ -62,12 +62,18 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity) {
   return false;
 }
 
-__device__ __forceinline__ void tma_load_3d(void *dst, const CUtensorMap *map, int x, int y, int z, uint64_t *bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::
-          "r"(smem_u32(dst)),
-      "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(z), "r"(smem_u32(bar))
-      : "memory");
+// bytes (a multiple of 16, both addresses 16-byte aligned) into shared memory
+__device__ __forceinline__ void bulk_load(void *dst, const void *src, uint32_t bytes, uint64_t *bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                   smem_u32(dst)),
+               "l"(src), "r"(bytes), "r"(smem_u32(bar))
+               : "memory");
+}
+
+// Byte of (row, column pair at 2 c) in a slice tile of 64-byte rows, the 64-byte
+// swizzle the descriptors below name: 16-byte chunk j of row r at j ^ (r / 2) % 4.
+__device__ __forceinline__ uint32_t swizzled(int r, int c) {
+  return (uint32_t)(r * 64 + ((((c >> 2) ^ (r >> 1)) & 3) << 4) + (c & 3) * 4);
 }
 
 // Shared-memory matrix descriptor: K-major, 64-byte swizzle, 8-row groups
@@ -176,21 +182,20 @@ __device__ __forceinline__ float pow2_scale(float m) {
   return ldexpf(1.0f, e);
 }
 
-// The u-th output tile of CTA `cta`: each CTA takes whole groups (every
-// a'-tile of one input tile, a'-tiles fastest), groups dealt round robin with
-// the tensor fastest.  Every group costs the same (the last a'-tile is
-// narrower), so the CTAs stay balanced; the group's input tile, read once
-// from HBM by its first a'-tile, is read again from L2 by the CTA's next
-// a'-tiles; and the tensors of one input tile run side by side on
-// neighbouring CTAs, so the fused update's coefficient tables (one per field
-// kind) come from HBM about once per input tile.
-// PARTS parts per a'-tile, the part fastest.
+// The u-th output tile of CTA `cta`: tiles dealt round robin over the CTAs, the
+// a'-tile fastest, then the tensor, then the input tile; the parts of a tile
+// one after the other on one CTA.  The a'-tiles of one input tile so run side
+// by side on neighbouring CTAs and its slices come from HBM once; a CTA taking
+// all of them itself came back to a part after 152 CTAs had read theirs, 90 MB
+// at 516^3, and read it from HBM again.  The tensors of one input tile run side
+// by side too, so the fused update's coefficient tables (one per field kind)
+// come from HBM about once per input tile.
 template <int PARTS>
 __device__ __forceinline__ TileIdx cta_tile(int u, int a_tiles, int count, int cta, int grid) {
   TileIdx x;
-  const int units = a_tiles * PARTS, grp = cta + (u / units) * grid, ug = u % units;
-  x.a_tile = ug / PARTS;
-  x.part = ug % PARTS;
+  const int tile = cta + (u / PARTS) * grid, grp = tile / a_tiles;
+  x.a_tile = tile - grp * a_tiles;
+  x.part = u % PARTS;
   x.t = grp % count;
   x.r_tile = grp / count;
   return x;
@@ -208,21 +213,6 @@ static inline PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
       fn = (PFN_cuTensorMapEncodeTiled_v12000)p;
   }
   return fn;
-}
-
-// k-blocked slice planes [depth][kp / BK][rows][BK] as a 3-D tensor {BK, rows,
-// depth * kp / BK}: a box is one k-block of box_rows consecutive rows.
-static inline cudaError_t make_map(CUtensorMap *map, const void *ptr, int kp, long long rows, int depth, int box_rows) {
-  auto fn = encode_fn();
-  if (!fn) return cudaErrorNotSupported;
-  cuuint64_t dims[3] = {(cuuint64_t)tc::BK, (cuuint64_t)rows, (cuuint64_t)depth * (cuuint64_t)(kp / tc::BK)};
-  cuuint64_t strides[2] = {(cuuint64_t)tc::BK * 2, (cuuint64_t)tc::BK * 2 * (cuuint64_t)rows};
-  cuuint32_t box[3] = {(cuuint32_t)tc::BK, (cuuint32_t)box_rows, 1};
-  cuuint32_t estr[3] = {1, 1, 1};
-  CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void *>(ptr), dims, strides, box, estr,
-                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
 }
 
 }  // namespace sclet
