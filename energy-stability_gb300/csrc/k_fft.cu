@@ -15,8 +15,10 @@
 // G_p(k) = (F_p(k) + conj F_p(-k)) / 2 of each product spectrum
 // F_p = sum_q B_pq H_q (B is not even at the Nyquist planes), whose inverse
 // transform is exactly that real part, before packing G_0 + i G_1.
-// Each 1D pass keeps tiles of lines in shared memory (Stockham autosort,
-// radices 4, 2, 3, 5); lines along y and z are loaded as runs of adjacent x.
+// Each 1D pass keeps tiles of lines in shared memory; lines along y and z are
+// loaded as runs of adjacent x.  FP32 edges of 16 N1 take register transforms and
+// one kernel for z forward, contraction and z backward (green_kernel), the
+// others Stockham stages (radices 4, 2, 3, 5) and a contraction of its own.
 #include <mutex>
 #include <math.h>
 #include <stdlib.h>
@@ -253,6 +255,50 @@ __global__ void __launch_bounds__(256) fft_lines_kernel(typename Cx<T>::t *data0
   }
 }
 
+__host__ __device__ inline int pq_slot(int p, int q) {
+  if (p > q) { int t = p; p = q; q = t; }
+  // (0,0)0 (0,1)1 (0,2)2 (0,3)3 (1,1)4 (1,2)5 (1,3)6 (2,2)7 (2,3)8 (3,3)9
+  return p * 4 - p * (p - 1) / 2 + (q - p);
+}
+
+// Contraction of one pair {k, -k}; see the file comment.  In: the packed spectra
+// at k (a = eta_0 + i eta_1, b = eta_2 + i eta_3) and -k (am, bm), the Green
+// tensor at both.  Out: the packed products there.
+template <typename T, typename C>
+__device__ __forceinline__ void contract_pair(C &a, C &am, C &b, C &bm, const T (&bk)[10], const T (&bkm)[10], int nac) {
+  C H[4], Hm[4];
+  // split Z = A + iB into the two real fields' spectra
+  H[0].x = (T)0.5 * (a.x + am.x); H[0].y = (T)0.5 * (a.y - am.y);
+  H[1].x = (T)0.5 * (a.y + am.y); H[1].y = (T)0.5 * (am.x - a.x);
+  H[2].x = (T)0.5 * (b.x + bm.x); H[2].y = (T)0.5 * (b.y - bm.y);
+  H[3].x = (T)0.5 * (b.y + bm.y); H[3].y = (T)0.5 * (bm.x - b.x);
+#pragma unroll
+  for (int q = 0; q < 4; q++) {
+    if (q >= nac) { H[q].x = 0; H[q].y = 0; }
+    Hm[q] = cconj(H[q]);
+  }
+  C G[4];
+#pragma unroll
+  for (int p = 0; p < 4; p++) {
+    C f, fm;
+    f.x = 0; f.y = 0; fm = f;
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      const T c = bk[pq_slot(p, q)], cm = bkm[pq_slot(p, q)];
+      f.x += c * H[q].x; f.y += c * H[q].y;
+      fm.x += cm * Hm[q].x; fm.y += cm * Hm[q].y;
+    }
+    // Hermitian part: its inverse transform is Re(IFFT(F_p))
+    G[p].x = (T)0.5 * (f.x + fm.x);
+    G[p].y = (T)0.5 * (f.y - fm.y);
+    if (p >= nac) { G[p].x = 0; G[p].y = 0; }
+  }
+  a.x = G[0].x - G[1].y; a.y = G[0].y + G[1].x;    // G0 + i G1
+  am.x = G[0].x + G[1].y; am.y = -G[0].y + G[1].x; // conj(G0) + i conj(G1)
+  b.x = G[2].x - G[3].y; b.y = G[2].y + G[3].x;
+  bm.x = G[2].x + G[3].y; bm.y = -G[2].y + G[3].x;
+}
+
 // ---- FP32 fast path: line FFTs of N = N1 * N2 points in two register passes
 //
 // X[k1 + N1 k2] = sum_t W_N2^(t k2) W_N^(t k1) sum_n1 x[t + N2 n1] W_N1^(n1 k1)
@@ -389,7 +435,7 @@ struct LineIO {
 };
 
 // L lines per CTA.  axis 0: lines along x, lane order over t (pass A) and k1
-// (pass B); axes 1 and 2: L adjacent x-lines, lane order over x.
+// (pass B); axis 1: L adjacent lines along y, lane order over x.
 template <int N1, int N2, int L, int AXIS, int SIGN, int IO>
 __global__ void __launch_bounds__(L *(N1 > N2 ? N1 : N2))
     lines_kernel(float2 *data0, float2 *data1, const float2 *__restrict__ tw, LineIO io) {
@@ -412,9 +458,9 @@ __global__ void __launch_bounds__(L *(N1 > N2 ? N1 : N2))
     ps = 1;
   } else {
     constexpr int ntx = N / L;
-    const int xt = blockIdx.x % ntx, w = blockIdx.x / ntx;  // w = z (axis 1) or y (axis 2)
-    base = (AXIS == 1 ? (long long)w * NN : (long long)w * N) + (long long)xt * L;
-    ps = AXIS == 1 ? N : NN;
+    const int xt = blockIdx.x % ntx, z = blockIdx.x / ntx;
+    base = z * NN + (long long)xt * L;
+    ps = N;
   }
   auto at = [&](int l, int k1, int t) -> int {
     return AXIS == 0 ? (l * N1 + k1) * RS + t : (k1 * N2 + t) * L + l;
@@ -499,20 +545,135 @@ static cudaError_t launch_one(float2 *z0, float2 *z1, const float2 *tw, const Li
   return cudaGetLastError();
 }
 
-// forward: x (reading the order parameters), y, z; inverse: z, y, x (writing felas)
-template <int N1, int N2>
-static cudaError_t launch_pass(int sign, int k, float2 *z0, float2 *z1, const float2 *tw, const LineIO &io,
-                               cudaStream_t s) {
-  if (sign < 0) {
-    switch (k) {
-      case 0: return launch_one<N1, N2, 0, -1, 1>(z0, z1, tw, io, s);
-      case 1: return launch_one<N1, N2, 1, -1, 0>(z0, z1, tw, io, s);
-      default: return launch_one<N1, N2, 2, -1, 0>(z0, z1, tw, io, s);
+// The z-lines forward, the contraction and the z-lines backward in one kernel: a
+// CTA takes L adjacent z-lines of a row y and their mirrors (N - x, N - y) of
+// both grids, transforms them in shared memory, multiplies by the Green tensor
+// pair by pair and transforms back, so a grid is read and written once where
+// three kernels did it three times.  The inverse transform runs its two passes
+// with the factors exchanged: the thread that left X[k1 + N1 k2] (all k2) in
+// shared memory takes up those slots again.  Half of the threads do a line's own
+// side, half the mirror's.  A line that is its own mirror (x and y each 0 or
+// N / 2) is done once.  Bound by memory, the grids once each way and half the
+// Green tensor, and by the latency of its phases at one or two CTAs an SM.
+// Elastic stage with three kernels and this one: 512^3 7.4 -> 5.8 ms (with the
+// factors of launch()), 192^3 357 -> 298 us, 32^3 39 -> 33 us.
+template <int N1, int N2, int L>
+__global__ void __launch_bounds__(2 * L *(N1 > N2 ? N1 : N2))
+    green_kernel(float2 *z01, float2 *z23, const float2 *__restrict__ tw, const float *__restrict__ bn, int nac) {
+  constexpr int N = N1 * N2, SIDE = L * (N1 > N2 ? N1 : N2), SET = N * L;
+  constexpr long long NN = (long long)N * N, N3 = NN * N;
+  extern __shared__ float2 tab[];  // [grid][side][slot of k][line]
+  const int side = threadIdx.x / SIDE, tid = threadIdx.x % SIDE;
+  const int xt = blockIdx.x % (N / L), y = blockIdx.x / (N / L), ym = y ? N - y : 0;
+  const int grids = z23 ? 2 : 1;
+  z01 += blockIdx.y * N3;  // blockIdx.y = run
+  if (z23) z23 += blockIdx.y * N3;
+  auto slot = [](int k1, int k2, int l) { return (k1 * N2 + k2) * L + l; };
+  // both passes give one line to L-strided threads
+  const int l = tid % L, t = tid / L;
+  const int x = xt * L + l, xm = x ? N - x : 0;
+  // a row that is its own mirror holds each pair of lines twice
+  const bool self = y == ym && x == xm, own = (y != ym || x <= xm) && !(side && self);
+  const int col = side ? ym * N + xm : y * N + x;
+  if (t < N2 && own) {
+    for (int q = 0; q < grids; q++) {
+      const float2 *src = (q ? z23 : z01) + col;
+      float2 *set = tab + (2 * q + side) * SET;
+      float2 v[N1];
+#pragma unroll
+      for (int n1 = 0; n1 < N1; n1++) v[n1] = src[(t + N2 * n1) * NN];
+      Dft<N1, -1>::run(v);
+#pragma unroll
+      for (int k1 = 0; k1 < N1; k1++) set[slot(k1, t, l)] = k1 > 0 && t > 0 ? cmul(v[k1], tw[t * k1]) : v[k1];
     }
   }
+  __syncthreads();
+  if (t < N1 && own) {
+    for (int q = 0; q < grids; q++) {
+      float2 *set = tab + (2 * q + side) * SET;
+      float2 v[N2];
+#pragma unroll
+      for (int k2 = 0; k2 < N2; k2++) v[k2] = set[slot(t, k2, l)];
+      Dft<N2, -1>::run(v);
+#pragma unroll
+      for (int k2 = 0; k2 < N2; k2++) set[slot(t, k2, l)] = v[k2];
+    }
+  }
+  __syncthreads();
+  // k at the line's own side, -k at the mirror's (or its own, of which half the k then)
+  for (int k = threadIdx.x / L; k < N; k += 2 * SIDE / L) {
+    if ((y == ym && x > xm) || (self && k > N / 2)) continue;
+    const int km = k ? N - k : 0;
+    const int i = slot(k % N1, k / N1, l), im = slot(km % N1, km / N1, l) + (self ? 0 : SET);
+    const long long g = k * NN + y * N + x, gm = km * NN + ym * N + xm;
+    const bool even = !(k == N / 2 || y == N / 2 || x == N / 2);  // B(-k) = B(k), see contract_kernel
+    float bk[10], bkm[10];
+#pragma unroll
+    for (int j = 0; j < 10; j++) bk[j] = bn[j * N3 + g];
+#pragma unroll
+    for (int j = 0; j < 10; j++) bkm[j] = even ? bk[j] : bn[j * N3 + gm];
+    float2 a = tab[i], am = tab[im], b = make_float2(0.0f, 0.0f), bm = b;
+    if (grids > 1) b = tab[2 * SET + i], bm = tab[2 * SET + im];
+    contract_pair<float, float2>(a, am, b, bm, bk, bkm, nac);
+    tab[i] = a;
+    if (im != i) tab[im] = am;
+    if (grids > 1) {
+      tab[2 * SET + i] = b;
+      if (im != i) tab[2 * SET + im] = bm;
+    }
+  }
+  __syncthreads();
+  if (t < N1 && own) {
+    for (int q = 0; q < grids; q++) {
+      float2 *set = tab + (2 * q + side) * SET;
+      float2 v[N2];
+#pragma unroll
+      for (int k2 = 0; k2 < N2; k2++) v[k2] = set[slot(t, k2, l)];
+      Dft<N2, 1>::run(v);
+#pragma unroll
+      for (int j = 0; j < N2; j++) set[slot(t, j, l)] = j > 0 && t > 0 ? cmul(v[j], cconj(tw[t * j])) : v[j];
+    }
+  }
+  __syncthreads();
+  if (t < N2 && own) {
+    for (int q = 0; q < grids; q++) {
+      float2 *dst = (q ? z23 : z01) + col;
+      const float2 *set = tab + (2 * q + side) * SET;
+      float2 v[N1];
+#pragma unroll
+      for (int n1 = 0; n1 < N1; n1++) v[n1] = set[slot(n1, t, l)];
+      Dft<N1, 1>::run(v);
+#pragma unroll
+      for (int m = 0; m < N1; m++) dst[(t + N2 * m) * NN] = v[m];
+    }
+  }
+}
+
+template <int N1, int N2>
+static cudaError_t launch_green(float2 *z0, float2 *z1, const float2 *tw, const float *bn, int nac, int runs,
+                                cudaStream_t s) {
+  // 8 lines where 16 would not fit shared memory, or leave SMs without a CTA
+  constexpr int N = N1 * N2, L = N > 256 || N <= 64 ? 8 : 16;
+  const size_t sm = sizeof(float2) * 2 * N * L * (z1 ? 2 : 1);
+  auto k = green_kernel<N1, N2, L>;
+  if (sm > 48 * 1024) {
+    const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    if (e != cudaSuccess) return e;
+  }
+  k<<<dim3((N / 2 + 1) * (N / L), runs), 2 * L * (N1 > N2 ? N1 : N2), sm, s>>>(z0, z1, tw, bn, nac);
+  return cudaGetLastError();
+}
+
+// pass 0 x (reading the order parameters), 1 y; 2 z with the contraction, both
+// ways; 3 y, 4 x backward (writing felas)
+template <int N1, int N2>
+static cudaError_t launch_pass(int k, float2 *z0, float2 *z1, const float2 *tw, const float *bn, const LineIO &io,
+                               cudaStream_t s) {
   switch (k) {
-    case 0: return launch_one<N1, N2, 2, 1, 0>(z0, z1, tw, io, s);
-    case 1: return launch_one<N1, N2, 1, 1, 0>(z0, z1, tw, io, s);
+    case 0: return launch_one<N1, N2, 0, -1, 1>(z0, z1, tw, io, s);
+    case 1: return launch_one<N1, N2, 1, -1, 0>(z0, z1, tw, io, s);
+    case 2: return launch_green<N1, N2>(z0, z1, tw, bn, io.nac, io.runs, s);
+    case 3: return launch_one<N1, N2, 1, 1, 0>(z0, z1, tw, io, s);
     default: return launch_one<N1, N2, 0, 1, 2>(z0, z1, tw, io, s);
   }
 }
@@ -526,20 +687,22 @@ static int pass_n1(int N) {
   return 0;
 }
 
-// pass k (0..2) of the forward (sign -1) or inverse (+1) 3-D transform
-static cudaError_t launch(int N, int sign, int k, float2 *z0, float2 *z1, const float2 *tw, const LineIO &io,
+// pass k (0..4) of the elastic force
+static cudaError_t launch(int N, int k, float2 *z0, float2 *z1, const float2 *tw, const float *bn, const LineIO &io,
                           cudaStream_t s) {
   switch (pass_n1(N)) {
-    case 2: return launch_pass<2, 16>(sign, k, z0, z1, tw, io, s);
-    case 3: return launch_pass<3, 16>(sign, k, z0, z1, tw, io, s);
-    case 4: return launch_pass<4, 16>(sign, k, z0, z1, tw, io, s);
-    case 5: return launch_pass<5, 16>(sign, k, z0, z1, tw, io, s);
-    case 6: return launch_pass<6, 16>(sign, k, z0, z1, tw, io, s);
-    case 8: return launch_pass<8, 16>(sign, k, z0, z1, tw, io, s);
-    case 10: return launch_pass<10, 16>(sign, k, z0, z1, tw, io, s);
-    case 12: return launch_pass<12, 16>(sign, k, z0, z1, tw, io, s);
-    case 16: return launch_pass<16, 16>(sign, k, z0, z1, tw, io, s);
-    default: return launch_pass<32, 16>(sign, k, z0, z1, tw, io, s);
+    case 2: return launch_pass<2, 16>(k, z0, z1, tw, bn, io, s);
+    case 3: return launch_pass<3, 16>(k, z0, z1, tw, bn, io, s);
+    case 4: return launch_pass<4, 16>(k, z0, z1, tw, bn, io, s);
+    case 5: return launch_pass<5, 16>(k, z0, z1, tw, bn, io, s);
+    case 6: return launch_pass<6, 16>(k, z0, z1, tw, bn, io, s);
+    case 8: return launch_pass<8, 16>(k, z0, z1, tw, bn, io, s);
+    case 10: return launch_pass<10, 16>(k, z0, z1, tw, bn, io, s);
+    case 12: return launch_pass<12, 16>(k, z0, z1, tw, bn, io, s);
+    case 16: return launch_pass<16, 16>(k, z0, z1, tw, bn, io, s);
+    // 16-point transforms where global memory is read and written, by all threads
+    // (32-point ones by half of them: 6.7 ms an elastic force of 512^3, now 5.8)
+    default: return launch_pass<16, 32>(k, z0, z1, tw, bn, io, s);
   }
 }
 
@@ -578,12 +741,6 @@ __global__ void pack_kernel(const T *__restrict__ u, typename Cx<T>::t *__restri
     z01[g] = a;
     if (z23) z23[g] = b;
   }
-}
-
-__host__ __device__ inline int pq_slot(int p, int q) {
-  if (p > q) { int t = p; p = q; q = t; }
-  // (0,0)0 (0,1)1 (0,2)2 (0,3)3 (1,1)4 (1,2)5 (1,3)6 (2,2)7 (2,3)8 (3,3)9
-  return p * 4 - p * (p - 1) / 2 + (q - p);
 }
 
 // Green-tensor kernel on the full grid, 10 symmetric slots (FP64, once).
@@ -642,16 +799,13 @@ __global__ void bn_kernel(B *__restrict__ bn, int N, BnConst bc) {
   }
 }
 
-// Contraction on pairs {k, -k}; see the file comment.  A row (y, z) is done
+// Contraction over the grid.  A row (y, z) is done
 // together with its mirror row (-y, -z), by the lower of the two.
 template <typename T, typename B>
 __global__ void contract_kernel(typename Cx<T>::t *z01, typename Cx<T>::t *z23, const B *__restrict__ bn, int N,
                                 int nac) {
   typedef typename Cx<T>::t C;
   const long long N3 = (long long)N * N * N;
-  // blockIdx.y = run: its grids at run N^3
-  z01 += blockIdx.y * N3;
-  if (z23) z23 += blockIdx.y * N3;
   auto mid = [&](int v) { return v == N / 2 || N - v == N / 2; };
   for (int row = blockIdx.x; row < N * N; row += gridDim.x) {
   const int z = row / N, y = row - z * N;
@@ -665,52 +819,21 @@ __global__ void contract_kernel(typename Cx<T>::t *z01, typename Cx<T>::t *z23, 
     // B(-k) has B(k)'s bits where no component's wave number is its own or its
     // neighbour's mirror (N / 2, or the two middle ones of an odd N): one read
     const bool even = !(mid(z) || mid(y) || mid(x));
-    C H[4], Hm[4];
     C a = z01[g], am = z01[gm];
     C b, bm;
     b.x = 0; b.y = 0; bm = b;
     if (z23) { b = z23[g]; bm = z23[gm]; }
-    // split Z = A + iB into the two real fields' spectra
-    H[0].x = (T)0.5 * (a.x + am.x); H[0].y = (T)0.5 * (a.y - am.y);
-    H[1].x = (T)0.5 * (a.y + am.y); H[1].y = (T)0.5 * (am.x - a.x);
-    H[2].x = (T)0.5 * (b.x + bm.x); H[2].y = (T)0.5 * (b.y - bm.y);
-    H[3].x = (T)0.5 * (b.y + bm.y); H[3].y = (T)0.5 * (bm.x - b.x);
-#pragma unroll
-    for (int q = 0; q < 4; q++) {
-      if (q >= nac) { H[q].x = 0; H[q].y = 0; }
-      Hm[q] = cconj(H[q]);
-    }
     T bk[10], bkm[10];
 #pragma unroll
     for (int i = 0; i < 10; i++) bk[i] = (T)bn[i * N3 + g];
 #pragma unroll
     for (int i = 0; i < 10; i++) bkm[i] = even ? bk[i] : (T)bn[i * N3 + gm];
-    C G[4];
-#pragma unroll
-    for (int p = 0; p < 4; p++) {
-      C f, fm;
-      f.x = 0; f.y = 0; fm = f;
-#pragma unroll
-      for (int q = 0; q < 4; q++) {
-        const T c = bk[pq_slot(p, q)], cm = bkm[pq_slot(p, q)];
-        f.x += c * H[q].x; f.y += c * H[q].y;
-        fm.x += cm * Hm[q].x; fm.y += cm * Hm[q].y;
-      }
-      // Hermitian part: its inverse transform is Re(IFFT(F_p))
-      G[p].x = (T)0.5 * (f.x + fm.x);
-      G[p].y = (T)0.5 * (f.y - fm.y);
-      if (p >= nac) { G[p].x = 0; G[p].y = 0; }
-    }
-    C w01, w23, w01m, w23m;
-    w01.x = G[0].x - G[1].y; w01.y = G[0].y + G[1].x;    // G0 + i G1
-    w01m.x = G[0].x + G[1].y; w01m.y = -G[0].y + G[1].x; // conj(G0) + i conj(G1)
-    w23.x = G[2].x - G[3].y; w23.y = G[2].y + G[3].x;
-    w23m.x = G[2].x + G[3].y; w23m.y = -G[2].y + G[3].x;
-    z01[g] = w01;
-    if (gm != g) z01[gm] = w01m;
+    contract_pair<T, C>(a, am, b, bm, bk, bkm, nac);
+    z01[g] = a;
+    if (gm != g) z01[gm] = am;
     if (z23) {
-      z23[g] = w23;
-      if (gm != g) z23[gm] = w23m;
+      z23[g] = b;
+      if (gm != g) z23[gm] = bm;
     }
   }
   }
@@ -919,16 +1042,8 @@ cudaError_t elastic_compute(ElasticPlan *p, const T *u, T *felas, int n, T *shel
     io.ustride = ustride;
     io.fstride = (long long)p->nac * n3;
     const float2 *tw = (const float2 *)p->tw;
-    for (int k = 0; k < 3; k++) {
-      cudaError_t e = fft2::launch(N, -1, k, (float2 *)z01, (float2 *)z23, tw, io, s);
-      launch_counter()++;
-      if (e != cudaSuccess) return e;
-    }
-    contract_kernel<T, float><<<dim3(rows_grid(N).x, p->runs), rows_block(N), 0, s>>>(z01, z23, (const float *)p->bn,
-                                                                                       N, p->nac);
-    launch_counter()++;
-    for (int k = 0; k < 3; k++) {
-      cudaError_t e = fft2::launch(N, +1, k, (float2 *)z01, (float2 *)z23, tw, io, s);
+    for (int k = 0; k < 5; k++) {
+      cudaError_t e = fft2::launch(N, k, (float2 *)z01, (float2 *)z23, tw, (const float *)p->bn, io, s);
       launch_counter()++;
       if (e != cudaSuccess) return e;
     }
