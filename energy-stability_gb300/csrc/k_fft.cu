@@ -13,8 +13,9 @@
 // 2 inverse complex transforms.  The reference keeps only the real part of
 // each inverse transform; the contraction therefore builds the Hermitian part
 // G_p(k) = (F_p(k) + conj F_p(-k)) / 2 of each product spectrum
-// F_p = sum_q B_pq H_q (B is not even at the Nyquist planes), whose inverse
-// transform is exactly that real part, before packing G_0 + i G_1.
+// F_p = sum_q B_pq H_q, whose inverse transform is exactly that real part, before
+// packing G_0 + i G_1.  It is the mean of B(k) and B(-k), which differ at the
+// Nyquist planes only, times H.
 // Each 1D pass keeps tiles of lines in shared memory; lines along y and z are
 // loaded as runs of adjacent x.  FP32 edges of 16 N1 take register transforms and
 // one kernel for z forward, contraction and z backward (green_kernel), the
@@ -45,6 +46,14 @@ __device__ inline C cmul(C a, C b) {
   C r;
   r.x = a.x * b.x - a.y * b.y;
   r.y = a.x * b.y + a.y * b.x;
+  return r;
+}
+// a conj(b)
+template <typename C>
+__device__ inline C cmulc(C a, C b) {
+  C r;
+  r.x = a.x * b.x + a.y * b.y;
+  r.y = a.y * b.x - a.x * b.y;
   return r;
 }
 template <typename C>
@@ -101,13 +110,17 @@ __device__ __forceinline__ int fdiv(int e, float inv) { return __float2int_rd(((
 // inputs (real coefficients: 12 and 32 additions and multiplications per
 // butterfly against 36 and 120 of the plain sums; FP64 operations are what the
 // FP64 plan's passes cost).
-template <int R, typename T, typename C>
+// FIRST: the stage of Ns = 1, whose twiddles are all one (a twiddle of one is
+// multiplied all the same elsewhere: whole warps pay for the others).  With the
+// direction a constant and the contraction in half the operations, the elastic
+// stage of 64^3 in FP64 took 272 us, now 231, of 128^3 1.64 -> 1.33 ms.
+template <int R, int SIGN, bool FIRST, typename T, typename C>
 __device__ __forceinline__ void fft_stage(const C *__restrict__ src, C *__restrict__ dst, int tile, int N, int ls, int Ns,
-                                          float inv_nb, float inv_ns, const C *__restrict__ tw, int sign) {
+                                          float inv_nb, float inv_ns, const C *__restrict__ tw) {
   const int nb = N / R;
   for (int e = threadIdx.x; e < tile * nb; e += blockDim.x) {
     const int line = fdiv(e, inv_nb), j = e - line * nb;
-    const int jq = fdiv(j, inv_ns), k = j - jq * Ns;
+    const int jq = FIRST ? j : fdiv(j, inv_ns), k = FIRST ? 0 : j - jq * Ns;
     const C *s = src + line * ls;
     C *d = dst + line * ls;
     C v[R];
@@ -116,18 +129,14 @@ __device__ __forceinline__ void fft_stage(const C *__restrict__ src, C *__restri
 #pragma unroll
     for (int r = 0; r < R; r++) {
       v[r] = s[j + r * nb];
-      if (r > 0 && k > 0) {
-        C w = tw[r * tstep];
-        if (sign > 0) w.y = -w.y;
-        v[r] = cmul(v[r], w);
-      }
+      if (!FIRST && r > 0) v[r] = SIGN > 0 ? cmulc(v[r], tw[r * tstep]) : cmul(v[r], tw[r * tstep]);
     }
     C o[R];
     // multiply by -i (forward) or +i (backward)
     auto turn = [&](C a) {
       C b;
-      b.x = sign < 0 ? a.y : -a.y;
-      b.y = sign < 0 ? -a.x : a.x;
+      b.x = SIGN < 0 ? a.y : -a.y;
+      b.y = SIGN < 0 ? -a.x : a.x;
       return b;
     };
     if (R == 2) {
@@ -186,10 +195,10 @@ __device__ __forceinline__ void fft_stage(const C *__restrict__ src, C *__restri
 // adjacent x (a tile that divides an odd N is one line, 16 bytes per access).
 // Elastic stage of 75^3 in FP64 2.00 -> 0.68 ms a second-order step, of 100^3 in
 // FP32 1.02 -> 0.46 ms, with the radix-3 and 5 butterflies above.
-template <typename T>
+template <typename T, int SIGN>
 __global__ void __launch_bounds__(256) fft_lines_kernel(typename Cx<T>::t *data0, typename Cx<T>::t *data1, int N,
                                                         int axis, int ltile, const typename Cx<T>::t *__restrict__ tw,
-                                                        int sign, Radices rad, StageDiv sd) {
+                                                        Radices rad, StageDiv sd) {
   typedef typename Cx<T>::t C;
   extern __shared__ unsigned char smem_raw[];
   const int tile = 1 << ltile, ls = N + 1;
@@ -229,12 +238,17 @@ __global__ void __launch_bounds__(256) fft_lines_kernel(typename Cx<T>::t *data0
   for (int st = 0; st < rad.count; st++) {
     const int R = rad.r[st];
     const float inb = sd.inv_nb[st], ins = sd.inv_ns[st];
+#define SCLET_STAGE(R)                                                                                \
+  if (st == 0) fft_stage<R, SIGN, true, T, C>(src, dst, lines, N, ls, Ns, inb, ins, tw);               \
+  else fft_stage<R, SIGN, false, T, C>(src, dst, lines, N, ls, Ns, inb, ins, tw);                      \
+  break;
     switch (R) {
-      case 4: fft_stage<4, T, C>(src, dst, lines, N, ls, Ns, inb, ins, tw, sign); break;
-      case 2: fft_stage<2, T, C>(src, dst, lines, N, ls, Ns, inb, ins, tw, sign); break;
-      case 3: fft_stage<3, T, C>(src, dst, lines, N, ls, Ns, inb, ins, tw, sign); break;
-      default: fft_stage<5, T, C>(src, dst, lines, N, ls, Ns, inb, ins, tw, sign); break;
+      case 4: SCLET_STAGE(4)
+      case 2: SCLET_STAGE(2)
+      case 3: SCLET_STAGE(3)
+      default: SCLET_STAGE(5)
     }
+#undef SCLET_STAGE
     __syncthreads();
     C *t = src;
     src = dst;
@@ -262,41 +276,33 @@ __host__ __device__ inline int pq_slot(int p, int q) {
 }
 
 // Contraction of one pair {k, -k}; see the file comment.  In: the packed spectra
-// at k (a = eta_0 + i eta_1, b = eta_2 + i eta_3) and -k (am, bm), the Green
-// tensor at both.  Out: the packed products there.
+// at k (a = eta_0 + i eta_1, b = eta_2 + i eta_3) and -k (am, bm) and the mean of
+// the Green tensor at k and -k: F_p's Hermitian part is that mean times H.  Out:
+// the packed products there, doubled (the inverse transform's scale halves them).
 template <typename T, typename C>
-__device__ __forceinline__ void contract_pair(C &a, C &am, C &b, C &bm, const T (&bk)[10], const T (&bkm)[10], int nac) {
-  C H[4], Hm[4];
+__device__ __forceinline__ void contract_pair(C &a, C &am, C &b, C &bm, const T (&bk)[10], int nac) {
+  C H[4];  // doubled
   // split Z = A + iB into the two real fields' spectra
-  H[0].x = (T)0.5 * (a.x + am.x); H[0].y = (T)0.5 * (a.y - am.y);
-  H[1].x = (T)0.5 * (a.y + am.y); H[1].y = (T)0.5 * (am.x - a.x);
-  H[2].x = (T)0.5 * (b.x + bm.x); H[2].y = (T)0.5 * (b.y - bm.y);
-  H[3].x = (T)0.5 * (b.y + bm.y); H[3].y = (T)0.5 * (bm.x - b.x);
-#pragma unroll
-  for (int q = 0; q < 4; q++) {
-    if (q >= nac) { H[q].x = 0; H[q].y = 0; }
-    Hm[q] = cconj(H[q]);
-  }
+  H[0].x = a.x + am.x; H[0].y = a.y - am.y;
+  H[1].x = a.y + am.y; H[1].y = am.x - a.x;
+  H[2].x = b.x + bm.x; H[2].y = b.y - bm.y;
+  H[3].x = b.y + bm.y; H[3].y = bm.x - b.x;
   C G[4];
 #pragma unroll
   for (int p = 0; p < 4; p++) {
-    C f, fm;
-    f.x = 0; f.y = 0; fm = f;
+    G[p].x = G[p].y = 0;
 #pragma unroll
-    for (int q = 0; q < 4; q++) {
-      const T c = bk[pq_slot(p, q)], cm = bkm[pq_slot(p, q)];
-      f.x += c * H[q].x; f.y += c * H[q].y;
-      fm.x += cm * Hm[q].x; fm.y += cm * Hm[q].y;
-    }
-    // Hermitian part: its inverse transform is Re(IFFT(F_p))
-    G[p].x = (T)0.5 * (f.x + fm.x);
-    G[p].y = (T)0.5 * (f.y - fm.y);
+    for (int q = 0; q < 4; q++)
+      if (q < nac) {
+        const T c = bk[pq_slot(p, q)];
+        G[p].x += c * H[q].x; G[p].y += c * H[q].y;
+      }
     if (p >= nac) { G[p].x = 0; G[p].y = 0; }
   }
   a.x = G[0].x - G[1].y; a.y = G[0].y + G[1].x;    // G0 + i G1
-  am.x = G[0].x + G[1].y; am.y = -G[0].y + G[1].x; // conj(G0) + i conj(G1)
+  am.x = G[0].x + G[1].y; am.y = G[1].x - G[0].y;  // conj(G0) + i conj(G1)
   b.x = G[2].x - G[3].y; b.y = G[2].y + G[3].x;
-  bm.x = G[2].x + G[3].y; bm.y = -G[2].y + G[3].x;
+  bm.x = G[2].x + G[3].y; bm.y = G[3].x - G[2].y;
 }
 
 // ---- FP32 fast path: line FFTs of N = N1 * N2 points in two register passes
@@ -421,13 +427,13 @@ struct Dft<5, SIGN> {
 // Grids and blocks of one elastic call.  io 1 (first forward x-pass): lines
 // are read from the order parameters (grid y = q holds eta_2q + i eta_2q+1 of
 // the owned cells) instead of data; io 2 (last inverse x-pass): the real and
-// imaginary parts, scaled by 1 / N^3, go to felas_2q and felas_2q+1.
+// imaginary parts, scaled by 1 / (2 N^3), go to felas_2q and felas_2q+1.
 struct LineIO {
   const float *u;  // order parameters, nac blocks of n^3
   float *felas;    // elastic force, nac blocks of n^3
   int n, nac;
   long long n3;
-  float scale;     // 1 / N^3
+  float scale;     // 1 / (2 N^3)
   // runs side by side: run r's grids at r N^3 of data0 / data1, its order
   // parameters at u + r ustride, its force at felas + r fstride
   int runs;
@@ -607,14 +613,16 @@ __global__ void __launch_bounds__(2 * L *(N1 > N2 ? N1 : N2))
     const int i = slot(k % N1, k / N1, l), im = slot(km % N1, km / N1, l) + (self ? 0 : SET);
     const long long g = k * NN + y * N + x, gm = km * NN + ym * N + xm;
     const bool even = !(k == N / 2 || y == N / 2 || x == N / 2);  // B(-k) = B(k), see contract_kernel
-    float bk[10], bkm[10];
+    float bk[10];
 #pragma unroll
     for (int j = 0; j < 10; j++) bk[j] = bn[j * N3 + g];
+    if (!even) {
 #pragma unroll
-    for (int j = 0; j < 10; j++) bkm[j] = even ? bk[j] : bn[j * N3 + gm];
+      for (int j = 0; j < 10; j++) bk[j] = 0.5f * (bk[j] + bn[j * N3 + gm]);
+    }
     float2 a = tab[i], am = tab[im], b = make_float2(0.0f, 0.0f), bm = b;
     if (grids > 1) b = tab[2 * SET + i], bm = tab[2 * SET + im];
-    contract_pair<float, float2>(a, am, b, bm, bk, bkm, nac);
+    contract_pair<float, float2>(a, am, b, bm, bk, nac);
     tab[i] = a;
     if (im != i) tab[im] = am;
     if (grids > 1) {
@@ -823,12 +831,14 @@ __global__ void contract_kernel(typename Cx<T>::t *z01, typename Cx<T>::t *z23, 
     C b, bm;
     b.x = 0; b.y = 0; bm = b;
     if (z23) { b = z23[g]; bm = z23[gm]; }
-    T bk[10], bkm[10];
+    T bk[10];
 #pragma unroll
     for (int i = 0; i < 10; i++) bk[i] = (T)bn[i * N3 + g];
+    if (!even) {
 #pragma unroll
-    for (int i = 0; i < 10; i++) bkm[i] = even ? bk[i] : (T)bn[i * N3 + gm];
-    contract_pair<T, C>(a, am, b, bm, bk, bkm, nac);
+      for (int i = 0; i < 10; i++) bk[i] = (T)0.5 * (bk[i] + (T)bn[i * N3 + gm]);
+    }
+    contract_pair<T, C>(a, am, b, bm, bk, nac);
     z01[g] = a;
     if (gm != g) z01[gm] = am;
     if (z23) {
@@ -839,13 +849,13 @@ __global__ void contract_kernel(typename Cx<T>::t *z01, typename Cx<T>::t *z23, 
   }
 }
 
-// Interior of felas_p from the inverse transforms, scaled by 1/N^3.
+// Interior of felas_p from the inverse transforms, scaled by 1 / (2 N^3).
 template <typename T>
 __global__ void unpack_kernel(const typename Cx<T>::t *__restrict__ w01, const typename Cx<T>::t *__restrict__ w23,
                               T *__restrict__ felas, int N, int nac) {
   const int n = N + 4;
   const long long n3 = (long long)n * n * n, N3 = (long long)N * N * N;
-  const double s = 1.0 / (double)N3;
+  const double s = 0.5 / (double)N3;  // the contraction doubled
   for (int row = blockIdx.x; row < N * N; row += gridDim.x)
   for (int x = threadIdx.x; x < N; x += blockDim.x) {
     const int z = row / N, y = row - z * N;
@@ -993,18 +1003,19 @@ static cudaError_t fft3d(ElasticPlan *p, typename Cx<T>::t *z0, typename Cx<T>::
   // the shared-memory attribute is per device
   constexpr int MAXDEV = 64;
   static std::mutex mu;
-  static bool attr_set[MAXDEV][2] = {};
-  const int which = sizeof(T) == 4 ? 1 : 0;
+  static bool attr_set[MAXDEV] = {};  // of this T
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
   if (dev < 0 || dev >= MAXDEV) return cudaErrorInvalidDevice;
   {
     std::lock_guard<std::mutex> lock(mu);
-    if (!attr_set[dev][which]) {
-      e = cudaFuncSetAttribute(fft_lines_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    if (!attr_set[dev]) {
+      e = cudaFuncSetAttribute(fft_lines_kernel<T, -1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+      if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(fft_lines_kernel<T, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
       if (e != cudaSuccess) return e;
-      attr_set[dev][which] = true;
+      attr_set[dev] = true;
     }
   }
   const long long across = (long long)N * ((N + p->tile - 1) / p->tile), along = ((long long)N * N + p->tile - 1) / p->tile;
@@ -1013,7 +1024,8 @@ static cudaError_t fft3d(ElasticPlan *p, typename Cx<T>::t *z0, typename Cx<T>::
   if (sign > 0) { order[0] = 2; order[2] = 0; }
   for (int k = 0; k < 3; k++) {
     const dim3 grid((unsigned)(order[k] == 0 ? along : across), z1 ? 2u : 1u);
-    fft_lines_kernel<T><<<grid, 256, p->smem, s>>>(z0, z1, N, order[k], p->ltile, tw, sign, p->rad, p->sd);
+    if (sign < 0) fft_lines_kernel<T, -1><<<grid, 256, p->smem, s>>>(z0, z1, N, order[k], p->ltile, tw, p->rad, p->sd);
+    else fft_lines_kernel<T, 1><<<grid, 256, p->smem, s>>>(z0, z1, N, order[k], p->ltile, tw, p->rad, p->sd);
     launch_counter()++;
   }
   return cudaGetLastError();
@@ -1037,7 +1049,7 @@ cudaError_t elastic_compute(ElasticPlan *p, const T *u, T *felas, int n, T *shel
     io.n = n;
     io.nac = p->nac;
     io.n3 = n3;
-    io.scale = (float)(1.0 / ((double)N * N * N));
+    io.scale = (float)(0.5 / ((double)N * N * N));  // the contraction doubled
     io.runs = p->runs;
     io.ustride = ustride;
     io.fstride = (long long)p->nac * n3;
