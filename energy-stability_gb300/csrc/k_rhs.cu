@@ -136,8 +136,8 @@ constexpr int RX = 32, RY = 8;
 // Bound by the FP32 issue and L1 (FP64: the FP64 pipe).  Before, every case
 // took the five-plane shared-memory ring below with the lifting inside; all
 // right-hand sides of a step, then and now: 4 fields of 36^3, FP32, no tensor
-// 103 -> 8 us; 4 + 1 fields of 196^3, diagonal tensors 525 -> 257 us, of 516^3
-// 5.74 -> 3.69 ms; 4 fields of 68^3 in FP64 303 -> 61 us.
+// 103 -> 8 us; 4 + 1 fields of 196^3, diagonal tensors 525 -> 240 us, of 516^3
+// 5.74 -> 3.59 ms; 4 fields of 68^3 in FP64 303 -> 47 us.
 template <typename PL, typename T, int NAC, bool DIAG>
 __global__ void __launch_bounds__(RX * RY, sizeof(T) == 4 ? 3 : 2)
     rhs_ac_diag_kernel(P<T> p0, const T *__restrict__ u, const T *__restrict__ felas, T *__restrict__ out, int zblocks) {
@@ -152,8 +152,9 @@ __global__ void __launch_bounds__(RX * RY, sizeof(T) == 4 ? 3 : 2)
     u += (size_t)run * p.F * n3;
     felas += (size_t)run * NAC * n3;
     out += (size_t)run * p.F * n3;
-    const int x = blockIdx.x * RX + threadIdx.x, y = blockIdx.y * RY + threadIdx.y;
-    if (x < 1 || x > n - 2 || y < 1 || y > n - 2) return;
+    const int c0 = blockIdx.x * (RX * RY) + threadIdx.x, m2 = n - 2;  // cell of the interior plane
+    if (c0 >= m2 * m2) return;
+    const int y = c0 / m2 + 1, x = c0 - (y - 1) * m2 + 1;
     const int z0 = max(1, zci * p.zc), z1 = min(n - 1, (zci + 1) * p.zc);
     if (z0 >= z1) return;
     size_t l = (size_t)z0 * nn + (size_t)y * n + x;
@@ -207,9 +208,8 @@ __global__ void __launch_bounds__(RX * RY, sizeof(T) == 4 ? 3 : 2)
   }
   // face cells of every run
   const int per = face_cells(n), total = per * p.runs;
-  const int stride = (int)(gridDim.z - zblocks) * gridDim.y * gridDim.x * (RX * RY);
-  int i = (((int)blockIdx.z - zblocks) * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
-  for (i = i * (RX * RY) + threadIdx.y * RX + threadIdx.x; i < total; i += stride) {
+  const int stride = (int)(gridDim.z - zblocks) * gridDim.x * (RX * RY);
+  for (int i = (((int)blockIdx.z - zblocks) * gridDim.x + blockIdx.x) * (RX * RY) + threadIdx.x; i < total; i += stride) {
     const int run = i / per;
     int z, y, x;
     face_cell(n, i - run * per, z, y, x);
@@ -428,8 +428,9 @@ __global__ void __launch_bounds__(RX * RY) rhs_ch_t_kernel(P<T> p0, const T *__r
   if ((int)blockIdx.z < zblocks) {
     const int zch = (n + p.zc - 1) / p.zc;
     const int run = blockIdx.z / zch, zci = blockIdx.z - run * zch;
-    const int x = blockIdx.x * RX + threadIdx.x, y = blockIdx.y * RY + threadIdx.y;
-    if (x < 1 || x > n - 2 || y < 1 || y > n - 2) return;
+    const int c0 = blockIdx.x * (RX * RY) + threadIdx.x, m2 = n - 2;  // cell of the interior plane
+    if (c0 >= m2 * m2) return;
+    const int y = c0 / m2 + 1, x = c0 - (y - 1) * m2 + 1;
     if (p0.krun) p.K[0] = (T)p0.krun[run];
     u += (size_t)run * p.F * n3;
     t += (size_t)run * n3;
@@ -442,9 +443,8 @@ __global__ void __launch_bounds__(RX * RY) rhs_ch_t_kernel(P<T> p0, const T *__r
     return;
   }
   const int per = face_cells(n), total = per * p.runs;
-  const int stride = (int)(gridDim.z - zblocks) * gridDim.y * gridDim.x * (RX * RY);
-  int i = (((int)blockIdx.z - zblocks) * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
-  for (i = i * (RX * RY) + threadIdx.y * RX + threadIdx.x; i < total; i += stride) {
+  const int stride = (int)(gridDim.z - zblocks) * gridDim.x * (RX * RY);
+  for (int i = (((int)blockIdx.z - zblocks) * gridDim.x + blockIdx.x) * (RX * RY) + threadIdx.x; i < total; i += stride) {
     const int run = i / per;
     int z, y, x;
     face_cell(n, i - run * per, z, y, x);
@@ -474,8 +474,9 @@ __global__ void __launch_bounds__(RX * RY) rhs_ch_lap_kernel(P<T> p0, const T *_
   if ((int)blockIdx.z < zblocks) {
     const int zch = (n + p.zc - 1) / p.zc;
     const int run = blockIdx.z / zch, zci = blockIdx.z - run * zch;
-    const int x = blockIdx.x * RX + threadIdx.x, y = blockIdx.y * RY + threadIdx.y;
-    if (x < 1 || x > n - 2 || y < 1 || y > n - 2) return;
+    const int c0 = blockIdx.x * (RX * RY) + threadIdx.x, m2 = n - 2;  // cell of the interior plane
+    if (c0 >= m2 * m2) return;
+    const int y = c0 / m2 + 1, x = c0 - (y - 1) * m2 + 1;
     t += (size_t)run * n3;
     out += (size_t)run * p.F * n3;
     const int z0 = max(1, zci * p.zc), z1 = min(n - 1, (zci + 1) * p.zc);
@@ -495,9 +496,8 @@ __global__ void __launch_bounds__(RX * RY) rhs_ch_lap_kernel(P<T> p0, const T *_
     return;
   }
   const int per = face_cells(n), total = per * p.runs;
-  const int stride = (int)(gridDim.z - zblocks) * gridDim.y * gridDim.x * (RX * RY);
-  int i = (((int)blockIdx.z - zblocks) * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
-  for (i = i * (RX * RY) + threadIdx.y * RX + threadIdx.x; i < total; i += stride) {
+  const int stride = (int)(gridDim.z - zblocks) * gridDim.x * (RX * RY);
+  for (int i = (((int)blockIdx.z - zblocks) * gridDim.x + blockIdx.x) * (RX * RY) + threadIdx.x; i < total; i += stride) {
     const int run = i / per;
     int z, y, x;
     face_cell(n, i - run * per, z, y, x);
@@ -687,9 +687,11 @@ __global__ void __launch_bounds__(RX * RY) mob_n_kernel(P<T> p0, const T *__rest
 // r = N - H u = N + LE (epn2 sum_a kk_a T_a u - KE u) of the Allen-Cahn fields,
 // T_a the second difference along axis a with zero values outside the block
 // (the operator the eigenbasis diagonalises).  A thread marches an (x, y)
-// column; differences are taken first, so a smooth field loses no digits.
-// q0 + blockIdx.z = (run, field) x chunk of planes.  Bound by HBM (u and N read,
-// r written).
+// column; in FP32 differences are taken first, so a smooth field loses no
+// digits; FP64, bound by its pipe, takes 7 operations instead of 14 (r's
+// rounding, dt H 2^-53 of u with dt H <= 4, is below the products').
+// q0 + blockIdx.z = (run, field) x chunk of planes.  FP32 is bound by HBM (u and
+// N read, r written).
 template <typename T>
 __global__ void __launch_bounds__(RX * RY) increment_rhs_kernel(P<T> p, const T *__restrict__ u,
                                                                 const T *__restrict__ rhs, T *__restrict__ r, T cx, T cy,
@@ -698,32 +700,44 @@ __global__ void __launch_bounds__(RX * RY) increment_rhs_kernel(P<T> p, const T 
   const size_t nn = (size_t)n * n, n3 = nn * n;
   const int zch = (n + p.zc - 1) / p.zc, q = q0 + blockIdx.z;
   const int t = q / zch, zci = q - t * zch;  // t = run nac + m
-  const int x = blockIdx.x * RX + threadIdx.x, y = blockIdx.y * RY + threadIdx.y;
-  if (x >= n || y >= n) return;
+  const int c = blockIdx.x * (RX * RY) + threadIdx.x;  // cell of the plane: no idle threads in warps
+  if (c >= n * n) return;
+  const int y = c / n, x = c - y * n;
   const size_t f = (size_t)(t / p.nac) * p.F + t % p.nac;
   const int z0 = zci * p.zc, z1 = min(n, z0 + p.zc);
-  size_t l = (size_t)z0 * nn + (size_t)y * n + x;
+  size_t l = (size_t)z0 * nn + c;
   const T *uf = u + f * n3, *nf = rhs + f * n3;
   T *rf = r + (size_t)t * n3;
+  const T cc = -(p.LE * p.KE + (T)2 * (cx + cy + cz));
   T um = z0 > 0 ? uf[l - nn] : (T)0, uc = uf[l];
 #pragma unroll 2
   for (int z = z0; z < z1; z++, l += nn) {
     const T up = z < n - 1 ? uf[l + nn] : (T)0;
     const T xm = x > 0 ? uf[l - 1] : (T)0, xp = x < n - 1 ? uf[l + 1] : (T)0;
     const T ym = y > 0 ? uf[l - n] : (T)0, yp = y < n - 1 ? uf[l + n] : (T)0;
-    const T lx = (xm - uc) + (xp - uc), ly = (ym - uc) + (yp - uc), lz = (um - uc) + (up - uc);
-    rf[l] = (nf[l] - p.LE * p.KE * uc) + (cx * lx + cy * ly + cz * lz);
+    if (sizeof(T) == 8) {
+      rf[l] = fma(cx, xm + xp, fma(cy, ym + yp, fma(cz, um + up, fma(cc, uc, nf[l]))));
+    } else {
+      const T lx = (xm - uc) + (xp - uc), ly = (ym - uc) + (yp - uc), lz = (um - uc) + (up - uc);
+      rf[l] = (nf[l] - p.LE * p.KE * uc) + (cx * lx + cy * ly + cz * lz);
+    }
     um = uc;
     uc = up;
   }
 }
 
+// CTAs over a plane's cells in order, a thread each: 32 x 8 tiles of an edge a
+// little above a multiple of 32, as every N + 4 is, left up to 44 % of the
+// threads idle, which costs FP64 pipe time all the same (4 fields of 68^3 in
+// FP64: right-hand side 61 -> 47 us, and the increments 62 -> 30 with their
+// fewer operations)
+static int plane_tiles(int cells) { return (cells + RX * RY - 1) / (RX * RY); }
+
 // z-planes per CTA: the tuned value if any, else the most of `zmax`, zmax / 2,
 // .. 2 that still gives every SM four CTAs (a small block marched 32 planes a
 // CTA left 20 CTAs on 152 SMs: 121 us at 36^3).
-static int planes_per_cta(const Phys &ph, int tuned, int zmax, int runs) {
+static int planes_per_cta(const Phys &ph, int tuned, int zmax, long long tiles, int runs) {
   if (tuned > 0) return tuned;
-  const long long tiles = (long long)((ph.n + RX - 1) / RX) * ((ph.n + RY - 1) / RY) * runs;
   int zc = zmax;
   if ((long long)((ph.n + zc - 1) / zc) * runs > 32767) zc = 32;  // the grid's z extent
   while (zc > 2 && tiles * ((ph.n + zc - 1) / zc) < 4 * 152) zc /= 2;
@@ -733,14 +747,14 @@ static int planes_per_cta(const Phys &ph, int tuned, int zmax, int runs) {
 template <typename T>
 cudaError_t launch_increment_rhs(const Phys &ph, const T *u, const T *rhs, T *r, cudaStream_t s) {
   P<T> p = to_p<T>(ph);
-  const int gx = (ph.n + RX - 1) / RX, gy = (ph.n + RY - 1) / RY, count = p.runs * ph.nac;
-  p.zc = planes_per_cta(ph, 0, 16, count);
+  const int count = p.runs * ph.nac, tiles = plane_tiles(ph.n * ph.n);
+  p.zc = planes_per_cta(ph, 0, 16, (long long)tiles * count, count);
   T c[3];
   for (int a = 0; a < 3; a++) c[a] = (T)(ph.LE * ph.epn2 * ph.kk[a] / (ph.h[a] * ph.h[a]));
   const int total = ((ph.n + p.zc - 1) / p.zc) * count;
   for (int q0 = 0; q0 < total; q0 += 65535) {  // the grid's z extent
-    increment_rhs_kernel<T><<<dim3(gx, gy, std::min(65535, total - q0)), dim3(RX, RY), 0, s>>>(p, u, rhs, r, c[0], c[1],
-                                                                                             c[2], q0);
+    increment_rhs_kernel<T><<<dim3(tiles, 1, std::min(65535, total - q0)), RX * RY, 0, s>>>(p, u, rhs, r, c[0], c[1],
+                                                                                            c[2], q0);
     launch_counter()++;
   }
   return cudaGetLastError();
@@ -754,14 +768,16 @@ static cudaError_t launch_rhs_pl(const Phys &ph, const T *u, const T *felas, T *
   long long n3 = (long long)ph.n * ph.n * ph.n;
   const int gx = (ph.n + RX - 1) / RX, gy = (ph.n + RY - 1) / RY;
   const dim3 blk(RX, RY), grd(gx, gy, ((ph.n + PZ - 1) / PZ) * p.runs);
-  // CTAs (in z) for the face cells of the kernels that take them apart
-  const int zfaces = (int)(((long long)face_cells(ph.n) * p.runs + RX * RY * gx * gy - 1) / ((long long)RX * RY * gx * gy));
+  // interior cells of a plane in order, and CTAs (in z) for the face cells, in the
+  // kernels that take them apart
+  const int tiles = plane_tiles((ph.n - 2) * (ph.n - 2));
+  const int zfaces = (int)(((long long)face_cells(ph.n) * p.runs + RX * RY * tiles - 1) / ((long long)RX * RY * tiles));
   if (ph.nac > 0) {
     bool diag = true;  // every gradient tensor diagonal
     for (int m = 0; m < ph.nac; m++)
       for (int k = 0; k < 9; k++) diag = diag && (k % 4 == 0 || p.kan[m][k] == (T)0);
     const bool ring = ph.anisotropic && !diag;
-    p.zc = planes_per_cta(ph, ph.rhs_zc, ph.anisotropic ? 32 : 8, p.runs);
+    p.zc = planes_per_cta(ph, ph.rhs_zc, ph.anisotropic ? 32 : 8, (long long)(ring ? gx * gy : tiles) * p.runs, p.runs);
     const int zblocks = ((ph.n + p.zc - 1) / p.zc) * p.runs;
     const int zface = std::min(zfaces, 65535 - zblocks);  // the face cells' loop covers the rest
     const size_t smem = sizeof(T) * ph.nac * 5 * PLANE;
@@ -769,10 +785,10 @@ static cudaError_t launch_rhs_pl(const Phys &ph, const T *u, const T *felas, T *
     switch (ph.nac * 3 + (ring ? 2 : ph.anisotropic ? 1 : 0)) {
 #define SCLET_RHS_AC(NAC)                                                                                         \
   case NAC * 3:                                                                                                   \
-    rhs_ac_diag_kernel<PL, T, NAC, false><<<dim3(gx, gy, zblocks + zface), blk, 0, s>>>(p, u, felas, out, zblocks); \
+    rhs_ac_diag_kernel<PL, T, NAC, false><<<dim3(tiles, 1, zblocks + zface), RX * RY, 0, s>>>(p, u, felas, out, zblocks); \
     break;                                                                                                        \
   case NAC * 3 + 1:                                                                                               \
-    rhs_ac_diag_kernel<PL, T, NAC, true><<<dim3(gx, gy, zblocks + zface), blk, 0, s>>>(p, u, felas, out, zblocks);  \
+    rhs_ac_diag_kernel<PL, T, NAC, true><<<dim3(tiles, 1, zblocks + zface), RX * RY, 0, s>>>(p, u, felas, out, zblocks);  \
     break;                                                                                                        \
   case NAC * 3 + 2:                                                                                               \
     e = cudaFuncSetAttribute(rhs_ac_kernel<PL, T, NAC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);   \
@@ -797,11 +813,11 @@ static cudaError_t launch_rhs_pl(const Phys &ph, const T *u, const T *felas, T *
   } else if (PL::max_nch > 0) {
     for (int m = 0; m < ph.nch; m++) {
       // one conserved field (the plugins' CH_f is defined for c_0 only)
-      p.zc = planes_per_cta(ph, 0, 16, p.runs);
+      p.zc = planes_per_cta(ph, 0, 16, (long long)tiles * p.runs, p.runs);
       const int zblocks = ((ph.n + p.zc - 1) / p.zc) * p.runs;
-      const dim3 gch(gx, gy, zblocks + zfaces);
-      rhs_ch_t_kernel<PL, T><<<gch, blk, 0, s>>>(p, u, scratch, zblocks);
-      rhs_ch_lap_kernel<PL, T><<<gch, blk, 0, s>>>(p, u, scratch, out + (long long)ph.nac * n3, zblocks);  // per run: + r F n^3
+      const dim3 gch(tiles, 1, zblocks + zfaces);
+      rhs_ch_t_kernel<PL, T><<<gch, RX * RY, 0, s>>>(p, u, scratch, zblocks);
+      rhs_ch_lap_kernel<PL, T><<<gch, RX * RY, 0, s>>>(p, u, scratch, out + (long long)ph.nac * n3, zblocks);  // per run: + r F n^3
       launch_counter() += 2;
     }
   }
