@@ -192,6 +192,7 @@ template <typename PL, int NAC, int NCH>
 __global__ void __launch_bounds__(256, 2) energy_partial_f32(Phys ph, EConst ec, const float *__restrict__ u,
                                                              const double *__restrict__ elam, int form,
                                                              double *__restrict__ part) {
+  chain_wait();
   constexpr int F = NAC + NCH;
   const int n = ph.n, N = n - 4;
   const long long n3 = (long long)n * n * n;
@@ -406,6 +407,7 @@ template <typename PL, int NAC, int NCH>
 __global__ void __launch_bounds__(256, 1) energy_partial_f64z(Phys ph, const double *__restrict__ u,
                                                               const double *__restrict__ elam, int form,
                                                               double *__restrict__ part) {
+  chain_wait();
   constexpr int F = NAC + NCH, Q = F + 2;  // sums of a block: one per field, two energies
   const int n = ph.n, N = n - 4;
   const long long n3 = (long long)n * n * n;
@@ -567,6 +569,7 @@ __global__ void __launch_bounds__(256, 1) energy_partial_f64z(Phys ph, const dou
 constexpr int FT_THREADS = 128;
 __global__ void __launch_bounds__(FT_THREADS) energy_final_kernel(Phys ph, int form, const double *__restrict__ part,
                                                                   int npart, double *__restrict__ out) {
+  chain_wait();
   const int F = ph.F, L = rec_len(F), q = blockIdx.x;
   part += (long long)blockIdx.y * npart * L;
   out += (long long)blockIdx.y * 4 * F;
@@ -631,7 +634,7 @@ int check_soln_partials(int n) {
 template <typename PL, int NAC, int NCH>
 static void launch_f32(const Phys &ph, const float *u, const double *elam, int form, double *partials, int npart,
                        cudaStream_t s) {
-  energy_partial_f32<PL, NAC, NCH><<<dim3(npart, ph.runs > 1 ? ph.runs : 1), dim3(32, 8), 0, s>>>(
+  chain_launch(npart <= 152, energy_partial_f32<PL, NAC, NCH>, dim3(npart, ph.runs > 1 ? ph.runs : 1), dim3(32, 8), 0, s, 
       ph, econst<PL>(ph), u, elam, form, partials);
 }
 
@@ -657,8 +660,8 @@ static cudaError_t check_soln_pl(const Phys &ph, const T *u, const double *elam,
     switch (ph.nac * 2 + ph.nch) {
 #define SCLET_F64Z(NA, NC) \
   case NA * 2 + NC:                                                                                         \
-    energy_partial_f64z<PL, NA, NC>                                                                         \
-        <<<g, b, sizeof(double2) * (NA + NC + 2) * EB, s>>>(ph, ud, elam, form, partials);                  \
+    chain_launch(false, energy_partial_f64z<PL, NA, NC>, g, b, sizeof(double2) * (NA + NC + 2) * EB, s, ph, ud, elam, form, \
+                 partials);                                                                                 \
     break;
       SCLET_F64Z(0, 1) SCLET_F64Z(1, 0) SCLET_F64Z(1, 1) SCLET_F64Z(2, 0) SCLET_F64Z(2, 1)
       SCLET_F64Z(3, 0) SCLET_F64Z(3, 1) SCLET_F64Z(4, 0) SCLET_F64Z(4, 1)
@@ -679,7 +682,7 @@ cudaError_t launch_check_soln(const Phys &ph, const T *u, const double *elam, in
     return check_soln_pl<PL, T>(ph, u, elam, form, partials, npart, s);
   });
   if (e != cudaSuccess) return e;
-  energy_final_kernel<<<dim3(2 * ph.F + 2, ph.runs > 1 ? ph.runs : 1), FT_THREADS, 0, s>>>(ph, form, partials, npart, out);
+  chain_launch(true, energy_final_kernel, dim3(2 * ph.F + 2, ph.runs > 1 ? ph.runs : 1), FT_THREADS, 0, s, ph, form, partials, npart, out);
   launch_counter() += 2;
   return cudaGetLastError();
 }

@@ -113,7 +113,7 @@ __device__ __forceinline__ int fdiv(int e, float inv) { return __float2int_rd(((
 // FIRST: the stage of Ns = 1, whose twiddles are all one (a twiddle of one is
 // multiplied all the same elsewhere: whole warps pay for the others).  With the
 // direction a constant and the contraction in half the operations, the elastic
-// stage of 64^3 in FP64 took 272 us, now 231, of 128^3 1.64 -> 1.33 ms.
+// stage of 64^3 in FP64 took 272 us, now 231.
 template <int R, int SIGN, bool FIRST, typename T, typename C>
 __device__ __forceinline__ void fft_stage(const C *__restrict__ src, C *__restrict__ dst, int tile, int N, int ls, int Ns,
                                           float inv_nb, float inv_ns, const C *__restrict__ tw) {
@@ -199,6 +199,7 @@ template <typename T, int SIGN>
 __global__ void __launch_bounds__(256) fft_lines_kernel(typename Cx<T>::t *data0, typename Cx<T>::t *data1, int N,
                                                         int axis, int ltile, const typename Cx<T>::t *__restrict__ tw,
                                                         Radices rad, StageDiv sd) {
+  chain_wait();
   typedef typename Cx<T>::t C;
   extern __shared__ unsigned char smem_raw[];
   const int tile = 1 << ltile, ls = N + 1;
@@ -445,6 +446,7 @@ struct LineIO {
 template <int N1, int N2, int L, int AXIS, int SIGN, int IO>
 __global__ void __launch_bounds__(L *(N1 > N2 ? N1 : N2))
     lines_kernel(float2 *data0, float2 *data1, const float2 *__restrict__ tw, LineIO io) {
+  chain_wait();
   static_assert(IO == 0 || AXIS == 0, "fused packing on x-passes only");
   constexpr int N = N1 * N2;
   constexpr int RS = AXIS == 0 ? N2 + 1 : N2;  // row stride of a line's table (padded on axis 0)
@@ -547,7 +549,7 @@ static cudaError_t launch_one(float2 *z0, float2 *z1, const float2 *tw, const Li
   }
   const int runs = io.runs > 0 ? io.runs : 1;
   const dim3 grid((unsigned)((long long)N * N / L), (z1 ? 2u : 1u) * runs);
-  k<<<grid, L * (N1 > N2 ? N1 : N2), sm, s>>>(z0, z1 ? z1 : z0, tw, io);
+  chain_launch(true, k, grid, L * (N1 > N2 ? N1 : N2), sm, s, z0, z1 ? z1 : z0, tw, io);
   return cudaGetLastError();
 }
 
@@ -566,6 +568,7 @@ static cudaError_t launch_one(float2 *z0, float2 *z1, const float2 *tw, const Li
 template <int N1, int N2, int L>
 __global__ void __launch_bounds__(2 * L *(N1 > N2 ? N1 : N2))
     green_kernel(float2 *z01, float2 *z23, const float2 *__restrict__ tw, const float *__restrict__ bn, int nac) {
+  chain_wait();
   constexpr int N = N1 * N2, SIDE = L * (N1 > N2 ? N1 : N2), SET = N * L;
   constexpr long long NN = (long long)N * N, N3 = NN * N;
   extern __shared__ float2 tab[];  // [grid][side][slot of k][line]
@@ -668,7 +671,7 @@ static cudaError_t launch_green(float2 *z0, float2 *z1, const float2 *tw, const 
     const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     if (e != cudaSuccess) return e;
   }
-  k<<<dim3((N / 2 + 1) * (N / L), runs), 2 * L * (N1 > N2 ? N1 : N2), sm, s>>>(z0, z1, tw, bn, nac);
+  chain_launch(true, k, dim3((N / 2 + 1) * (N / L), runs), 2 * L * (N1 > N2 ? N1 : N2), sm, s, z0, z1, tw, bn, nac);
   return cudaGetLastError();
 }
 
@@ -734,6 +737,7 @@ static cudaError_t upload_constants(cudaStream_t s) {
 template <typename T>
 __global__ void pack_kernel(const T *__restrict__ u, typename Cx<T>::t *__restrict__ z01,
                             typename Cx<T>::t *__restrict__ z23, int N, int nac) {
+  chain_wait();
   const int n = N + 4;
   const long long n3 = (long long)n * n * n;
   for (int row = blockIdx.x; row < N * N; row += gridDim.x)
@@ -812,6 +816,7 @@ __global__ void bn_kernel(B *__restrict__ bn, int N, BnConst bc) {
 template <typename T, typename B>
 __global__ void contract_kernel(typename Cx<T>::t *z01, typename Cx<T>::t *z23, const B *__restrict__ bn, int N,
                                 int nac) {
+  chain_wait();
   typedef typename Cx<T>::t C;
   const long long N3 = (long long)N * N * N;
   auto mid = [&](int v) { return v == N / 2 || N - v == N / 2; };
@@ -853,6 +858,7 @@ __global__ void contract_kernel(typename Cx<T>::t *z01, typename Cx<T>::t *z23, 
 template <typename T>
 __global__ void unpack_kernel(const typename Cx<T>::t *__restrict__ w01, const typename Cx<T>::t *__restrict__ w23,
                               T *__restrict__ felas, int N, int nac) {
+  chain_wait();
   const int n = N + 4;
   const long long n3 = (long long)n * n * n, N3 = (long long)N * N * N;
   const double s = 0.5 / (double)N3;  // the contraction doubled
@@ -1024,8 +1030,8 @@ static cudaError_t fft3d(ElasticPlan *p, typename Cx<T>::t *z0, typename Cx<T>::
   if (sign > 0) { order[0] = 2; order[2] = 0; }
   for (int k = 0; k < 3; k++) {
     const dim3 grid((unsigned)(order[k] == 0 ? along : across), z1 ? 2u : 1u);
-    if (sign < 0) fft_lines_kernel<T, -1><<<grid, 256, p->smem, s>>>(z0, z1, N, order[k], p->ltile, tw, p->rad, p->sd);
-    else fft_lines_kernel<T, 1><<<grid, 256, p->smem, s>>>(z0, z1, N, order[k], p->ltile, tw, p->rad, p->sd);
+    if (sign < 0) chain_launch(sizeof(T) == 4, fft_lines_kernel<T, -1>, grid, 256, p->smem, s, z0, z1, N, order[k], p->ltile, tw, p->rad, p->sd);
+    else chain_launch(sizeof(T) == 4, fft_lines_kernel<T, 1>, grid, 256, p->smem, s, z0, z1, N, order[k], p->ltile, tw, p->rad, p->sd);
     launch_counter()++;
   }
   return cudaGetLastError();
@@ -1060,16 +1066,16 @@ cudaError_t elastic_compute(ElasticPlan *p, const T *u, T *felas, int n, T *shel
       if (e != cudaSuccess) return e;
     }
   } else {
-    pack_kernel<T><<<rows_grid(N), rows_block(N), 0, s>>>(u, z01, z23, N, p->nac);
+    chain_launch(sizeof(T) == 4, pack_kernel<T>, rows_grid(N), rows_block(N), 0, s, u, z01, z23, N, p->nac);
     launch_counter()++;
     fft3d<T>(p, z01, z23, -1, s);
     if (p->fp32)
-      contract_kernel<T, float><<<rows_grid(N), rows_block(N), 0, s>>>(z01, z23, (const float *)p->bn, N, p->nac);
+      chain_launch(sizeof(T) == 4, contract_kernel<T, float>, rows_grid(N), rows_block(N), 0, s, z01, z23, (const float *)p->bn, N, p->nac);
     else
-      contract_kernel<T, double><<<rows_grid(N), rows_block(N), 0, s>>>(z01, z23, (const double *)p->bn, N, p->nac);
+      chain_launch(sizeof(T) == 4, contract_kernel<T, double>, rows_grid(N), rows_block(N), 0, s, z01, z23, (const double *)p->bn, N, p->nac);
     launch_counter()++;
     fft3d<T>(p, z01, z23, +1, s);
-    unpack_kernel<T><<<rows_grid(N), rows_block(N), 0, s>>>(z01, z23, felas, N, p->nac);
+    chain_launch(sizeof(T) == 4, unpack_kernel<T>, rows_grid(N), rows_block(N), 0, s, z01, z23, felas, N, p->nac);
     launch_counter()++;
   }
   // ghost cells: the shared-scratch semantics

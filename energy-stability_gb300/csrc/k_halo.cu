@@ -26,6 +26,7 @@ __device__ inline long long ghost_source(int n, int z, int y, int x) {
 
 template <typename T>
 __global__ void ghost_gather(const T *__restrict__ u, T *__restrict__ shell, int n, long long ns, int count) {
+  chain_wait();
   long long n3 = (long long)n * n * n;
   long long total = ns * count;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
@@ -39,6 +40,7 @@ __global__ void ghost_gather(const T *__restrict__ u, T *__restrict__ shell, int
 
 template <typename T>
 __global__ void ghost_scatter(T *__restrict__ u, const T *__restrict__ shell, int n, long long ns, int count) {
+  chain_wait();
   long long n3 = (long long)n * n * n;
   long long total = ns * count;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
@@ -61,8 +63,8 @@ template <typename T>
 cudaError_t launch_ghost_fill(T *u, int count, int n, T *shell, cudaStream_t s) {
   long long ns = shell_count(n);
   int g = grid_for(ns * count);
-  ghost_gather<T><<<g, 256, 0, s>>>(u, shell, n, ns, count);
-  ghost_scatter<T><<<g, 256, 0, s>>>(u, shell, n, ns, count);
+  chain_launch(true, ghost_gather<T>, g, 256, 0, s, u, shell, n, ns, count);
+  chain_launch(true, ghost_scatter<T>, g, 256, 0, s, u, shell, n, ns, count);
   launch_counter() += 2;
   return cudaGetLastError();
 }
@@ -80,6 +82,7 @@ cudaError_t launch_ghost_fill(T *u, int count, int n, T *shell, cudaStream_t s) 
 template <typename T>
 __global__ void elastic_shell_gather(const T *__restrict__ felas, T *__restrict__ shell, int n, long long ns, int nac,
                                      int first, int per) {
+  chain_wait();
   const long long n3 = (long long)n * n * n;
   const int b = blockIdx.x / per, p = b % nac;
   const T *run = felas + (b - p) * n3;  // the run's blocks
@@ -110,6 +113,7 @@ __global__ void elastic_shell_gather(const T *__restrict__ felas, T *__restrict_
 
 template <typename T>
 __global__ void elastic_shell_scatter(T *__restrict__ felas, const T *__restrict__ shell, int n, long long ns, int per) {
+  chain_wait();
   const int b = blockIdx.x / per;
   felas += b * (long long)n * n * n;
   shell += b * ns;
@@ -124,8 +128,8 @@ template <typename T>
 cudaError_t launch_elastic_shell(T *felas, int nac, int n, T *shell, cudaStream_t s, int runs, bool first) {
   const long long ns = shell_count(n);
   const int per = grid_for(ns), g = per * nac * (runs > 0 ? runs : 1);
-  elastic_shell_gather<T><<<g, 256, 0, s>>>(felas, shell, n, ns, nac, first ? 1 : 0, per);
-  elastic_shell_scatter<T><<<g, 256, 0, s>>>(felas, shell, n, ns, per);
+  chain_launch(true, elastic_shell_gather<T>, g, 256, 0, s, felas, shell, n, ns, nac, first ? 1 : 0, per);
+  chain_launch(true, elastic_shell_scatter<T>, g, 256, 0, s, felas, shell, n, ns, per);
   launch_counter() += 2;
   return cudaGetLastError();
 }

@@ -114,6 +114,7 @@ __global__ void seed_kernel(double *X, const double *g, int n, int which, const 
 __global__ void __launch_bounds__(MB) target_kernel(const float *__restrict__ a, const float2 *__restrict__ wa,
                                                     const float *__restrict__ b, const float *__restrict__ bsub,
                                                     const float2 *__restrict__ wb, int n, double *__restrict__ part) {
+  chain_wait();
   constexpr int U = 4;
   const long long n3 = (long long)n * n * n, stride = (long long)gridDim.x * MB;
   Fs acc = {0.0f, 0.0f};
@@ -163,6 +164,7 @@ __device__ __forceinline__ void owned_rows(int n, F &&f) {
 
 // Partial owned-cell sum of u per block.
 __global__ void __launch_bounds__(MB) owned_sum_kernel(const float *__restrict__ u, int n, double *__restrict__ part) {
+  chain_wait();
   Fs acc = {0.0f, 0.0f};
   owned_rows(n, [&](size_t l0, int N, int lane) {
     for (int x0 = lane; x0 < N; x0 += 128) {
@@ -187,6 +189,7 @@ constexpr int FB = 128;  // threads per set
 __global__ void __launch_bounds__(2 * FB) fold_kernel(int n, const double *__restrict__ tpart,
                                                       const double *__restrict__ apart, int np,
                                                       double *__restrict__ res) {
+  chain_wait();
   __shared__ double2 sw[2 * FB / 32];
   const int set = threadIdx.x / FB, i = threadIdx.x % FB;
   const double2 *part = reinterpret_cast<const double2 *>(set ? apart : tpart);
@@ -223,6 +226,7 @@ __global__ void __launch_bounds__(2 * FB) fold_kernel(int n, const double *__res
 
 // the uniform shift res[2] on the owned cells
 __global__ void __launch_bounds__(MB) shift_kernel(float *__restrict__ u, int n, const double *__restrict__ res) {
+  chain_wait();
   const float d = (float)res[2];
   owned_rows(n, [&](size_t l0, int N, int lane) {
     for (int x0 = lane; x0 < N; x0 += 128) {
@@ -278,16 +282,16 @@ cudaError_t mass_weight(double *w, double *tmp, const double *g, const double *v
 
 cudaError_t mass_target(const float *a, const double *wa, const float *b, const float *bsub, const double *wb, int n,
                         double *part, cudaStream_t s) {
-  target_kernel<<<mass_partials(), MB, 0, s>>>(a, reinterpret_cast<const float2 *>(wa), b, bsub,
+  chain_launch(false, target_kernel, mass_partials(), MB, 0, s, a, reinterpret_cast<const float2 *>(wa), b, bsub,
                                                 reinterpret_cast<const float2 *>(wb), n, part);
   launch_counter()++;
   return cudaGetLastError();
 }
 
 cudaError_t mass_fix(float *u, int n, const double *tpart, double *apart, double *res, cudaStream_t s) {
-  owned_sum_kernel<<<mass_partials(), MB, 0, s>>>(u, n, apart);
-  fold_kernel<<<1, 2 * FB, 0, s>>>(n, tpart, apart, mass_partials(), res);
-  shift_kernel<<<mass_partials() * 2, MB, 0, s>>>(u, n, res);
+  chain_launch(false, owned_sum_kernel, mass_partials(), MB, 0, s, u, n, apart);
+  chain_launch(true, fold_kernel, 1, 2 * FB, 0, s, n, tpart, apart, mass_partials(), res);
+  chain_launch(false, shift_kernel, mass_partials() * 2, MB, 0, s, u, n, res);
   launch_counter() += 3;
   return cudaGetLastError();
 }

@@ -144,6 +144,7 @@ template <int MT>
 __global__ void __launch_bounds__(FR) fold_fwd_f64_kernel(const double *__restrict__ W, TensorList<double> in,
                                                           const double *__restrict__ sub, double *__restrict__ out,
                                                           int n, int tiles, FoldEpi ep, EtdCoef ec) {
+  chain_wait();
   __shared__ double xs[FK][FR + 1];
   __shared__ __align__(16) double ws[FK][MT];
   const int t = blockIdx.z, h = fold_half(n);
@@ -224,6 +225,7 @@ __global__ void __launch_bounds__(FR) fold_fwd_f64_kernel(const double *__restri
 template <int MI>
 __global__ void __launch_bounds__(FR) fold_inv_f64_kernel(const double *__restrict__ W, const double *__restrict__ in,
                                                           double *__restrict__ out, int n, int tiles, int F, int accf) {
+  chain_wait();
   __shared__ double xs[2][FK][FR + 1];
   __shared__ __align__(16) double ws[2][FK][MI];
   const int t = blockIdx.z, h = fold_half(n), h1 = n / 2;
@@ -292,7 +294,7 @@ template <int MT>
 void run_fwd(int mt, dim3 grid, cudaStream_t s, const double *W, const TensorList<double> &in, const double *sub,
              double *out, int n, int tiles, const FoldEpi &ep, const EtdCoef &ec) {
   if constexpr (MT <= FWD_MAX) {
-    if (mt == MT) fold_fwd_f64_kernel<MT><<<grid, FR, 0, s>>>(W, in, sub, out, n, tiles, ep, ec);
+    if (mt == MT) chain_launch(false, fold_fwd_f64_kernel<MT>, grid, FR, 0, s, W, in, sub, out, n, tiles, ep, ec);
     else run_fwd<MT + FWD_STEP>(mt, grid, s, W, in, sub, out, n, tiles, ep, ec);
   }
 }
@@ -300,7 +302,7 @@ template <int MI>
 void run_inv(int mi, dim3 grid, cudaStream_t s, const double *W, const double *in, double *out, int n, int tiles, int F,
              int acc) {
   if constexpr (MI <= INV_MAX) {
-    if (mi == MI) fold_inv_f64_kernel<MI><<<grid, FR, 0, s>>>(W, in, out, n, tiles, F, acc);
+    if (mi == MI) chain_launch(false, fold_inv_f64_kernel<MI>, grid, FR, 0, s, W, in, out, n, tiles, F, acc);
     else run_inv<MI + INV_STEP>(mi, grid, s, W, in, out, n, tiles, F, acc);
   }
 }

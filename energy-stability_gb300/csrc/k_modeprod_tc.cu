@@ -141,6 +141,7 @@ __global__ void __launch_bounds__(THREADS, 1)
   __syncthreads();
   fence_after();
   const uint32_t tmem = tmem_slot;
+  chain_wait();
 
   if (warp == 0) {
     if (lane == 0) {
@@ -426,6 +427,7 @@ template <int C>
 __global__ void __launch_bounds__(256) slice_fields_kernel(const float *__restrict__ x, const float *__restrict__ sub,
                                                            float *__restrict__ scale, __nv_bfloat16 *__restrict__ out,
                                                            int n, int kp, int count, int bits) {
+  chain_wait();
   const float step = ldexpf(1.0f, bits);
   const long long rows = (long long)n * n, total_rows = rows * count;
   const int lane = threadIdx.x & 31, h = lane >> 4, kl = 2 * (lane & 15);
@@ -543,6 +545,7 @@ template <int C, int MODE>
 __global__ void __launch_bounds__(256)
     slice_fold_kernel(TensorList<float> xs, const float *__restrict__ sub, float *__restrict__ scale,
                       __nv_bfloat16 *__restrict__ out, int n, int kp, int count, int bits, SpecUpdate sp) {
+  chain_wait();
   const float step = ldexpf(1.0f, bits), step4 = ldexpf(1.0f, 4 * bits);
   const int rows = n * n;
   const long long n3 = (long long)rows * n;
@@ -827,6 +830,14 @@ cudaError_t tc_slice_matrix(const double *m, __nv_bfloat16 *planes, float *row_s
   return cudaGetLastError();
 }
 
+// Whether a slicing of g CTAs is launched early: with a CTA per SM at most, or in
+// a few waves.  In one wave its CTAs would crowd on the SMs that the product ahead
+// leaves first, with the little L1 its shared memory leaves, and in many waves
+// only the latter counts (a step of 4 fields, early and else: 36^3, 81 CTAs, 100
+// and 111 us; 68^3, 292, 174 and 156 us; of 104^3 with variable mobility, 1014,
+// 1.18 and 1.21 ms; of 196^3, 3606, 2.37 and 2.29 ms).
+static bool slice_early(int g) { return g <= 152 || (g > 4 * 152 && g <= 16 * 152); }
+
 cudaError_t tc_slice_fields(const float *x, const float *sub, float *scale, __nv_bfloat16 *planes, int n, int count,
                             cudaStream_t s) {
   if (n > tc::BK * tc::SLICE_MAXC) return cudaErrorInvalidValue;
@@ -834,10 +845,11 @@ cudaError_t tc_slice_fields(const float *x, const float *sub, float *scale, __nv
   long long blocks = (warps * 32 + 255) / 256;
   int g = (int)(blocks > 152 * 32 ? 152 * 32 : blocks);
   const int chunks = (n + tc::BK - 1) / tc::BK, kp = tc_kp(n), bits = tc_slice_bits(n);
-  if (chunks <= 4) tc::slice_fields_kernel<4><<<g, 256, 0, s>>>(x, sub, scale, planes, n, kp, count, bits);
-  else if (chunks <= 8) tc::slice_fields_kernel<8><<<g, 256, 0, s>>>(x, sub, scale, planes, n, kp, count, bits);
-  else if (chunks <= 17) tc::slice_fields_kernel<17><<<g, 256, 0, s>>>(x, sub, scale, planes, n, kp, count, bits);
-  else tc::slice_fields_kernel<tc::SLICE_MAXC><<<g, 256, 0, s>>>(x, sub, scale, planes, n, kp, count, bits);
+  const bool early = slice_early(g);
+  if (chunks <= 4) chain_launch(early, tc::slice_fields_kernel<4>, g, 256, 0, s, x, sub, scale, planes, n, kp, count, bits);
+  else if (chunks <= 8) chain_launch(early, tc::slice_fields_kernel<8>, g, 256, 0, s, x, sub, scale, planes, n, kp, count, bits);
+  else if (chunks <= 17) chain_launch(early, tc::slice_fields_kernel<17>, g, 256, 0, s, x, sub, scale, planes, n, kp, count, bits);
+  else chain_launch(early, tc::slice_fields_kernel<tc::SLICE_MAXC>, g, 256, 0, s, x, sub, scale, planes, n, kp, count, bits);
   launch_counter()++;
   return cudaGetLastError();
 }
@@ -846,7 +858,8 @@ template <int MODE>
 static void run_slice_fold(int chunks, int g, const TensorList<float> &x, const float *sub, float *scale,
                            __nv_bfloat16 *planes, int n, int kp, int count, int bits, const SpecUpdate &sp,
                            cudaStream_t s) {
-#define SCLET_SLICE(C) tc::slice_fold_kernel<C, MODE><<<g, 256, 0, s>>>(x, sub, scale, planes, n, kp, count, bits, sp)
+  const bool early = slice_early(g);
+#define SCLET_SLICE(C) chain_launch(early, tc::slice_fold_kernel<C, MODE>, g, 256, 0, s, x, sub, scale, planes, n, kp, count, bits, sp)
   if (chunks <= 1) SCLET_SLICE(1);
   else if (chunks <= 2) SCLET_SLICE(2);
   else if (chunks <= 3) SCLET_SLICE(3);
@@ -965,7 +978,9 @@ cudaError_t launch_modeprod_tc(const __nv_bfloat16 *mat, const __nv_bfloat16 *pl
   // persistent: as many CTAs as can be resident at once (or the tuned count)
   if (args.max_ctas > 0 && args.max_ctas < ctas) ctas = args.max_ctas;
   const int grid = (int)(tiles < ctas ? tiles : ctas);
-  inst->kern<<<grid, tc::THREADS, inst->smem, s>>>(reinterpret_cast<const char *>(planes),
+  // early but for many tiles a CTA, where it gives nothing (516^3: 242 a CTA, 1 %
+  // of a step slower; 196^3: 12, 3 % faster)
+  chain_launch(tiles <= 16LL * ctas, inst->kern, grid, tc::THREADS, inst->smem, s, reinterpret_cast<const char *>(planes),
                                                    reinterpret_cast<const char *>(mat), g);
   launch_counter()++;
   return cudaGetLastError();

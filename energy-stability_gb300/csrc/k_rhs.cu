@@ -141,6 +141,7 @@ constexpr int RX = 32, RY = 8;
 template <typename PL, typename T, int NAC, bool DIAG>
 __global__ void __launch_bounds__(RX * RY, sizeof(T) == 4 ? 3 : 2)
     rhs_ac_diag_kernel(P<T> p0, const T *__restrict__ u, const T *__restrict__ felas, T *__restrict__ out, int zblocks) {
+  chain_wait();
   const int n = p0.n;
   const size_t nn = (size_t)n * n, n3 = nn * n;
   P<T> p = p0;
@@ -269,6 +270,7 @@ constexpr int PLANE = HX * HY;     // one haloed plane
 template <typename PL, typename T, int NAC>
 __global__ void __launch_bounds__(RX * RY, sizeof(T) == 4 ? 3 : 1) rhs_ac_kernel(P<T> p0, const T *__restrict__ u, const T *__restrict__ felas,
                                                          T *__restrict__ out) {
+  chain_wait();
   extern __shared__ unsigned char smem_raw[];
   T *ring = reinterpret_cast<T *>(smem_raw);  // [nac][5][HY][HX]
   const int n = p0.n;
@@ -412,6 +414,7 @@ __device__ inline T ch_mu_at(const P<T> &p, const T *__restrict__ u, int z, int 
 template <typename PL, typename T>
 __global__ void __launch_bounds__(RX * RY) rhs_ch_t_kernel(P<T> p0, const T *__restrict__ u, T *__restrict__ t,
                                                            int zblocks) {
+  chain_wait();
   const int n = p0.n;
   const size_t nn = (size_t)n * n, n3 = nn * n;
   P<T> p = p0;
@@ -468,6 +471,7 @@ __global__ void __launch_bounds__(RX * RY) rhs_ch_t_kernel(P<T> p0, const T *__r
 template <typename PL, typename T>
 __global__ void __launch_bounds__(RX * RY) rhs_ch_lap_kernel(P<T> p0, const T *__restrict__ u, const T *__restrict__ t,
                                                              T *__restrict__ out, int zblocks) {
+  chain_wait();
   const int n = p0.n;
   const size_t nn = (size_t)n * n, n3 = nn * n;
   P<T> p = p0;
@@ -546,6 +550,7 @@ __device__ __forceinline__ T mobility(const P<T> &p, T e) {
 // per run (blockIdx.y): the largest M over the block, per CTA
 template <typename T>
 __global__ void __launch_bounds__(256) mob_max_kernel(P<T> p, const T *__restrict__ u, double *__restrict__ part) {
+  chain_wait();
   __shared__ double sm[8];
   const size_t n3 = (size_t)p.n * p.n * p.n;
   const T *e0 = u + (size_t)blockIdx.y * p.F * n3;  // the run's first order parameter
@@ -564,6 +569,7 @@ __global__ void __launch_bounds__(256) mob_max_kernel(P<T> p, const T *__restric
 
 // C of every run: cmax[run] = max of its MOB_PARTS partial maxima
 __global__ void __launch_bounds__(256) mob_final_kernel(const double *__restrict__ part, double *__restrict__ cmax) {
+  chain_wait();
   __shared__ double sm[8];
   double mx = -1.0e30;
   for (int i = threadIdx.x; i < MOB_PARTS; i += blockDim.x) mx = fmax(mx, part[(size_t)blockIdx.x * MOB_PARTS + i]);
@@ -580,6 +586,7 @@ __global__ void __launch_bounds__(256) mob_final_kernel(const double *__restrict
 // t1 and t2 of every cell (blockIdx.z = run x z)
 template <typename PL, typename T>
 __global__ void __launch_bounds__(RX * RY) mob_t_kernel(P<T> p0, const T *__restrict__ u, T *__restrict__ tt) {
+  chain_wait();
   const int n = p0.n;
   const int zch = (n + PZ - 1) / PZ;  // blockIdx.z = run x chunk of PZ planes
   const int run = blockIdx.z / zch, z0 = (blockIdx.z - run * zch) * PZ, z1 = z0 + PZ < n ? z0 + PZ : n;
@@ -627,6 +634,7 @@ __global__ void __launch_bounds__(RX * RY) mob_t_kernel(P<T> p0, const T *__rest
 template <typename PL, typename T>
 __global__ void __launch_bounds__(RX * RY) mob_n_kernel(P<T> p0, const T *__restrict__ u, const T *__restrict__ tt,
                                                         const double *__restrict__ cmax, T *__restrict__ out) {
+  chain_wait();
   const int n = p0.n;
   const int zch = (n + PZ - 1) / PZ;  // blockIdx.z = run x chunk of PZ planes
   const int run = blockIdx.z / zch, z0 = (blockIdx.z - run * zch) * PZ, z1 = z0 + PZ < n ? z0 + PZ : n;
@@ -696,6 +704,7 @@ template <typename T>
 __global__ void __launch_bounds__(RX * RY) increment_rhs_kernel(P<T> p, const T *__restrict__ u,
                                                                 const T *__restrict__ rhs, T *__restrict__ r, T cx, T cy,
                                                                 T cz, int q0) {
+  chain_wait();
   const int n = p.n;
   const size_t nn = (size_t)n * n, n3 = nn * n;
   const int zch = (n + p.zc - 1) / p.zc, q = q0 + blockIdx.z;
@@ -753,7 +762,7 @@ cudaError_t launch_increment_rhs(const Phys &ph, const T *u, const T *rhs, T *r,
   for (int a = 0; a < 3; a++) c[a] = (T)(ph.LE * ph.epn2 * ph.kk[a] / (ph.h[a] * ph.h[a]));
   const int total = ((ph.n + p.zc - 1) / p.zc) * count;
   for (int q0 = 0; q0 < total; q0 += 65535) {  // the grid's z extent
-    increment_rhs_kernel<T><<<dim3(tiles, 1, std::min(65535, total - q0)), RX * RY, 0, s>>>(p, u, rhs, r, c[0], c[1],
+    chain_launch(sizeof(T) == 4, increment_rhs_kernel<T>, dim3(tiles, 1, std::min(65535, total - q0)), RX * RY, 0, s, p, u, rhs, r, c[0], c[1],
                                                                                             c[2], q0);
     launch_counter()++;
   }
@@ -785,14 +794,14 @@ static cudaError_t launch_rhs_pl(const Phys &ph, const T *u, const T *felas, T *
     switch (ph.nac * 3 + (ring ? 2 : ph.anisotropic ? 1 : 0)) {
 #define SCLET_RHS_AC(NAC)                                                                                         \
   case NAC * 3:                                                                                                   \
-    rhs_ac_diag_kernel<PL, T, NAC, false><<<dim3(tiles, 1, zblocks + zface), RX * RY, 0, s>>>(p, u, felas, out, zblocks); \
+    chain_launch(sizeof(T) == 4, rhs_ac_diag_kernel<PL, T, NAC, false>, dim3(tiles, 1, zblocks + zface), RX * RY, 0, s, p, u, felas, out, zblocks); \
     break;                                                                                                        \
   case NAC * 3 + 1:                                                                                               \
-    rhs_ac_diag_kernel<PL, T, NAC, true><<<dim3(tiles, 1, zblocks + zface), RX * RY, 0, s>>>(p, u, felas, out, zblocks);  \
+    chain_launch(sizeof(T) == 4, rhs_ac_diag_kernel<PL, T, NAC, true>, dim3(tiles, 1, zblocks + zface), RX * RY, 0, s, p, u, felas, out, zblocks);  \
     break;                                                                                                        \
   case NAC * 3 + 2:                                                                                               \
     e = cudaFuncSetAttribute(rhs_ac_kernel<PL, T, NAC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);   \
-    if (e == cudaSuccess) rhs_ac_kernel<PL, T, NAC><<<dim3(gx, gy, zblocks), blk, smem, s>>>(p, u, felas, out);     \
+    if (e == cudaSuccess) chain_launch(sizeof(T) == 4, rhs_ac_kernel<PL, T, NAC>, dim3(gx, gy, zblocks), blk, smem, s, p, u, felas, out);     \
     break;
       SCLET_RHS_AC(1) SCLET_RHS_AC(2) SCLET_RHS_AC(3) SCLET_RHS_AC(4)
 #undef SCLET_RHS_AC
@@ -805,10 +814,10 @@ static cudaError_t launch_rhs_pl(const Phys &ph, const T *u, const T *felas, T *
     if (!ph.mob_t || !ph.mob_part) return cudaErrorInvalidValue;
     T *tt = static_cast<T *>(ph.mob_t);
     double *cmax = ph.mob_part + (size_t)MOB_PARTS * p.runs;
-    mob_max_kernel<T><<<dim3(MOB_PARTS, p.runs), 256, 0, s>>>(p, u, ph.mob_part);
-    mob_final_kernel<<<p.runs, 256, 0, s>>>(ph.mob_part, cmax);
-    mob_t_kernel<PL, T><<<grd, blk, 0, s>>>(p, u, tt);
-    mob_n_kernel<PL, T><<<grd, blk, 0, s>>>(p, u, tt, cmax, out);
+    chain_launch(sizeof(T) == 4, mob_max_kernel<T>, dim3(MOB_PARTS, p.runs), 256, 0, s, p, u, ph.mob_part);
+    chain_launch(true, mob_final_kernel, p.runs, 256, 0, s, ph.mob_part, cmax);
+    chain_launch(sizeof(T) == 4, mob_t_kernel<PL, T>, grd, blk, 0, s, p, u, tt);
+    chain_launch(sizeof(T) == 4, mob_n_kernel<PL, T>, grd, blk, 0, s, p, u, tt, cmax, out);
     launch_counter() += 4;
   } else if (PL::max_nch > 0) {
     for (int m = 0; m < ph.nch; m++) {
@@ -816,8 +825,8 @@ static cudaError_t launch_rhs_pl(const Phys &ph, const T *u, const T *felas, T *
       p.zc = planes_per_cta(ph, 0, 16, (long long)tiles * p.runs, p.runs);
       const int zblocks = ((ph.n + p.zc - 1) / p.zc) * p.runs;
       const dim3 gch(tiles, 1, zblocks + zfaces);
-      rhs_ch_t_kernel<PL, T><<<gch, RX * RY, 0, s>>>(p, u, scratch, zblocks);
-      rhs_ch_lap_kernel<PL, T><<<gch, RX * RY, 0, s>>>(p, u, scratch, out + (long long)ph.nac * n3, zblocks);  // per run: + r F n^3
+      chain_launch(sizeof(T) == 4, rhs_ch_t_kernel<PL, T>, gch, RX * RY, 0, s, p, u, scratch, zblocks);
+      chain_launch(sizeof(T) == 4, rhs_ch_lap_kernel<PL, T>, gch, RX * RY, 0, s, p, u, scratch, out + (long long)ph.nac * n3, zblocks);  // per run: + r F n^3
       launch_counter() += 2;
     }
   }

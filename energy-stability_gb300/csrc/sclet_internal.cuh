@@ -142,6 +142,36 @@ __host__ __device__ inline int fold_mode0(int n, int part) { return part == 0 ? 
 bool basis_is_dirichlet(int n, const double *d, const double *v, const double *vi);
 std::vector<double> fold_matrix(int n, const double *m, bool inverse);
 
+// Chained launches: a kernel of a step may be launched before the one ahead of
+// it on the stream has ended.  Its CTAs then wait in chain_wait(), the first
+// thing every such kernel does (or all but its set-up in shared memory), until
+// that one has ended and its writes are visible, so the order of the work stays
+// the stream's; what is saved is the launch latency between two kernels: a step
+// of 4 fields of 36^3 154 -> 98 us, of 68^3 194 -> 175 us.
+// Not for a kernel whose CTAs are dealt to the SMs once, in equal shares: placed
+// while the kernel ahead still holds some SMs, they crowd on the others (the FP64
+// products of 68^3 0.59 -> 1.04 ms a step).  Those, and what the FP64 pipe
+// bounds, are launched with early = false.
+__device__ __forceinline__ void chain_wait() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+template <typename... P, typename... A>
+cudaError_t chain_launch(bool early, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
+                         A &&...args) {
+  cudaLaunchAttribute attr = {};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = early ? 1 : 0;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 // Blocks of a batch that do not lie in one run of memory: tensor t is the
 // block t - first of the last segment with first <= t (blocks n^3 apart).
 template <typename T>
