@@ -1042,7 +1042,7 @@ static dim3 rows_grid(int N) { return dim3((unsigned)(N * N < 152 * 16 ? N * N :
 static dim3 rows_block(int N) { return dim3((unsigned)(N >= 256 ? 256 : (N + 31) / 32 * 32)); }
 
 template <typename T>
-cudaError_t elastic_compute(ElasticPlan *p, const T *u, T *felas, int n, T *shell, cudaStream_t s, long long ustride) {
+cudaError_t elastic_compute(ElasticPlan *p, const T *u, T *felas, int n, cudaStream_t s, long long ustride) {
   typedef typename Cx<T>::t C;
   const int N = p->N;
   const long long n3 = (long long)n * n * n;
@@ -1079,15 +1079,13 @@ cudaError_t elastic_compute(ElasticPlan *p, const T *u, T *felas, int n, T *shel
     launch_counter()++;
   }
   // ghost cells: the shared-scratch semantics
-  cudaError_t e = launch_elastic_shell<T>(felas, p->nac, n, shell, s, p->runs, p->first);
+  cudaError_t e = launch_elastic_ghosts<T>(felas, p->nac, n, s, p->runs, p->first);
   if (e != cudaSuccess) return e;
   p->first = false;
   return cudaGetLastError();
 }
 
-template cudaError_t elastic_compute<double>(ElasticPlan *, const double *, double *, int, double *, cudaStream_t,
-                                             long long);
-template cudaError_t elastic_compute<float>(ElasticPlan *, const float *, float *, int, float *, cudaStream_t,
-                                            long long);
+template cudaError_t elastic_compute<double>(ElasticPlan *, const double *, double *, int, cudaStream_t, long long);
+template cudaError_t elastic_compute<float>(ElasticPlan *, const float *, float *, int, cudaStream_t, long long);
 
 }  // namespace sclet

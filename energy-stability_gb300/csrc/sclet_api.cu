@@ -56,7 +56,7 @@ struct sclet_ctx {
   int *dev_err = nullptr;  // bounded-wait failures of device kernels
   // FP64 form: state2 = [u (F) | rhs1 (F)]
   double *state2 = nullptr, *rhs2 = nullptr, *A = nullptr, *B = nullptr;
-  double *felas = nullptr, *scratch = nullptr, *shell = nullptr;
+  double *felas = nullptr, *scratch = nullptr;
   double *V[3] = {nullptr, nullptr, nullptr}, *Vi[3] = {nullptr, nullptr, nullptr};
   double *phi1[2] = {nullptr, nullptr}, *phi2[2] = {nullptr, nullptr};
   // the basis is the block's own Dirichlet one (sclet_basis.cu): folded
@@ -67,7 +67,7 @@ struct sclet_ctx {
   // MIXED form: fstate2 = [u (F) | rhs1 (F)] in FP32; FP32 work tensors W1, W2
   // (2F blocks each); slice planes P of up to 2F tensors with their row scales
   // scaleP; sliced matrices with row scales
-  float *fstate2 = nullptr, *frhs2 = nullptr, *ffelas = nullptr, *fscratch = nullptr, *fshell = nullptr;
+  float *fstate2 = nullptr, *frhs2 = nullptr, *ffelas = nullptr, *fscratch = nullptr;
   float *W1 = nullptr, *W2 = nullptr, *scaleP = nullptr, *rsV = nullptr, *rsVi = nullptr;
   __nv_bfloat16 *P = nullptr, *matV = nullptr, *matVi = nullptr;
   float4 *coef[2] = {nullptr, nullptr};   // ETD1 coefficient pairs per field kind (full form)
@@ -507,9 +507,9 @@ void sclet_destroy(sclet_ctx *ctx) {
   if (ctx->stream) cudaStreamSynchronize(ctx->stream);
   if (ctx->copy_in) cudaStreamSynchronize(ctx->copy_in);
   if (ctx->copy_out) cudaStreamSynchronize(ctx->copy_out);
-  void *bufs[] = {ctx->state2, ctx->rhs2, ctx->A, ctx->B, ctx->felas, ctx->scratch, ctx->shell, ctx->elam,
+  void *bufs[] = {ctx->state2, ctx->rhs2, ctx->A, ctx->B, ctx->felas, ctx->scratch, ctx->elam,
                   ctx->partials, ctx->phi1[0], ctx->phi1[1], ctx->phi2[0], ctx->phi2[1], ctx->dev_err,
-                  ctx->fstate2, ctx->frhs2, ctx->ffelas, ctx->fscratch, ctx->fshell, ctx->W1, ctx->W2, ctx->P,
+                  ctx->fstate2, ctx->frhs2, ctx->ffelas, ctx->fscratch, ctx->W1, ctx->W2, ctx->P,
                   ctx->scaleP, ctx->rsV, ctx->rsVi, ctx->matV, ctx->matVi, ctx->stage64,
                   ctx->coef[0], ctx->coef[1], ctx->coef1[0], ctx->coef1[1], ctx->coef2[0],
                   ctx->coef2[1], ctx->massW, ctx->massPart,
@@ -656,9 +656,7 @@ int sclet_create_runs(const sclet_params *p, int runs, const double *krun, int p
     CC(cudaMalloc(&ctx->B, 2 * F * blk));
     CC(cudaMalloc(&ctx->felas, nfel * blk));
     CC(cudaMemsetAsync(ctx->felas, 0, nfel * blk, s));
-    // CH scratch of the right-hand side, or the elastic ghost shells of all fields
-    CC(cudaMalloc(&ctx->scratch, std::max(2 * blk, sizeof(double) * nfel * (size_t)shell_count(n))));
-    CC(cudaMalloc(&ctx->shell, sizeof(double) * F * shell_count(n)));
+    CC(cudaMalloc(&ctx->scratch, 2 * blk));  // CH scratch of the right-hand side
     for (int a = 0; a < 3; a++) {
       CC(cudaMalloc(&ctx->V[a], sizeof(double) * n * n));
       CC(cudaMalloc(&ctx->Vi[a], sizeof(double) * n * n));
@@ -679,9 +677,7 @@ int sclet_create_runs(const sclet_params *p, int runs, const double *krun, int p
     if (p->etd2) CC(cudaMalloc(&ctx->frhs2, FT * blk));
     CC(cudaMalloc(&ctx->ffelas, nfel * runs * blk));
     CC(cudaMemsetAsync(ctx->ffelas, 0, nfel * runs * blk, s));
-    // elastic ghost shells of every run's fields or the CH scratch of every run
-    CC(cudaMalloc(&ctx->fscratch, std::max((runs + 1) * blk, sizeof(float) * nfel * runs * (size_t)shell_count(n))));
-    CC(cudaMalloc(&ctx->fshell, sizeof(float) * FT * shell_count(n)));
+    CC(cudaMalloc(&ctx->fscratch, (runs + 1) * blk));  // CH scratch of every run
     CC(cudaMalloc(&ctx->W1, 2 * FT * blk));
     CC(cudaMalloc(&ctx->W2, 2 * FT * blk));
     CC(cudaMalloc(&ctx->P, sizeof(__nv_bfloat16) * plane_elems(ctx) * 2 * FT));
@@ -897,8 +893,8 @@ int sclet_transfer(sclet_ctx *ctx) {
   StageEv ev;
   long long l0 = launch_counter();
   stage_begin(ctx, 3, ev);
-  if (mixed(ctx)) CK(launch_ghost_fill<float>(fu_of(ctx), ctx->FT, ctx->n, ctx->fshell, ctx->stream));
-  else CK(launch_ghost_fill<double>(u_of(ctx), ctx->F, ctx->n, ctx->shell, ctx->stream));
+  if (mixed(ctx)) CK(launch_ghost_fill<float>(fu_of(ctx), ctx->FT, ctx->n, ctx->stream));
+  else CK(launch_ghost_fill<double>(u_of(ctx), ctx->F, ctx->n, ctx->stream));
   stage_end(ctx, ev, l0);
   return SCLET_OK;
 }
@@ -909,10 +905,10 @@ int sclet_elastic_calculate(sclet_ctx *ctx) {
   long long l0 = launch_counter();
   stage_begin(ctx, 2, ev);
   if (mixed(ctx))
-    CK(elastic_compute<float>(ctx->elastic, fu_of(ctx), ctx->ffelas, ctx->n, ctx->fscratch, ctx->stream,
+    CK(elastic_compute<float>(ctx->elastic, fu_of(ctx), ctx->ffelas, ctx->n, ctx->stream,
                               (long long)ctx->F * ctx->n3));
   else
-    CK(elastic_compute<double>(ctx->elastic, u_of(ctx), ctx->felas, ctx->n, ctx->scratch, ctx->stream));
+    CK(elastic_compute<double>(ctx->elastic, u_of(ctx), ctx->felas, ctx->n, ctx->stream));
   stage_end(ctx, ev, l0);
   return SCLET_OK;
 }

@@ -65,57 +65,15 @@ __host__ __device__ inline int wrap1(int n, int v) {
   return v < 2 ? v + N : (v >= n - 2 ? v - N : v);
 }
 
-// Number of ghost cells of an n^3 block: 4 z-planes, 4 y-slabs of the inner
-// z range, 4 x-columns of the inner z,y range.
-__host__ __device__ inline long long shell_count(int n) {
-  long long N = n - 4;
-  return 4LL * n * n + 4LL * N * n + 4LL * N * N;
-}
-// Maps a shell index to its cell.
-__device__ inline void shell_cell(int n, long long s, int &z, int &y, int &x) {
-  long long N = n - 4;
-  long long nz = 4LL * n * n;
-  if (s < nz) {
-    int p = (int)(s / ((long long)n * n));
-    long long r = s - (long long)p * n * n;
-    z = p < 2 ? p : n - 4 + p;
-    y = (int)(r / n);
-    x = (int)(r % n);
-    return;
-  }
-  s -= nz;
-  long long ny = 4LL * N * n;
-  if (s < ny) {
-    int zz = (int)(s / (4LL * n));
-    long long r = s - (long long)zz * 4 * n;
-    int p = (int)(r / n);
-    z = 2 + zz;
-    y = p < 2 ? p : n - 4 + p;
-    x = (int)(r % n);
-    return;
-  }
-  s -= ny;
-  {
-    int zz = (int)(s / (4LL * N));
-    long long r = s - (long long)zz * 4 * N;
-    int yy = (int)(r / 4);
-    int p = (int)(r % 4);
-    z = 2 + zz;
-    y = 2 + yy;
-    x = p < 2 ? p : n - 4 + p;
-  }
-}
-
 // ---- kernel launchers (each returns the launch's cudaError_t) -------------
-// Ghost fill of `count` blocks (stride n^3) in place; shell: scratch of
-// count * shell_count(n) elements.
+// Ghost fill of `count` blocks (stride n^3) in place.
 template <typename T>
-cudaError_t launch_ghost_fill(T *u, int count, int n, T *shell, cudaStream_t s);
+cudaError_t launch_ghost_fill(T *u, int count, int n, cudaStream_t s);
 // Ghost cells of the elastic force of every field and run (nac blocks per run
-// side by side) by the shared-scratch semantics, see k_halo.cu.  shell holds
-// nac * runs * shell_count(n) values; first: no previous call.
+// side by side) by the shared-scratch semantics, see k_halo.cu.  first: no
+// previous call.
 template <typename T>
-cudaError_t launch_elastic_shell(T *felas, int nac, int n, T *shell, cudaStream_t s, int runs, bool first);
+cudaError_t launch_elastic_ghosts(T *felas, int nac, int n, cudaStream_t s, int runs, bool first);
 
 // Right-hand sides of all fields into out (F blocks).  felas: nac blocks.
 template <typename T>
@@ -222,10 +180,9 @@ cudaError_t elastic_plan_create(ElasticPlan **plan, int big_n, int nac, const do
 void elastic_plan_destroy(ElasticPlan *plan);
 // felas (nac blocks of n^3) from the AC fields u (first nac blocks).
 // runs (the plan's): run r's order parameters at u + r ustride, its force at
-// felas + r nac n^3; shell holds nac * runs * shell_count(n) values
+// felas + r nac n^3
 template <typename T>
-cudaError_t elastic_compute(ElasticPlan *plan, const T *u, T *felas, int n, T *shell, cudaStream_t s,
-                            long long ustride = 0);
+cudaError_t elastic_compute(ElasticPlan *plan, const T *u, T *felas, int n, cudaStream_t s, long long ustride = 0);
 
 // Diagnostics: out (F*4 doubles, device) per field max, min, vol, energy.
 template <typename T>
