@@ -53,7 +53,7 @@
 // The folded forms (the default basis) halve the MMAs of a product and, with
 // the increment form, a field needs six products instead of nine.  Kernel time
 // of a step, dense and nine products before, now: 4 + 1 fields of 516^3
-// 52.8 -> 20.8 ms, of 196^3 1.64 -> 0.84 ms, 4 fields of 68^3 124 -> 72 us; the
+// 52.8 -> 18.9 ms, of 196^3 1.64 -> 0.82 ms, 4 fields of 68^3 124 -> 72 us; the
 // step's error against 64 bits fell from 2.2e-7 to 0.6e-7 (196^3, ten steps).
 // Warp 0 issues the copies, warp 1 issues MMAs (one elected thread each) and owns the
 // tensor memory (4 classes x 128 columns).  Warps 2-5 run the epilogue (TMEM
@@ -262,7 +262,39 @@ __global__ void __launch_bounds__(THREADS, 1)
     const float wt[NACC] = {ldexpf(1.0f, -2 * g.bits), ldexpf(1.0f, -3 * g.bits), ldexpf(1.0f, -4 * g.bits),
                             ldexpf(1.0f, -5 * g.bits)};
     int j = 0;
-    float even[FORM == 2 ? CPW : 1][32];  // the even part's tile of an inverse product
+    // An inverse product's even part E until the odd part's O is there.  With one
+    // accumulator set (DEFER) E - O then waits for the next tile: E + O is stored
+    // while the next even part's MMAs run, E - O while the odd part's do, instead
+    // of both under the even part's and nothing under the odd one's (products of
+    // 516^3 21.0 -> 18.9 ms a step, of 196^3 0.85 -> 0.82 ms).  With two sets the
+    // MMAs do not wait for the stores, and it would only add a pass over the tile
+    // (104^3: 0.26 -> 0.28 ms).
+    constexpr bool DEFER = FORM == 2 && NBUF == 1;
+    float even[FORM == 2 ? CPW : 1][32];
+    // E - O of tile tp, to the mirrored positions
+    auto store_mirror = [&](const TileIdx &tp) {
+      const long long r = (long long)tp.r_tile * BM + q * 32 + lane;
+      const int nch = (min(BN, h - tp.a_tile * BN) + 31) / 32;
+      float *outT = g.out + (long long)tp.t * g.n * rows;
+      const bool add = OUT == 2 && tp.t % g.F < g.acc;
+#pragma unroll
+      for (int cl = 0; cl < CPW; cl++) {
+        const int a0 = tp.a_tile * BN + (c_first + cl) * 32;
+        const int lim = min(32, g.n / 2 - a0);  // an odd block's middle cell has no mirror
+        const uint32_t q0 = (uint32_t)(g.n - 1 - a0) * (uint32_t)rows + (uint32_t)r;
+        if (c_first + cl < nch && r < rows) {
+#pragma unroll
+          for (int jj = 0; jj < 32; jj++)
+            if (jj < lim) {
+              float *oz = outT + (q0 - (uint32_t)jj * (uint32_t)rows);
+              if (add) atomicAdd(oz, even[cl][jj]);
+              else *oz = even[cl][jj];
+            }
+        }
+      }
+    };
+    TileIdx prev;
+    bool ok_all = true;
     for (int u = 0; u < mine; u++, j++) {
       const int b = j % NBUF;
       const TileIdx ti = cta_tile<PARTS>(u, a_tiles, g.count, blockIdx.x, gridDim.x);
@@ -286,6 +318,7 @@ __global__ void __launch_bounds__(THREADS, 1)
       ok = __shfl_sync(0xffffffffu, ok, 0);
       if (!ok) {
         if (lane == 0) failed = 1;
+        ok_all = false;
         break;
       }
       fence_after();
@@ -314,6 +347,7 @@ __global__ void __launch_bounds__(THREADS, 1)
       fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&tempty_bar[b]);
+      if (DEFER && ti.part == 0 && u > 0) store_mirror(prev);
       const bool ch = ti.t % g.F >= g.nac;  // field kind: Cahn-Hilliard
       const bool add = OUT == 2 && (FORM != 2 || ti.t % g.F < g.acc);
       const float4 *cf = ch ? g.coef[1] : g.coef[0];
@@ -340,10 +374,11 @@ __global__ void __launch_bounds__(THREADS, 1)
 #pragma unroll
             for (int jj = 0; jj < 32; jj++) {
               const float od = acc[cl][jj] * (si * __shfl_sync(0xffffffffu, rs, jj));
+              const float y = even[cl][jj] + od, z = even[cl][jj] - od;
+              if (DEFER) even[cl][jj] = z;
               if (jj < lim && live) {
-                const float y = even[cl][jj] + od, z = even[cl][jj] - od;
                 float *oy = outT + (o0 + (uint32_t)jj * urows), *oz = outT + (q0 - (uint32_t)jj * urows);
-                const bool mirror = a0 + jj < g.n / 2;  // an odd block's middle cell has none
+                const bool mirror = !DEFER && a0 + jj < g.n / 2;  // an odd block's middle cell has none
                 if (add) {
                   atomicAdd(oy, y);
                   if (mirror) atomicAdd(oz, z);
@@ -401,8 +436,13 @@ __global__ void __launch_bounds__(THREADS, 1)
           }
         }
       }
-      if (__any_sync(0xffffffffu, *(volatile int *)&failed != 0)) break;
+      prev = ti;
+      if (__any_sync(0xffffffffu, *(volatile int *)&failed != 0)) {
+        ok_all = false;
+        break;
+      }
     }
+    if (DEFER && mine > 0 && ok_all) store_mirror(prev);
   }
   __syncthreads();
   if (threadIdx.x == 0 && failed) atomicExch(g.err, 1);
