@@ -66,22 +66,33 @@ __device__ __forceinline__ GhostTree ghost_tree(int n, int r) {
   return t;
 }
 
-// `per` CTAs for each of the blocks of u.
+// `per` CTAs for each group of FILL blocks of u (a tree's cells are found once for
+// the group; finding them is most of the work).
+constexpr int FILL = 3;
 template <typename T>
-__global__ void ghost_fill(T *__restrict__ u, int n, int per) {
+__global__ void ghost_fill(T *__restrict__ u, int count, int n, int per) {
   chain_wait();
-  const int b = blockIdx.x / per, roots = 12 * (n - 4) * (n - 4);
-  u += b * ((long long)n * n * n);
+  const int b = blockIdx.x / per, roots = 12 * (n - 4) * (n - 4), live = min(FILL, count - b * FILL);
+  const long long n3 = (long long)n * n * n;
+  u += b * FILL * n3;
   for (int r = (blockIdx.x - b * per) * blockDim.x + threadIdx.x; r < roots; r += per * blockDim.x) {
     const GhostTree t = ghost_tree(n, r);
-    const T v = u[t.source];
-    T g = (T)0, h = (T)0;
-    if (t.c[0] >= 0 || t.c[1] >= 0) g = u[t.cell];
-    if (t.c[2] >= 0) h = u[t.c[1]];
-    u[t.cell] = v;
-    if (t.c[0] >= 0) u[t.c[0]] = g;
-    if (t.c[1] >= 0) u[t.c[1]] = g;
-    if (t.c[2] >= 0) u[t.c[2]] = h;
+    T v[FILL], g[FILL], h[FILL];
+#pragma unroll
+    for (int f = 0; f < FILL; f++)
+      if (f < live) {
+        v[f] = u[f * n3 + t.source];
+        if (t.c[0] >= 0 || t.c[1] >= 0) g[f] = u[f * n3 + t.cell];
+        if (t.c[2] >= 0) h[f] = u[f * n3 + t.c[1]];
+      }
+#pragma unroll
+    for (int f = 0; f < FILL; f++)
+      if (f < live) {
+        u[f * n3 + t.cell] = v[f];
+        if (t.c[0] >= 0) u[f * n3 + t.c[0]] = g[f];
+        if (t.c[1] >= 0) u[f * n3 + t.c[1]] = g[f];
+        if (t.c[2] >= 0) u[f * n3 + t.c[2]] = h[f];
+      }
   }
 }
 
@@ -94,7 +105,7 @@ static int tree_ctas(int n) {
 template <typename T>
 cudaError_t launch_ghost_fill(T *u, int count, int n, cudaStream_t s) {
   const int per = tree_ctas(n);
-  chain_launch(true, ghost_fill<T>, per * count, 256, 0, s, u, n, per);
+  chain_launch(true, ghost_fill<T>, per * ((count + FILL - 1) / FILL), 256, 0, s, u, count, n, per);
   launch_counter()++;
   return cudaGetLastError();
 }

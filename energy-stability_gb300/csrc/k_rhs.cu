@@ -136,10 +136,10 @@ constexpr int RX = 32, RY = 8;
 // Bound by the FP32 issue and L1 (FP64: the FP64 pipe).  Before, every case
 // took the five-plane shared-memory ring below with the lifting inside; all
 // right-hand sides of a step, then and now: 4 fields of 36^3, FP32, no tensor
-// 103 -> 8 us; 4 + 1 fields of 196^3, diagonal tensors 525 -> 240 us, of 516^3
-// 5.74 -> 3.59 ms; 4 fields of 68^3 in FP64 303 -> 47 us.
+// 103 -> 8 us; 4 + 1 fields of 196^3, diagonal tensors 525 -> 197 us, of 516^3
+// 5.74 -> 2.89 ms; 4 fields of 68^3 in FP64 303 -> 47 us.
 template <typename PL, typename T, int NAC, bool DIAG>
-__global__ void __launch_bounds__(RX * RY, sizeof(T) == 4 ? 3 : 2)
+__global__ void __launch_bounds__(RX * RY, (sizeof(T) == 4 ? 4 : 2) + (DIAG ? 0 : 1))
     rhs_ac_diag_kernel(P<T> p0, const T *__restrict__ u, const T *__restrict__ felas, T *__restrict__ out, int zblocks) {
   chain_wait();
   const int n = p0.n;
@@ -467,9 +467,11 @@ __global__ void __launch_bounds__(RX * RY) rhs_ch_t_kernel(P<T> p0, const T *__r
   }
 }
 
-// N_c = lap(t) (zero outside), minus mu(outside)/h^2 on faces.
+// N_c = lap(t) (zero outside), minus mu(outside)/h^2 on faces.  Six CTAs an SM:
+// the face cells' code would take 106 registers and leave the march two (54 us at
+// 196^3, now 30).
 template <typename PL, typename T>
-__global__ void __launch_bounds__(RX * RY) rhs_ch_lap_kernel(P<T> p0, const T *__restrict__ u, const T *__restrict__ t,
+__global__ void __launch_bounds__(RX * RY, sizeof(T) == 4 ? 6 : 4) rhs_ch_lap_kernel(P<T> p0, const T *__restrict__ u, const T *__restrict__ t,
                                                              T *__restrict__ out, int zblocks) {
   chain_wait();
   const int n = p0.n;
