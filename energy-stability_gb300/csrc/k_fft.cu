@@ -861,7 +861,7 @@ __global__ void unpack_kernel(const typename Cx<T>::t *__restrict__ w01, const t
   chain_wait();
   const int n = N + 4;
   const long long n3 = (long long)n * n * n, N3 = (long long)N * N * N;
-  const double s = 0.5 / (double)N3;  // the contraction doubled
+  const T s = (T)(0.5 / (double)N3);  // the contraction doubled
   for (int row = blockIdx.x; row < N * N; row += gridDim.x)
   for (int x = threadIdx.x; x < N; x += blockDim.x) {
     const int z = row / N, y = row - z * N;

@@ -17,13 +17,13 @@
 // AC_f and CH_f come from the run's physics plugin (the drop-in form of
 // formula.c:9-56, sclet_physics.cuh), a template parameter of every kernel.
 #include <algorithm>
+#include <type_traits>
 
 #include "sclet_internal.cuh"
 #include "sclet_physics.cuh"
 
 namespace sclet {
 
-constexpr int PZ = 16;  // z-planes per CTA of the variable-mobility kernels
 
 template <typename T>
 struct P {
@@ -556,9 +556,10 @@ __global__ void __launch_bounds__(256) mob_max_kernel(P<T> p, const T *__restric
   __shared__ double sm[8];
   const size_t n3 = (size_t)p.n * p.n * p.n;
   const T *e0 = u + (size_t)blockIdx.y * p.F * n3;  // the run's first order parameter
-  double mx = -1.0e30;
+  T top = (T)-1.0e30;
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n3; i += (size_t)gridDim.x * blockDim.x)
-    mx = fmax(mx, (double)mobility(p, e0[i]));
+    top = max(top, mobility(p, e0[i]));
+  double mx = (double)top;
 #pragma unroll
   for (int off = 16; off > 0; off >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, off));
   if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = mx;
@@ -585,21 +586,21 @@ __global__ void __launch_bounds__(256) mob_final_kernel(const double *__restrict
   }
 }
 
-// t1 and t2 of every cell (blockIdx.z = run x z)
+// The two kernels over the cells: planes of the march away from the faces, the
+// face cells apart in the launch's last CTAs, as the constant-mobility ones, and
+// for FP32 four CTAs an SM (with the liftings inside the march and two CTAs an SM
+// 27 and 43 us at 104^3, now 13 and 17).
+// t1 and t2 of every cell.
 template <typename PL, typename T>
-__global__ void __launch_bounds__(RX * RY) mob_t_kernel(P<T> p0, const T *__restrict__ u, T *__restrict__ tt) {
+__global__ void __launch_bounds__(RX * RY, sizeof(T) == 4 ? 4 : 2) mob_t_kernel(P<T> p0, const T *__restrict__ u0,
+                                                                                T *__restrict__ tt, int zblocks) {
   chain_wait();
   const int n = p0.n;
-  const int zch = (n + PZ - 1) / PZ;  // blockIdx.z = run x chunk of PZ planes
-  const int run = blockIdx.z / zch, z0 = (blockIdx.z - run * zch) * PZ, z1 = z0 + PZ < n ? z0 + PZ : n;
-  const int x = blockIdx.x * RX + threadIdx.x, y = blockIdx.y * RY + threadIdx.y;
-  if (x >= n || y >= n) return;
-  const size_t n3 = (size_t)n * n * n, nn = (size_t)n * n;
+  const size_t nn = (size_t)n * n, n3 = nn * n;
   P<T> p = p0;
-  if (p0.krun) p.K[0] = (T)p0.krun[run];
-  u += (size_t)run * p.F * n3;
-  T *t1 = tt + (size_t)run * 2 * n3, *t2 = t1 + n3;
-  for (int z = z0; z < z1; z++) {
+  auto cell = [&](auto face, int run, int z, int y, int x) {
+    const T *u = u0 + (size_t)run * p.F * n3;
+    T *t1 = tt + (size_t)run * 2 * n3, *t2 = t1 + n3;
     const size_t l = (size_t)z * nn + (size_t)y * n + x;
     const T *cf = u + p.nac * n3;
     T e[4] = {(T)0, (T)0, (T)0, (T)0};
@@ -617,7 +618,7 @@ __global__ void __launch_bounds__(RX * RY) mob_t_kernel(P<T> p0, const T *__rest
     la += (cz + ck - (T)2 * c) * p.ih2z;
     T a = -f0 + p.KCI * c;
     T b = p.epn2 * la - f0;
-    if (x == 0 || x == n - 1 || y == 0 || y == n - 1 || z == 0 || z == n - 1) {
+    if (decltype(face)::value) {
       const int iz = img1(n, z), iy = img1(n, y), ix = img1(n, x), lo = img1(n, -1), hi = img1(n, n);
       T w;
       if (x == 0) { w = p.epn2 * cf[L3(n, iz, iy, lo)] * p.ih2x; a += w; b += w; }
@@ -629,27 +630,44 @@ __global__ void __launch_bounds__(RX * RY) mob_t_kernel(P<T> p0, const T *__rest
     }
     t1[l] = a;
     t2[l] = b;
+  };
+  if ((int)blockIdx.z < zblocks) {
+    const int zch = (n + p.zc - 1) / p.zc;
+    const int run = blockIdx.z / zch, zci = blockIdx.z - run * zch;
+    const int c0 = blockIdx.x * (RX * RY) + threadIdx.x, m2 = n - 2;  // cell of the interior plane
+    if (c0 >= m2 * m2) return;
+    const int y = c0 / m2 + 1, x = c0 - (y - 1) * m2 + 1;
+    if (p0.krun) p.K[0] = (T)p0.krun[run];
+    const int z0 = max(1, zci * p.zc), z1 = min(n - 1, (zci + 1) * p.zc);
+    for (int z = z0; z < z1; z++) cell(std::false_type(), run, z, y, x);
+    return;
+  }
+  const int per = face_cells(n), total = per * p.runs;
+  const int stride = (int)(gridDim.z - zblocks) * gridDim.x * (RX * RY);
+  for (int i = (((int)blockIdx.z - zblocks) * gridDim.x + blockIdx.x) * (RX * RY) + threadIdx.x; i < total; i += stride) {
+    const int run = i / per;
+    int z, y, x;
+    face_cell(n, i - run * per, z, y, x);
+    if (p0.krun) p.K[0] = (T)p0.krun[run];
+    cell(std::true_type(), run, z, y, x);
   }
 }
 
-// N = LCI (f1 + f2) of every cell (blockIdx.z = run x z)
+// N = LCI (f1 + f2) of every cell.
 template <typename PL, typename T>
-__global__ void __launch_bounds__(RX * RY) mob_n_kernel(P<T> p0, const T *__restrict__ u, const T *__restrict__ tt,
-                                                        const double *__restrict__ cmax, T *__restrict__ out) {
+__global__ void __launch_bounds__(RX * RY, sizeof(T) == 4 ? 4 : 2) mob_n_kernel(P<T> p0, const T *__restrict__ u0,
+                                                                                const T *__restrict__ tt,
+                                                                                const double *__restrict__ cmax,
+                                                                                T *__restrict__ out0, int zblocks) {
   chain_wait();
   const int n = p0.n;
-  const int zch = (n + PZ - 1) / PZ;  // blockIdx.z = run x chunk of PZ planes
-  const int run = blockIdx.z / zch, z0 = (blockIdx.z - run * zch) * PZ, z1 = z0 + PZ < n ? z0 + PZ : n;
-  const int x = blockIdx.x * RX + threadIdx.x, y = blockIdx.y * RY + threadIdx.y;
-  if (x >= n || y >= n) return;
-  const size_t n3 = (size_t)n * n * n, nn = (size_t)n * n;
+  const size_t nn = (size_t)n * n, n3 = nn * n;
   P<T> p = p0;
-  if (p0.krun) p.K[0] = (T)p0.krun[run];
-  u += (size_t)run * p.F * n3;
-  out += (size_t)run * p.F * n3;
-  const T *t1 = tt + (size_t)run * 2 * n3, *t2 = t1 + n3;
-  const T C = (T)cmax[run];
-  for (int z = z0; z < z1; z++) {
+  auto cell = [&](auto face, int run, int z, int y, int x) {
+    const T *u = u0 + (size_t)run * p.F * n3;
+    T *out = out0 + (size_t)run * p.F * n3;
+    const T *t1 = tt + (size_t)run * 2 * n3, *t2 = t1 + n3;
+    const T C = (T)cmax[run];
     const size_t l = (size_t)z * nn + (size_t)y * n + x;
     // f1 = -C lap0(t1) - C mu_out / h^2
     const T tc = t1[l];
@@ -660,7 +678,7 @@ __global__ void __launch_bounds__(RX * RY) mob_n_kernel(P<T> p0, const T *__rest
     la += (at + ab - (T)2 * tc) * p.ih2y;
     la += (af + ak - (T)2 * tc) * p.ih2z;
     T f1 = -C * la;
-    if (x == 0 || x == n - 1 || y == 0 || y == n - 1 || z == 0 || z == n - 1) {
+    if (decltype(face)::value) {
       const int iz = img1(n, z), iy = img1(n, y), ix = img1(n, x), lo = img1(n, -1), hi = img1(n, n);
       if (x == 0) f1 -= C * ch_mu_at<PL>(p, u, iz, iy, lo) * p.ih2x;
       if (x == n - 1) f1 -= C * ch_mu_at<PL>(p, u, iz, iy, hi) * p.ih2x;
@@ -691,6 +709,26 @@ __global__ void __launch_bounds__(RX * RY) mob_n_kernel(P<T> p0, const T *__rest
     nb(z < n - 1, l + nn, bq, mq);
     d += (mq + mc) * (bq - bc) * hz;
     out[(size_t)p.nac * n3 + l] = p.LCI * (f1 - d);
+  };
+  if ((int)blockIdx.z < zblocks) {
+    const int zch = (n + p.zc - 1) / p.zc;
+    const int run = blockIdx.z / zch, zci = blockIdx.z - run * zch;
+    const int c0 = blockIdx.x * (RX * RY) + threadIdx.x, m2 = n - 2;  // cell of the interior plane
+    if (c0 >= m2 * m2) return;
+    const int y = c0 / m2 + 1, x = c0 - (y - 1) * m2 + 1;
+    if (p0.krun) p.K[0] = (T)p0.krun[run];
+    const int z0 = max(1, zci * p.zc), z1 = min(n - 1, (zci + 1) * p.zc);
+    for (int z = z0; z < z1; z++) cell(std::false_type(), run, z, y, x);
+    return;
+  }
+  const int per = face_cells(n), total = per * p.runs;
+  const int stride = (int)(gridDim.z - zblocks) * gridDim.x * (RX * RY);
+  for (int i = (((int)blockIdx.z - zblocks) * gridDim.x + blockIdx.x) * (RX * RY) + threadIdx.x; i < total; i += stride) {
+    const int run = i / per;
+    int z, y, x;
+    face_cell(n, i - run * per, z, y, x);
+    if (p0.krun) p.K[0] = (T)p0.krun[run];
+    cell(std::true_type(), run, z, y, x);
   }
 }
 
@@ -778,7 +816,7 @@ static cudaError_t launch_rhs_pl(const Phys &ph, const T *u, const T *felas, T *
   P<T> p = to_p<T>(ph);
   long long n3 = (long long)ph.n * ph.n * ph.n;
   const int gx = (ph.n + RX - 1) / RX, gy = (ph.n + RY - 1) / RY;
-  const dim3 blk(RX, RY), grd(gx, gy, ((ph.n + PZ - 1) / PZ) * p.runs);
+  const dim3 blk(RX, RY);
   // interior cells of a plane in order, and CTAs (in z) for the face cells, in the
   // kernels that take them apart
   const int tiles = plane_tiles((ph.n - 2) * (ph.n - 2));
@@ -818,8 +856,11 @@ static cudaError_t launch_rhs_pl(const Phys &ph, const T *u, const T *felas, T *
     double *cmax = ph.mob_part + (size_t)MOB_PARTS * p.runs;
     chain_launch(sizeof(T) == 4, mob_max_kernel<T>, dim3(MOB_PARTS, p.runs), 256, 0, s, p, u, ph.mob_part);
     chain_launch(true, mob_final_kernel, p.runs, 256, 0, s, ph.mob_part, cmax);
-    chain_launch(sizeof(T) == 4, mob_t_kernel<PL, T>, grd, blk, 0, s, p, u, tt);
-    chain_launch(sizeof(T) == 4, mob_n_kernel<PL, T>, grd, blk, 0, s, p, u, tt, cmax, out);
+    p.zc = planes_per_cta(ph, 0, 16, (long long)tiles * p.runs, p.runs);
+    const int zblocks = ((ph.n + p.zc - 1) / p.zc) * p.runs;
+    const dim3 gmb(tiles, 1, zblocks + std::min(zfaces, 65535 - zblocks));
+    chain_launch(sizeof(T) == 4, mob_t_kernel<PL, T>, gmb, RX * RY, 0, s, p, u, tt, zblocks);
+    chain_launch(sizeof(T) == 4, mob_n_kernel<PL, T>, gmb, RX * RY, 0, s, p, u, tt, cmax, out, zblocks);
     launch_counter() += 4;
   } else if (PL::max_nch > 0) {
     for (int m = 0; m < ph.nch; m++) {

@@ -4,6 +4,8 @@ where the faces, the two-cell neighbourhoods and the (x, y) tiles meet."""
 import numpy as np
 import pytest
 
+import cases
+
 pytestmark = pytest.mark.gpu
 
 
@@ -79,3 +81,15 @@ def test_no_gradient_tensor_is_pointwise_plus_lifting(N, nac, precision_name, sc
                 sl[ax] = at
                 want[tuple(sl)] += w * face
         assert np.linalg.norm(got[m] - want) <= tol * np.linalg.norm(want), m
+
+
+@pytest.mark.parametrize("N,nac", [(4, 1), (5, 2), (30, 1)])
+def test_variable_mobility_edges(N, nac, tmp_path, sclet_lib, oracle_lib):
+    """The variable-mobility kernels' march and face cells where the block's
+    edge meets their planes and CTAs, two steps against the oracle: roundings of
+    2^-53 in sums of about thirty terms, amplified by h^-4 and the step."""
+    from test_gpu_parity import _oracle_vs_gpu
+    case = cases.Case(big_n=N, nac=nac, nch=1, elastic=0, steps=2, seed=N, eta_range=(0.0, 0.9), variable_mobility=1,
+                      suffix="vme")
+    errs, _, _ = _oracle_vs_gpu(tmp_path, sclet_lib, oracle_lib, case, 2)
+    assert max(errs) <= 1e-10, errs
