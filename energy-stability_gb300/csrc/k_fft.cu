@@ -20,6 +20,7 @@
 // loaded as runs of adjacent x.  FP32 edges of 16 N1 take register transforms and
 // one kernel for z forward, contraction and z backward (green_kernel), the
 // others Stockham stages (radices 4, 2, 3, 5) and a contraction of its own.
+#include <algorithm>
 #include <mutex>
 #include <math.h>
 #include <stdlib.h>
@@ -98,7 +99,11 @@ static Radices factor(int n) {
 // keeps up to 2^ltile lines in shared memory; element-to-line maps use shifts, and
 // the per-stage quotients use a float reciprocal, exact for these ranges (a
 // quotient's fractional part stays >= 0.5 / divisor away from the next
-// integer, far above float rounding at operands below 2^16).
+// integer, far above float rounding at operands below 2^16).  The twiddles lie in
+// shared memory beside the lines and the stage tables in the constant bank: read
+// through L1 and from a copy on the stack, they were what a stage waited for
+// (elastic stage of 100^3 in FP32 351 -> 258 us a second-order step, of 64^3 in
+// FP64 227 -> 200).
 struct StageDiv {
   float inv_nb[16], inv_ns[16];
 };
@@ -116,7 +121,7 @@ __device__ __forceinline__ int fdiv(int e, float inv) { return __float2int_rd(((
 // stage of 64^3 in FP64 took 272 us, now 231.
 template <int R, int SIGN, bool FIRST, typename T, typename C>
 __device__ __forceinline__ void fft_stage(const C *__restrict__ src, C *__restrict__ dst, int tile, int N, int ls, int Ns,
-                                          float inv_nb, float inv_ns, const C *__restrict__ tw) {
+                                          float inv_nb, float inv_ns, const C *tw) {
   const int nb = N / R;
   for (int e = threadIdx.x; e < tile * nb; e += blockDim.x) {
     const int line = fdiv(e, inv_nb), j = e - line * nb;
@@ -198,13 +203,16 @@ __device__ __forceinline__ void fft_stage(const C *__restrict__ src, C *__restri
 template <typename T, int SIGN>
 __global__ void __launch_bounds__(256) fft_lines_kernel(typename Cx<T>::t *data0, typename Cx<T>::t *data1, int N,
                                                         int axis, int ltile, const typename Cx<T>::t *__restrict__ tw,
-                                                        Radices rad, StageDiv sd) {
+                                                        const __grid_constant__ Radices rad,
+                                                        const __grid_constant__ StageDiv sd) {
   chain_wait();
   typedef typename Cx<T>::t C;
   extern __shared__ unsigned char smem_raw[];
   const int tile = 1 << ltile, ls = N + 1;
   C *buf0 = reinterpret_cast<C *>(smem_raw);
   C *buf1 = buf0 + (size_t)tile * ls;
+  C *tws = buf1 + (size_t)tile * ls;  // the twiddles
+  for (int e = threadIdx.x; e < N; e += blockDim.x) tws[e] = tw[e];
   C *data = blockIdx.y == 0 ? data0 : data1;
   const long long NN = (long long)N * N;
   // Line set of this CTA
@@ -240,8 +248,8 @@ __global__ void __launch_bounds__(256) fft_lines_kernel(typename Cx<T>::t *data0
     const int R = rad.r[st];
     const float inb = sd.inv_nb[st], ins = sd.inv_ns[st];
 #define SCLET_STAGE(R)                                                                                \
-  if (st == 0) fft_stage<R, SIGN, true, T, C>(src, dst, lines, N, ls, Ns, inb, ins, tw);               \
-  else fft_stage<R, SIGN, false, T, C>(src, dst, lines, N, ls, Ns, inb, ins, tw);                      \
+  if (st == 0) fft_stage<R, SIGN, true, T, C>(src, dst, lines, N, ls, Ns, inb, ins, tws);              \
+  else fft_stage<R, SIGN, false, T, C>(src, dst, lines, N, ls, Ns, inb, ins, tws);                     \
   break;
     switch (R) {
       case 4: SCLET_STAGE(4)
@@ -885,7 +893,7 @@ struct ElasticPlan {
   void *tw;       // twiddles, complex of the working precision
   void *z01, *z23;
   void *bn;       // 10 * N^3 Green-tensor slots, double (FP64 plan) or float
-  int tile, ltile;
+  int tile, ltile, threads;
   int fast;       // FP32 plan with a two-pass register path for N
   StageDiv sd;
   size_t smem;
@@ -971,13 +979,18 @@ cudaError_t elastic_plan_create(ElasticPlan **out, int N, int nac, const double 
     if ((e = cudaGetLastError()) != cudaSuccess) goto fail;
   }
   {
-    // tile of lines per CTA: two ping-pong buffers within ~72 KB (three CTAs an SM)
-    int tile = 16;
+    // tile of lines per CTA: two ping-pong buffers within ~72 KB (three CTAs an
+    // SM).  Of 16, 8 and 4 lines 8 are best (64-byte runs at least): elastic stage
+    // of 64^3 in FP64 200, 177 and 183 us, of 100^3 in FP32 258, 230 and 244
+    int tile = 8;
     while (tile > 1 && 2 * (size_t)tile * (N + 1) * csz > 72 * 1024) tile /= 2;
     p->tile = tile;
     p->ltile = 0;
     while ((1 << p->ltile) < tile) p->ltile++;
-    p->smem = 2 * (size_t)tile * (N + 1) * csz;
+    // FP32: a thread per butterfly of four; FP64: 256, so that a tile's loads are in
+    // flight together (128 threads at 64^3: 184 us for 177)
+    p->threads = fp32 ? std::max(64, std::min(256, (tile * N / 4 + 31) / 32 * 32)) : 256;
+    p->smem = (2 * (size_t)tile * (N + 1) + N) * csz;
     int ns = 1;
     for (int st = 0; st < p->rad.count; st++) {
       p->sd.inv_nb[st] = 1.0f / (float)(N / p->rad.r[st]);
@@ -1030,8 +1043,8 @@ static cudaError_t fft3d(ElasticPlan *p, typename Cx<T>::t *z0, typename Cx<T>::
   if (sign > 0) { order[0] = 2; order[2] = 0; }
   for (int k = 0; k < 3; k++) {
     const dim3 grid((unsigned)(order[k] == 0 ? along : across), z1 ? 2u : 1u);
-    if (sign < 0) chain_launch(sizeof(T) == 4, fft_lines_kernel<T, -1>, grid, 256, p->smem, s, z0, z1, N, order[k], p->ltile, tw, p->rad, p->sd);
-    else chain_launch(sizeof(T) == 4, fft_lines_kernel<T, 1>, grid, 256, p->smem, s, z0, z1, N, order[k], p->ltile, tw, p->rad, p->sd);
+    if (sign < 0) chain_launch(sizeof(T) == 4, fft_lines_kernel<T, -1>, grid, p->threads, p->smem, s, z0, z1, N, order[k], p->ltile, tw, p->rad, p->sd);
+    else chain_launch(sizeof(T) == 4, fft_lines_kernel<T, 1>, grid, p->threads, p->smem, s, z0, z1, N, order[k], p->ltile, tw, p->rad, p->sd);
     launch_counter()++;
   }
   return cudaGetLastError();
