@@ -254,6 +254,9 @@ __global__ void __launch_bounds__(256, 2) energy_partial_f32(Phys ph, EConst ec,
     if (NCH > 0) ca = corner_pair(a[F - 1]);
     row += (long long)n * n;
     fetch(row);
+    // unrolled, so that a plane's sums change names instead of registers: 4 + 1
+    // fields of 196^3 182 -> 150 us, of 516^3 2.92 -> 2.31 ms
+#pragma unroll 4
     for (int k = k0; k < k1; k++) {
       Face4<float> b[F];  // plane k + 1
 #pragma unroll
