@@ -33,6 +33,7 @@ constexpr long long NPARAM = LAYERS * (WPER + CH);
 struct sclet_net {
   int device = 0;
   cudaStream_t stream = nullptr;
+  cudaEvent_t order = nullptr;  // between stream and a caller's (forward)
   std::string err;
   float out_scale = 1.0f;
   long long adam_t = 0;
@@ -137,11 +138,17 @@ ConvArgs conv_args(sclet_net *net, int N, int batch, int mode, int layer, const 
   return a;
 }
 
-// forward pass into net->pred (or out), keeping every activation
+// forward pass into net->pred (or out), keeping every activation; on a caller's
+// stream after the network's own work (cleared activations, weight copies) and
+// before its next
 int forward(sclet_net *net, int N, int batch, const float *in, float *out, cudaStream_t s) {
   int rc = ensure_acts(net, N, batch);
   if (rc != SCLET_OK) return rc;
   if ((rc = sync_weights(net)) != SCLET_OK) return rc;
+  if (s != net->stream) {
+    NK(cudaEventRecord(net->order, net->stream));
+    NK(cudaStreamWaitEvent(s, net->order, 0));
+  }
   NK(launch_conv_pack(in, SCLET_NET_IN, N, batch, net->x, s));
   NK(launch_conv(net->x, wl(net->wf, 0), conv_args(net, N, batch, CONV_RELU, 0, nullptr, net->h[0]), s));
   for (int k = 0; k < SCLET_NET_BLOCKS; k++) {
@@ -153,6 +160,10 @@ int forward(sclet_net *net, int N, int batch, const float *in, float *out, cudaS
   ConvArgs a = conv_args(net, N, batch, CONV_OUT_F32, LAYERS - 1, nullptr, nullptr);
   a.outf = out ? out : net->pred;
   NK(launch_conv(net->h[SCLET_NET_BLOCKS], wl(net->wf, LAYERS - 1), a, s));
+  if (s != net->stream) {
+    NK(cudaEventRecord(net->order, s));
+    NK(cudaStreamWaitEvent(net->stream, net->order, 0));
+  }
   return SCLET_OK;
 }
 
@@ -245,6 +256,7 @@ int sclet_net_create(int device, unsigned long long seed, float out_scale, sclet
   } while (0)
   NC(cudaSetDevice(device));
   NC(cudaStreamCreateWithFlags(&net->stream, cudaStreamNonBlocking));
+  NC(cudaEventCreateWithFlags(&net->order, cudaEventDisableTiming));
   const size_t pb = sizeof(float) * NPARAM;
   NC(cudaMalloc(&net->p, pb));
   NC(cudaMalloc(&net->m, pb));
@@ -281,6 +293,7 @@ void sclet_net_destroy(sclet_net *net) {
   cudaFree(net->dev_err);
   cudaFree(net->part);
   if (net->part_host) cudaFreeHost(net->part_host);
+  if (net->order) cudaEventDestroy(net->order);
   if (net->stream) cudaStreamDestroy(net->stream);
   delete net;
 }

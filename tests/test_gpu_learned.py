@@ -181,6 +181,29 @@ def _solvers(learned, sg, seed, N=24):
     return case, fine, coarse, u0
 
 
+def test_first_forward_on_the_runs_stream(learned, sclet_lib):
+    """The learned step runs the network on the coarse run's stream: a network
+    that has not run yet (activations cleared, weight copies made on its own
+    stream first) steps as one that has.  Sums of the increment's squares in any
+    order, one FP32 rounding of its scale: 1e-6 of the field."""
+    out = []
+    for warm in (False, True):
+        torch = _torch()
+        _, fine, coarse, u0 = _solvers(learned, sclet_lib, 5, N=64)
+        net = learned.Net(seed=2, out_scale=0.01)
+        net.set_params(co.random_params(4).astype(np.float32))
+        if warm:
+            x = torch.zeros((1, 8, 64, 64, 64), dtype=torch.float32, device="cuda")
+            net.forward(x, torch.zeros((1, 4, 64, 64, 64), dtype=torch.float32, device="cuda"))
+        coarse.set_fields(u0)
+        fine.set_fields(u0)
+        learned.learned_steps(coarse, fine, net, 8, 1, check_every=0, energy_tol=1e9)
+        out.append(coarse.get_fields())
+        for x in (fine, coarse, net):
+            x.close()
+    assert np.linalg.norm(out[0] - out[1]) <= 1e-6 * np.linalg.norm(out[1])
+
+
 def test_failed_steps_fall_back_to_fine_steps(learned, sclet_lib):
     """A corrector that raises the energy fails the energy check on every
     step; each step is replaced by eight fine steps, so the run equals the
