@@ -172,10 +172,16 @@ __global__ void __launch_bounds__(THREADS, 1)
   fence_after();
   const uint32_t tmem = tmem_slot;
 
+  // The launch is early (chain_launch): the weights, which no kernel since the
+  // input's packing wrote, load while the layer ahead ends.  A forward pass of
+  // 4 x 64^3 873 -> 850 us.
+  if (warp == 0 && lane == 0) {
+    mbar_expect_tx(&w_bar, TAPS * WTILE);
+    for (int t = 0; t < TAPS; t++) tma_load_2d(wsm + t * WTILE, &tmW, 0, t * CH, &w_bar);
+  }
+  chain_wait();
   if (warp == 0) {
     if (lane == 0) {
-      mbar_expect_tx(&w_bar, TAPS * WTILE);
-      for (int t = 0; t < TAPS; t++) tma_load_2d(wsm + t * WTILE, &tmW, 0, t * CH, &w_bar);
       int q = 0;  // planes loaded
       for (int t = t0; t < t1 && !*(volatile int *)&failed;) {
         // the tiles of one column: planes zh - 1 of the first .. zh + 1 of the last
@@ -435,7 +441,7 @@ cudaError_t launch_conv(const __nv_bfloat16 *in, const __nv_bfloat16 *w, const C
   const long long tiles = (long long)args.batch * N * per_plane;
   if (tiles > 0x7fffffffLL) return cudaErrorInvalidValue;
   const int grid = (int)(tiles < ctas ? tiles : ctas);
-  conv::conv_tc_kernel<<<grid, conv::THREADS, gm.smem, s>>>(ma, mw, args, gm);
+  chain_launch(true, conv::conv_tc_kernel, grid, conv::THREADS, gm.smem, s, ma, mw, args, gm);
   launch_counter()++;
   return cudaGetLastError();
 }

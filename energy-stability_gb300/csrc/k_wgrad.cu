@@ -128,6 +128,7 @@ __global__ void __launch_bounds__(WG_THREADS, 1)
   __syncthreads();
   fence_after();
   const uint32_t tmem = tmem_slot;
+  chain_wait();
 
   if (warp == 0) {
     if (lane == 0) {
@@ -316,7 +317,7 @@ cudaError_t launch_conv_wgrad(const __nv_bfloat16 *in, const __nv_bfloat16 *g, i
   if ((e = make_map_lines(&mg, g, lines, wg::G_ROWS)) != cudaSuccess) return e;
   const long long tiles = (long long)batch * N * (((long long)N * (N + 2) + ROWS - 1) / ROWS);
   const int grid = (int)(tiles < sms ? tiles : sms);
-  wg::wgrad_tc_kernel<<<grid, wg::WG_THREADS, gm.smem, s>>>(mx, mg, N, batch, dw, db, err, gm);
+  chain_launch(true, wg::wgrad_tc_kernel, grid, wg::WG_THREADS, gm.smem, s, mx, mg, N, batch, dw, db, err, gm);
   launch_counter()++;
   return cudaGetLastError();
 }
