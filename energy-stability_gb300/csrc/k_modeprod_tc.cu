@@ -53,10 +53,10 @@
 // The folded forms (the default basis) halve the MMAs of a product and, with
 // the increment form, a field needs six products instead of nine.  Kernel time
 // of a step, dense and nine products before, now: 4 + 1 fields of 516^3
-// 52.8 -> 18.9 ms, of 196^3 1.64 -> 0.82 ms, 4 fields of 68^3 124 -> 72 us; the
+// 52.8 -> 17.3 ms, of 196^3 1.64 -> 0.65 ms, 4 fields of 68^3 124 -> 72 us; the
 // step's error against 64 bits fell from 2.2e-7 to 0.6e-7 (196^3, ten steps).
 // Warp 0 issues the copies, warp 1 issues MMAs (one elected thread each) and owns the
-// tensor memory (4 classes x 128 columns).  Warps 2-5 run the epilogue (TMEM
+// tensor memory (4 classes x 128 columns).  Warps 2-9 run the epilogue (TMEM
 // lane quadrant warp % 4): the four classes of the tile are combined into
 // registers and the tensor memory is released at once, then the scaling, the
 // fused ETD update (ac_updateU_new / ch_updateU_new, calc.c:489-535) or phi2
@@ -329,6 +329,29 @@ __global__ void __launch_bounds__(THREADS, 1)
       for (int cl = 0; cl < CPW; cl++) {
         const int c = c_first + cl;
         if (c < nch) {
+          if constexpr (DEFER) {
+            // Beside E: eight columns of the four classes at a time, so that
+            // nothing spills.  Spilled values went to L2, shared memory taking
+            // all of L1: products of 516^3 18.9 -> 17.3 ms a step, of 196^3
+            // 0.82 -> 0.65 ms.
+#pragma unroll
+            for (int c8 = 0; c8 < 4; c8++) {
+              const uint32_t col = ta + (uint32_t)(c * 32 + c8 * 8);
+              uint32_t ra[8], rb[8], rc[8], rd[8];
+              tmem_ld8_async(col + 3 * BN, ra);
+              tmem_ld8_async(col + 2 * BN, rb);
+              tmem_ld8_async(col + BN, rc);
+              tmem_ld8_async(col, rd);
+              tmem_wait_ld();
+              float *o = acc[cl] + c8 * 8;
+#pragma unroll
+              for (int jj = 0; jj < 8; jj++)
+                o[jj] = fmaf(__uint_as_float(rd[jj]), wt[0],
+                             fmaf(__uint_as_float(rc[jj]), wt[1],
+                                  fmaf(__uint_as_float(rb[jj]), wt[2], __uint_as_float(ra[jj]) * wt[3])));
+            }
+            continue;
+          }
           uint32_t ra[32], rb[32];
           tmem_ld32_async(ta + 3 * BN + c * 32, ra);
           tmem_ld32_async(ta + 2 * BN + c * 32, rb);
