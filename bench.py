@@ -54,9 +54,10 @@ import cases  # noqa: E402
 METRIC = "cell-updates/s on 1 GB300: mixed/learned vs plain FP64 at ≤1e-5 rel L2"
 UNIT = "cell-updates/s"
 # DRAM bytes (read + write) of one tensor-core product launch over its
-# algorithmic bytes, from an ncu capture of a ten-tensor launch at 192^3:
-# (692.4 + 273.6) MB over 10 x 196^3 x (8 + 4) B = 903.6 MB.
-TC_TRAFFIC_RATIO = 1.069
+# algorithmic bytes, from an ncu capture of a six-tensor launch at 192^3:
+# (475.6 + 150.8) MB over 6 x 196^3 x (8 + 4) B = 542.1 MB (the slices' columns
+# beyond the 98 of a part, zeros up to 128, are read too).
+TC_TRAFFIC_RATIO = 1.155
 FP64_PEAK_TFLOPS = 1.25  # nominal GB300 FP64 rate (the measured peaks cover HBM and bf16 only)
 
 
@@ -289,19 +290,29 @@ def profiled_stages(s, steps=2):
     return dict(zip(STAGES, ms)), dict(zip(STAGES, launches))
 
 
+def step_products(case):
+    """Mode-n products of a first-order step: the order parameters advance by
+    increments (three products each way), the conserved fields from u and N (six
+    forward, three back)."""
+    return 6 * case.nac + 9 * case.nch
+
+
 def tc_mma_flops(n):
-    """Physical BF16 MMA flops of one split product (n x n matrix times an n^3
-    tensor) as the tensor-core kernel issues them: eleven MMAs per k-step of
-    16, input rows padded to 128-row tiles (M), the eigen-modes in 128-wide
-    tiles with the last one N = its live modes rounded up to 16, and k-steps
-    over the 32-wide k-blocks with the last k-block's second k-step skipped
-    when it holds only zero columns."""
+    """Physical BF16 MMA flops of one parity-folded split product (two matrices
+    of half the block's edge, h, each times h columns of n^2 lines) as the
+    tensor-core kernel issues them: eleven MMAs per k-step of 16, lines padded to
+    128-row tiles (M), the h modes in tiles of 128 (64 for h <= 64) with the last
+    one N = its live modes rounded up to 16, and k-steps over the 32-wide
+    k-blocks with the last k-block's second k-step skipped when it holds only
+    zero columns."""
+    h = (n + 1) // 2
     r_pad = (n * n + 127) // 128 * 128
-    full, last = divmod(n, 128)
-    a_eff = 128 * full + ((last + 15) // 16 * 16 if last else 0)
-    nkb = (n + 31) // 32
-    ksteps = 2 * (nkb - 1) + (2 if n - 32 * (nkb - 1) > 16 else 1)
-    return 11 * 2.0 * r_pad * a_eff * 16 * ksteps
+    bn = 64 if h <= 64 else 128
+    full, last = divmod(h, bn)
+    a_eff = bn * full + (last + 15) // 16 * 16
+    nkb = (h + 31) // 32
+    ksteps = 2 * (nkb - 1) + (2 if h - 32 * (nkb - 1) > 16 else 1)
+    return 2 * 11 * 2.0 * r_pad * a_eff * 16 * ksteps
 
 
 def tc_roofline(case, stage_ms, stage_launches, steps):
@@ -309,18 +320,16 @@ def tc_roofline(case, stage_ms, stage_launches, steps):
     steps.  The kernel is bound by the tensor pipe: `achieved` counts the
     physical BF16 MMA flops of the split product (tc_mma_flops) over its live
     CUDA-event time, against the measured sustained bf16 rate (the kernel runs
-    inside a long step); the algorithmic flops (2 n^4 per product) are
+    inside a long step); the algorithmic flops (n^4 per folded product) are
     `algorithmic_tflops`.  The HBM view (`hbm`): the bytes the kernel must
     move given its interface, the four BF16 slice planes of the input (8 B per
     element; the zero columns up to the next multiple of 32 are not counted)
-    and the FP32 output (4 B per element), plus, for the fused ETD update of
-    one product in nine, the other operand (4 B) and the coefficient pairs
-    (16 B)."""
-    n, F = case.n, case.nac + case.nch
-    per_step_products = 9 * F
+    and the FP32 output (4 B per element)."""
+    n = case.n
+    per_step_products = step_products(case)
     elems = n ** 3
-    bytes_step = per_step_products * elems * (8.0 + 4.0) + F * elems * 20.0
-    flops_step = per_step_products * 2.0 * n ** 4
+    bytes_step = per_step_products * elems * (8.0 + 4.0)
+    flops_step = per_step_products * float(n) ** 4
     mma_step = per_step_products * tc_mma_flops(n)
     t = stage_ms["tc_kernel"] / 1000.0
     launches = max(stage_launches["tc_kernel"], 1)
@@ -335,8 +344,8 @@ def tc_roofline(case, stage_ms, stage_launches, steps):
         "achieved_counts": "physical BF16 MMA flops of the split product (eleven MMAs per term)",
         "frac_of_burst_peak": mma / bf16b, "algorithmic_tflops": flops_step * steps / t / 1e12,
         "traffic": per_launch * TC_TRAFFIC_RATIO,
-        "traffic_source": f"ncu DRAM read+write / algorithmic bytes = {TC_TRAFFIC_RATIO} on one 192^3 launch of ten "
-                          "tensors (--set full capture), scaled to this launch size",
+        "traffic_source": f"ncu DRAM read+write / algorithmic bytes = {TC_TRAFFIC_RATIO} on one 192^3 launch of six "
+                          "tensors, scaled to this launch size",
         "peak_source": src, "avg_launch_ms": stage_ms["tc_kernel"] / launches,
         "hbm": {"achieved": gbs, "peak": hbm, "unit": "GB/s", "frac": gbs / hbm,
                 "algorithmic_bytes_per_launch": per_launch, "bytes_per_step": bytes_step},
@@ -549,9 +558,9 @@ def run_gpu(args, world, rank, local):
     if precision == sg.MIXED:
         roofline = tc_roofline(case, stage_ms, stage_launches, 2)
     else:
-        flops_products = 2.0 * n ** 4 * 9 * F * 2
+        flops_products = float(n) ** 4 * step_products(case) * 2
         achieved = flops_products / (stage_ms["products"] / 1000.0) / 1e12
-        roofline = {"bound": "fp64", "kernel": "modeprod_f64 (eigenbasis mode-n products)", "achieved": achieved,
+        roofline = {"bound": "fp64", "kernel": "fold_fwd_f64, fold_inv_f64 (parity-folded eigenbasis mode-n products)", "achieved": achieved,
                     "peak": FP64_PEAK_TFLOPS, "unit": "TFLOP/s", "frac": achieved / FP64_PEAK_TFLOPS, "traffic": None,
                     "peak_source": "nominal GB300 FP64",
                     "avg_launch_ms": stage_ms["products"] / max(stage_launches["products"], 1)}
