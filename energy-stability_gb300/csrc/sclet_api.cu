@@ -99,6 +99,9 @@ struct sclet_ctx {
   // one step captured as a CUDA graph (sclet_graph_step)
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t graph_exec = nullptr;
+  // counts what changes the launches of a step (the basis, the tuned shapes):
+  // a graph captured under an earlier count is captured again
+  long long launch_form = 0;
 };
 
 static std::string g_create_error;
@@ -213,6 +216,15 @@ int fail(sclet_ctx *ctx, int code, const std::string &msg) {
 int mass_weights_setup(sclet_ctx *ctx, const double *v, const double *vi);
 int queue_diagnostics(sclet_ctx *ctx, int energy_form);
 int read_diagnostics(sclet_ctx *ctx, sclet_diag *out);
+
+// the captured step is of another form, or of other shapes, than the next one
+void drop_graph(sclet_ctx *ctx) {
+  if (ctx->graph_exec) cudaGraphExecDestroy(ctx->graph_exec);
+  if (ctx->graph) cudaGraphDestroy(ctx->graph);
+  ctx->graph_exec = nullptr;
+  ctx->graph = nullptr;
+  ctx->launch_form++;
+}
 
 // elements of one sliced tensor as allocated: room for either form
 long long plane_elems(const sclet_ctx *ctx) {
@@ -736,6 +748,10 @@ int sclet_create_runs(const sclet_params *p, int runs, const double *krun, int p
 
 int sclet_set_eigen(sclet_ctx *ctx, const double *d, const double *v, const double *vi) {
   CK(cudaSetDevice(ctx->device));
+  // the basis decides which kernels a step launches (folded products, increments)
+  // and how their matrices lie, so no captured step outlives it
+  CK(cudaStreamSynchronize(ctx->stream));
+  drop_graph(ctx);
   return upload_eigen(ctx, d, v, vi);
 }
 
@@ -1446,20 +1462,12 @@ int ctx_fail(sclet_ctx *ctx, int code, const char *msg) {
 }  // namespace sclet
 
 // ---- CUDA graphs and the autotuner ------------------------------------------
-namespace {
-void drop_graph(sclet_ctx *ctx) {
-  if (ctx->graph_exec) cudaGraphExecDestroy(ctx->graph_exec);
-  if (ctx->graph) cudaGraphDestroy(ctx->graph);
-  ctx->graph_exec = nullptr;
-  ctx->graph = nullptr;
-}
-}  // namespace
-
 namespace sclet {
 // one step of ctx captured on its own stream into the capture that stream is
 // part of (the caller began it)
 int ctx_capture_step(sclet_ctx *ctx) { return sclet_step(ctx, 1); }
 long long ctx_steps_done(const sclet_ctx *ctx) { return ctx->steps_done; }
+long long ctx_launch_form(const sclet_ctx *ctx) { return ctx->launch_form; }
 }  // namespace sclet
 
 extern "C" {

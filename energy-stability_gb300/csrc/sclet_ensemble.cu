@@ -15,6 +15,7 @@
 namespace sclet {
 int ctx_capture_step(sclet_ctx *ctx);
 long long ctx_steps_done(const sclet_ctx *ctx);
+long long ctx_launch_form(const sclet_ctx *ctx);
 int ctx_device(const sclet_ctx *ctx);
 int ctx_fail(sclet_ctx *ctx, int code, const char *msg);
 }  // namespace sclet
@@ -29,6 +30,7 @@ struct sclet_ensemble {
   std::vector<cudaEvent_t> join;
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
+  std::vector<long long> form;  // each context's launch form as captured
   std::string err;
 };
 
@@ -109,6 +111,17 @@ int sclet_ensemble_step(sclet_ensemble *e, int nsteps) {
     if (rc != SCLET_OK) return rc;
     nsteps--;
   }
+  // a context whose basis or tuned shapes changed launches other kernels than the
+  // captured ones
+  std::vector<long long> form;
+  for (auto *c : e->ctx) form.push_back(ctx_launch_form(c));
+  if (e->exec && form != e->form) {
+    EK(cudaStreamSynchronize(e->master));
+    EK(cudaGraphExecDestroy(e->exec));
+    e->exec = nullptr;
+    EK(cudaGraphDestroy(e->graph));
+    e->graph = nullptr;
+  }
   if (!e->exec) {
     EK(cudaStreamBeginCapture(e->master, cudaStreamCaptureModeRelaxed));
     int rc = queue_all(e);
@@ -121,6 +134,7 @@ int sclet_ensemble_step(sclet_ensemble *e, int nsteps) {
     EK(x);
     e->graph = g;
     EK(cudaGraphInstantiate(&e->exec, e->graph, 0));
+    e->form = form;
   }
   for (int k = 0; k < nsteps; k++) EK(cudaGraphLaunch(e->exec, e->master));
   return SCLET_OK;

@@ -296,7 +296,9 @@ int sclet_stage_times(const sclet_ctx *ctx, float *ms, int *launches, int nclass
 /* No counterpart in the reference.  sclet_step's work captured once as a
  * CUDA graph (on the first call; a context that has not stepped yet takes
  * its first step uncaptured) and replayed nsteps times on the context's
- * stream: the same launches with the host's launch cost paid once. */
+ * stream: the same launches with the host's launch cost paid once.
+ * sclet_set_eigen and sclet_tune change the launches: the next call captures
+ * again (an ensemble's too). */
 int sclet_graph_step(sclet_ctx *ctx, int nsteps);
 /* No counterpart in the reference.  Autotuner of the mixed form's launch
  * shapes: times `trials` steps of each candidate (z-planes per CTA of the

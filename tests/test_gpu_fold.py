@@ -155,3 +155,58 @@ def test_basis_can_change_back_and_forth(sclet_lib):
     s.close()
     np.testing.assert_array_equal(out[0], out[2])
     np.testing.assert_array_equal(out[1], out[3])
+
+
+@pytest.mark.parametrize("precision_name", ["FP64", "MIXED"])
+@pytest.mark.parametrize("folded_first", [True, False])
+def test_captured_steps_follow_the_basis(folded_first, precision_name, sclet_lib):
+    """A step captured for one basis is not replayed for the next: each basis
+    launches kernels and matrix layouts of its own.  Bit for bit."""
+    sg = sclet_lib
+    p = _params(sg, 31, 2, 1)
+    u0 = np.random.default_rng(2).uniform(-0.3, 0.3, size=(3, 35, 35, 35))
+    bases = [cases.eigen_variant(35, 3), _swapped(35)]
+    if not folded_first:
+        bases.reverse()
+    s = sg.Solver(p, getattr(sg, precision_name))
+    for basis in bases + bases[:1]:
+        s.set_eigen(*basis)
+        s.set_fields(u0)
+        s.graph_step(3)
+        got = s.get_fields()
+        one = sg.Solver(p, getattr(sg, precision_name))
+        one.set_eigen(*basis)
+        one.set_fields(u0)
+        one.step(3)
+        np.testing.assert_array_equal(got, one.get_fields())
+        one.close()
+    s.sync()
+    s.close()
+
+
+def test_ensemble_steps_follow_the_basis(sclet_lib):
+    """The same of the graph an ensemble holds over its contexts."""
+    sg = sclet_lib
+    made = []
+    for N in (31, 20):
+        p = _params(sg, N, 2, 0)
+        u0 = np.random.default_rng(N).uniform(-0.3, 0.3, size=(2, N + 4, N + 4, N + 4))
+        made.append((p, u0, sg.Solver(p, sg.MIXED)))
+    ens = sg.Ensemble([s for _, _, s in made])
+    for basis in (cases.eigen_variant(35, 3), _swapped(35), cases.eigen_variant(35, 3)):
+        made[0][2].set_eigen(*basis)
+        for _, u0, s in made:
+            s.set_fields(u0)
+        ens.step(3)
+        ens.sync()
+        for k, (p, u0, s) in enumerate(made):
+            one = sg.Solver(p, sg.MIXED)
+            if k == 0:
+                one.set_eigen(*basis)
+            one.set_fields(u0)
+            one.step(3)
+            np.testing.assert_array_equal(s.get_fields(), one.get_fields())
+            one.close()
+    ens.close()
+    for _, _, s in made:
+        s.close()
