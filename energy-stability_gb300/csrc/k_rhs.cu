@@ -782,22 +782,29 @@ __global__ void __launch_bounds__(RX * RY) increment_rhs_kernel(P<T> p, const T 
 // fewer operations)
 static int plane_tiles(int cells) { return (cells + RX * RY - 1) / (RX * RY); }
 
-// z-planes per CTA: the tuned value if any, else the most of `zmax`, zmax / 2,
-// .. 2 that still gives every SM four CTAs (a small block marched 32 planes a
-// CTA left 20 CTAs on 152 SMs: 121 us at 36^3).
-static int planes_per_cta(const Phys &ph, int tuned, int zmax, long long tiles, int runs) {
-  if (tuned > 0) return tuned;
+// z-planes per CTA: the most of `zmax`, zmax / 2, .. 2 that still gives every SM
+// four CTAs (a small block marched 32 planes a CTA left 20 CTAs on 152 SMs:
+// 121 us at 36^3).
+static int planes_per_cta(int n, int zmax, long long tiles, int runs) {
   int zc = zmax;
-  if ((long long)((ph.n + zc - 1) / zc) * runs > 32767) zc = 32;  // the grid's z extent
-  while (zc > 2 && tiles * ((ph.n + zc - 1) / zc) < 4 * 152) zc /= 2;
+  if ((long long)((n + zc - 1) / zc) * runs > 32767) zc = std::max(zc, 32);  // the grid's z extent
+  while (zc > 2 && tiles * ((n + zc - 1) / zc) < 4 * 152) zc /= 2;
   return zc;
+}
+
+// z-planes per CTA of the Allen-Cahn right-hand side (tiles: CTAs of one plane of
+// every run).  A tuned value takes the place of the default bound, so whatever the
+// tuner chooses fills the SMs as the default does, and the default is one of its
+// candidates.
+int rhs_ac_planes(int n, int tuned, bool tensors, long long tiles, int runs) {
+  return planes_per_cta(n, tuned > 0 ? tuned : tensors ? 32 : 8, tiles, runs);
 }
 
 template <typename T>
 cudaError_t launch_increment_rhs(const Phys &ph, const T *u, const T *rhs, T *r, cudaStream_t s) {
   P<T> p = to_p<T>(ph);
   const int count = p.runs * ph.nac, tiles = plane_tiles(ph.n * ph.n);
-  p.zc = planes_per_cta(ph, 0, 16, (long long)tiles * count, count);
+  p.zc = planes_per_cta(ph.n, 16, (long long)tiles * count, count);
   T c[3];
   for (int a = 0; a < 3; a++) c[a] = (T)(ph.LE * ph.epn2 * ph.kk[a] / (ph.h[a] * ph.h[a]));
   const int total = ((ph.n + p.zc - 1) / p.zc) * count;
@@ -826,7 +833,7 @@ static cudaError_t launch_rhs_pl(const Phys &ph, const T *u, const T *felas, T *
     for (int m = 0; m < ph.nac; m++)
       for (int k = 0; k < 9; k++) diag = diag && (k % 4 == 0 || p.kan[m][k] == (T)0);
     const bool ring = ph.anisotropic && !diag;
-    p.zc = planes_per_cta(ph, ph.rhs_zc, ph.anisotropic ? 32 : 8, (long long)(ring ? gx * gy : tiles) * p.runs, p.runs);
+    p.zc = rhs_ac_planes(ph.n, ph.rhs_zc, ph.anisotropic, (long long)(ring ? gx * gy : tiles) * p.runs, p.runs);
     const int zblocks = ((ph.n + p.zc - 1) / p.zc) * p.runs;
     const int zface = std::min(zfaces, 65535 - zblocks);  // the face cells' loop covers the rest
     const size_t smem = sizeof(T) * ph.nac * 5 * PLANE;
@@ -856,7 +863,7 @@ static cudaError_t launch_rhs_pl(const Phys &ph, const T *u, const T *felas, T *
     double *cmax = ph.mob_part + (size_t)MOB_PARTS * p.runs;
     chain_launch(sizeof(T) == 4, mob_max_kernel<T>, dim3(MOB_PARTS, p.runs), 256, 0, s, p, u, ph.mob_part);
     chain_launch(true, mob_final_kernel, p.runs, 256, 0, s, ph.mob_part, cmax);
-    p.zc = planes_per_cta(ph, 0, 16, (long long)tiles * p.runs, p.runs);
+    p.zc = planes_per_cta(ph.n, 16, (long long)tiles * p.runs, p.runs);
     const int zblocks = ((ph.n + p.zc - 1) / p.zc) * p.runs;
     const dim3 gmb(tiles, 1, zblocks + std::min(zfaces, 65535 - zblocks));
     chain_launch(sizeof(T) == 4, mob_t_kernel<PL, T>, gmb, RX * RY, 0, s, p, u, tt, zblocks);
@@ -865,7 +872,7 @@ static cudaError_t launch_rhs_pl(const Phys &ph, const T *u, const T *felas, T *
   } else if (PL::max_nch > 0) {
     for (int m = 0; m < ph.nch; m++) {
       // one conserved field (the plugins' CH_f is defined for c_0 only)
-      p.zc = planes_per_cta(ph, 0, 16, (long long)tiles * p.runs, p.runs);
+      p.zc = planes_per_cta(ph.n, 16, (long long)tiles * p.runs, p.runs);
       const int zblocks = ((ph.n + p.zc - 1) / p.zc) * p.runs;
       const dim3 gch(tiles, 1, zblocks + zfaces);
       chain_launch(sizeof(T) == 4, rhs_ch_t_kernel<PL, T>, gch, RX * RY, 0, s, p, u, scratch, zblocks);

@@ -1548,11 +1548,12 @@ int sclet_tune(sclet_ctx *ctx, int trials, int *choice) {
   int dev = 0, sms = 0;
   CK(cudaGetDevice(&dev));
   CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  // coordinate search: z-planes per CTA of the RHS, then the persistent CTAs
-  // of the tensor-core products
+  // coordinate search: z-planes per CTA of the RHS (the most of them: see
+  // rhs_ac_planes; 8 or, with gradient tensors, 32 is the default), then the
+  // persistent CTAs of the tensor-core products (all SMs is the default)
   const int zcs[] = {8, 16, 32, 64};
   const int ctas[] = {sms, sms * 3 / 4, sms / 2};
-  int best_zc = 32, best_ctas = 0, rc = SCLET_OK;
+  int best_zc = 0, best_ctas = 0, rc = SCLET_OK;  // 0: the default
   float best = 1e30f, ms = 0.0f;
   for (int zc : zcs) {
     if ((rc = trial(zc, 0, &ms)) != SCLET_OK) break;

@@ -38,7 +38,7 @@ struct Phys {
   int runs;
   const double *krun;
   // launch shape chosen by the autotuner (0: the default)
-  int rhs_zc;       // z-planes per CTA of the Allen-Cahn right-hand side
+  int rhs_zc;       // most z-planes per CTA of the Allen-Cahn right-hand side (0: default)
   int tc_ctas;      // persistent CTAs of the tensor-core products
   // variable-mobility Cahn-Hilliard (VariableMobility = 1): M(eta0) =
   // mob_m0 (1 - eta0 + mob_dg eta0) (mobility_constants); device scratch of
@@ -78,6 +78,7 @@ cudaError_t launch_elastic_ghosts(T *felas, int nac, int n, cudaStream_t s, int 
 // Right-hand sides of all fields into out (F blocks).  felas: nac blocks.
 template <typename T>
 cudaError_t launch_rhs(const Phys &ph, const T *u, const T *felas, T *out, T *scratch, cudaStream_t s);
+int rhs_ac_planes(int n, int tuned, bool tensors, long long tiles, int runs);
 
 // Mode-n product with rotation, FP64: for `count` tensors,
 // out_t[a'*n*n + r] = sum_a M[a'*n + a] in_t[r*n + a]  (M row-major).

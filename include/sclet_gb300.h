@@ -301,11 +301,12 @@ int sclet_stage_times(const sclet_ctx *ctx, float *ms, int *launches, int nclass
  * again (an ensemble's too). */
 int sclet_graph_step(sclet_ctx *ctx, int nsteps);
 /* No counterpart in the reference.  Autotuner of the mixed form's launch
- * shapes: times `trials` steps of each candidate (z-planes per CTA of the
- * Allen-Cahn right-hand side: 8, 16, 32, 64; then persistent CTAs of the
- * tensor-core products: all SMs, 3/4, 1/2), keeps the fastest and puts the
- * state back after every trial, so results do not change.  choice (2 ints,
- * may be NULL) receives the z-planes and the CTA count (0: all SMs). */
+ * shapes: times `trials` steps of each candidate (the most z-planes per CTA of
+ * the Allen-Cahn right-hand side: 8, 16, 32, 64, fewer where that would leave
+ * SMs without work; then persistent CTAs of the tensor-core products: all SMs,
+ * 3/4, 1/2), keeps the fastest and puts the state back after every trial, so
+ * results do not change.  The default shapes are among the candidates.  choice
+ * (2 ints, may be NULL) receives the z-planes and the CTA count (0: all SMs). */
 int sclet_tune(sclet_ctx *ctx, int trials, int *choice);
 /* The batched ensemble (no counterpart in the reference): contexts of
  * several block sizes (each holding its runs side by side) advanced
