@@ -146,9 +146,10 @@ __global__ void __launch_bounds__(RX * RY, (sizeof(T) == 4 ? 4 : 2) + (DIAG ? 0 
   const size_t nn = (size_t)n * n, n3 = nn * n;
   P<T> p = p0;
   const bool el = p.elastic == 1, has_c = p.nch > 0;
-  if ((int)blockIdx.z < zblocks) {
+  const int bz = blockIdx.y * gridDim.z + blockIdx.z;  // the march's (run, chunk of planes), then the face cells'
+  if (bz < zblocks) {
     const int zchunks = (n + p.zc - 1) / p.zc;
-    const int run = blockIdx.z / zchunks, zci = blockIdx.z - run * zchunks;
+    const int run = bz / zchunks, zci = bz - run * zchunks;
     if (p0.krun) p.K[0] = (T)p0.krun[run];
     u += (size_t)run * p.F * n3;
     felas += (size_t)run * NAC * n3;
@@ -209,8 +210,8 @@ __global__ void __launch_bounds__(RX * RY, (sizeof(T) == 4 ? 4 : 2) + (DIAG ? 0 
   }
   // face cells of every run
   const int per = face_cells(n), total = per * p.runs;
-  const int stride = (int)(gridDim.z - zblocks) * gridDim.x * (RX * RY);
-  for (int i = (((int)blockIdx.z - zblocks) * gridDim.x + blockIdx.x) * (RX * RY) + threadIdx.x; i < total; i += stride) {
+  const int stride = (int)(gridDim.y * gridDim.z - zblocks) * gridDim.x * (RX * RY);
+  for (int i = ((bz - zblocks) * gridDim.x + blockIdx.x) * (RX * RY) + threadIdx.x; i < total; i += stride) {
     const int run = i / per;
     int z, y, x;
     face_cell(n, i - run * per, z, y, x);
@@ -834,17 +835,21 @@ static cudaError_t launch_rhs_pl(const Phys &ph, const T *u, const T *felas, T *
       for (int k = 0; k < 9; k++) diag = diag && (k % 4 == 0 || p.kan[m][k] == (T)0);
     const bool ring = ph.anisotropic && !diag;
     p.zc = rhs_ac_planes(ph.n, ph.rhs_zc, ph.anisotropic, (long long)(ring ? gx * gy : tiles) * p.runs, p.runs);
+    // more runs than a grid of 32 planes a CTA holds in z are refused
+    if ((long long)((ph.n + 31) / 32) * p.runs > 65535) return cudaErrorInvalidConfiguration;
     const int zblocks = ((ph.n + p.zc - 1) / p.zc) * p.runs;
-    const int zface = std::min(zfaces, 65535 - zblocks);  // the face cells' loop covers the rest
+    // the face cells' CTAs come after the march's; what z does not hold goes to y
+    const int gyz = (zblocks + zfaces + 65534) / 65535;
+    const dim3 gdiag(tiles, gyz, (zblocks + zfaces + gyz - 1) / gyz);
     const size_t smem = sizeof(T) * ph.nac * 5 * PLANE;
     cudaError_t e = cudaSuccess;
     switch (ph.nac * 3 + (ring ? 2 : ph.anisotropic ? 1 : 0)) {
 #define SCLET_RHS_AC(NAC)                                                                                         \
   case NAC * 3:                                                                                                   \
-    chain_launch(sizeof(T) == 4, rhs_ac_diag_kernel<PL, T, NAC, false>, dim3(tiles, 1, zblocks + zface), RX * RY, 0, s, p, u, felas, out, zblocks); \
+    chain_launch(sizeof(T) == 4, rhs_ac_diag_kernel<PL, T, NAC, false>, gdiag, RX * RY, 0, s, p, u, felas, out, zblocks); \
     break;                                                                                                        \
   case NAC * 3 + 1:                                                                                               \
-    chain_launch(sizeof(T) == 4, rhs_ac_diag_kernel<PL, T, NAC, true>, dim3(tiles, 1, zblocks + zface), RX * RY, 0, s, p, u, felas, out, zblocks);  \
+    chain_launch(sizeof(T) == 4, rhs_ac_diag_kernel<PL, T, NAC, true>, gdiag, RX * RY, 0, s, p, u, felas, out, zblocks);  \
     break;                                                                                                        \
   case NAC * 3 + 2:                                                                                               \
     e = cudaFuncSetAttribute(rhs_ac_kernel<PL, T, NAC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);   \
@@ -865,7 +870,7 @@ static cudaError_t launch_rhs_pl(const Phys &ph, const T *u, const T *felas, T *
     chain_launch(true, mob_final_kernel, p.runs, 256, 0, s, ph.mob_part, cmax);
     p.zc = planes_per_cta(ph.n, 16, (long long)tiles * p.runs, p.runs);
     const int zblocks = ((ph.n + p.zc - 1) / p.zc) * p.runs;
-    const dim3 gmb(tiles, 1, zblocks + std::min(zfaces, 65535 - zblocks));
+    const dim3 gmb(tiles, 1, zblocks + zfaces);  // one run: nch > 0
     chain_launch(sizeof(T) == 4, mob_t_kernel<PL, T>, gmb, RX * RY, 0, s, p, u, tt, zblocks);
     chain_launch(sizeof(T) == 4, mob_n_kernel<PL, T>, gmb, RX * RY, 0, s, p, u, tt, cmax, out, zblocks);
     launch_counter() += 4;

@@ -98,3 +98,30 @@ def test_ensemble_of_sizes_matches_each_context(sclet_lib):
         s.step(5)
         np.testing.assert_array_equal(g, s.get_fields())
         s.close()
+
+
+def test_as_many_runs_as_the_grid_holds(sclet_lib):
+    """65535 runs fill the right-hand side's grid in z with their march alone; the
+    face cells are computed all the same.  One run more is refused."""
+    sg = sclet_lib
+    p = sg.default_params()
+    p.nx = p.ny = p.nz = 8
+    p.xmax = p.ymax = p.zmax = 4.0
+    p.nac, p.nch, p.elastic = 1, 0, 0
+    runs = 65535
+    u0 = np.random.default_rng(5).uniform(-0.3, 0.3, size=(runs, 8, 8, 8))
+    s = sg.Solver(p, sg.MIXED, runs=runs)
+    s.set_fields(u0)
+    s.step(2)
+    got = s.get_fields()
+    s.close()
+    for r in (0, 1, 40000, runs - 1):
+        one = sg.Solver(p, sg.MIXED)
+        one.set_fields(u0[r:r + 1])
+        one.step(2)
+        np.testing.assert_array_equal(got[r:r + 1], one.get_fields(), err_msg=str(r))
+        one.close()
+    s = sg.Solver(p, sg.MIXED, runs=runs + 1)
+    with pytest.raises(RuntimeError):
+        s.step(1)
+    s.close()
