@@ -9,9 +9,9 @@
 // corrector (correct_U_new, calc.c:569-583) adds <w2, N2 - N1>, w2 from phi2.
 // The weights are computed once in FP64 from the FP64 basis and kept as FP32
 // (hi, lo) pairs.  Each mixed step forms the target from the stored state with
-// error-free FP32 products and sums per thread (about 48 bits, no FP64
-// instructions per cell) and compensated FP64 sums across threads in a fixed
-// order, then shifts the owned cells of the new state uniformly so their sum
+// error-free FP32 products and sums of up to 256 cells per thread (about 48
+// bits, no FP64 instructions per cell) and compensated FP64 sums of these and
+// across threads in a fixed order, then shifts the owned cells of the new state uniformly so their sum
 // meets it.  The FP32 state itself rounds that sum at the level of its own
 // storage (about 1e-11 relative at 192^3).
 #include "sclet_internal.cuh"
@@ -60,28 +60,49 @@ struct Fs {
   }
 };
 
-// Block-wide sum of the threads' pairs: exact-pair butterflies in FP32 (a
-// merge's rounding acts on the low halves only), the warps' pairs in FP64 in
-// order; thread 0 receives the pair.  (An FP64 tree over 256 threads is 70 warp
-// instructions of 16 cycles each on this GPU, more than the block's sums.)
-__device__ Ks block_reduce(Fs v) {
-  __shared__ Fs sw[MB / 32];
+// A thread's sum over many cells: FP32 pairs of up to FLUSH_CELLS cells, whose low
+// half is plain FP32, collected in an FP64 pair.
+constexpr int FLUSH_CELLS = 256;
+struct Sum {
+  Fs f = {0.0f, 0.0f};
+  Ks d = {0.0, 0.0};
+  __device__ void flush() {
+    d.add((double)f.s);
+    d.c += (double)f.e;
+    f = Fs{0.0f, 0.0f};
+  }
+};
+
+// Block-wide sum of the threads' FP64 pairs (compensated throughout), by one warp
+// through shared memory: eight threads a lane, then the lanes.  Lane 0 of that
+// warp receives the pair, normalised, and `true`.  Bound by FP64 instructions, 64
+// cycles of a scheduler each: 100 of one warp instead of 320 of a butterfly in
+// every warp; the warp changes from block to block, so that the four blocks of
+// an SM use its four schedulers.  (FP32 pairs merged by butterflies and kept for
+// all of a thread's cells: target and correction of a 196^3 block 28 + 40 us for
+// now 30 + 44, and at 516^3 an error of 1.2e-16 of the terms' sum for 0.5e-17.)
+__device__ bool block_reduce(Sum v, Ks &r) {
+  __shared__ double2 sp[MB];
+  v.flush();
+  sp[threadIdx.x] = make_double2(v.d.s, v.d.c);
+  __syncthreads();
+  if ((int)(threadIdx.x >> 5) != (int)(blockIdx.x * 4LL / gridDim.x)) return false;
+  const int lane = threadIdx.x & 31;
+  Ks k = {sp[lane].x, sp[lane].y};
+#pragma unroll
+  for (int w = 1; w < MB / 32; w++) {
+    const double2 o = sp[w * 32 + lane];
+    k.add(o.x);
+    k.c += o.y;
+  }
 #pragma unroll
   for (int off = 16; off > 0; off >>= 1) {
-    const float os = __shfl_xor_sync(0xffffffffu, v.s, off), oe = __shfl_xor_sync(0xffffffffu, v.e, off);
-    const float t = v.s + os, bp = t - v.s;
-    v.e = (v.e + oe) + ((v.s - (t - bp)) + (os - bp));
-    v.s = t;
+    const double os = __shfl_xor_sync(0xffffffffu, k.s, off), oc = __shfl_xor_sync(0xffffffffu, k.c, off);
+    k.add(os);
+    k.c += oc;
   }
-  if ((threadIdx.x & 31) == 0) sw[threadIdx.x >> 5] = v;
-  __syncthreads();
-  Ks r = {0.0, 0.0};
-  if (threadIdx.x == 0)
-    for (int w = 0; w < MB / 32; w++) {
-      r.add((double)sw[w].s);
-      r.c += (double)sw[w].e;
-    }
-  return r;
+  two_sum(k.s, k.c, r.s, r.c);
+  return lane == 0;
 }
 
 // X[k][j][i] = g[i] g[j] g[k] * coefficient of CH eigen-mode (i, j, k):
@@ -110,14 +131,16 @@ __global__ void seed_kernel(double *X, const double *g, int n, int which, const 
 
 // Partial target per block: sum of wa*a (or of a over owned cells when wa is
 // null) plus sum of wb*(b - bsub).  Each thread takes cells a grid apart, four
-// at a time (their loads are in flight together), and accumulates an FP32 pair.
+// at a time (their loads are in flight together).
 __global__ void __launch_bounds__(MB) target_kernel(const float *__restrict__ a, const float2 *__restrict__ wa,
                                                     const float *__restrict__ b, const float *__restrict__ bsub,
                                                     const float2 *__restrict__ wb, int n, double *__restrict__ part) {
   chain_wait();
   constexpr int U = 4;
   const long long n3 = (long long)n * n * n, stride = (long long)gridDim.x * MB;
-  Fs acc = {0.0f, 0.0f};
+  Sum sum;
+  Fs &acc = sum.f;
+  int cells = 0;
   for (long long l0 = blockIdx.x * (long long)MB + threadIdx.x; l0 < n3; l0 += U * stride) {
     float va[U], vb[U], vs[U];
     float2 pa[U], pb[U];
@@ -143,9 +166,10 @@ __global__ void __launch_bounds__(MB) target_kernel(const float *__restrict__ a,
       if (bsub) acc.add_product_diff(pb[k], vb[k], vs[k]);
       else acc.add_product(pb[k], vb[k]);
     }
+    if ((cells += U) % FLUSH_CELLS == 0) sum.flush();
   }
-  const Ks r = block_reduce(acc);
-  if (threadIdx.x == 0) {
+  Ks r;
+  if (block_reduce(sum, r)) {
     part[2 * blockIdx.x] = r.s;
     part[2 * blockIdx.x + 1] = r.c;
   }
@@ -165,26 +189,28 @@ __device__ __forceinline__ void owned_rows(int n, F &&f) {
 // Partial owned-cell sum of u per block.
 __global__ void __launch_bounds__(MB) owned_sum_kernel(const float *__restrict__ u, int n, double *__restrict__ part) {
   chain_wait();
-  Fs acc = {0.0f, 0.0f};
+  Sum sum;
+  int rows = 0;
   owned_rows(n, [&](size_t l0, int N, int lane) {
     for (int x0 = lane; x0 < N; x0 += 128) {
       float v[4];
 #pragma unroll
       for (int k = 0; k < 4; k++) v[k] = x0 + 32 * k < N ? u[l0 + x0 + 32 * k] : 0.0f;
 #pragma unroll
-      for (int k = 0; k < 4; k++) acc.add(v[k]);
+      for (int k = 0; k < 4; k++) sum.f.add(v[k]);
     }
+    if (++rows % 16 == 0) sum.flush();  // 256 cells of rows of 512
   });
-  const Ks r = block_reduce(acc);
-  if (threadIdx.x == 0) {
+  Ks r;
+  if (block_reduce(sum, r)) {
     part[2 * blockIdx.x] = r.s;
     part[2 * blockIdx.x + 1] = r.c;
   }
 }
 
 // One block folds both partial sets in a fixed order, half of its warps each,
-// and records (target, before, shift) in res.  Bound by FP64 instructions (64
-// cycles of a scheduler each): few warps, a pair's low half added plainly.
+// and records (target, before, shift) in res.  Bound by FP64 instructions: few
+// warps, a pair's low half (2^-53 of the high one) added plainly.
 constexpr int FB = 128;  // threads per set
 __global__ void __launch_bounds__(2 * FB) fold_kernel(int n, const double *__restrict__ tpart,
                                                       const double *__restrict__ apart, int np,
@@ -253,8 +279,8 @@ __global__ void to_pairs_kernel(double *w, long long count) {
 
 // Four blocks per SM, each thread with four cells in flight.  (Sixteen blocks per
 // SM spent their time in their reductions and left 2432 pairs for the one block
-// that folds them: target, sum, fold and shift of a 196^3 block 44, 37, 31 and
-// 25 us, now 31, 16, 12 and 22.)
+// that folds them: target, and sum, fold and shift, of a 196^3 block 45 and 90 us,
+// now 30 and 44.)
 int mass_partials() { return 152 * 4; }
 
 cudaError_t mass_weight(double *w, double *tmp, const double *g, const double *viT, int n, int which, const EtdCoef &ec,
