@@ -96,9 +96,9 @@ __device__ __forceinline__ KS shfl_ks(KS v, int off) {
 // of eight.  The conserved field's corner average is an exact FP32 pair sum
 // finished in pair arithmetic (no FP64 instructions per cell).  Blocks loop
 // over units; one partial record per block (rec_len).  Bound by FP32 issue:
-// diagnostics of a 4-field 36^3 block 31 -> 19 us, of a 196^3 block with five
-// fields 191 -> 160 us, since a plane's sums are shared by the cubes on both of
-// its sides and no reduction runs through FP64.
+// diagnostics of a 4-field 36^3 block 31 -> 18 us, of a 196^3 block with five
+// fields 191 -> 150 us, since a plane's sums are shared by the cubes on both of
+// its sides and FP64 adds only the warps' sums.
 constexpr int EZ = 8;  // planes per unit
 
 __host__ __device__ inline int energy_units(int N) { return ((N + 31) / 32) * ((N + 7) / 8) * ((N + EZ - 1) / EZ); }
@@ -321,10 +321,11 @@ __global__ void __launch_bounds__(256, 2) energy_partial_f32(Phys ph, EConst ec,
       ca = cb;
     }
   }
-  // warp butterflies, then the warps' values by one warp, in FP32 (max, min) and
-  // exact-pair arithmetic (sums); only the record is FP64, a lane per field (an
-  // FP64 warp instruction is 64 cycles of its scheduler: the block's merges in
-  // FP64, one field after the other, took longer than a small block's cells)
+  // warp butterflies in FP32 (max, min) and exact-pair arithmetic (sums), then the
+  // warps' values, sums in FP64 pairs, eight lanes a quantity (an FP64 warp
+  // instruction is 64 cycles of its scheduler: the block's merges in FP64, one
+  // field after the other, took longer than a small block's cells; in FP32 pairs
+  // they would hold 48 bits, for 17.1 us of diagnostics at 36^3 instead of 18.3)
 #pragma unroll
   for (int off = 16; off > 0; off >>= 1) {
 #pragma unroll
@@ -356,33 +357,32 @@ __global__ void __launch_bounds__(256, 2) energy_partial_f32(Phys ph, EConst ec,
     wc[wid] = cnt;
   }
   __syncthreads();
-  if (wid == 0 && lane < F + 2) {
-    // lane f: field f; lanes F and F + 1: the two energies
-    double *dst = part + (long long)blockIdx.x * rec_len(F);
-    const int at = lane < F ? 4 * lane + 2 : 4 * F + 2 * (lane - F);
-    Acc<float> s;
-    float top = -1.0e30f, low = 1.0e30f;
-    int count = 0;
-    for (int w = 0; w < NW; w++) {
-      s.add(wv[at][w]);
-      s.e += wv[at + 1][w];
-      if (lane < F) {
-        top = fmaxf(top, wv[4 * lane][w]);
-        low = fminf(low, wv[4 * lane + 1][w]);
-        count += wc[w];
-      }
+  if (wid < 2) {
+    // quantity q (field q's sum, max and min, or an energy) of warp w
+    static_assert(NW == 8 && F + 2 <= 8, "eight quantities over two warps");
+    const int q = (wid * 32 + lane) >> 3, w = lane & 7;
+    const bool on = q < F + 2, field = q < F;
+    const int at = field ? 4 * q + 2 : 4 * F + 2 * (q - F);
+    KS v = {on ? (double)wv[at][w] : 0.0, on ? (double)wv[at + 1][w] : 0.0};
+    float top = field ? wv[4 * q][w] : -1.0e30f, low = field ? wv[4 * q + 1][w] : 1.0e30f;
+    int count = wc[w];
+#pragma unroll
+    for (int off = 4; off > 0; off >>= 1) {
+      v = shfl_ks(v, off);
+      top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, off));
+      low = fminf(low, __shfl_xor_sync(0xffffffffu, low, off));
+      count += __shfl_xor_sync(0xffffffffu, count, off);
     }
-    if (lane < F) {
-      const double sh = lane >= NAC ? ph.cshift : 0.0;
-      KS v = {(double)s.s, (double)s.e};
-      ks_add(v, (double)count * (sh + 1.0));  // sum of (value + 1)
-      dst[4 * lane] = (double)top + sh;
-      dst[4 * lane + 1] = (double)low + sh;
-      dst[4 * lane + 2] = v.s;
-      dst[4 * lane + 3] = v.c;
-    } else {
-      dst[at] = (double)s.s;
-      dst[at + 1] = (double)s.e;
+    if (on && w == 0) {
+      double *dst = part + (long long)blockIdx.x * rec_len(F);
+      if (field) {
+        const double sh = q >= NAC ? ph.cshift : 0.0;
+        ks_add(v, (double)count * (sh + 1.0));  // sum of (value + 1)
+        dst[4 * q] = (double)top + sh;
+        dst[4 * q + 1] = (double)low + sh;
+      }
+      dst[at] = v.s;
+      dst[at + 1] = v.c;
     }
   }
 }

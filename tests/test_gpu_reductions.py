@@ -1,7 +1,6 @@
 """Diagnostics of check_soln_new where the reduction's shapes meet their edges:
 owned edges around the 32 x 8 column tile and the eight-plane unit, several
-field counts, both energy forms, against numpy.  (The FP32 form of the same walk
-is held to the FP64 one by test_gpu_mixed.py's energy curves.)"""
+field counts, both energy forms, against numpy, in both precisions."""
 import numpy as np
 import pytest
 
@@ -67,3 +66,67 @@ def test_diagnostics_match_numpy(N, nac, nch, form, sclet_lib):
     want = _numpy(p, u, form)
     np.testing.assert_array_equal(got[:, :2], want[:, :2])
     np.testing.assert_allclose(got[:, 2:], want[:, 2:], rtol=1e-13)
+
+
+def _magnitudes(p, u, form):
+    """The energies of _numpy with every term taken by its size."""
+    q = type(p)()
+    for k, _ in p._fields_:
+        setattr(q, k, getattr(p, k))
+    q.landau[:] = [abs(v) for v in p.landau]
+    nac, own = p.nac, u[:, 2:-2, 2:-2, 2:-2]
+    if form == 1:
+        # the coupling th d s, d = c - c0, is the one term that _numpy subtracts
+        e = _numpy(q, u, 1)[:, 3]
+        if p.nch:
+            h3 = p.xmax * p.ymax * p.zmax / own[0].size
+            e = e + 2 * q.landau[4] * h3 * sum((np.abs(own[nac] - q.landau[5]).max() * (f ** 2).sum()) for f in own[:nac])
+        return e
+    s = (own[:nac] ** 2).sum(0) if nac else 0.0
+    h3 = p.xmax * p.ymax * p.zmax / own[0].size
+    add = 2 * (7128.0 + 12 * 2372) / 2372 / 3 * (np.abs(own[:nac]) ** 3).sum() if nac else 0.0
+    e = _numpy(p, u, 0)[:, 3]
+    return np.array([abs(e[f]) + h3 * (add if f < nac else ((own[nac] ** 2 + 1) ** 2).sum()) for f in range(len(own))])
+
+
+@pytest.mark.parametrize("N,nac,nch", [(4, 1, 0), (7, 0, 1), (8, 4, 1), (9, 2, 1), (33, 4, 0), (41, 3, 1), (65, 4, 1)])
+@pytest.mark.parametrize("form", [0, 1])
+def test_fp32_diagnostics_match_numpy(N, nac, nch, form, sclet_lib):
+    """The FP32 form on the values the state holds: maxima and minima exact, FP64
+    sums of the FP32 values, energies to the FP32 roundings of a cell, at most 40
+    of 2^-24 of its terms' sizes."""
+    sg = sclet_lib
+    p = sg.default_params()
+    n = N + 4
+    p.nx = p.ny = p.nz = n
+    p.xmax, p.ymax, p.zmax = 0.5 * N, 0.4 * N, 0.6 * N
+    p.kkx, p.kky, p.kkz = 1.0, 0.7, 0.4
+    p.nac, p.nch, p.elastic = nac, nch, 0
+    u = np.random.default_rng(N).uniform(0.2, 0.9, size=(nac + nch, n, n, n))
+    s = sg.Solver(p, sg.MIXED)
+    s.set_fields(u)
+    u = s.get_fields()
+    got = s.check_soln(form)
+    s.close()
+    want = _numpy(p, u, form)
+    np.testing.assert_array_equal(got[:, :2], want[:, :2])
+    np.testing.assert_allclose(got[:, 2], want[:, 2], rtol=1e-12)  # pairs of 13 terms: 13^2 2^-49
+    assert np.all(np.abs(got[:, 3] - want[:, 3]) <= 40 * 2.0 ** -24 * _magnitudes(p, u, form))
+
+
+def test_fp32_volume_keeps_more_than_an_fp32_pair(sclet_lib):
+    """One cell each of two warps' columns away from -1, the sum 2 + 2^-20 + 2^-43 +
+    2^-45: every warp's sum is an exact FP32 pair, theirs together is not."""
+    sg = sclet_lib
+    p = sg.default_params()
+    p.nx = p.ny = p.nz = 12
+    p.xmax = p.ymax = p.zmax = 8.0
+    p.nac, p.nch, p.elastic = 1, 0, 0
+    u = np.full((1, 12, 12, 12), -1.0)
+    u[0, 2, 2, 2] = 2.0 ** -20 + 2.0 ** -43
+    u[0, 2, 3, 2] = 2.0 ** -45
+    s = sg.Solver(p, sg.MIXED)
+    s.set_fields(u)
+    np.testing.assert_array_equal(s.get_fields(), u)
+    assert s.check_soln(1)[0, 2] == 2.0 + 2.0 ** -20 + 2.0 ** -43 + 2.0 ** -45
+    s.close()
