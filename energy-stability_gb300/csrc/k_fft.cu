@@ -862,26 +862,30 @@ __global__ void contract_kernel(typename Cx<T>::t *z01, typename Cx<T>::t *z23, 
   }
 }
 
-// Interior of felas_p from the inverse transforms, scaled by 1 / (2 N^3).
+// Interior of felas_p from the inverse transforms, scaled by 1 / (2 N^3) (the
+// contraction doubled).  In FP32 the scale is a (hi, lo) pair, so that the product
+// rounds once, as an FP64 multiplication would, which took 37 us a call at 104^3;
+// the rounded scale alone puts a second rounding on every value unless N is a
+// power of two.
 template <typename T>
 __global__ void unpack_kernel(const typename Cx<T>::t *__restrict__ w01, const typename Cx<T>::t *__restrict__ w23,
-                              T *__restrict__ felas, int N, int nac) {
+                              T *__restrict__ felas, int N, int nac, T hi, T lo) {
   chain_wait();
   const int n = N + 4;
-  const long long n3 = (long long)n * n * n, N3 = (long long)N * N * N;
-  const T s = (T)(0.5 / (double)N3);  // the contraction doubled
+  const long long n3 = (long long)n * n * n;
+  auto scaled = [&](T v) { return sizeof(T) == 4 ? fma(v, hi, v * lo) : v * hi; };
   for (int row = blockIdx.x; row < N * N; row += gridDim.x)
   for (int x = threadIdx.x; x < N; x += blockDim.x) {
     const int z = row / N, y = row - z * N;
     const long long g = (long long)row * N + x;
     long long l = ((long long)(z + 2) * n + (y + 2)) * n + (x + 2);
     typename Cx<T>::t a = w01[g];
-    felas[l] = (T)(a.x * s);
-    if (nac > 1) felas[n3 + l] = (T)(a.y * s);
+    felas[l] = scaled(a.x);
+    if (nac > 1) felas[n3 + l] = scaled(a.y);
     if (nac > 2) {
       typename Cx<T>::t b = w23[g];
-      felas[2 * n3 + l] = (T)(b.x * s);
-      if (nac > 3) felas[3 * n3 + l] = (T)(b.y * s);
+      felas[2 * n3 + l] = scaled(b.x);
+      if (nac > 3) felas[3 * n3 + l] = scaled(b.y);
     }
   }
 }
@@ -1088,7 +1092,9 @@ cudaError_t elastic_compute(ElasticPlan *p, const T *u, T *felas, int n, cudaStr
       chain_launch(sizeof(T) == 4, contract_kernel<T, double>, rows_grid(N), rows_block(N), 0, s, z01, z23, (const double *)p->bn, N, p->nac);
     launch_counter()++;
     fft3d<T>(p, z01, z23, +1, s);
-    chain_launch(sizeof(T) == 4, unpack_kernel<T>, rows_grid(N), rows_block(N), 0, s, z01, z23, felas, N, p->nac);
+    const double scale = 0.5 / ((double)N * N * N);
+    chain_launch(sizeof(T) == 4, unpack_kernel<T>, rows_grid(N), rows_block(N), 0, s, z01, z23, felas, N, p->nac, (T)scale,
+                 (T)(scale - (double)(T)scale));
     launch_counter()++;
   }
   // ghost cells: the shared-scratch semantics

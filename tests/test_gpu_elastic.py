@@ -1,5 +1,6 @@
 """The elastic force's fused contraction (z-lines forward, Green tensor, z-lines
-backward in one kernel) against the FP64 form's separate passes."""
+backward in one kernel) against the FP64 form's separate passes, and what the
+generic passes round."""
 import numpy as np
 import pytest
 
@@ -30,3 +31,31 @@ def test_fused_contraction(N, nac, sclet_lib):
     for m in range(nac):
         a, b = out[sg.MIXED][m][own], out[sg.FP64][m][own]
         assert np.linalg.norm(a - b) <= 2e-6 * np.linalg.norm(b), (N, nac, m)
+
+
+@pytest.mark.parametrize("N", [6, 12, 18, 24])
+def test_generic_force_is_scaled_with_one_rounding(N, sclet_lib):
+    """A uniform field: every sum of the generic FP32 transforms is exact, so the
+    force is the Green tensor's product at k = 0 times 1 / N^3, each rounded once."""
+    sg = sclet_lib
+    p = sg.default_params()
+    p.nx = p.ny = p.nz = N + 4
+    p.xmax = p.ymax = p.zmax = float(N)
+    p.nac, p.nch, p.elastic = 1, 0, 1
+
+    def force(s, c):
+        s.set_fields(np.full((1, N + 4, N + 4, N + 4), c))
+        s.elastic()
+        f = s.get_felas()[0][2:-2, 2:-2, 2:-2]
+        assert np.all(f == f[0, 0, 0])
+        return f[0, 0, 0]
+
+    s = sg.Solver(p, sg.FP64)
+    b0 = np.float32(force(s, 1.0))
+    s.close()
+    s = sg.Solver(p, sg.MIXED)
+    for m in range(1, 256, 5):
+        c = m / 256.0
+        x = b0 * np.float32(2.0 * N ** 3 * c)
+        assert force(s, c) == np.float32(np.float64(x) * (0.5 / N ** 3)), m
+    s.close()
