@@ -15,16 +15,20 @@
 // (dx moved to the gradient: sum_c g[c] x[c + dx] = sum_c' g[c' - dx] x[c'].)
 // What such MMAs cost is reading their operands from shared memory: the three dx
 // of one input operand read it once, through the A collector.  The nine in-plane
-// taps have 32 accumulator columns each in tensor memory, kept across tiles, and are
-// drained into FP32 registers every DRAIN tiles with round-to-nearest adds (the
-// accumulator's own rounding then acts on at most 8 DRAIN sums); each CTA adds
-// its sums to the gradient once, at the end.  Warp 0 issues TMA, warp 1 the
-// MMAs, warps 2-3 write the gradient's shifted copies with the slots outside the
-// owned cells cleared (the halo holds periodic images, which the data gradient
-// needs), warps 4-15 drain.
+// taps have 32 accumulator columns each in tensor memory, drained into FP32
+// registers after every tile with round-to-nearest adds, a stencil row's three
+// taps by four warps while the other rows' MMAs run: the accumulator itself
+// rounds toward zero, so its eight accumulations are all that may carry that.
+// (Drained every eight tiles a layer of 4 x 64^3 took 98 us for 108, but sums of one
+// sign were low by 1.2e-6 and those of either sign 1.5 times as far off as with
+// FP32 FMAs.  Now, relative to the gradient's norm, FP32 FMAs and this: 4 x 64^3
+// 4.8e-7 and 2.7e-7, one sign 2.2e-7 and 1.8e-7; 112^3 5.9e-7 and 2.9e-7, one sign
+// 2.5e-7 and 2.1e-7.)  Each CTA adds its sums to the gradient once, at the end.
+// Warp 0 issues TMA, warp 1 the MMAs, warps 2-3 write the gradient's shifted
+// copies with the slots outside the owned cells cleared (the halo holds periodic
+// images, which the data gradient needs), warps 4-15 drain.
 //
-// A layer on 4 x 64^3: 2.22 ms as an FP32-issue kernel, 0.10 ms with an operand
-// read per tap, 0.09 ms now.
+// A layer on 4 x 64^3: 2.22 ms as an FP32-issue kernel, 0.11 ms now.
 #include <mutex>
 
 #include "sclet_conv_tc.cuh"
@@ -45,7 +49,6 @@ constexpr int EPI = 12;                     // draining warps, three per TMEM la
 constexpr int TAPS_PER_WARP = TAPS2 / 3;
 constexpr int WG_THREADS = 32 * (2 + SHIFTERS + EPI);
 constexpr int WG_TMEM = 512;                // 288 columns used; allocations are powers of two
-constexpr int DRAIN = 8;                    // tiles per drain
 
 // Runs of the input per stage as in k_conv.cu's ny: 1 one run of 128 + 2 Np
 // slots per plane and chunk, 3 one run of 128 slots per stencil row.  A stage:
@@ -71,14 +74,18 @@ static Geom geom_for(int N, int ny) {
   return g;
 }
 
+// SPLIT: drains of an accumulator per tile
+template <int SPLIT>
 __global__ void __launch_bounds__(WG_THREADS, 1)
     wgrad_tc_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmG, int N, int batch,
                     float *__restrict__ dw, float *__restrict__ db, int *err, Geom gm) {
+  constexpr int KSTEPS = ROWS / 16 / SPLIT;  // accumulations between drains
   extern __shared__ uint8_t smem_raw[];
   __shared__ __align__(8) uint64_t full_bar[MAX_STAGES];
   __shared__ __align__(8) uint64_t ready_bar[MAX_STAGES];  // shifted copies written
   __shared__ __align__(8) uint64_t empty_bar[MAX_STAGES];
-  __shared__ __align__(8) uint64_t acc_full, acc_empty, done_bar;
+  __shared__ __align__(8) uint64_t acc_full[3], acc_empty[3];  // per stencil row: three taps' accumulators
+  __shared__ __align__(8) uint64_t done_bar;
   __shared__ uint32_t tmem_slot;
   __shared__ int failed;
 
@@ -111,8 +118,10 @@ __global__ void __launch_bounds__(WG_THREADS, 1)
       mbar_init(&ready_bar[s], SHIFTERS);
       mbar_init(&empty_bar[s], 1);
     }
-    mbar_init(&acc_full, 1);
-    mbar_init(&acc_empty, EPI);
+    for (int dy = 0; dy < 3; dy++) {
+      mbar_init(&acc_full[dy], 1);
+      mbar_init(&acc_empty[dy], EPI / 3);
+    }
     mbar_init(&done_bar, 1);
     failed = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -164,34 +173,39 @@ __global__ void __launch_bounds__(WG_THREADS, 1)
     const uint32_t g_hi = (uint32_t)(dg0 >> 32), x_hi = (uint32_t)(dx0 >> 32);
     bool ok = true;
     for (int it = 0; it < mine && ok; it++) {
-      const int grp = it / DRAIN, s = it % stages;
-      if (it % DRAIN == 0 && grp > 0) ok = mbar_wait(&acc_empty, (grp - 1) & 1);
-      ok = __all_sync(0xffffffffu, ok && mbar_wait(&ready_bar[s], (it / stages) & 1));
+      const int s = it % stages;
+      ok = __all_sync(0xffffffffu, mbar_wait(&ready_bar[s], (it / stages) & 1));
       if (!ok) break;
       fence_after();
       const Tile ti = tile_of(blockIdx.x + it * gridDim.x, N, Np, per_plane);
       const uint32_t st = (uint32_t)(s * gm.stage_bytes >> 4);
-      const uint32_t first_tile = it % DRAIN == 0 ? 0u : 1u;
+      for (int part = 0; part < SPLIT && ok; part++) {
+        const int use = it * SPLIT + part;  // of each stencil row's accumulators
 #pragma unroll
-      for (int dy = 0; dy < 3; dy++) {
-        // the run holding stencil row dy and its first slot within it
-        const uint32_t first = (uint32_t)(ti.s0 + (ny == 1 ? -Np : (dy - 1) * Np));
-        const uint32_t x_lo = (uint32_t)dx0 + st + (ny == 1 ? 0u : (uint32_t)(dy * gm.row_bytes) >> 4) + (first & 7) +
-                              (ny == 1 ? (uint32_t)(dy * Np) : 0u);
+        for (int dy = 0; dy < 3; dy++) {
+          if (use > 0) ok = ok && mbar_wait(&acc_empty[dy], (use - 1) & 1);
+          ok = __all_sync(0xffffffffu, ok);
+          fence_after();
+          // the run holding stencil row dy and its first slot within it
+          const uint32_t first = (uint32_t)(ti.s0 + (ny == 1 ? -Np : (dy - 1) * Np));
+          const uint32_t x_lo = (uint32_t)dx0 + st + (ny == 1 ? 0u : (uint32_t)(dy * gm.row_bytes) >> 4) + (first & 7) +
+                                (ny == 1 ? (uint32_t)(dy * Np) : 0u);
 #pragma unroll
-        for (int ks = 0; ks < ROWS / 16; ks++) {
-          // one input operand, the three dx
-          const uint32_t acc = tmem + (uint32_t)(dy * 3 * CH), x = x_lo + (uint32_t)(ks * 16);
-          const uint32_t g = (uint32_t)dg0 + st + (uint32_t)(ks * 16), on = ks == 0 ? first_tile : 1u;
-          constexpr uint32_t DX = (uint32_t)(4 * S_BYTES) >> 4;
-          mma_bf16_from<A_FILL>(issue, acc, x, x_hi, g, g_hi, idesc, on);
-          mma_bf16_from<A_USE>(issue, acc + CH, x, x_hi, g + DX, g_hi, idesc, on);
-          mma_bf16_from<A_LAST>(issue, acc + 2 * CH, x, x_hi, g + 2 * DX, g_hi, idesc, on);
+          for (int k = 0; k < KSTEPS; k++) {
+            // one input operand, the three dx
+            const uint32_t acc = tmem + (uint32_t)(dy * 3 * CH), k16 = (uint32_t)((part * KSTEPS + k) * 16), x = x_lo + k16;
+            const uint32_t g = (uint32_t)dg0 + st + k16, on = k == 0 ? 0u : 1u;
+            constexpr uint32_t DX = (uint32_t)(4 * S_BYTES) >> 4;
+            const bool go = issue && ok;
+            mma_bf16_from<A_FILL>(go, acc, x, x_hi, g, g_hi, idesc, on);
+            mma_bf16_from<A_USE>(go, acc + CH, x, x_hi, g + DX, g_hi, idesc, on);
+            mma_bf16_from<A_LAST>(go, acc + 2 * CH, x, x_hi, g + 2 * DX, g_hi, idesc, on);
+          }
+          if (ok) mma_commit_from(issue, &acc_full[dy]);
         }
       }
       mma_commit_from(issue, &empty_bar[s]);
-      if (it % DRAIN == DRAIN - 1 || it == mine - 1) mma_commit_from(issue, &acc_full);
-      ok = !__any_sync(0xffffffffu, *(volatile int *)&failed);
+      ok = ok && !__any_sync(0xffffffffu, *(volatile int *)&failed);
     }
     if (!ok && lane == 0) failed = 1;
     mma_commit_from(issue, &done_bar);
@@ -232,13 +246,12 @@ __global__ void __launch_bounds__(WG_THREADS, 1)
     }
   } else {
     // D row 32 q + lane = (dz = q, ci = lane), row 96 the sums of g; column co
-    const int q = warp & 3, t0 = ((warp - 2 - SHIFTERS) >> 2) * TAPS_PER_WARP;
+    const int q = warp & 3, row = (warp - 2 - SHIFTERS) >> 2, t0 = row * TAPS_PER_WARP;  // the stencil row dy
     float sum[TAPS_PER_WARP][CH] = {};
-    const int groups = (mine + DRAIN - 1) / DRAIN;
     bool good = true;
-    for (int grp = 0; grp < groups; grp++) {
+    for (int use = 0; use < mine * SPLIT; use++) {
       int ok = 1;
-      if (lane == 0) ok = mbar_wait(&acc_full, grp & 1) ? 1 : 0;
+      if (lane == 0) ok = mbar_wait(&acc_full[row], use & 1) ? 1 : 0;
       ok = __shfl_sync(0xffffffffu, ok, 0);
       if (!ok) {
         if (lane == 0) failed = 1;
@@ -248,15 +261,23 @@ __global__ void __launch_bounds__(WG_THREADS, 1)
       fence_after();
 #pragma unroll
       for (int t = 0; t < TAPS_PER_WARP; t++) {
-        uint32_t r[32];
-        tmem_ld32_async(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)((t0 + t) * CH), r);
-        tmem_wait_ld();
+        const uint32_t col = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)((t0 + t) * CH);
 #pragma unroll
-        for (int c = 0; c < CH; c++) sum[t][c] += __uint_as_float(r[c]);
+        for (int c0 = 0; c0 < CH; c0 += 16) {  // 16 columns at a time: nothing spills
+          uint32_t ra[8], rb[8];
+          tmem_ld8_async(col + c0, ra);
+          tmem_ld8_async(col + c0 + 8, rb);
+          tmem_wait_ld();
+#pragma unroll
+          for (int c = 0; c < 8; c++) {
+            sum[t][c0 + c] += __uint_as_float(ra[c]);
+            sum[t][c0 + 8 + c] += __uint_as_float(rb[c]);
+          }
+        }
       }
       fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(&acc_empty);
+      if (lane == 0) mbar_arrive(&acc_empty[row]);
     }
     if (good) {
 #pragma unroll
@@ -297,7 +318,9 @@ cudaError_t launch_conv_wgrad(const __nv_bfloat16 *in, const __nv_bfloat16 *g, i
   {
     std::lock_guard<std::mutex> lock(mu);
     if (!sms_of[dev]) {
-      e = cudaFuncSetAttribute(wg::wgrad_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_LIMIT);
+      e = cudaFuncSetAttribute(wg::wgrad_tc_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_LIMIT);
+      if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(wg::wgrad_tc_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_LIMIT);
       if (e != cudaSuccess) return e;
       e = cudaDeviceGetAttribute(&sms_of[dev], cudaDevAttrMultiProcessorCount, dev);
       if (e != cudaSuccess) return e;
@@ -317,7 +340,9 @@ cudaError_t launch_conv_wgrad(const __nv_bfloat16 *in, const __nv_bfloat16 *g, i
   if ((e = make_map_lines(&mg, g, lines, wg::G_ROWS)) != cudaSuccess) return e;
   const long long tiles = (long long)batch * N * (((long long)N * (N + 2) + ROWS - 1) / ROWS);
   const int grid = (int)(tiles < sms ? tiles : sms);
-  chain_launch(true, wg::wgrad_tc_kernel, grid, wg::WG_THREADS, gm.smem, s, mx, mg, N, batch, dw, db, err, gm);
+  // a tile per CTA at most: nothing averages the accumulators' rounding, so half as
+  // many accumulations (16^3: error 1.13e-7 and 0.97e-7, 7.2 and 7.8 us; FP32 FMAs 1.09e-7)
+  chain_launch(true, tiles <= sms ? wg::wgrad_tc_kernel<2> : wg::wgrad_tc_kernel<1>, grid, wg::WG_THREADS, gm.smem, s, mx, mg, N, batch, dw, db, err, gm);
   launch_counter()++;
   return cudaGetLastError();
 }

@@ -3,6 +3,8 @@
 pass and every parameter's gradient --, training on solver-generated pairs
 with the gain over the coarse step without the corrector on held-out runs,
 and the plain-ETD judge of sclet_learned_step (energy, deviation, fallback)."""
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -252,3 +254,41 @@ def test_deviation_bound_is_checked(learned, sclet_lib):
     np.testing.assert_array_equal(coarse.get_fields()[own], plain.get_fields()[own])
     for s in (plain, fine, coarse):
         s.close()
+
+
+@pytest.mark.parametrize("N,B", [(16, 1), (48, 4)])
+def test_weight_gradient_of_one_sign_is_not_biased(N, B, sclet_lib):
+    """One layer's weight gradient with activations and gradients above zero,
+    against FP64 sums of the same BF16 values.  Sums rounded to nearest have
+    errors of either sign; the accumulators round toward zero, the k-th of a
+    tile's eight accumulations by at most 2^-23 of k / 8 of the tile's sum:
+    4.5 x 2^-23 of a sum at most."""
+    torch = _torch()
+    Np = N + 2
+    cs = (Np * Np + 7) // 8 * 8
+    gen = torch.Generator(device="cuda").manual_seed(N)
+    v = (torch.rand((2, B, N, N, N, 32), generator=gen, device="cuda") + 0.1).to(torch.bfloat16)
+
+    def stored(a):  # chunk-planar with a periodic halo
+        i = (torch.arange(Np, device="cuda") - 1) % N
+        a = a[:, i][:, :, i][:, :, :, i].reshape(B, Np, Np * Np, 4, 8).permute(0, 1, 3, 2, 4)
+        o = torch.zeros((B, Np, 4, cs, 8), dtype=torch.bfloat16, device="cuda")
+        o[:, :, :, :Np * Np] = a
+        return o
+
+    x, g = stored(v[0]), stored(v[1])
+    dw, db = torch.zeros((27, 32, 32), device="cuda"), torch.zeros(32, device="cuda")
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+    f = sclet_lib.lib()._ZN5sclet17launch_conv_wgradEPK13__nv_bfloat16S2_iiPfS3_PiP11CUstream_st
+    ptr = ctypes.c_void_p
+    f.restype, f.argtypes = ctypes.c_int, [ptr, ptr, ctypes.c_int, ctypes.c_int, ptr, ptr, ptr, ptr]
+    torch.cuda.synchronize()
+    assert f(x.data_ptr(), g.data_ptr(), N, B, dw.data_ptr(), db.data_ptr(), err.data_ptr(), None) == 0
+    torch.cuda.synchronize()
+    assert err.item() == 0
+    gd = v[1].double().reshape(-1, 32)
+    want = torch.stack([gd.T @ torch.roll(v[0].double(), (1 - t // 9, 1 - t // 3 % 3, 1 - t % 3), (1, 2, 3)).reshape(-1, 32)
+                        for t in range(27)])
+    bias = ((dw.double() - want) / want).mean().item()
+    assert abs(bias) <= 4.5 * 2.0 ** -23, bias
+    assert abs(((db.double() - gd.sum(0)) / gd.sum(0)).mean().item()) <= 4.5 * 2.0 ** -23
