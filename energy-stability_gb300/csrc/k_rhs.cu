@@ -146,10 +146,9 @@ __global__ void __launch_bounds__(RX * RY, (sizeof(T) == 4 ? 4 : 2) + (DIAG ? 0 
   const size_t nn = (size_t)n * n, n3 = nn * n;
   P<T> p = p0;
   const bool el = p.elastic == 1, has_c = p.nch > 0;
-  const int bz = blockIdx.y * gridDim.z + blockIdx.z;  // the march's (run, chunk of planes), then the face cells'
-  if (bz < zblocks) {
+  if ((int)blockIdx.z < zblocks) {
     const int zchunks = (n + p.zc - 1) / p.zc;
-    const int run = bz / zchunks, zci = bz - run * zchunks;
+    const int run = blockIdx.z / zchunks, zci = blockIdx.z - run * zchunks;
     if (p0.krun) p.K[0] = (T)p0.krun[run];
     u += (size_t)run * p.F * n3;
     felas += (size_t)run * NAC * n3;
@@ -210,8 +209,8 @@ __global__ void __launch_bounds__(RX * RY, (sizeof(T) == 4 ? 4 : 2) + (DIAG ? 0 
   }
   // face cells of every run
   const int per = face_cells(n), total = per * p.runs;
-  const int stride = (int)(gridDim.y * gridDim.z - zblocks) * gridDim.x * (RX * RY);
-  for (int i = ((bz - zblocks) * gridDim.x + blockIdx.x) * (RX * RY) + threadIdx.x; i < total; i += stride) {
+  const int stride = (int)(gridDim.z - zblocks) * gridDim.x * (RX * RY);
+  for (int i = (((int)blockIdx.z - zblocks) * gridDim.x + blockIdx.x) * (RX * RY) + threadIdx.x; i < total; i += stride) {
     const int run = i / per;
     int z, y, x;
     face_cell(n, i - run * per, z, y, x);
@@ -838,19 +837,23 @@ static cudaError_t launch_rhs_pl(const Phys &ph, const T *u, const T *felas, T *
     // more runs than a grid of 32 planes a CTA holds in z are refused
     if ((long long)((ph.n + 31) / 32) * p.runs > 65535) return cudaErrorInvalidConfiguration;
     const int zblocks = ((ph.n + p.zc - 1) / p.zc) * p.runs;
-    // the face cells' CTAs come after the march's; what z does not hold goes to y
-    const int gyz = (zblocks + zfaces + 65534) / 65535;
-    const dim3 gdiag(tiles, gyz, (zblocks + zfaces + gyz - 1) / gyz);
+    // the face cells' CTAs come after the march's, in a launch of their own where
+    // the grid's z does not hold both (split over y too, the kernel's block index
+    // cost the march its registers: 196^3 197 -> 274 us)
+    const bool apart = zblocks + zfaces > 65535;
+    auto diag_kernels = [&](auto kernel) {
+      const dim3 grid(tiles, 1, apart ? zblocks : zblocks + zfaces);
+      chain_launch(sizeof(T) == 4, kernel, grid, RX * RY, 0, s, p, u, felas, out, zblocks);
+      if (!apart) return;
+      chain_launch(sizeof(T) == 4, kernel, dim3(tiles, 1, std::min(zfaces, 65535)), RX * RY, 0, s, p, u, felas, out, 0);
+      launch_counter()++;
+    };
     const size_t smem = sizeof(T) * ph.nac * 5 * PLANE;
     cudaError_t e = cudaSuccess;
     switch (ph.nac * 3 + (ring ? 2 : ph.anisotropic ? 1 : 0)) {
 #define SCLET_RHS_AC(NAC)                                                                                         \
-  case NAC * 3:                                                                                                   \
-    chain_launch(sizeof(T) == 4, rhs_ac_diag_kernel<PL, T, NAC, false>, gdiag, RX * RY, 0, s, p, u, felas, out, zblocks); \
-    break;                                                                                                        \
-  case NAC * 3 + 1:                                                                                               \
-    chain_launch(sizeof(T) == 4, rhs_ac_diag_kernel<PL, T, NAC, true>, gdiag, RX * RY, 0, s, p, u, felas, out, zblocks);  \
-    break;                                                                                                        \
+  case NAC * 3: diag_kernels(rhs_ac_diag_kernel<PL, T, NAC, false>); break;                                       \
+  case NAC * 3 + 1: diag_kernels(rhs_ac_diag_kernel<PL, T, NAC, true>); break;                                    \
   case NAC * 3 + 2:                                                                                               \
     e = cudaFuncSetAttribute(rhs_ac_kernel<PL, T, NAC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);   \
     if (e == cudaSuccess) chain_launch(sizeof(T) == 4, rhs_ac_kernel<PL, T, NAC>, dim3(gx, gy, zblocks), blk, smem, s, p, u, felas, out);     \
