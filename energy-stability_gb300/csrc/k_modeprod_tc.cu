@@ -894,12 +894,14 @@ cudaError_t tc_slice_matrix(const double *m, __nv_bfloat16 *planes, float *row_s
 }
 
 // Whether a slicing of g CTAs is launched early: with a CTA per SM at most, or in
-// a few waves.  In one wave its CTAs would crowd on the SMs that the product ahead
-// leaves first, with the little L1 its shared memory leaves, and in many waves
-// only the latter counts (a step of 4 fields, early and else: 36^3, 81 CTAs, 100
-// and 111 us; 68^3, 292, 174 and 156 us; of 104^3 with variable mobility, 1014,
-// 1.18 and 1.21 ms; of 196^3, 3606, 2.37 and 2.29 ms).
-static bool slice_early(int g) { return g <= 152 || (g > 4 * 152 && g <= 16 * 152); }
+// four to seven waves.  In fewer waves its CTAs would crowd on the SMs that the
+// product ahead leaves first, with the little L1 its shared memory leaves; in more
+// the launch latency saved is nothing.  Step times, early over late, of 34 edges
+// from 12^3 to 320^3 with 1, 4 and 4 + 1 fields, plain launches and graphs: up to
+// 152 CTAs 0.84 to 0.97 and 0.95 to 1.05, 200 to 560 1.01 to 1.16 and 1.02 to
+// 1.25, 610 to 1060 0.97 to 1.01 and 0.99 to 1.06, beyond 0.99 to 1.04 and 1.00 to
+// 1.05 (1200 to 2400: 1.00 to 1.04 both).
+static bool slice_early(int g) { return g <= 152 || (g > 4 * 152 && g <= 7 * 152); }
 
 cudaError_t tc_slice_fields(const float *x, const float *sub, float *scale, __nv_bfloat16 *planes, int n, int count,
                             cudaStream_t s) {
@@ -1041,8 +1043,10 @@ cudaError_t launch_modeprod_tc(const __nv_bfloat16 *mat, const __nv_bfloat16 *pl
   // persistent: as many CTAs as can be resident at once (or the tuned count)
   if (args.max_ctas > 0 && args.max_ctas < ctas) ctas = args.max_ctas;
   const int grid = (int)(tiles < ctas ? tiles : ctas);
-  // early but for many tiles a CTA, where it gives nothing (516^3: 242 a CTA, 1 %
-  // of a step slower; 196^3: 12, 3 % faster)
+  // early but for many tiles a CTA, where it gives nothing (step times, early over
+  // late, of 20 edges from 16^3 to 432^3 with 1, 4 and 4 + 1 fields, plain launches
+  // and graphs: up to 1 tile a CTA 0.83 to 0.93 and 0.93 to 0.98, 2 to 5 0.94 to 0.98
+  // and 0.98 to 1.00, 5 to 16 0.98 to 1.00 both, beyond 1.00 both)
   chain_launch(tiles <= 16LL * ctas, inst->kern, grid, tc::THREADS, inst->smem, s, reinterpret_cast<const char *>(planes),
                                                    reinterpret_cast<const char *>(mat), g);
   launch_counter()++;
