@@ -68,6 +68,7 @@
 #include <stdint.h>
 
 #include <mutex>
+#include <type_traits>
 
 #include "sclet_internal.cuh"
 #include "sclet_tc.cuh"
@@ -83,11 +84,12 @@ namespace tc {
 // in two parts (even, odd modes) of h = ceil(n / 2) columns, a tile's parts one
 // after the other.  The forward epilogue interleaves
 // the parts' modes; the inverse one keeps the even part's tile E in registers
-// until the odd part's O is there and stores E + O and E - O.
+// until the odd part's O is there and stores E + O and E - O, or, for fields that
+// are no increments, E at its positions and O at their mirrors (see unfold_kernel, k_mass.cu).
 // EPI 0 store, 1 ETD1 update, 2 phi scaling (FORM 0; the folded transforms apply
 // them where the lines are sliced for the inverse, slice_fold_kernel).
-// OUT 1 store, 2 accumulate (FORM 2: of fields below g.acc, the others store;
-// as reductions at the L2, so that no epilogue warp waits for the old values).
+// OUT 1 store, 2 accumulate (FORM 2: of fields below g.acc, the others store E and
+// O; as reductions at the L2, so that no epilogue warp waits for the old values).
 // BN: a'-tile width.  128 columns of the four classes fill tensor memory; with
 // 64, for halves up to 64, two accumulator sets alternate.
 template <int FORM, int EPI, int OUT, int BN>
@@ -276,7 +278,7 @@ __global__ void __launch_bounds__(THREADS, 1)
       const long long r = (long long)tp.r_tile * BM + q * 32 + lane;
       const int nch = (min(BN, h - tp.a_tile * BN) + 31) / 32;
       float *outT = g.out + (long long)tp.t * g.n * rows;
-      const bool add = OUT == 2 && tp.t % g.F < g.acc;
+      if (tp.t % g.F >= g.acc) return;  // stored as it came
 #pragma unroll
       for (int cl = 0; cl < CPW; cl++) {
         const int a0 = tp.a_tile * BN + (c_first + cl) * 32;
@@ -287,7 +289,7 @@ __global__ void __launch_bounds__(THREADS, 1)
           for (int jj = 0; jj < 32; jj++)
             if (jj < lim) {
               float *oz = outT + (q0 - (uint32_t)jj * (uint32_t)rows);
-              if (add) atomicAdd(oz, even[cl][jj]);
+              if (OUT == 2) atomicAdd(oz, even[cl][jj]);
               else *oz = even[cl][jj];
             }
         }
@@ -372,7 +374,6 @@ __global__ void __launch_bounds__(THREADS, 1)
       if (lane == 0) mbar_arrive(&tempty_bar[b]);
       if (DEFER && ti.part == 0 && u > 0) store_mirror(prev);
       const bool ch = ti.t % g.F >= g.nac;  // field kind: Cahn-Hilliard
-      const bool add = OUT == 2 && (FORM != 2 || ti.t % g.F < g.acc);
       const float4 *cf = ch ? g.coef[1] : g.coef[0];
       const float2 *cf2 = ch ? g.coef2[1] : g.coef2[0];
       const long long tb = (long long)ti.t * g.n * rows;
@@ -387,13 +388,24 @@ __global__ void __launch_bounds__(THREADS, 1)
           const int lim = min(32, h - a0);  // live a' in the chunk
           const float rs = rsv[cl];
           if (FORM == 2) {
+            const uint32_t o0 = (uint32_t)a0 * urows + (uint32_t)(live ? r : 0);
+            const uint32_t q0 = (uint32_t)(g.n - 1 - a0) * urows + (uint32_t)(live ? r : 0);  // mirrored position
+            if (ti.t % g.F >= g.acc) {
+              // E at its positions, O at the mirrored ones (an odd block's middle cell has none)
+              const int end = ti.part == 0 ? lim : min(lim, g.n / 2 - a0);
+              const uint32_t at = ti.part == 0 ? o0 : q0, step = ti.part == 0 ? urows : 0u - urows;
+#pragma unroll
+              for (int jj = 0; jj < 32; jj++) {
+                const float v = acc[cl][jj] * (si * __shfl_sync(0xffffffffu, rs, jj));
+                if (jj < end && live) outT[at + (uint32_t)jj * step] = v;
+              }
+              continue;
+            }
             if (ti.part == 0) {
 #pragma unroll
               for (int jj = 0; jj < 32; jj++) even[cl][jj] = acc[cl][jj] * (si * __shfl_sync(0xffffffffu, rs, jj));
               continue;
             }
-            const uint32_t o0 = (uint32_t)a0 * urows + (uint32_t)(live ? r : 0);
-            const uint32_t q0 = (uint32_t)(g.n - 1 - a0) * urows + (uint32_t)(live ? r : 0);  // mirrored position
 #pragma unroll
             for (int jj = 0; jj < 32; jj++) {
               const float od = acc[cl][jj] * (si * __shfl_sync(0xffffffffu, rs, jj));
@@ -402,7 +414,7 @@ __global__ void __launch_bounds__(THREADS, 1)
               if (jj < lim && live) {
                 float *oy = outT + (o0 + (uint32_t)jj * urows), *oz = outT + (q0 - (uint32_t)jj * urows);
                 const bool mirror = !DEFER && a0 + jj < g.n / 2;  // an odd block's middle cell has none
-                if (add) {
+                if (OUT == 2) {
                   atomicAdd(oy, y);
                   if (mirror) atomicAdd(oz, z);
                 } else {
@@ -595,7 +607,8 @@ __device__ __forceinline__ uint32_t bf16_pair(float lo, float hi) {
 //   MODE 1 (inverse): the even and the odd modes of the line, interleaved in x
 //   MODE 2: the same after the step's update of the eigen-modes: phi x for
 //        tensors t < sp.nI, e u^ + phi1 N^ for the others (u^ the block t, N^
-//        the block t + count - nI)
+//        the block t + count - nI), these as pairs whose low half joins the last
+//        slice
 // A CTA takes SLICE_ROWS lines of one tensor, the tensors of the same lines in
 // neighbouring CTAs (the coefficients of MODE 2 come from HBM about once).  A
 // line is held in registers, all its loads in flight at once.  (Reading it twice
@@ -638,7 +651,8 @@ __global__ void __launch_bounds__(256)
     const float *x = xt + l0;
     // columns k, k + 1 (k < h): MODE 0: a = x[k], x[k+1], b = their mirrors; else
     // a = the even part's two modes, b = the odd part's
-    auto load = [&](int k, float &a0, float &a1, float &b0, float &b1) {
+    uint32_t alo[MODE == 2 ? C : 1], blo[MODE == 2 ? C : 1];  // MODE 2: the values' low parts, BF16 pairs
+    auto load = [&](int k, int c, float &a0, float &a1, float &b0, float &b1) {
       if (MODE == 0) {
         const int q = n - 1 - k;
         a1 = b1 = 0.0f;
@@ -681,14 +695,20 @@ __global__ void __launch_bounds__(256)
         };
         four(x, v);
         if (MODE == 2) {
+          float lo[4] = {0.0f, 0.0f, 0.0f, 0.0f};
           if (etd) {
             float nh[4];
             four(x + nhat, nh);
 #pragma unroll
             for (int i = 0; i < 4; i++)
               if (k2 + i < n) {
+                // e u^ + phi1 N^ with what its products and sums round off
                 const float4 f = __ldg(ce + l0 + k2 + i);  // (e_hi, e_lo, phi1_hi, phi1_lo)
-                v[i] = fmaf(f.x, v[i], fmaf(f.y, v[i], fmaf(f.z, nh[i], f.w * nh[i])));
+                const float u = v[i], w = fmaf(f.y, u, f.w * nh[i]), p = f.x * u, q = fmaf(f.z, nh[i], w);
+                v[i] = __fadd_rn(p, q);
+                const float b = __fadd_rn(v[i], -p);
+                lo[i] = __fadd_rn(__fadd_rn(p, -__fadd_rn(v[i], -b)), __fadd_rn(q, -b)) +
+                        (fmaf(f.x, u, -p) + (fmaf(f.z, nh[i], -q) + w));
               }
           } else {
             float2 f[4];
@@ -704,6 +724,10 @@ __global__ void __launch_bounds__(256)
 #pragma unroll
             for (int i = 0; i < 4; i++) v[i] = fmaf(f[i].x, v[i], f[i].y * v[i]);  // (phi_hi, phi_lo)
           }
+          if (etd) {
+            alo[c] = bf16_pair(odd0 ? lo[0] : lo[1], odd0 ? lo[2] : lo[3]);
+            blo[c] = bf16_pair(odd0 ? lo[1] : lo[0], odd0 ? lo[3] : lo[2]);
+          }
         }
         a0 = odd0 ? v[0] : v[1];
         a1 = odd0 ? v[2] : v[3];
@@ -715,7 +739,8 @@ __global__ void __launch_bounds__(256)
 #pragma unroll
     for (int c = 0; c < C; c++) {
       a0[c] = a1[c] = b0[c] = b1[c] = 0.0f;
-      if (kl + BK * c < h) load(kl + BK * c, a0[c], a1[c], b0[c], b1[c]);
+      if (MODE == 2) alo[c] = blo[c] = 0;
+      if (kl + BK * c < h) load(kl + BK * c, c, a0[c], a1[c], b0[c], b1[c]);
     }
     float me = 0.0f, mo = 0.0f;
 #pragma unroll
@@ -771,12 +796,18 @@ __global__ void __launch_bounds__(256)
         fold(k + 1 == mid ? 0.0f : a1[c], k + 1 == mid ? 0.0f : -b1[c], io, d1);
         put(odd);
       } else {
-        digits(a0[c] * ie, 0.0f, step, step4, d0);
-        digits(a1[c] * ie, 0.0f, step, step4, d1);
-        put(even);
-        digits(b0[c] * io, 0.0f, step, step4, d0);
-        digits(b1[c] * io, 0.0f, step, step4, d1);
-        put(odd);
+        auto store = [&](auto low) {
+          constexpr bool LOW = decltype(low)::value;
+          const uint32_t la = LOW ? alo[c] : 0, lb = LOW ? blo[c] : 0;
+          digits(a0[c] * ie, LOW ? __uint_as_float(la << 16) * ie : 0.0f, step, step4, d0);
+          digits(a1[c] * ie, LOW ? __uint_as_float(la & 0xffff0000u) * ie : 0.0f, step, step4, d1);
+          put(even);
+          digits(b0[c] * io, LOW ? __uint_as_float(lb << 16) * io : 0.0f, step, step4, d0);
+          digits(b1[c] * io, LOW ? __uint_as_float(lb & 0xffff0000u) * io : 0.0f, step, step4, d1);
+          put(odd);
+        };
+        if (MODE == 2 && etd) store(std::integral_constant<bool, MODE == 2>());
+        else store(std::false_type());
       }
     }
   }

@@ -978,7 +978,7 @@ static cudaError_t tc_prod(sclet_ctx *ctx, bool inverse, const __nv_bfloat16 *pl
   stage_begin(ctx, 5, ev);
   TcArgs g = tc_args(ctx, inverse, count, out, epi, aux, outmode);
   g.in_scale = scale;
-  if (acc >= 0) g.acc = acc;  // fields the folded inverse accumulates
+  if (acc >= 0) g.acc = acc;  // of a folded inverse: the fields that are increments
   cudaError_t e = launch_modeprod_tc(inverse ? ctx->matV : ctx->matVi, planes, count, g, ctx->stream);
   stage_end(ctx, ev, l0);
   return e;
@@ -1030,11 +1030,20 @@ static int etd_update_fold(sclet_ctx *ctx) {
   sp.F = ctx->F;
   sp.nac = ctx->nac;
   CK(tc_slice_parts(ctx, false, list(ctx->W1), nullptr, F, &sp));
-  CK(tc_prod(ctx, true, ctx->P, ctx->scaleP, F, ctx->W1, 0, nullptr, 1));
+  const int inc = nI ? ctx->nac : 0;  // a run's fields that are increments
+  CK(tc_prod(ctx, true, ctx->P, ctx->scaleP, F, ctx->W1, 0, nullptr, 1, inc));
   CK(tc_slice_parts(ctx, false, list(ctx->W1), nullptr, F));
-  CK(tc_prod(ctx, true, ctx->P, ctx->scaleP, F, ctx->W2, 0, nullptr, 1));
+  CK(tc_prod(ctx, true, ctx->P, ctx->scaleP, F, ctx->W2, 0, nullptr, 1, inc));
   CK(tc_slice_parts(ctx, false, list(ctx->W2), nullptr, F));
-  CK(tc_prod(ctx, true, ctx->P, ctx->scaleP, F, fu_of(ctx), 0, nullptr, nI ? 2 : 1, nI ? ctx->nac : 0));
+  CK(tc_prod(ctx, true, ctx->P, ctx->scaleP, F, fu_of(ctx), 0, nullptr, nI ? 2 : 1, inc));
+  // the parts of the other fields: order parameters of every run (of one run where
+  // there is a conserved field), then the conserved field with its owned cells' sum
+  if (!nI) {
+    if (ctx->nch == 0) CK(launch_unfold(fu_of(ctx), ctx->n, F, n3, nullptr, ctx->stream));
+    else CK(launch_unfold(fu_of(ctx), ctx->n, ctx->nac, n3, nullptr, ctx->stream));
+  }
+  if (ctx->nch > 0)
+    CK(launch_unfold(fu_of(ctx) + ctx->nac * n3, ctx->n, 1, n3, ctx->massPart + 2 * mass_partials(), ctx->stream));
   return SCLET_OK;
 }
 
@@ -1067,9 +1076,13 @@ static int etd_update_mixed(sclet_ctx *ctx) {
     CK(tc_slice(ctx, ctx->W1, nullptr, F));
     CK(tc_prod(ctx, true, ctx->P, ctx->scaleP, F, fu_of(ctx), 0, nullptr, 1));
   }
-  if (ctx->nch > 0)
-    CK(mass_fix(fu_of(ctx) + ctx->nac * n3, ctx->n, ctx->massPart, ctx->massPart + 2 * mass_partials(), ctx->massRes,
-                ctx->stream));
+  if (ctx->nch > 0) {
+    float *c = fu_of(ctx) + ctx->nac * n3;
+    double *apart = ctx->massPart + 2 * mass_partials();
+    // the folded form summed the owned cells where it unfolded them
+    if (ctx->dirichlet) CK(mass_shift(c, ctx->n, ctx->massPart, apart, ctx->massRes, ctx->stream));
+    else CK(mass_fix(c, ctx->n, ctx->massPart, apart, ctx->massRes, ctx->stream));
+  }
   return SCLET_OK;
 }
 

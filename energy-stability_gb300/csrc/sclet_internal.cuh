@@ -202,8 +202,14 @@ int mass_partials();
 // null) + wb.(b - bsub); wa, wb hold the weight pairs of mass_weight
 cudaError_t mass_target(const float *a, const double *wa, const float *b, const float *bsub, const double *wb, int n,
                         double *part, cudaStream_t s);
-// shifts the owned cells of u so that their sum meets the target partials
+// shifts the owned cells of u so that their sum meets the target partials;
+// mass_shift: apart holds that sum's partials already
 cudaError_t mass_fix(float *u, int n, const double *tpart, double *apart, double *res, cudaStream_t s);
+cudaError_t mass_shift(float *u, int n, const double *tpart, const double *apart, double *res, cudaStream_t s);
+// The parts of `count` blocks after three inverse products (TcArgs::acc), block b
+// at u + b stride, -> the fields, in place; apart (of one block, may be null): the
+// partial sums of its owned cells as mass_fix forms them.
+cudaError_t launch_unfold(float *u, int n, int count, long long stride, double *apart, cudaStream_t s);
 
 // 16-bit codes of one field block (see k_codec.cu); kind 0 AC, 1 CH; the
 // stored values plus shift are the field's values.

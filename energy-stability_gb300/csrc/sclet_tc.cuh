@@ -20,7 +20,8 @@ struct TcArgs {
   int form;                 // 0 any basis, 1 folded forward, 2 folded inverse product
   int epi;                  // 0 none, 1 ETD1 update (aux = uhat), 2 phi scaling
   int outmode;              // 1 FP32 store, 2 FP32 accumulate
-  int acc;                  // form 2, outmode 2: fields t % F < acc accumulate, the others store
+  int acc;                  // form 2: fields t % F < acc are increments (outmode 2 accumulates them); of the
+                            // others E and O are stored, for launch_unfold
   const float *aux;         // [count][n^3] FP32 uhat, same layout as out
   float *out;               // [count][n^3] FP32, rotated layout
   const float *in_scale;    // [count][n*n] power-of-two scale of each input row's slices ([count][2][n*n] folded)

@@ -210,3 +210,62 @@ def test_ensemble_steps_follow_the_basis(sclet_lib):
     ens.close()
     for _, _, s in made:
         s.close()
+
+
+@pytest.mark.parametrize("N", [20, 31])
+def test_conserved_update_rounds_no_more_than_the_general_path(N, sclet_lib):
+    """One update of a conserved field, which is no increment, against the exact
+    update of the same state and right-hand side in FP64: with dense sums seven
+    roundings of the state's size (three products, the modes' update, three
+    products), folded as many at most.  Means over the cells; 3 % for their chance."""
+    sg = sclet_lib
+    p = _params(sg, N, 0, 1)
+    p.ymax = p.zmax = p.xmax
+    n = N + 4
+    d, v, vi = cases.eigen_variant(n, 3)
+    h2 = (p.xmax / N) ** 2
+    T = (d[:, None, None] + d[None, :, None] + d[None, None, :]) / h2
+    lci, kci, c0 = p.landau[9], p.landau[10], p.landau[5]
+    H = lci * (T * T * p.epn2 - kci * T)
+    phi = -np.expm1(-p.dt * H) / H
+
+    def transform(m, a):
+        return np.einsum("ia,jb,kc,abc->ijk", m, m, m, a, optimize=True)
+
+    err = []
+    for basis in ((d, v, vi), _swapped(n)):
+        sq = 0.0
+        for seed in range(4):
+            s = sg.Solver(p, sg.MIXED)
+            s.set_eigen(*basis)
+            s.set_fields(c0 + 0.05 * np.random.default_rng(seed).uniform(-0.5, 0.5, size=(1, n, n, n)))
+            s.transfer()
+            s.calc_rhs(1)
+            u, rhs = s.get_fields()[0] - c0, s.get_rhs(1)[0]
+            assert s.L.sclet_etd_update(s.h) == 0
+            got = s.get_fields()[0] - c0
+            s.close()
+            q = (got - transform(v, np.exp(-p.dt * H) * transform(vi, u) + phi * transform(vi, rhs)))[(slice(2, -2),) * 3]
+            sq += np.mean((q - q.mean()) ** 2)  # the mass correction is a uniform shift
+        err.append(np.sqrt(sq / 4))
+    assert err[0] <= 1.03 * err[1], err
+
+
+@pytest.mark.parametrize("N", [4, 5, 21])
+def test_full_form_runs_side_by_side(N, sclet_lib):
+    """Strong damping: order parameters in the full form, their parts unfolded after
+    the products, in every run as in a run of its own."""
+    sg = sclet_lib
+    p = _params(sg, N, 2, 0, dt=5.0)
+    u0 = np.random.default_rng(N).uniform(-0.1, 0.1, size=(3 * 2, N + 4, N + 4, N + 4))
+    s = sg.Solver(p, sg.MIXED, runs=3)
+    s.set_fields(u0)
+    s.step(2)
+    got = s.get_fields()
+    s.close()
+    for r in range(3):
+        one = sg.Solver(p, sg.MIXED)
+        one.set_fields(u0[2 * r:2 * r + 2])
+        one.step(2)
+        np.testing.assert_array_equal(got[2 * r:2 * r + 2], one.get_fields())
+        one.close()
