@@ -38,20 +38,11 @@ __device__ inline KS ks_merge(KS a, KS b) {
 
 constexpr int EB = 256;  // threads per block
 
-// Per-thread sum of T values with FP64-class accuracy.  For FP32 values the
-// running sum is a float pair (s, e) updated by the error-free TwoSum (Knuth),
-// about 48 bits, so a thread's few dozen terms cost FP32 instructions, not
-// FP64 ones (the FP64 pipe of this GPU is 1/64 of the FP32 rate).
-template <typename T>
-struct Acc;
-template <>
-struct Acc<double> {
-  double s = 0.0;
-  __device__ void add(double v) { s += v; }
-  __device__ double value() const { return s; }
-};
-template <>
-struct Acc<float> {
+// Per-thread sum of FP32 values with FP64-class accuracy: a float pair (s, e)
+// updated by the error-free TwoSum (Knuth), about 48 bits, so a thread's few dozen
+// terms cost FP32 instructions, not FP64 ones (the FP64 pipe of this GPU is 1/64 of
+// the FP32 rate).
+struct Acc {
   float s = 0.0f, e = 0.0f;
   __device__ void add(float v) {
     const float t = s + v;
@@ -59,7 +50,6 @@ struct Acc<float> {
     e += (s - (t - bp)) + (v - bp);
     s = t;
   }
-  __device__ double value() const { return (double)s + (double)e; }
   // pair sum with the partner lane at xor distance off; both lanes end with
   // the same pair (TwoSum is exact and the merge symmetric)
   __device__ void merge_lane(int off) {
@@ -207,7 +197,7 @@ __global__ void __launch_bounds__(256, 2) energy_partial_f32(Phys ph, EConst ec,
   part += (long long)blockIdx.y * gridDim.x * rec_len(F);
   const float p2 = ec.p2, p3 = ec.p3, p4 = ec.p4;
   float mx[F], mn[F];
-  Acc<float> vsum[F], eac_p, ech_p;
+  Acc vsum[F], eac_p, ech_p;
   int cnt = 0;
 #pragma unroll
   for (int f = 0; f < F; f++) {

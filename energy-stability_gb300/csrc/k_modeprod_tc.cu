@@ -1066,7 +1066,6 @@ cudaError_t launch_modeprod_tc(const __nv_bfloat16 *mat, const __nv_bfloat16 *pl
   if ((long long)kp > (1LL << (24 - 2 * bits))) return cudaErrorInvalidValue;
   if ((long long)n * n * n > 0xffffffffLL) return cudaErrorInvalidValue;  // 32-bit offsets within a tensor
   TcArgs g = args;
-  g.kp = kp;
   g.kblocks = kp / tc::BK;
   g.bits = bits;
   const long long tiles = (((long long)n * n + tc::BM - 1) / tc::BM) * count * ((h + bn - 1) / bn);

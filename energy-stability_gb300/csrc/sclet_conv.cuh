@@ -1,4 +1,4 @@
-// Declarations of the corrector network's kernels (k_conv.cu, k_conv_train.cu).
+// Declarations of the corrector network's kernels (k_conv.cu, k_conv_train.cu, k_wgrad.cu).
 #pragma once
 
 #include <cuda_bf16.h>

@@ -106,7 +106,7 @@ std::vector<double> fold_matrix(int n, const double *m, bool inverse);
 // thing every such kernel does (or all but its set-up in shared memory), until
 // that one has ended and its writes are visible, so the order of the work stays
 // the stream's; what is saved is the launch latency between two kernels: a step
-// of 4 fields of 36^3 154 -> 98 us, of 68^3 194 -> 175 us.
+// of 4 fields of 36^3 154 -> 98 us, of 68^3 194 -> 156 us.
 // Not for a kernel whose CTAs are dealt to the SMs once, in equal shares: placed
 // while the kernel ahead still holds some SMs, they crowd on the others (the FP64
 // products of 68^3 0.59 -> 1.04 ms a step).  Those, and what the FP64 pipe
@@ -162,7 +162,7 @@ cudaError_t launch_increment_rhs(const Phys &ph, const T *u, const T *rhs, T *r,
 // Inverse: out += for tensors with t % F < acc, a store for the others.
 struct FoldEpi {
   const double *phi[2];
-  int scaled, etd, t0, acc;
+  int scaled, etd, t0;
 };
 cudaError_t launch_fold_fwd_f64(const double *W, const TensorList<double> &in, const double *sub, double *out, int count,
                                 int n, const FoldEpi &ep, const EtdCoef &ec, cudaStream_t s);

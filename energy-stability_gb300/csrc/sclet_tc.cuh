@@ -9,13 +9,13 @@
 namespace sclet {
 
 constexpr int TC_PLANES = 4;    // fixed-point slices per data operand (tc_slice_bits each)
-constexpr int TC_PLANES_M = 5;  // slices per matrix: four 6-bit slices and a fifth
-                                // stored pre-scaled by 1/64 (see k_modeprod_tc.cu)
+constexpr int TC_PLANES_M = 5;  // slices per matrix: four of tc_slice_bits and a fifth, stored
+                                // pre-scaled by 2^-bits (see k_modeprod_tc.cu)
 constexpr int TC_BM = 128;      // lines per tile of input slices
 constexpr int TC_BK = 32;       // columns per k-block
 
 struct TcArgs {
-  int n, kp, kblocks, count;
+  int n, kblocks, count;
   int bits;                 // slice width (set by launch_modeprod_tc)
   int form;                 // 0 any basis, 1 folded forward, 2 folded inverse product
   int epi;                  // 0 none, 1 ETD1 update (aux = uhat), 2 phi scaling
