@@ -53,11 +53,11 @@ import cases  # noqa: E402
 
 METRIC = "cell-updates/s on 1 GB300: mixed/learned vs plain FP64 at ≤1e-5 rel L2"
 UNIT = "cell-updates/s"
-# DRAM bytes (read + write) of one tensor-core product launch over its
-# algorithmic bytes, from an ncu capture of a six-tensor launch at 192^3:
-# (475.6 + 150.8) MB over 6 x 196^3 x (8 + 4) B = 542.1 MB (the slices' columns
-# beyond the 98 of a part, zeros up to 128, are read too).
-TC_TRAFFIC_RATIO = 1.155
+# DRAM bytes (read + write) of one tensor-core product launch over the bytes it
+# addresses (the slices' columns beyond a part's, zeros up to whole k-blocks of 32,
+# are read too), from an ncu capture of a six-tensor launch at 192^3: (475.6 +
+# 150.8) MB over 6 x 196^3 x (8 x 128 / 98 + 4) B = 652.8 MB.
+TC_TRAFFIC_RATIO = 0.960
 FP64_PEAK_TFLOPS = 1.25  # nominal GB300 FP64 rate (the measured peaks cover HBM and bf16 only)
 
 
@@ -328,6 +328,7 @@ def tc_roofline(case, stage_ms, stage_launches, steps):
     n = case.n
     per_step_products = step_products(case)
     elems = n ** 3
+    kp = ((n + 1) // 2 + 31) // 32 * 32  # columns of a part, whole k-blocks
     bytes_step = per_step_products * elems * (8.0 + 4.0)
     flops_step = per_step_products * float(n) ** 4
     mma_step = per_step_products * tc_mma_flops(n)
@@ -343,9 +344,9 @@ def tc_roofline(case, stage_ms, stage_launches, steps):
         "achieved": mma, "peak": bf16s, "unit": "TFLOP/s", "frac": mma / bf16s,
         "achieved_counts": "physical BF16 MMA flops of the split product (eleven MMAs per term)",
         "frac_of_burst_peak": mma / bf16b, "algorithmic_tflops": flops_step * steps / t / 1e12,
-        "traffic": per_launch * TC_TRAFFIC_RATIO,
-        "traffic_source": f"ncu DRAM read+write / algorithmic bytes = {TC_TRAFFIC_RATIO} on one 192^3 launch of six "
-                          "tensors, scaled to this launch size",
+        "traffic": per_launch * (16.0 * kp / n + 4.0) / 12.0 * TC_TRAFFIC_RATIO,
+        "traffic_source": f"ncu DRAM read+write / addressed bytes (parts of {(n + 1) // 2} columns padded to {kp}) = "
+                          f"{TC_TRAFFIC_RATIO} on one 192^3 launch of six tensors, scaled to this launch size",
         "peak_source": src, "avg_launch_ms": stage_ms["tc_kernel"] / launches,
         "hbm": {"achieved": gbs, "peak": hbm, "unit": "GB/s", "frac": gbs / hbm,
                 "algorithmic_bytes_per_launch": per_launch, "bytes_per_step": bytes_step},
