@@ -11,9 +11,9 @@
 // (hi, lo) pairs.  Each mixed step forms the target from the stored state with
 // error-free FP32 products and sums of up to 256 cells per thread (about 48
 // bits, no FP64 instructions per cell) and compensated FP64 sums of these and
-// across threads in a fixed order, then shifts the owned cells of the new state uniformly so their sum
-// meets it.  The FP32 state itself rounds that sum at the level of its own
-// storage (about 1e-11 relative at 192^3).
+// across threads in a fixed order, then shifts the owned cells of the new state
+// uniformly so their sum meets it.  The FP32 state itself rounds that sum at the
+// level of its own storage (about 1e-11 relative at 192^3).
 #include <algorithm>
 
 #include "sclet_internal.cuh"
